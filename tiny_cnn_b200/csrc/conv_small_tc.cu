@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(TFS_THREADS, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
   float *bias_s = reinterpret_cast<float *>(tmem_slot + 4);      // [OCp], zeros without a bias
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int s_begin = (int)((long long)blockIdx.x * a.nsteps / a.nblocks);
   const int s_end = (int)((long long)(blockIdx.x + 1) * a.nsteps / a.nblocks);
   constexpr int W_TMA = TFS_EPI_WARPS + TFS_CONV_WARPS, W_MMA = W_TMA + 1;
@@ -166,26 +166,26 @@ __global__ void __launch_bounds__(TFS_THREADS, 1)
       tma_load_4d(stage0 + (size_t)st * STAGE, &x_map, xs, pos.yb * TFS_ROWS - a.pad_t, 0, pos.b,
                   &tma_full[st]);
     }
-  } else if (warp == W_MMA && lane == 0) {
-    // ---- MMA issuer ------------------------------------------------------------------------------
+  } else if (warp == W_MMA) {
+    // ---- MMA issuer (the whole warp stays converged: see elect_one) ---
     const uint32_t idesc1 = umma_idesc_tf32(128, a.OCp), idesc2 = umma_idesc_tf32(128, 2 * a.OCp);
     const uint64_t b0 = umma_desc(smem_u32(wt), 16, 1024, 2);
     long long w = 0, w2 = 0, t0 = tc_clock(), tq;
     for (int s = s_begin; s < s_end; ++s) {
       const uint32_t i = s - s_begin, ab = i & 1;
       tq = tc_clock();
-      if (!mbar_wait_bounded(&a_full[ab], (i >> 1) & 1)) {
+      if (!mbar_wait_warp(&a_full[ab], (i >> 1) & 1)) {
         failed = true;
         break;
       }
       w += tc_clock() - tq;
       tq = tc_clock();
-      if (i >= 2 && !mbar_wait_bounded(&acc_empty[ab], ((i >> 1) - 1) & 1)) {
+      if (i >= 2 && !mbar_wait_warp(&acc_empty[ab], ((i >> 1) - 1) & 1)) {
         failed = true;
         break;
       }
       w2 += tc_clock() - tq;
-      if (a.dbg && s == s_end - 1) {
+      if (a.dbg && lane == 0 && s == s_end - 1) {
         a.dbg[blockIdx.x * 12 + 2] = tc_clock() - t0;
         a.dbg[blockIdx.x * 12 + 3] = w;
         a.dbg[blockIdx.x * 12 + 4] = w2;
@@ -194,14 +194,17 @@ __global__ void __launch_bounds__(TFS_THREADS, 1)
       const uint32_t acc = tmem_base + ab * 2u * (uint32_t)a.OCp;
       const uint32_t ahi = tmem_a + ab * 2u * Kp, alo = ahi + Kp;
       // the descriptor of K step ks is the first one plus its byte offset / 16 in the address field
+      if (elect_one()) {
 #pragma unroll 4
-      for (int ks = 0; ks < a.ksteps; ++ks) {
-        const uint64_t b = b0 + (uint64_t)(((uint32_t)(ks >> 2) * WT + (uint32_t)(ks & 3) * 32u) >> 4);
-        umma_tf32_ta(acc, ahi + ks * 8, b, idesc2, ks != 0);
-        umma_tf32_ta(acc, alo + ks * 8, b, idesc1, 1);
+        for (int ks = 0; ks < a.ksteps; ++ks) {
+          const uint64_t b = b0 + (uint64_t)(((uint32_t)(ks >> 2) * WT + (uint32_t)(ks & 3) * 32u) >> 4);
+          umma_tf32_ta(acc, ahi + ks * 8, b, idesc2, ks != 0);
+          umma_tf32_ta(acc, alo + ks * 8, b, idesc1, 1);
+        }
+        umma_commit(&a_empty[ab]);
+        umma_commit(&acc_full[ab]);
       }
-      umma_commit(&a_empty[ab]);
-      umma_commit(&acc_full[ab]);
+      __syncwarp();
     }
   } else if (warp >= TFS_EPI_WARPS && warp < W_TMA) {
     // ---- converters ------------------------------------------------------------------------------

@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(TCV_THREADS, 1)
   uint64_t *filt_empty = filt_full + a.nf;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(filt_empty + a.nf);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&halo_full[i], 1);
@@ -471,15 +471,15 @@ __global__ void __launch_bounds__(TCV_THREADS, 1)
         }
       }
     }
-  } else if (warp == 5 && lane == 0) {
-    // ---- MMA issuer -----------------------------------------------------------------------
+  } else if (warp == 5) {
+    // ---- MMA issuer (the whole warp stays converged: see elect_one) ---
     const uint32_t idesc = umma_idesc_tf32(128, Ng);
     uint32_t u = 0, f = 0, it = 0;
     long long w_acc = 0, w_halo = 0, w_filt = 0, t_begin = tc_clock(), tq, t_first = 0;
     for (int unit = blockIdx.x; unit < nunits && !failed; unit += gridDim.x, ++it) {
       const uint32_t ab = it % a.nb, ause = it / a.nb;
       tq = tc_clock();
-      if (ause > 0 && !mbar_wait_bounded(&acc_empty[ab], (ause - 1) & 1)) {
+      if (ause > 0 && !mbar_wait_warp(&acc_empty[ab], (ause - 1) & 1)) {
         failed = true;
         break;
       }
@@ -489,50 +489,49 @@ __global__ void __launch_bounds__(TCV_THREADS, 1)
       for (int slab = 0; slab < a.slabs && !failed; ++slab, ++u) {
         const uint32_t hb = u % a.nh;
         tq = tc_clock();
-        if (!mbar_wait_bounded(&halo_full[hb], (u / a.nh) & 1)) {
+        if (!mbar_wait_warp(&halo_full[hb], (u / a.nh) & 1)) {
           failed = true;
           break;
         }
         w_halo += tc_clock() - tq;
         if (t_first == 0) t_first = tc_clock() - t_entry;  // kernel entry -> first operand tile in place
         tc_fence_after();
-        const uint32_t hbase = smem_u32(halo + (size_t)hb * 2 * HB);
+        // A: the haloed tile, addressed kx pixels (rows of 128 bytes) further on for every kx
+        const uint64_t a0 = umma_desc(smem_u32(halo + (size_t)hb * 2 * HB), 16, a.hw * 128, 2);
         for (int kx = 0; kx < a.KW && !failed; ++kx) {
-          {
-            // A: the haloed tile addressed kx pixels (rows of 128 bytes) further on
-            const uint32_t abase = hbase + (uint32_t)kx * 128u;
-            const uint32_t d = tmem_d;
-            for (int part = 0; part < 2; ++part, ++f) {  // the hi filter tile, then the lo tile
-              const uint32_t fs = f % a.nf;
-              tq = tc_clock();
-              if (!mbar_wait_bounded(&filt_full[fs], (f / a.nf) & 1)) {
-                failed = true;
-                break;
-              }
-              w_filt += tc_clock() - tq;
-              tc_fence_after();
-              const uint32_t bbase = smem_u32(filt + (size_t)fs * FB);
+          for (int part = 0; part < 2; ++part, ++f) {  // the hi filter tile, then the lo tile
+            const uint32_t fs = f % a.nf;
+            tq = tc_clock();
+            if (!mbar_wait_warp(&filt_full[fs], (f / a.nf) & 1)) {
+              failed = true;
+              break;
+            }
+            w_filt += tc_clock() - tq;
+            tc_fence_after();
+            const uint64_t b0 = umma_desc(smem_u32(filt + (size_t)fs * FB), 16, 1024, 2);
+            if (elect_one()) {
 #pragma unroll
               for (int k4 = 0; k4 < 4; ++k4) {
-                const uint64_t ahi = umma_desc(abase + k4 * 32, 16, a.hw * 128, 2);
-                const uint64_t b = umma_desc(bbase + k4 * 32, 16, 1024, 2);
+                const uint64_t ahi = a0 + (uint32_t)(kx * 8 + k4 * 2), b = b0 + k4 * 2;
                 if (part == 0) {
-                  const uint64_t alo = umma_desc(abase + HB + k4 * 32, 16, a.hw * 128, 2);
-                  umma_tf32(d, alo, b, idesc, (slab | kx | k4) != 0);
-                  umma_tf32(d, ahi, b, idesc, 1);
+                  umma_tf32(tmem_d, ahi + (HB >> 4), b, idesc, (slab | kx | k4) != 0);
+                  umma_tf32(tmem_d, ahi, b, idesc, 1);
                 } else {
-                  umma_tf32(d, ahi, b, idesc, 1);
+                  umma_tf32(tmem_d, ahi, b, idesc, 1);
                 }
               }
               umma_commit(&filt_empty[fs]);
             }
+            __syncwarp();
           }
         }
-        if (!failed) umma_commit(&halo_empty[hb]);
+        if (!failed && elect_one()) umma_commit(&halo_empty[hb]);
+        __syncwarp();
       }
-      if (!failed) umma_commit(&acc_full[ab]);
+      if (!failed && elect_one()) umma_commit(&acc_full[ab]);
+      __syncwarp();
     }
-    if (a.dbg) {
+    if (a.dbg && lane == 0) {
       long long *d = a.dbg + (size_t)blockIdx.x * 8;
       d[0] = tc_clock() - t_begin;
       d[1] = w_acc;
@@ -694,7 +693,7 @@ __global__ void __launch_bounds__(TCV_THREADS, 1)
   uint64_t *accum = empty + TCW_STAGES;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accum + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int ocs = blockIdx.y / a.ic_slabs, ics = blockIdx.y % a.ic_slabs;
   const int s_begin = (int)((long long)blockIdx.x * a.nstages / a.ksplits);
   const int s_end = (int)((long long)(blockIdx.x + 1) * a.nstages / a.ksplits);
@@ -732,41 +731,41 @@ __global__ void __launch_bounds__(TCV_THREADS, 1)
       tma_load_3d(p + 2 * DYB, &x_hi, ics * 32, u0, t0 - a.pad_t, &full[st]);
       tma_load_3d(p + 2 * DYB + XB, &x_lo, ics * 32, u0, t0 - a.pad_t, &full[st]);
     }
-  } else if (warp == 5 && lane == 0) {
+  } else if (warp == 5) {  // the whole warp stays converged: see elect_one
     const uint32_t idesc = umma_idesc_tf32_major(128, N, 1, 1);
-    uint32_t accumulate = 0;
     long long w_full = 0, t_begin = tc_clock(), tq;
     for (int s = s_begin; s < s_end && !failed; ++s) {
       const uint32_t i = s - s_begin, st = i % TCW_STAGES;
       tq = tc_clock();
-      if (!mbar_wait_bounded(&full[st], (i / TCW_STAGES) & 1)) {
+      if (!mbar_wait_warp(&full[st], (i / TCW_STAGES) & 1)) {
         failed = true;
         break;
       }
       w_full += tc_clock() - tq;
       tc_fence_after();
       const uint32_t base = smem_u32(smem + st * STAGE);
-      for (int r = 0; r < TCW_ROWS; ++r) {
-        // B: X rows r .. r+KH-1 of this 8-column strip, one 32 x 8-pixel block per ky
-        const uint32_t xb = base + 2 * DYB + (uint32_t)r * 1024u;
-        const uint64_t bhi = umma_desc(xb, 1024, 512, 1);
-        const uint64_t blo = umma_desc(xb + XB, 1024, 512, 1);
-        for (int ch = 0; ch < chunks; ++ch) {
-          // A: dY pixels shifted by j = 4*ch .. 4*ch+3 columns (kx = KW-1-j), one block per shift
-          const uint32_t ab = base + (uint32_t)(r * 16 + ch * 4) * 128u;
-          const uint64_t ahi = umma_desc(ab, 128, 512, 1);
-          const uint64_t alo = umma_desc(ab + DYB, 128, 512, 1);
-          const uint32_t d = tmem_base + (uint32_t)(ch * N);
-          umma_tf32(d, alo, bhi, idesc, accumulate);
-          umma_tf32(d, ahi, blo, idesc, 1);
-          umma_tf32(d, ahi, bhi, idesc, 1);
+      // B: X rows r .. r+KH-1 of the 8-column strip, one 32 x 8-pixel block per ky
+      const uint64_t b0 = umma_desc(base + 2 * DYB, 1024, 512, 1);
+      // A: dY pixels shifted by j = 4*ch .. 4*ch+3 columns (kx = KW-1-j), one block per shift
+      const uint64_t a0 = umma_desc(base, 128, 512, 1);
+      if (elect_one()) {
+#pragma unroll 4
+        for (int r = 0; r < TCW_ROWS; ++r) {
+          const uint64_t bhi = b0 + (uint32_t)r * 64u, blo = bhi + (XB >> 4);
+          for (int ch = 0; ch < chunks; ++ch) {
+            const uint64_t ahi = a0 + (uint32_t)(r * 16 + ch * 4) * 8u, alo = ahi + (DYB >> 4);
+            const uint32_t d = tmem_base + (uint32_t)(ch * N);
+            umma_tf32(d, alo, bhi, idesc, (i | (uint32_t)r) != 0);
+            umma_tf32(d, ahi, blo, idesc, 1);
+            umma_tf32(d, ahi, bhi, idesc, 1);
+          }
         }
-        accumulate = 1;
+        umma_commit(&empty[st]);
       }
-      umma_commit(&empty[st]);
+      __syncwarp();
     }
-    if (!failed) umma_commit(accum);
-    if (a.dbg) {
+    if (!failed && elect_one()) umma_commit(accum);
+    if (a.dbg && lane == 0) {
       long long *d = a.dbg + (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * 8;
       d[0] = tc_clock() - t_begin;
       d[1] = w_full;
@@ -1443,7 +1442,7 @@ __global__ void __launch_bounds__(TCS_THREADS, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accum + 1);
   float *bsum_s = reinterpret_cast<float *>(tmem_slot + 4);   // [group][8 pixel quads][OCp] bias partials
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int s_begin = (int)((long long)blockIdx.x * a.nsteps / a.ksplits);
   const int s_end = (int)((long long)(blockIdx.x + 1) * a.nsteps / a.ksplits);
   if (tid == 0) {
@@ -1488,8 +1487,8 @@ __global__ void __launch_bounds__(TCS_THREADS, 1)
       tma_load_4d(p, &dy_map, x0, 0, y, b, &tma_full[st]);
       tma_load_4d(p + 2 * BB, &x_map, xs, y - a.pad_t, 0, b, &tma_full[st]);
     }
-  } else if (warp == TCS_CONV_WARPS + 1 && lane == 0) {
-    // ---- MMA issuer ---------------------------------------------------------------------------
+  } else if (warp == TCS_CONV_WARPS + 1) {
+    // ---- MMA issuer (the whole warp stays converged: see elect_one) ---
     // the hi and lo gradient tiles are neighbours in shared memory: A_hi * [B_hi | B_lo] is one
     // instruction of width 2*OCp (columns OCp.. hold the A_hi*B_lo part, added in the epilogue)
     const uint32_t idesc1 = umma_idesc_tf32(128, a.OCp), idesc2 = umma_idesc_tf32(128, 2 * a.OCp);
@@ -1497,28 +1496,30 @@ __global__ void __launch_bounds__(TCS_THREADS, 1)
     for (int s = s_begin; s < s_end && !failed; ++s) {
       const uint32_t i = s - s_begin, st = i % a.nst;
       tq = tc_clock();
-      if (!mbar_wait_bounded(&op_full[st], (i / a.nst) & 1)) {
+      if (!mbar_wait_warp(&op_full[st], (i / a.nst) & 1)) {
         failed = true;
         break;
       }
       w += tc_clock() - tq;
-      if (a.dbg && s == s_end - 1) {
+      if (a.dbg && lane == 0 && s == s_end - 1) {
         a.dbg[blockIdx.x * 8 + 2] = tc_clock() - t0;
         a.dbg[blockIdx.x * 8 + 3] = w;
       }
       tc_fence_after();
-      const uint32_t base = smem_u32(smem + (size_t)st * STAGE);
+      const uint64_t b0 = umma_desc(smem_u32(smem + (size_t)st * STAGE), 16, 1024, 2);
       const uint32_t ta = tmem_a + (i & 1u) * 64u;
+      if (elect_one()) {
 #pragma unroll
-      for (int k4 = 0; k4 < 4; ++k4) {
-        const uint64_t b = umma_desc(base + k4 * 32, 16, 1024, 2);
-        umma_tf32_ta(tmem_base, ta + k4 * 8, b, idesc2, (i | k4) != 0);
-        umma_tf32_ta(tmem_base, ta + 32 + k4 * 8, b, idesc1, 1);
+        for (int k4 = 0; k4 < 4; ++k4) {
+          umma_tf32_ta(tmem_base, ta + k4 * 8, b0 + k4 * 2, idesc2, (i | k4) != 0);
+          umma_tf32_ta(tmem_base, ta + 32 + k4 * 8, b0 + k4 * 2, idesc1, 1);
+        }
+        umma_commit(&op_empty[st]);
+        umma_commit(&a_empty[i & 1u]);
       }
-      umma_commit(&op_empty[st]);
-      umma_commit(&a_empty[i & 1u]);
+      __syncwarp();
     }
-    if (!failed) umma_commit(accum);
+    if (!failed && elect_one()) umma_commit(accum);
   } else if (warp < TCS_CONV_WARPS) {
     // ---- converters: im2col rows and the hi / lo split, then the epilogue ----------------------
     const int KK = a.KH * a.KW;

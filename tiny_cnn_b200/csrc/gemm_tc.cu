@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   uint64_t *accum = empty + TC_STAGES;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accum + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int m0 = blockIdx.y * TC_BM, n0 = blockIdx.x * BN;
   const int nkb = (a.K + TC_BK - 1) / TC_BK;
 
@@ -133,31 +133,33 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       tma_load_2d(st + 2 * A_BYTES, &mapBhi, kb * TC_BK, n0, &full[s]);
       tma_load_2d(st + 2 * A_BYTES + B_BYTES, &mapBlo, kb * TC_BK, n0, &full[s]);
     }
-  } else if (warp == 5 && lane == 0) {
-    // ---- MMA issuer -------------------------------------------------------------
+  } else if (warp == 5) {
+    // ---- MMA issuer (the whole warp stays converged: see elect_one) ---
     constexpr uint32_t idesc = umma_idesc_tf32(TC_BM, BN);
-    for (int kb = 0; kb < nkb && !failed; ++kb) {
+    for (int kb = 0; kb < nkb; ++kb) {
       const int s = kb % TC_STAGES;
-      if (!mbar_wait_bounded(&full[s], (kb / TC_STAGES) & 1)) {
+      if (!mbar_wait_warp(&full[s], (kb / TC_STAGES) & 1)) {
         failed = true;
         break;
       }
       tc_fence_after();
-      const uint32_t base = smem_u32(smem + s * STAGE_BYTES);
+      const uint64_t a0 = umma_desc_k128(smem_u32(smem + s * STAGE_BYTES));
+      const uint64_t b0 = a0 + (2 * A_BYTES >> 4);
+      if (elect_one()) {
 #pragma unroll
-      for (int k4 = 0; k4 < TC_BK / 8; ++k4) {
-        // one instruction consumes 8 floats (32 bytes) of k: advance inside the swizzle row
-        const uint64_t ahi = umma_desc_k128(base + k4 * 32);
-        const uint64_t alo = umma_desc_k128(base + A_BYTES + k4 * 32);
-        const uint64_t bhi = umma_desc_k128(base + 2 * A_BYTES + k4 * 32);
-        const uint64_t blo = umma_desc_k128(base + 2 * A_BYTES + B_BYTES + k4 * 32);
-        umma_tf32(tmem_base, alo, bhi, idesc, (kb | k4) != 0);
-        umma_tf32(tmem_base, ahi, blo, idesc, 1);
-        umma_tf32(tmem_base, ahi, bhi, idesc, 1);
+        for (int k4 = 0; k4 < TC_BK / 8; ++k4) {
+          // one instruction consumes 8 floats (32 bytes) of k: advance inside the swizzle row
+          const uint64_t ahi = a0 + k4 * 2, alo = ahi + (A_BYTES >> 4);
+          const uint64_t bhi = b0 + k4 * 2, blo = bhi + (B_BYTES >> 4);
+          umma_tf32(tmem_base, alo, bhi, idesc, (kb | k4) != 0);
+          umma_tf32(tmem_base, ahi, blo, idesc, 1);
+          umma_tf32(tmem_base, ahi, bhi, idesc, 1);
+        }
+        umma_commit(&empty[s]);  // the stage may be refilled once these MMAs have read it
       }
-      umma_commit(&empty[s]);  // the stage may be refilled once these MMAs have read it
+      __syncwarp();
     }
-    if (!failed) umma_commit(accum);  // accumulator complete
+    if (!failed && elect_one()) umma_commit(accum);  // accumulator complete
   } else if (warp < 4) {
     // ---- epilogue ------------------------------------------------------------------
     if (!mbar_wait_bounded(accum, 0)) failed = true;

@@ -15,6 +15,24 @@ __device__ __forceinline__ void split_tf32(float x, float &hi, float &lo) {
   lo = x - hi;                                              // exact in fp32
 }
 
+// One lane of a converged warp (the same one every time).  The warps that issue tcgen05.mma stay
+// converged -- every lane runs the loops and the waits, and only the instruction itself is left to
+// the elected lane -- because descriptors and addresses then live in uniform registers, which the
+// instruction wants: issued from an `if (lane == 0)` branch, every MMA first moves its operands
+// there, 120 - 145 cycles an instruction whatever its width; issued this way the tensor pipe is the
+// limit (measured back to back on TF32, M = 128: 48 cycles at N = 64, 64 at 128, 96 at 192, 128 at 256).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p != 0;
+}
+// the warp's number, known to the compiler to be the same in all of its lanes
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// bounded wait of a whole warp: the same answer in every lane
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+}
+
 __device__ __forceinline__ void tma_load_2d(void *smem_dst, const CUtensorMap *map, int c0, int c1,
                                             uint64_t *bar) {
   asm volatile(
