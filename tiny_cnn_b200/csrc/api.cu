@@ -29,17 +29,20 @@ int conv_fwd_impl(b200_ctx *ctx, const b200_conv_desc *d, const float *in, const
   B200_TRY(conv_geom_from_desc(ctx, d, &g));
   if (batch == 0) return 0;  // empty batch: nothing to read or write
   B200_REQUIRE(in && W && out && (bias || !g.has_bias), "conv2d_fwd: NULL buffer");
-  ConvTcUse tc = conv_tc_use(ctx, g, d->algo);
-  B200_REQUIRE(d->algo != 3 || tc.fwd || tc.fwd_small,
-               "conv2d_fwd: tensor-core kernels need stride 1, dilation 1, windows <= 8x8, <= 256 channels");
+  const ConvTcUse tc = conv_tc_use(ctx, g, d->algo);
+  if (tc.fc) {
+    void *scratch = nullptr;
+    B200_TRY(ctx_scratch(ctx, fc_scratch_floats(ctx, g.C * g.HI * g.WI, g.OC, batch) * sizeof(float), &scratch));
+    return fc_fwd(ctx, g.C * g.HI * g.WI, g.OC, in, W, g.has_bias ? bias : nullptr, out, batch, B200_ACT_NONE,
+                  static_cast<float *>(scratch), true);
+  }
   if (tc.fwd_small) return conv_fwd_small(ctx, g, in, W, bias, out, batch, B200_ACT_NONE);
   if (tc.fwd) {
-    size_t n_x = align_up(conv_tc_tall_floats(g, batch, 0), 64);
     void *scratch = nullptr;
-    B200_TRY(ctx_scratch(ctx, (n_x + conv_tc_filter_floats(ctx, g, 0)) * sizeof(float), &scratch));
-    float *xs = static_cast<float *>(scratch);
-    B200_TRY(conv_tc_tall_x(ctx, g, in, batch, xs));
-    return conv_tc_fwd(ctx, g, xs, W, bias, out, batch, B200_ACT_NONE, xs + n_x);
+    B200_TRY(ctx_scratch(ctx, conv_gather_filter_floats(ctx, g, 0) * sizeof(float), &scratch));
+    float *wt = static_cast<float *>(scratch);
+    B200_TRY(conv_gather_prep(ctx, g, W, wt, nullptr));
+    return conv_gather_fwd(ctx, g, in, wt, bias, out, batch, B200_ACT_NONE);
   }
   bool tiled = use_tiled(d, g);
   B200_REQUIRE(tiled || d->algo != 2, "conv2d_fwd: tiled kernels need stride 1, dilation 1, 3x3/5x5");
@@ -69,50 +72,38 @@ int conv_bwd_impl(b200_ctx *ctx, const b200_conv_desc *d, const float *in, const
     }
     return 0;
   }
-  ConvTcUse tc = conv_tc_use(ctx, g, d->algo);
-  B200_REQUIRE(d->algo != 3 || tc.dw || tc.dw_small,
-               "conv2d_bwd: tensor-core kernels need stride 1, dilation 1, windows <= 8x8, <= 256 channels");
-  if (!din) tc.dx = false;
-  bool tiled = use_tiled(d, g) && g.OW <= 64;
+  const ConvTcUse tc = conv_tc_use(ctx, g, d->algo);
+  if (tc.fc) {
+    void *scratch = nullptr;
+    B200_TRY(ctx_scratch(ctx, fc_scratch_floats(ctx, g.C * g.HI * g.WI, g.OC, batch) * sizeof(float), &scratch));
+    return fc_bwd(ctx, g.C * g.HI * g.WI, g.OC, in, W, dout, din, dW, g.has_bias ? db : nullptr, accumulate, batch,
+                  static_cast<float *>(scratch), true);
+  }
+  const bool tc_dx = tc.dx && din;
+  const bool tiled = use_tiled(d, g) && g.OW <= 64;
   B200_REQUIRE(tiled || d->algo != 2,
                "conv2d_bwd: tiled kernels need stride 1, dilation 1, 3x3/5x5, out width <= 64");
-  // one carve-up of the context scratch for every pass of this call
-  const bool need_dys = tc.dx || tc.dw;
-  size_t n_dys = need_dys ? align_up(conv_tc_tall_floats(g, batch, 1), 64) : 0;
-  int bs_rows = tc.dw && g.has_bias ? conv_tc_bsum_rows(g, batch) : 0;
-  size_t n_bs = align_up((size_t)bs_rows * g.OC, 64);
-  size_t n_xs = tc.dw ? align_up(conv_tc_tall_floats(g, batch, 0), 64) : 0;
-  size_t n_wdx = tc.dx ? align_up(conv_tc_filter_floats(ctx, g, 1), 64) : 0;
-  size_t n_part = tc.dw ? align_up(conv_tc_dw_floats(ctx, g, batch), 64) : 0;
-  size_t n_tdx = (din && !tc.dx && tiled) ? align_up(conv_tiled_dx_scratch(g), 64) : 0;
-  size_t n_small = tc.dw_small ? align_up(conv_dw_small_floats(ctx, g, batch), 64) : 0;
-  size_t n_tdw = (!tc.dw && !tc.dw_small && tiled) ? conv_tiled_dw_scratch(ctx, g, batch) : 0;
+  // one carve-up of the context scratch for both passes of this call
+  const size_t n_dx = tc_dx ? conv_gather_filter_floats(ctx, g, 1) : din && tiled ? conv_tiled_dx_scratch(g) : 0;
+  const size_t n_dw = tc.dw_small ? conv_dw_small_floats(ctx, g, batch)
+                      : tc.dw     ? conv_gather_dw_floats(ctx, g, batch)
+                      : tiled     ? conv_tiled_dw_scratch(ctx, g, batch)
+                                  : 0;
   void *scratch = nullptr;
-  B200_TRY(ctx_scratch(ctx, (n_dys + n_bs + n_xs + n_wdx + n_part + n_small + n_tdx + n_tdw + 64) * sizeof(float),
-                       &scratch));
-  float *dys = static_cast<float *>(scratch);
-  float *bs = dys + n_dys, *xs = bs + n_bs, *wdx = xs + n_xs, *part = wdx + n_wdx;
-  float *small = part + n_part;
-  float *s_dx = small + n_small, *s_dw = s_dx + n_tdx;
-  if (need_dys) B200_TRY(conv_tc_tall_dy(ctx, g, dout, batch, dys, bs_rows ? bs : nullptr));
+  B200_TRY(ctx_scratch(ctx, (align_up(n_dx, 64) + n_dw + 64) * sizeof(float), &scratch));
+  float *s_dx = static_cast<float *>(scratch), *s_dw = s_dx + align_up(n_dx, 64);
   // dX
-  if (din) {
-    if (tc.dx)
-      B200_TRY(conv_tc_dx(ctx, g, dys, W, din, batch, wdx));
-    else if (tiled)
-      B200_TRY(conv_tiled_dx(ctx, g, W, dout, din, batch, s_dx));
-    else
-      B200_TRY(conv_general_dx(ctx, g, W, dout, din, batch));
+  if (tc_dx) {
+    B200_TRY(conv_gather_prep(ctx, g, W, nullptr, s_dx));
+    B200_TRY(conv_gather_dx(ctx, g, dout, s_dx, din, batch));
+  } else if (din && tiled) {
+    B200_TRY(conv_tiled_dx(ctx, g, W, dout, din, batch, s_dx));
+  } else if (din) {
+    B200_TRY(conv_general_dx(ctx, g, W, dout, din, batch));
   }
   // dW, db
-  if (tc.dw) {
-    B200_TRY(conv_tc_tall_x(ctx, g, in, batch, xs));
-    int splits = 0;
-    B200_TRY(conv_tc_dw(ctx, g, xs, dys, batch, part, &splits));
-    B200_TRY(conv_tc_dw_finish(ctx, g, part, splits, dW, accumulate, g.has_bias ? bs : nullptr, batch, db));
-    return 0;
-  }
-  if (tc.dw_small) return conv_dw_small(ctx, g, in, dout, batch, small, dW, db, accumulate);
+  if (tc.dw_small) return conv_dw_small(ctx, g, in, dout, batch, s_dw, dW, db, accumulate);
+  if (tc.dw) return conv_gather_dw(ctx, g, in, dout, batch, s_dw, dW, db, accumulate);
   if (!tiled) return conv_general_dw(ctx, g, in, dout, dW, db, accumulate, batch);
   int splits = 0;
   B200_TRY(conv_tiled_dw_partials(ctx, g, in, dout, batch, s_dw, &splits));
@@ -135,41 +126,39 @@ int conv_time_pass_impl(b200_ctx *ctx, const b200_conv_desc *d, const float *in,
   const bool use_tc = pass == 0 ? (tc.fwd || tc.fwd_small) : pass == 1 ? tc.dx : (tc.dw || tc.dw_small);
   B200_REQUIRE(use_tc || tiled, "conv2d_time_pass: only the tensor-core and the tiled kernels are timed");
   const size_t in_len = (size_t)batch * g.C * g.HI * g.WI, out_len = (size_t)batch * g.OC * g.OH * g.OW;
-  size_t n_res = align_up(in_len > out_len ? in_len : out_len, 64);
-  size_t n_xs = align_up(conv_tc_tall_floats(g, batch, 0), 64), n_dys = align_up(conv_tc_tall_floats(g, batch, 1), 64);
-  size_t n_wt = align_up(use_tc ? conv_tc_filter_floats(ctx, g, pass == 1) : 0, 64);
-  size_t n_part = use_tc ? align_up(tc.dw_small ? conv_dw_small_floats(ctx, g, batch) + conv_weight_len(g) + g.OC
-                                               : conv_tc_dw_floats(ctx, g, batch), 64) : 0;
-  size_t n_tiled = 0;
-  if (!use_tc)
-    n_tiled = pass == 0 ? conv_tiled_fwd_scratch(g) : pass == 1 ? conv_tiled_dx_scratch(g)
-                                                                 : conv_tiled_dw_scratch(ctx, g, batch);
+  const size_t n_res = align_up(in_len > out_len ? in_len : out_len, 64), n_w = align_up(conv_weight_len(g) + g.OC, 64);
+  const size_t n_s = !use_tc ? (pass == 0   ? conv_tiled_fwd_scratch(g)
+                                : pass == 1 ? conv_tiled_dx_scratch(g)
+                                            : conv_tiled_dw_scratch(ctx, g, batch))
+                     : pass < 2    ? conv_gather_filter_floats(ctx, g, pass)
+                     : tc.dw_small ? conv_dw_small_floats(ctx, g, batch)
+                                   : conv_gather_dw_floats(ctx, g, batch);
   void *scratch = nullptr;
-  B200_TRY(ctx_scratch(ctx, (n_res + n_xs + n_dys + n_wt + n_part + n_tiled + 64) * sizeof(float), &scratch));
-  float *res = static_cast<float *>(scratch), *xs = res + n_res, *dys = xs + n_xs, *wt = dys + n_dys;
-  float *part = wt + n_wt, *ts = part + n_part;
+  B200_TRY(ctx_scratch(ctx, (n_res + n_w + n_s + 64) * sizeof(float), &scratch));
+  float *res = static_cast<float *>(scratch), *gw = res + n_res, *s = gw + n_w;
   cudaEvent_t e0, e1;
   B200_CUDA(cudaEventCreate(&e0));
   B200_CUDA(cudaEventCreate(&e1));
   int splits = 0, rc = 0;
   auto run = [&](int prep) -> int {
-    if (use_tc) {
-      if (pass == 0 && tc.fwd_small) return conv_fwd_small(ctx, g, in, W, nullptr, res, batch, B200_ACT_NONE);
-      if (pass == 0) return conv_tc_fwd(ctx, g, xs, W, nullptr, res, batch, B200_ACT_NONE, wt, prep);
-      if (pass == 1) return conv_tc_dx(ctx, g, dys, W, res, batch, wt, prep);
-      if (tc.dw_small) {  // includes its finishing launch
-        float *gw = part + conv_dw_small_floats(ctx, g, batch);
-        return conv_dw_small(ctx, g, in, dout, batch, part, gw, gw + conv_weight_len(g), 0);
-      }
-      return conv_tc_dw(ctx, g, xs, dys, batch, part, &splits);
+    if (use_tc && pass == 0) {
+      if (tc.fwd_small) return conv_fwd_small(ctx, g, in, W, nullptr, res, batch, B200_ACT_NONE);
+      if (prep) B200_TRY(conv_gather_prep(ctx, g, W, s, nullptr));
+      return conv_gather_fwd(ctx, g, in, s, nullptr, res, batch, B200_ACT_NONE);
     }
-    if (pass == 0) return conv_tiled_fwd(ctx, g, in, W, nullptr, res, batch, B200_ACT_NONE, ts);
-    if (pass == 1) return conv_tiled_dx(ctx, g, W, dout, res, batch, ts);
-    return conv_tiled_dw_partials(ctx, g, in, dout, batch, ts, &splits);
+    if (use_tc && pass == 1) {
+      if (prep) B200_TRY(conv_gather_prep(ctx, g, W, nullptr, s));
+      return conv_gather_dx(ctx, g, dout, s, res, batch);
+    }
+    if (use_tc) {  // includes the finishing launch
+      float *gb = gw + conv_weight_len(g);
+      if (tc.dw_small) return conv_dw_small(ctx, g, in, dout, batch, s, gw, gb, 0);
+      return conv_gather_dw(ctx, g, in, dout, batch, s, gw, gb, 0);
+    }
+    if (pass == 0) return conv_tiled_fwd(ctx, g, in, W, nullptr, res, batch, B200_ACT_NONE, s);
+    if (pass == 1) return conv_tiled_dx(ctx, g, W, dout, res, batch, s);
+    return conv_tiled_dw_partials(ctx, g, in, dout, batch, s, &splits);
   };
-  const bool slab = use_tc && !(pass == 2 && tc.dw_small) && !(pass == 0 && tc.fwd_small);
-  if (slab && pass != 1) rc = conv_tc_tall_x(ctx, g, in, batch, xs);
-  if (!rc && slab && pass != 0) rc = conv_tc_tall_dy(ctx, g, dout, batch, dys, nullptr);
   if (!rc) rc = run(1);  // warm-up, filter matrices, tile choice
   if (!rc) rc = cudaEventRecord(e0, ctx->stream) == cudaSuccess ? 0 : 1;
   for (int i = 0; i < reps && !rc; ++i) rc = run(0);

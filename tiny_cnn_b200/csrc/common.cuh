@@ -156,75 +156,39 @@ int conv_tiled_dx(b200_ctx *ctx, const ConvGeom &g, const float *W, const float 
 int conv_tiled_dw_partials(b200_ctx *ctx, const ConvGeom &g, const float *in,
                            const float *dout, int B, float *scratch, int *splits);
 
-// tensor-core path (conv_tc.cu): stride 1, dilation 1, windows up to 8x8, at most 256 channels
-// either side.  The passes read "tall" split copies of the input (xs) and of dY (dys) that
-// conv_tc_tall_x / conv_tc_tall_dy write; sizes in floats from the *_floats functions.
-bool conv_tc_ok(const b200_ctx *ctx, const ConvGeom &g);
-// which passes of a layer run on the tensor cores: `algo` 3 = all (when conv_tc_ok), 1 / 2 =
-// none, 0 = by the context's conv_tensor_cores option
+// tensor-core forward and dX passes with the im2col operand made in tensor memory (conv_gather.cu): any
+// stride, window, padding and map size that fits; forward dilation.  `wt` holds the filter blocks of one
+// pass (conv_gather_filter_floats), made by conv_gather_prep.
+bool conv_gather_ok(const b200_ctx *ctx, const ConvGeom &g, int for_dx);
+size_t conv_gather_filter_floats(const b200_ctx *ctx, const ConvGeom &g, int for_dx);
+int conv_gather_prep(b200_ctx *ctx, const ConvGeom &g, const float *W, float *wt_fwd, float *wt_dx);
+int conv_gather_fwd(b200_ctx *ctx, const ConvGeom &g, const float *in, const float *wt, const float *bias, float *out,
+                    int B, int act);
+int conv_gather_dx(b200_ctx *ctx, const ConvGeom &g, const float *dout, const float *wt, float *din, int B);
+// dW and db the same way (conv_gather_dw.cu), any stride; `part` holds conv_gather_dw_floats
+bool conv_gather_dw_ok(const b200_ctx *ctx, const ConvGeom &g);
+size_t conv_gather_dw_floats(const b200_ctx *ctx, const ConvGeom &g, int B);
+int conv_gather_dw(b200_ctx *ctx, const ConvGeom &g, const float *in, const float *dout, int B, float *part, float *dW,
+                   float *db, int accumulate);
+
+// which passes of a layer run on the tensor cores: `algo` 3 = all that can, 1 / 2 = none, 0 = by the
+// context's conv_tensor_cores option
 struct ConvTcUse {
-  bool fwd, dx, dw;
+  bool fwd, dx, dw;  // conv_gather_*
   bool dw_small;   // dW through the im2col form for layers with few input channels (conv_dw_small)
   bool fwd_small;  // forward through the im2col form for the same layers (conv_fwd_small)
+  bool fc;         // the window is the whole input: a fully-connected layer with weights [out][in] (fc.cu)
 };
 // forward of layers with few input channels (in_c*KH*KW <= 96, <= 64 out channels) from the CHW input
 bool conv_fwd_small_ok(const b200_ctx *ctx, const ConvGeom &g);
 int conv_fwd_small(b200_ctx *ctx, const ConvGeom &g, const float *in, const float *W, const float *bias, float *out,
                    int B, int act);
 ConvTcUse conv_tc_use(const b200_ctx *ctx, const ConvGeom &g, int algo);
-size_t conv_tc_tall_floats(const ConvGeom &g, int B, int which);  // 0: input, 1: dY
-size_t conv_tc_filter_floats(const b200_ctx *ctx, const ConvGeom &g, int for_dx);
-int conv_tc_bsum_rows(const ConvGeom &g, int B);
-size_t conv_tc_dw_floats(const b200_ctx *ctx, const ConvGeom &g, int B);
-int conv_tc_tall_x(b200_ctx *ctx, const ConvGeom &g, const float *in, int B, float *xs);
-int conv_tc_tall_dy(b200_ctx *ctx, const ConvGeom &g, const float *dout, int B, float *dys, float *bsum);
-// the same conversions fused with the 2x2/2 max-pooling layer before the convolution (forward) and
-// with the gradient of the pooling layer (and relu) after it (backward)
-int conv_tc_tall_x_pool(b200_ctx *ctx, const ConvGeom &g, const float *in, float *pooled, int32_t *argmax, int B,
-                        float *xs);
-int conv_tc_tall_dy_unpool(b200_ctx *ctx, const ConvGeom &g, const float *gpool, const int32_t *argmax,
-                           const float *pooled_y, float *dout_chw, int B, float *dys, float *bsum);
-// filter matrices of the forward and / or dX pass (either may be nullptr) in one launch
-int conv_tc_prep(b200_ctx *ctx, const ConvGeom &g, const float *W, float *wt_fwd, float *wt_dx);
-// `prep` = 0 reuses the filter matrices an earlier call left in `wt` (same weights)
-int conv_tc_fwd(b200_ctx *ctx, const ConvGeom &g, const float *xs, const float *W, const float *bias,
-                float *out, int B, int act, float *wt, int prep = 1);
-int conv_tc_dx(b200_ctx *ctx, const ConvGeom &g, const float *dys, const float *W, float *din, int B,
-               float *wt, int prep = 1);
-int conv_tc_dw(b200_ctx *ctx, const ConvGeom &g, const float *xs, const float *dys, int B, float *part,
-               int *splits);
-// Arguments of one finishing pass of a tensor-core dW kernel: sums the partial rows in fixed order
-// and stores the totals in the reference layout.  Elements [0, row_w) are weight-gradient entries in
-// the producing kernel's own order; `layout` says which: 0 = [unit][j][ky][inc][o] of
-// conv_dw_tc_kernel (kx = KW-1-j), 1 = [k][o] of conv_dw_small_tc_kernel.  Elements
-// [row_w, row_w + OC) are bias-gradient sums taken from `bsrc` (bs_rows rows of bs_stride floats,
-// entry bs_off + o of each).  Unconnected pairs get no gradient.
-struct DwFinishArgs {
-  const float *part;
-  long long part_stride;
-  int splits;
-  const float *bsrc;
-  long long bs_stride, bs_off;
-  int bs_rows;
-  float *dW, *db;
-  int layout, row_w;
-  int C, OC, OCp, KH, KW, ic_slabs;
-  const uint8_t *tbl;
-  int accumulate;
-};
-constexpr int DW_FINISH_MAX = 4;  // layers per launch of dw_finish_many
-// finish: fixed-order sum of the partial rows into the reference layout, and (with bsum / db) the bias
-// gradient.  With `defer` the pass is not launched but described there, for dw_finish_many.
-int conv_tc_dw_finish(b200_ctx *ctx, const ConvGeom &g, float *part, int splits, float *dW, int accumulate,
-                      const float *bsum, int B, float *db, DwFinishArgs *defer = nullptr);
-// the finishing passes of several layers in one launch (same sums, element by element)
-int dw_finish_many(b200_ctx *ctx, const DwFinishArgs *list, int n);
-
 // dW of stride-1 layers with in_c*KH*KW <= 128 on the tensor cores, straight from the CHW tensors
 bool conv_dw_small_ok(const b200_ctx *ctx, const ConvGeom &g);
 size_t conv_dw_small_floats(const b200_ctx *ctx, const ConvGeom &g, int B);
 int conv_dw_small(b200_ctx *ctx, const ConvGeom &g, const float *in, const float *dout, int B, float *part,
-                  float *dW, float *db, int accumulate, DwFinishArgs *defer = nullptr);
+                  float *dW, float *db, int accumulate);
 
 // dst (+)= sum_r src[r*stride + i], rows summed in order; optional connection
 // mask for convolution weights (entries of unconnected pairs are left alone
@@ -250,7 +214,7 @@ int gemm_tc(b200_ctx *ctx, int M, int N, int K, const float *src_a, long long ld
 // sums small GEMMs are split into, or the split operands of the tensor-core path.
 size_t fc_scratch_floats(const b200_ctx *ctx, int in_size, int out_size, int B);
 int fc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
-           const float *bias, float *out, int B, int act, float *scratch);
+           const float *bias, float *out, int B, int act, float *scratch, bool w_rows = false);
 // sum of a bucket over the ranks of a data-parallel job through peer memory (peer_reduce.cu)
 struct PeerReduce {
   int rank = 0, world = 0;
@@ -274,7 +238,7 @@ int peer_reduce_run(b200_ctx *ctx, const PeerReduce *pr, float *grads);
 
 int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
            const float *dout, float *din, float *dW, float *db, int accumulate, int B,
-           float *scratch);
+           float *scratch, bool w_rows = false);
 
 int maxpool_fwd(b200_ctx *ctx, const b200_pool_desc &d, const float *in, float *out,
                 int32_t *argmax, int B);

@@ -477,4 +477,493 @@ int conv_fwd_small(b200_ctx *ctx, const ConvGeom &g, const float *in, const floa
   return 0;
 }
 
+// ---- dW of layers with few input channels: explicit transposed im2col operand -----------------
+//
+// When in_c * KH * KW <= 128 (the first layer of a network: 3 x 5 x 5 = 75) a 32-channel slab would
+// be almost all padding.  Here the contraction still runs over pixels, but both operands are
+// K-major with 32 consecutive pixels of one output row per 128-byte row:
+//   B[o][p]  = dY[b][o][y][x0 + p]                  a TMA tile straight from the CHW gradient
+//   A[k][p]  = Xpad[b][c][y + ky][x0 + p + kx]      k = (c*KH + ky)*KW + kx: a converter thread owns
+//              tap k, gathers its pixels from the raw input rows (one TMA tile), splits them and
+//              writes hi / lo into TMEM lane k (tcgen05.st); the MMAs take A from tensor memory, so
+//              the im2col rows never pass through shared memory
+//   D[k][o] += A * B^T                              M = 128 (k padded), N = out channels, 4 k-steps
+// so dW needs 8 MMAs per 32 pixels.  The converter warps also split B into hi / lo in place and
+// keep the bias-gradient sums.  Per-CTA partial results are merged in fixed order afterwards.
+
+namespace {
+
+// Arguments of the finishing pass of conv_dw_small_tc_kernel: sums the partial rows in fixed order and
+// stores the totals in the reference layout.  Elements [0, row_w) are weight-gradient entries [k][o];
+// the bias-gradient sums come from `bsrc` (bs_rows rows of bs_stride floats, entry bs_off + o of each).
+// Unconnected pairs get no gradient.
+struct DwFinishArgs {
+  const float *part;
+  long long part_stride;
+  int splits;
+  const float *bsrc;
+  long long bs_stride, bs_off;
+  int bs_rows;
+  float *dW, *db;
+  int row_w;
+  int C, OC, OCp, KH, KW;
+  const uint8_t *tbl;
+  int accumulate;
+};
+
+// One block of the finishing pass (DwFinishArgs): 8 row lanes per
+// element, lane k adds rows k, k+8, ... in order, lanes combined in order.
+__device__ __forceinline__ void dw_finish_block(const DwFinishArgs &a, const int block) {
+  constexpr int RL = 8;  // row lanes
+  __shared__ float lanes[RL][33];
+  __shared__ float tree[256];
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int wblocks = (a.row_w + 31) / 32;
+  if (block >= wblocks) {
+    // bias gradient: one block per output channel; its many short partial rows are spread over
+    // all 256 threads (thread k adds rows k, k+256, ... in order), combined by a fixed tree
+    const int o = block - wblocks, t = ty * 32 + tx;
+    if (a.db == nullptr || o >= a.OC) return;
+    const float *src = a.bsrc + a.bs_off + o;
+    float s = 0.f;
+    for (int r = t; r < a.bs_rows; r += 256) s += src[(size_t)r * a.bs_stride];
+    tree[t] = s;
+    __syncthreads();
+#pragma unroll
+    for (int w = 128; w > 0; w >>= 1) {
+      if (t < w) tree[t] += tree[t + w];
+      __syncthreads();
+    }
+    if (t == 0) a.db[o] = a.accumulate ? a.db[o] + tree[0] : tree[0];
+    return;
+  }
+  const int e = block * 32 + tx;
+  float s0 = 0.f, s1 = 0.f;
+  if (e < a.row_w) {
+    const float *src = a.part + e;
+    int r = ty;
+    for (; r + RL < a.splits; r += 2 * RL) {
+      s0 += src[(size_t)r * a.part_stride];
+      s1 += src[(size_t)(r + RL) * a.part_stride];
+    }
+    if (r < a.splits) s0 += src[(size_t)r * a.part_stride];
+  }
+  lanes[ty][tx] = s0 + s1;
+  __syncthreads();
+  if (ty == 0 && e < a.row_w) {
+    float s = lanes[0][tx];
+#pragma unroll
+    for (int k = 1; k < RL; ++k) s += lanes[k][tx];
+    const int k = e / a.OCp, KK = a.KH * a.KW, o = e - k * a.OCp, inc = k / KK;
+    const int t = k - inc * KK, ky = t / a.KW, kx = t - ky * a.KW;
+    if (o < a.OC && inc < a.C) {
+      if (a.tbl && !a.tbl[inc * a.OC + o]) s = 0.f;
+      float *d = a.dW + (((size_t)o * a.C + inc) * a.KH + ky) * a.KW + kx;
+      *d = a.accumulate ? *d + s : s;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) dw_finish_kernel(const DwFinishArgs a) { dw_finish_block(a, (int)blockIdx.x); }
+
+int dw_finish_blocks(const DwFinishArgs &a) { return (a.row_w + 31) / 32 + (a.db != nullptr ? a.OC : 0); }
+
+int launch_dw_finish(b200_ctx *ctx, const DwFinishArgs &a) {
+  dw_finish_kernel<<<dw_finish_blocks(a), dim3(32, 8), 0, ctx->stream>>>(a);
+  B200_LAUNCHED();
+  return 0;
+}
+
+}  // namespace
+
+namespace {
+
+constexpr int TCS_MAX_STAGES = 4;     // gradient tile + raw input rows per stage: a few KB each
+constexpr int TCS_PX = 32;          // pixels per step (one 128-byte operand row)
+constexpr int TCS_GROUPS = 2;       // converter groups; group g converts the steps i with i % 2 == g
+constexpr int TCS_GROUP_WARPS = 8;
+static_assert(TCS_GROUPS <= 2, "a group's first step must be the first use of its stage: stages >= groups");
+constexpr int TCS_CONV_WARPS = TCS_GROUPS * TCS_GROUP_WARPS;  // then one TMA warp and one MMA warp
+constexpr int TCS_THREADS = (TCS_CONV_WARPS + 2) * 32;
+
+struct TcDwSmallArgs {
+  float *part;          // [ksplits][row] with row = 128 * OCp (D[k][o]) + OCp (bias sums)
+  int *err;
+  int C, OC, OCp, KH, KW, pad_t, pad_l;
+  int OH, OW, nxb;      // output extent, 32-pixel blocks per output row
+  int Kreal;            // C * KH * KW
+  int bw;               // floats per raw input row in shared memory
+  int nsteps, ksplits;
+  int nst;              // pipeline stages
+  int tmem_cols;        // accumulator 2*OCp, then two A buffers of 32 hi + 32 lo columns
+  long long row;
+  long long *dbg;       // [blocks][8] cycle counters in a build with -DB200_TC_TIMING, else nullptr
+};
+
+__global__ void __launch_bounds__(TCS_THREADS, 1)
+  conv_dw_small_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap dy_map,
+                          const TcDwSmallArgs a) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const uint32_t BB = (uint32_t)a.OCp * 128u;           // B tile (hi or lo)
+  const uint32_t XB = ((uint32_t)(a.C * a.KH * a.bw * 4) + 1023u) & ~1023u;  // raw input rows
+  const uint32_t STAGE = 2 * BB + XB;
+  uint64_t *tma_full = reinterpret_cast<uint64_t *>(smem + (size_t)a.nst * STAGE);
+  uint64_t *op_full = tma_full + TCS_MAX_STAGES;
+  uint64_t *op_empty = op_full + TCS_MAX_STAGES;
+  uint64_t *a_empty = op_empty + TCS_MAX_STAGES;   // [2] A buffers in tensor memory, one per converter group
+  uint64_t *accum = a_empty + 2;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accum + 1);
+  float *bsum_s = reinterpret_cast<float *>(tmem_slot + 4);   // [group][8 pixel quads][OCp] bias partials
+
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
+  const int s_begin = (int)((long long)blockIdx.x * a.nsteps / a.ksplits);
+  const int s_end = (int)((long long)(blockIdx.x + 1) * a.nsteps / a.ksplits);
+  if (tid == 0) {
+    for (int s = 0; s < a.nst; ++s) {
+      mbar_init(&tma_full[s], 1);
+      mbar_init(&op_full[s], TCS_CONV_WARPS);
+      mbar_init(&op_empty[s], 1);
+    }
+    mbar_init(&a_empty[0], 1);
+    mbar_init(&a_empty[1], 1);
+    mbar_init(accum, 1);
+    mbar_fence_init();
+  }
+  if (warp == TCS_CONV_WARPS) tmem_alloc(tmem_slot, (uint32_t)a.tmem_cols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_a = tmem_base + 2u * (uint32_t)a.OCp;   // A buffer of group g: 64 columns from tmem_a + 64 g
+  bool failed = false;
+
+  if (warp == TCS_CONV_WARPS && lane == 0) {
+    // ---- TMA producer: raw input rows and the gradient tile of each step ----------------------
+    long long w = 0, t0 = tc_clock(), tq;
+    for (int s = s_begin; s < s_end; ++s) {
+      const uint32_t i = s - s_begin, st = i % a.nst, use = i / a.nst;
+      tq = tc_clock();
+      if (use > 0 && !mbar_wait_bounded(&op_empty[st], (use - 1) & 1)) {
+        failed = true;
+        break;
+      }
+      w += tc_clock() - tq;
+      if (a.dbg && s == s_end - 1) {
+        a.dbg[blockIdx.x * 8 + 0] = tc_clock() - t0;
+        a.dbg[blockIdx.x * 8 + 1] = w;
+      }
+      const int xb = s % a.nxb, by = s / a.nxb, y = by % a.OH, b = by / a.OH;
+      const int x0 = xb * TCS_PX;
+      const int xs = (x0 - a.pad_l) & ~3;  // aligned start column of the raw rows (floor to 4)
+      uint8_t *p = smem + (size_t)st * STAGE;
+      mbar_expect_tx(&tma_full[st], BB + (uint32_t)(a.C * a.KH * a.bw * 4));
+      tma_load_4d(p, &dy_map, x0, 0, y, b, &tma_full[st]);
+      tma_load_4d(p + 2 * BB, &x_map, xs, y - a.pad_t, 0, b, &tma_full[st]);
+    }
+  } else if (warp == TCS_CONV_WARPS + 1) {
+    // ---- MMA issuer (the whole warp stays converged: see elect_one) ---
+    // the hi and lo gradient tiles are neighbours in shared memory: A_hi * [B_hi | B_lo] is one
+    // instruction of width 2*OCp (columns OCp.. hold the A_hi*B_lo part, added in the epilogue)
+    const uint32_t idesc1 = umma_idesc_tf32(128, a.OCp), idesc2 = umma_idesc_tf32(128, 2 * a.OCp);
+    long long w = 0, t0 = tc_clock(), tq;
+    for (int s = s_begin; s < s_end && !failed; ++s) {
+      const uint32_t i = s - s_begin, st = i % a.nst;
+      tq = tc_clock();
+      if (!mbar_wait_warp(&op_full[st], (i / a.nst) & 1)) {
+        failed = true;
+        break;
+      }
+      w += tc_clock() - tq;
+      if (a.dbg && lane == 0 && s == s_end - 1) {
+        a.dbg[blockIdx.x * 8 + 2] = tc_clock() - t0;
+        a.dbg[blockIdx.x * 8 + 3] = w;
+      }
+      tc_fence_after();
+      const uint64_t b0 = umma_desc(smem_u32(smem + (size_t)st * STAGE), 16, 1024, 2);
+      const uint32_t ta = tmem_a + (i & 1u) * 64u;
+      if (elect_one()) {
+#pragma unroll
+        for (int k4 = 0; k4 < 4; ++k4) {
+          umma_tf32_ta(tmem_base, ta + k4 * 8, b0 + k4 * 2, idesc2, (i | k4) != 0);
+          umma_tf32_ta(tmem_base, ta + 32 + k4 * 8, b0 + k4 * 2, idesc1, 1);
+        }
+        umma_commit(&op_empty[st]);
+        umma_commit(&a_empty[i & 1u]);
+      }
+      __syncwarp();
+    }
+    if (!failed && elect_one()) umma_commit(accum);
+  } else if (warp < TCS_CONV_WARPS) {
+    // ---- converters: im2col rows and the hi / lo split, then the epilogue ----------------------
+    const int KK = a.KH * a.KW;
+    const int grp = warp / TCS_GROUP_WARPS, gtid = tid - grp * (TCS_GROUP_WARPS * 32);
+    constexpr int NCT = TCS_GROUP_WARPS * 32;  // threads of one group
+    // A: this thread owns tap k = its TMEM lane and half of the step's 32 pixels (two warps of a
+    // group share a lane quadrant); taps beyond the real ones are written as zeros
+    static_assert(TCS_GROUP_WARPS == 8, "two warps per TMEM lane quadrant in every converter group");
+    const int k = 32 * (warp & 3) + lane, phalf = ((warp - grp * TCS_GROUP_WARPS) >> 2) * 16;
+    int soff = -1;  // floats into the raw rows (without the step's column offset)
+    if (k < a.Kreal) {
+      const int c = k / KK, r = k - c * KK, ky = r / a.KW, kx = r - ky * a.KW;
+      soff = (c * a.KH + ky) * a.bw + kx + phalf;
+    }
+    const uint32_t ta_thread = tmem_a + (uint32_t)grp * 64u + ((uint32_t)(warp & 3) << 21) + (uint32_t)phalf;
+    constexpr int NB = 128 * 8 / NCT;  // at most 128 out channels x 8 quads per step
+    float bacc[NB];                    // bias partials of the (o, quad) items this thread owns
+#pragma unroll
+    for (int q = 0; q < NB; ++q) bacc[q] = 0.f;
+    long long w = 0, t0 = tc_clock(), tq;
+    // Every converter warp observes every step's barrier, in order, and takes part in the
+    // hand-over, although only the step's group converts: a warp that skipped phases of an
+    // mbarrier could no longer tell one phase from the one two later (the wait is by parity).
+    for (int s = s_begin; s < s_end; ++s) {
+      const uint32_t i = s - s_begin, st = i % a.nst;
+      tq = tc_clock();
+      if (!mbar_wait_bounded(&tma_full[st], (i / a.nst) & 1)) {
+        failed = true;
+        break;
+      }
+      w += tc_clock() - tq;
+      if ((int)(i % TCS_GROUPS) != grp) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&op_full[st]);
+        continue;
+      }
+      // this group's A buffer was read by the MMAs of its previous step
+      if (i >= 2 && !mbar_wait_bounded(&a_empty[grp], ((i >> 1) - 1) & 1)) {
+        failed = true;
+        break;
+      }
+      tc_fence_after();
+      uint8_t *p = smem + (size_t)st * STAGE;
+      const int x0 = (s % a.nxb) * TCS_PX;
+      const int d = (x0 - a.pad_l) - ((x0 - a.pad_l) & ~3);  // offset of the first needed column
+      const float *xr = reinterpret_cast<const float *>(p + 2 * BB) + d;
+      {
+        uint32_t h[16], l[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          float hv, lv;
+          split_tf32_rn(soff >= 0 ? xr[soff + q] : 0.f, hv, lv);
+          h[q] = __float_as_uint(hv);
+          l[q] = __float_as_uint(lv);
+        }
+        tmem_st16(ta_thread, h);
+        tmem_st16(ta_thread + 32, l);
+      }
+      // B: split the gradient tile in place (hi) and into the lo tile; bias partial sums
+#pragma unroll
+      for (int slot = 0; slot < NB; ++slot) {
+        const int it = gtid + NCT * slot;
+        if (it < a.OCp * 8) {
+          const int o = it >> 3, quad = it & 7;
+          const uint32_t off = (uint32_t)o * 128u + (uint32_t)((quad ^ (o & 7)) << 4);
+          float4 v = *reinterpret_cast<float4 *>(p + off);
+          float h[4], l[4];
+          split_tf32_rn(v.x, h[0], l[0]);
+          split_tf32_rn(v.y, h[1], l[1]);
+          split_tf32_rn(v.z, h[2], l[2]);
+          split_tf32_rn(v.w, h[3], l[3]);
+          *reinterpret_cast<float4 *>(p + off) = make_float4(h[0], h[1], h[2], h[3]);
+          *reinterpret_cast<float4 *>(p + BB + off) = make_float4(l[0], l[1], l[2], l[3]);
+          bacc[slot] += (v.x + v.y) + (v.z + v.w);
+        }
+      }
+      // generic-proxy writes -> visible to the tensor core (async proxy); the TMEM stores have
+      // landed; then hand over
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&op_full[st]);
+    }
+    if (a.dbg && tid == 0) {
+      a.dbg[blockIdx.x * 8 + 4] = tc_clock() - t0;
+      a.dbg[blockIdx.x * 8 + 5] = w;
+    }
+    // ---- epilogue ------------------------------------------------------------------------------
+    float *row = a.part + (size_t)blockIdx.x * a.row;
+#pragma unroll
+    for (int slot = 0; slot < NB; ++slot) {
+      const int it = gtid + NCT * slot;
+      if (it < a.OCp * 8) bsum_s[(grp * 8 + (it & 7)) * a.OCp + (it >> 3)] = bacc[slot];
+    }
+    asm volatile("bar.sync 1, %0;\n" ::"n"(TCS_CONV_WARPS * 32) : "memory");
+    for (int o = tid; o < a.OCp; o += TCS_CONV_WARPS * 32) {
+      float t = bsum_s[o];
+#pragma unroll
+      for (int q = 1; q < TCS_GROUPS * 8; ++q) t += bsum_s[q * a.OCp + o];
+      row[(size_t)128 * a.OCp + o] = t;
+    }
+    if (warp < 4 && s_end > s_begin && !failed) {
+      if (!mbar_wait_bounded(accum, 0)) failed = true;
+      tc_fence_after();
+    }
+    if (warp < 4 && !failed) {  // one warp per TMEM lane quadrant
+      const int k = warp * 32 + lane;
+      for (int c0 = 0; c0 < a.OCp; c0 += 16) {
+        float v[16];
+        if (s_end > s_begin) {
+          float w[16];
+          tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+          tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(a.OCp + c0), w);
+#pragma unroll
+          for (int q = 0; q < 16; ++q) v[q] += w[q];
+        } else {
+#pragma unroll
+          for (int q = 0; q < 16; ++q) v[q] = 0.f;
+        }
+        float4 *dst = reinterpret_cast<float4 *>(row + (size_t)k * a.OCp + c0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      }
+    }
+  }
+  if (failed && a.err) atomicExch(a.err, 5);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == TCS_CONV_WARPS) tmem_dealloc(tmem_base, (uint32_t)a.tmem_cols);
+}
+
+size_t dw_small_stage(const ConvGeom &g, int OCp, int bw) {
+  size_t XB = ((size_t)g.C * g.KH * bw * 4 + 1023) & ~(size_t)1023;
+  return 2 * (size_t)OCp * 128 + XB;
+}
+
+size_t dw_small_fixed(int OCp) {
+  return 1024 + (3 * TCS_MAX_STAGES + 3) * 8 + 32 + (size_t)TCS_GROUPS * 8 * OCp * 4 + 64;
+}
+
+// pipeline stages that fit (0: the kernel does not fit)
+int dw_small_stages(const b200_ctx *ctx, const ConvGeom &g, int OCp, int bw) {
+  size_t fixed = dw_small_fixed(OCp), stage = dw_small_stage(g, OCp, bw);
+  // at least as many stages as converter groups: a group waiting for the second use of a stage
+  // before its first use has happened would see the barrier's parity as already satisfied
+  if (ctx->smem_optin < fixed + TCS_GROUPS * stage) return 0;
+  size_t n = (ctx->smem_optin - fixed) / stage;
+  return (int)(n > TCS_MAX_STAGES ? TCS_MAX_STAGES : n);
+}
+
+int dw_small_bw(const ConvGeom &g) { return (TCS_PX + g.KW - 1 + 3 + 3) & ~3; }
+
+}  // namespace
+
+// true when the small-input-channel dW kernel applies
+bool conv_dw_small_ok(const b200_ctx *ctx, const ConvGeom &g) {
+  if (g.SH != 1 || g.SW != 1 || g.DH != 1 || g.DW != 1) return false;
+  if (g.C * g.KH * g.KW > 128 || g.OC > 128) return false;
+  if ((g.WI & 3) || (g.OW & 3)) return false;                 // TMA strides are multiples of 16 bytes
+  if (((size_t)g.HI * g.WI) & 3 || ((size_t)g.OH * g.OW) & 3) return false;
+  if (g.pad_t < 0 || g.pad_l < 0) return false;
+  if (g.OH + g.KH - 1 < g.HI + g.pad_t || g.OW + g.KW - 1 < g.WI + g.pad_l) return false;  // windows over all of it
+  const int OCp = (g.OC + 15) / 16 * 16;
+  return dw_small_stages(ctx, g, OCp, dw_small_bw(g)) >= TCS_GROUPS;
+}
+
+int conv_dw_small_splits(const b200_ctx *ctx, const ConvGeom &g, int B) {
+  long long nsteps = (long long)B * g.OH * ceil_div(g.OW, TCS_PX);
+  return (int)(nsteps < ctx->sm_count ? nsteps : ctx->sm_count);
+}
+
+size_t conv_dw_small_floats(const b200_ctx *ctx, const ConvGeom &g, int B) {
+  const int OCp = (g.OC + 15) / 16 * 16;
+  return ((size_t)conv_dw_small_splits(ctx, g, B) + 1) * ((size_t)129 * OCp);
+}
+
+// dW (+ db when the layer has a bias) from the CHW input and gradient; `part` holds conv_dw_small_floats
+int conv_dw_small(b200_ctx *ctx, const ConvGeom &g, const float *in, const float *dout, int B, float *part,
+                  float *dW, float *db, int accumulate) {
+  const int OCp = (g.OC + 15) / 16 * 16, bw = dw_small_bw(g);
+  EncodeTiledFn fn = encode_fn();
+  B200_REQUIRE(fn != nullptr, "cuTensorMapEncodeTiled is not available from the driver");
+  CUtensorMap x_map, dy_map;
+  {
+    cuuint64_t dims[4] = {(cuuint64_t)g.WI, (cuuint64_t)g.HI, (cuuint64_t)g.C, (cuuint64_t)B};
+    cuuint64_t strides[3] = {(cuuint64_t)g.WI * 4, (cuuint64_t)g.HI * g.WI * 4, (cuuint64_t)g.C * g.HI * g.WI * 4};
+    cuuint32_t box[4] = {(cuuint32_t)bw, (cuuint32_t)g.KH, (cuuint32_t)g.C, 1};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = fn(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(in), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    B200_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed (%d) for the input rows", (int)r);
+  }
+  {
+    // dimensions ordered (x, o, y, b) so that one box is the K-major tile [o][32 pixels]
+    cuuint64_t dims[4] = {(cuuint64_t)g.OW, (cuuint64_t)g.OC, (cuuint64_t)g.OH, (cuuint64_t)B};
+    cuuint64_t strides[3] = {(cuuint64_t)g.OH * g.OW * 4, (cuuint64_t)g.OW * 4, (cuuint64_t)g.OC * g.OH * g.OW * 4};
+    cuuint32_t box[4] = {TCS_PX, (cuuint32_t)OCp, 1, 1};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = fn(&dy_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(dout), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    B200_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed (%d) for the gradient tiles", (int)r);
+  }
+  TcDwSmallArgs a;
+  a.part = part;
+  a.err = ctx->dev_err;
+  a.C = g.C;
+  a.OC = g.OC;
+  a.OCp = OCp;
+  a.KH = g.KH;
+  a.KW = g.KW;
+  a.pad_t = g.pad_t;
+  a.pad_l = g.pad_l;
+  a.OH = g.OH;
+  a.OW = g.OW;
+  a.nxb = ceil_div(g.OW, TCS_PX);
+  a.Kreal = g.C * g.KH * g.KW;
+  a.bw = bw;
+  a.nsteps = B * g.OH * a.nxb;
+  a.ksplits = conv_dw_small_splits(ctx, g, B);
+  a.nst = dw_small_stages(ctx, g, OCp, bw);
+  B200_REQUIRE(a.nst >= TCS_GROUPS, "conv_dw_small: the tiles do not fit shared memory");
+  a.tmem_cols = pow2_cols(2 * OCp + 128);
+  a.row = (long long)129 * OCp;
+  const size_t smem = dw_small_fixed(OCp) + (size_t)a.nst * dw_small_stage(g, OCp, bw);
+  B200_CUDA(cudaFuncSetAttribute(conv_dw_small_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  a.dbg = nullptr;
+#ifdef B200_TC_TIMING
+  static const bool timing = getenv("B200_TC_TIMING") != nullptr;
+  if (timing) B200_CUDA(cudaMalloc(&a.dbg, (size_t)a.ksplits * 8 * sizeof(long long)));
+#endif
+  conv_dw_small_tc_kernel<<<a.ksplits, TCS_THREADS, smem, ctx->stream>>>(x_map, dy_map, a);
+  B200_LAUNCHED();
+#ifdef B200_TC_TIMING
+  if (timing) {  // diagnostic: cycles of the three roles and of their waits, averaged over blocks
+    std::vector<long long> h((size_t)a.ksplits * 8);
+    B200_CUDA(cudaStreamSynchronize(ctx->stream));
+    B200_CUDA(cudaMemcpy(h.data(), a.dbg, h.size() * sizeof(long long), cudaMemcpyDeviceToHost));
+    B200_CUDA(cudaFree(a.dbg));
+    double s[8] = {0};
+    for (int i = 0; i < a.ksplits; ++i)
+      for (int k = 0; k < 8; ++k) s[k] += (double)h[(size_t)i * 8 + k] / a.ksplits;
+    fprintf(stderr,
+            "[tc-timing] dW small: steps/block %.1f stages %d: producer %.0f clk (wait %.0f), mma %.0f (wait %.0f), "
+            "converter group 0 %.0f (wait %.0f)\n",
+            (double)a.nsteps / a.ksplits, a.nst, s[0], s[1], s[2], s[3], s[4], s[5]);
+  }
+#endif
+  DwFinishArgs f;
+  f.part = part;
+  f.part_stride = a.row;
+  f.splits = a.ksplits;
+  f.bsrc = part;            // the bias sums are the last OCp entries of every partial row
+  f.bs_stride = a.row;
+  f.bs_off = (long long)128 * OCp;
+  f.bs_rows = a.ksplits;
+  f.dW = dW;
+  f.db = g.has_bias ? db : nullptr;
+  f.row_w = 128 * OCp;
+  f.C = g.C;
+  f.OC = g.OC;
+  f.OCp = OCp;
+  f.KH = g.KH;
+  f.KW = g.KW;
+  f.tbl = g.tbl;
+  f.accumulate = accumulate;
+  B200_TRY(launch_dw_finish(ctx, f));
+  return 0;
+}
+
 }  // namespace b200

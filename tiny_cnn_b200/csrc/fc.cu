@@ -186,8 +186,8 @@ static bool use_tc(const b200_ctx *ctx, int M, int N, int K) {
 size_t fc_scratch_floats(const b200_ctx *ctx, int in_size, int out_size, int B) {
   size_t need = 0;
   if (ctx->fc_tensor_cores != 0) {
-    size_t t[3] = {gemm_tc_scratch_floats(B, out_size, in_size), gemm_tc_scratch_floats(B, in_size, out_size),
-                   gemm_tc_scratch_floats(in_size, out_size, B)};
+    size_t t[4] = {gemm_tc_scratch_floats(B, out_size, in_size), gemm_tc_scratch_floats(B, in_size, out_size),
+                   gemm_tc_scratch_floats(in_size, out_size, B), gemm_tc_scratch_floats(out_size, in_size, B)};
     for (size_t v : t)
       if (v > need) need = v;
   }
@@ -229,39 +229,45 @@ static int run_gemm(b200_ctx *ctx, int M, int N, int K, const float *A, long lon
   return 0;
 }
 
+// `w_rows`: the weights are stored [out][in] (a convolution whose window is the whole input), not [in][out]
 int fc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
-           const float *bias, float *out, int B, int act, float *scratch) {
+           const float *bias, float *out, int B, int act, float *scratch, bool w_rows) {
   if (scratch && use_tc(ctx, B, out_size, in_size))
     // A = in [B][in]; Bt = W^T: W is [in][out], i.e. K x N, transposed while splitting
-    return gemm_tc(ctx, B, out_size, in_size, in, in_size, false, W, out_size, true, out, bias, 0,
+    return gemm_tc(ctx, B, out_size, in_size, in, in_size, false, W, w_rows ? in_size : out_size, !w_rows, out, bias, 0,
                    act, scratch);
-  // M = B, N = out, K = in; A = in (k fast), Bm = W[k][n] (n fast)
+  // M = B, N = out, K = in; A = in (k fast), Bm(k, n) = W[k][n] (n fast) or W[n][k] (k fast)
+  if (w_rows)
+    return run_gemm<true, false>(ctx, B, out_size, in_size, in, in_size, 1, W, 1, in_size, out, bias, 0, act, scratch);
   return run_gemm<true, true>(ctx, B, out_size, in_size, in, in_size, 1, W, out_size, 1, out, bias,
                               0, act, scratch);
 }
 
 int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
            const float *dout, float *din, float *dW, float *db, int accumulate, int B,
-           float *scratch) {
+           float *scratch, bool w_rows) {
   if (din && scratch && use_tc(ctx, B, in_size, out_size)) {
     // din[B][in] = dout[B][out] * W^T: A = dout; Bt[n = c][k = o] = W[c*out + o] as stored
-    B200_TRY(gemm_tc(ctx, B, in_size, out_size, dout, out_size, false, W, out_size, false, din,
+    B200_TRY(gemm_tc(ctx, B, in_size, out_size, dout, out_size, false, W, w_rows ? in_size : out_size, w_rows, din,
                      nullptr, 0, 0, scratch));
+  } else if (din && w_rows) {
+    B200_TRY((run_gemm<true, true>(ctx, B, in_size, out_size, dout, out_size, 1, W, in_size, 1,
+                                   din, nullptr, 0, 0, scratch)));
   } else if (din) {
     // din[B][in] = dout[B][out] * W^T : M = B, N = in, K = out;
     // Bm(k = o, n = c) = W[c*out + o] -> b_k = 1, b_n = out (k fast)
     B200_TRY((run_gemm<true, false>(ctx, B, in_size, out_size, dout, out_size, 1, W, 1, out_size,
                                     din, nullptr, 0, 0, scratch)));
   }
-  if (dW && scratch && use_tc(ctx, in_size, out_size, B)) {
-    // dW[in][out] (+)= in^T * dout: A = in^T (in is B x in = K x M), Bt = dout^T (K x N)
-    B200_TRY(gemm_tc(ctx, in_size, out_size, B, in, in_size, true, dout, out_size, true, dW, nullptr,
-                     accumulate, 0, scratch));
-  } else if (dW) {
-    // dW[in][out] (+)= in^T * dout : M = in, N = out, K = B;
-    // A(m = c, k = n) = in[n*in + c] -> a_m = 1, a_k = in (m fast)
-    B200_TRY((run_gemm<false, true>(ctx, in_size, out_size, B, in, 1, in_size, dout, out_size, 1,
-                                    dW, nullptr, accumulate, 0, scratch)));
+  if (dW) {
+    // dW[in][out] (+)= in^T * dout, or dW[out][in] (+)= dout^T * in
+    const float *p = w_rows ? dout : in, *q = w_rows ? in : dout;
+    const int M = w_rows ? out_size : in_size, N = w_rows ? in_size : out_size;
+    if (scratch && use_tc(ctx, M, N, B))
+      B200_TRY(gemm_tc(ctx, M, N, B, p, M, true, q, N, true, dW, nullptr, accumulate, 0, scratch));
+    else
+      // A(m, k = n) = p[n*M + m] (m fast)
+      B200_TRY((run_gemm<false, true>(ctx, M, N, B, p, 1, M, q, N, 1, dW, nullptr, accumulate, 0, scratch)));
   }
   if (db) {
     col_sum_kernel<<<ceil_div(out_size, 32), dim3(32, 8), 0, ctx->stream>>>(dout, db, B, out_size,

@@ -31,11 +31,9 @@ struct Layer {
   int32_t *argmax = nullptr;
   bool tiled = false;
   float *wt_fwd = nullptr, *wt_dx = nullptr, *dw_part = nullptr;
-  // tensor-core passes: tall split copies of the input and of dY, per-block bias partials,
-  // filter matrices, partial weight gradients
-  ConvTcUse tc = {false, false, false, false};
-  float *tc_xs = nullptr, *tc_dys = nullptr, *tc_bsum = nullptr;
-  float *tc_wt_fwd = nullptr, *tc_wt_dx = nullptr, *tc_part = nullptr, *tc_small_part = nullptr;
+  // tensor-core passes: filter blocks of the forward and dX passes, partial weight gradients
+  ConvTcUse tc = {};
+  float *tc_wt_fwd = nullptr, *tc_wt_dx = nullptr, *tc_part = nullptr;
   float *fc_scratch = nullptr;  // k-slice partial sums of the small GEMMs
   float *fc_scratch_side = nullptr;  // the same for the dW GEMM when it runs on the side stream
   float act_param = 0.f;  // leaky relu: epsilon; elu: alpha
@@ -48,13 +46,8 @@ struct Layer {
   bool skipped = false;   // activation layer folded into the previous layer
   bool relu_bwd_fused = false;   // max-pool: also applies the gradient of the relu before it
   bool bwd_done_by_next = false; // relu: its gradient is produced by the pooling layer after it
-  // 2x2 max-pool next to a tensor-core convolution: the pooling kernels also write the tall split
-  // copies that convolution reads (its input in the forward pass, its dY in the backward pass)
   cudaEvent_t ev_prep = nullptr;  // convolution: its filter matrices / copies are ready (side stream)
   bool dx_prep_side = false;      // the FFMA dX filter copy of this step was made beside the forward pass
-  int feeds_conv = -1;     // max-pool: convolution layer whose input copy it writes
-  int grad_to_conv = -1;   // max-pool: convolution layer whose dY copy it writes
-  bool xs_from_pool = false, dys_from_pool = false;  // convolution: copies come from the pooling layers
 };
 
 }  // namespace
@@ -67,7 +60,6 @@ struct b200_net {
   // index of that fully-connected layer (-1: none) and of a relu directly before it (-1: none)
   int head_fc = -1, head_relu = -1;
   bool train_phase = true;  // net_phase::train (b200_net_set_phase)
-  bool batch_finishes = false;  // B200_NET_BATCH_FINISH=1
   std::vector<OptSegment> segs;  // trainable tensors in update order
   size_t n_params = 0;
   float *params = nullptr, *grads = nullptr, *state0 = nullptr, *state1 = nullptr;
@@ -104,7 +96,6 @@ struct b200_net {
   int fit_rows = 0;  // rows of x_dev / t_dev the last step of a fit call ran on
   bool fuse = true;
   bool input_grad = true;
-  bool keep_layer_grads = false;  // B200_NET_KEEP_GRADS=1: every layer's dE/d out also in CHW form
   PeerReduce peer;  // data-parallel replicas: the gradient bucket is summed over the ranks inside the step
   // the layers after `peer_early_layer` (inclusive) own bucket entries [peer.split, n): once their weight
   // gradients exist they are pushed to the peers from `comm`, beside the rest of the backward pass
@@ -171,7 +162,8 @@ int net_forward_impl(b200_net *net, const float *x, int B) {
         if (L.kind != B200_LAYER_CONV || !L.ev_prep) continue;
         const bool dx_copy = L.tiled && !L.tc.dx && L.g.OW <= 64 && L.wt_dx && (i > 0 || net->input_grad);
         if (pass == 0) L.dx_prep_side = false;
-        if (pass == 0 ? !L.tc.fwd : !dx_copy) continue;
+        const bool tc_dx = L.tc.dx && (i > 0 || net->input_grad);
+        if (pass == 0 ? !L.tc.fwd && !tc_dx : !dx_copy) continue;
         if (!prep_on_side) {
           B200_CUDA(cudaEventRecord(net->ev_fork, main_stream));
           B200_CUDA(cudaStreamWaitEvent(net->side, net->ev_fork, 0));
@@ -180,7 +172,7 @@ int net_forward_impl(b200_net *net, const float *x, int B) {
         ctx->stream = net->side;
         int rc;
         if (pass == 0) {
-          rc = conv_tc_prep(ctx, L.g, net->params + L.w_off, L.tc_wt_fwd, L.tc.dx ? L.tc_wt_dx : nullptr);
+          rc = conv_gather_prep(ctx, L.g, net->params + L.w_off, L.tc_wt_fwd, tc_dx ? L.tc_wt_dx : nullptr);
         } else {
           rc = conv_tiled_dx_prep(ctx, L.g, net->params + L.w_off, L.wt_dx);
           L.dx_prep_side = rc == 0;
@@ -201,22 +193,27 @@ int net_forward_impl(b200_net *net, const float *x, int B) {
     const float *W = net->params + L.w_off;
     const float *b = L.b_len ? net->params + L.b_off : nullptr;
     switch (L.kind) {
-      case B200_LAYER_CONV:
-        if (L.tc.fwd) {
-          if (!L.xs_from_pool) B200_TRY(conv_tc_tall_x(ctx, L.g, in, B, L.tc_xs));
-          // the dX pass of this step reads the same weights: both filter matrices in one launch
-          if (prep_on_side && L.ev_prep && L.tc.fwd)
+      case B200_LAYER_CONV: {
+        // the dX pass of this step reads the same weights: both passes' filter blocks in one launch
+        const bool tc_dx = L.tc.dx && (i > 0 || net->input_grad);
+        if (L.tc.fwd || tc_dx) {
+          if (prep_on_side && L.ev_prep)
             B200_CUDA(cudaStreamWaitEvent(ctx->stream, L.ev_prep, 0));
           else
-            B200_TRY(conv_tc_prep(ctx, L.g, W, L.tc_wt_fwd, L.tc.dx ? L.tc_wt_dx : nullptr));
-          B200_TRY(conv_tc_fwd(ctx, L.g, L.tc_xs, W, b, dst, B, L.fused_act, L.tc_wt_fwd, 0));
-        } else if (L.tc.fwd_small)
+            B200_TRY(conv_gather_prep(ctx, L.g, W, L.tc_wt_fwd, tc_dx ? L.tc_wt_dx : nullptr));
+        }
+        if (L.tc.fwd) {
+          B200_TRY(conv_gather_fwd(ctx, L.g, in, L.tc_wt_fwd, b, dst, B, L.fused_act));
+        } else if (L.tc.fc)
+          B200_TRY(fc_fwd(ctx, (int)L.in_dim, L.g.OC, in, W, b, dst, B, L.fused_act, L.fc_scratch, true));
+        else if (L.tc.fwd_small)
           B200_TRY(conv_fwd_small(ctx, L.g, in, W, b, dst, B, L.fused_act));
         else if (L.tiled)
           B200_TRY(conv_tiled_fwd(ctx, L.g, in, W, b, dst, B, L.fused_act, L.wt_fwd));
         else
           B200_TRY(conv_general_fwd(ctx, L.g, in, W, b, dst, B, L.fused_act));
         break;
+      }
       case B200_LAYER_FC:
         if ((int)i == net->head_fc)
           B200_TRY(fc_softmax_fwd(ctx, L.fc_in, L.fc_out, in, W, b, dst, net->layers[n - 1].out, B));
@@ -224,12 +221,7 @@ int net_forward_impl(b200_net *net, const float *x, int B) {
           B200_TRY(fc_fwd(ctx, L.fc_in, L.fc_out, in, W, b, dst, B, L.fused_act, L.fc_scratch));
         break;
       case B200_LAYER_MAXPOOL:
-        if (L.feeds_conv >= 0) {
-          Layer &Cv = net->layers[L.feeds_conv];
-          B200_TRY(conv_tc_tall_x_pool(ctx, Cv.g, in, dst, L.argmax, B, Cv.tc_xs));
-        } else {
-          B200_TRY(maxpool_fwd(ctx, L.pd, in, dst, L.argmax, B));
-        }
+        B200_TRY(maxpool_fwd(ctx, L.pd, in, dst, L.argmax, B));
         break;
       case B200_LAYER_AVGPOOL:
         B200_TRY(avgpool_fwd(ctx, L.pd, in, W, b, dst, B));
@@ -299,19 +291,17 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
     side_used = true;
     return 0;
   };
-  // The finishing passes of the tensor-core dW kernels (partial rows -> gradient in the reference
-  // layout) can be collected and launched together (before the gradients leave for the other
-  // replicas, and at the end of the pass) instead of after each dW kernel: B200_NET_BATCH_FINISH=1.
-  // Measured slower on the benchmark step (0.335 against 0.323 ms: the one launch then shares the SMs
-  // with the first layer's dX), so each pass follows its kernel by default.
-  std::vector<DwFinishArgs> finishes;
-  auto flush_finishes = [&]() -> int {
-    if (finishes.empty()) return 0;
-    ctx->stream = net->side;  // they were produced there (fork() ran)
-    int rc = dw_finish_many(ctx, finishes.data(), (int)finishes.size());
+  // a fully-connected layer, or a convolution that is one (w_rows)
+  auto fc_backward = [&](Layer &L, bool w_rows, const float *in, float *din, const float *W, float *dW, float *db,
+                         bool can_fork) -> int {
+    const int n_in = (int)L.in_dim, n_out = (int)L.out_dim;
+    if (!can_fork || !L.fc_scratch_side)
+      return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, dW, db, 0, B, L.fc_scratch, w_rows);
+    B200_TRY(fork());
+    rc_side = fc_bwd(ctx, n_in, n_out, in, W, L.grad, nullptr, dW, db, 0, B, L.fc_scratch_side, w_rows);
     ctx->stream = main_stream;
-    finishes.clear();
-    return rc;
+    if (rc_side) return 0;
+    return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, nullptr, nullptr, 0, B, L.fc_scratch, w_rows);
   };
   for (int i = tail_fused ? n - 2 : n - 1; i >= 0 && rc_side == 0; --i) {
     Layer &L = net->layers[i];
@@ -326,28 +316,19 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
     const bool can_fork = net->side != nullptr && (din != nullptr || head);
     switch (L.kind) {
       case B200_LAYER_CONV: {
+        if (L.tc.fc) {
+          B200_TRY(fc_backward(L, true, in, din, W, dW, db, can_fork));
+          break;
+        }
         bool tiled_bwd = L.tiled && L.g.OW <= 64;
         const bool tc_dx = L.tc.dx && din != nullptr;
-        if ((tc_dx || L.tc.dw) && !L.dys_from_pool)
-          B200_TRY(conv_tc_tall_dy(ctx, L.g, L.grad, B, L.tc_dys, L.tc.dw && db ? L.tc_bsum : nullptr));
         // dW first: its launch precedes the dX launch, so a one-block-per-SM dW kernel is resident
         // when the small blocks of an FFMA dX arrive and both share the SMs
-        const bool forked = can_fork && (L.tc.dw || L.tc.dw_small);
-        const bool batch_fin = forked && net->batch_finishes;
-        if (forked) B200_TRY(fork());
+        if (can_fork && (L.tc.dw || L.tc.dw_small)) B200_TRY(fork());
         if (L.tc.dw) {
-          if (!L.tc.fwd && !L.xs_from_pool) rc_side = conv_tc_tall_x(ctx, L.g, in, B, L.tc_xs);
-          int splits = 0;
-          if (!rc_side) rc_side = conv_tc_dw(ctx, L.g, L.tc_xs, L.tc_dys, B, L.tc_part, &splits);
-          DwFinishArgs later;
-          if (!rc_side)
-            rc_side = conv_tc_dw_finish(ctx, L.g, L.tc_part, splits, dW, 0, db ? L.tc_bsum : nullptr, B, db,
-                                        batch_fin ? &later : nullptr);
-          if (!rc_side && batch_fin) finishes.push_back(later);
+          rc_side = conv_gather_dw(ctx, L.g, in, L.grad, B, L.tc_part, dW, db, 0);
         } else if (L.tc.dw_small) {
-          DwFinishArgs later;
-          rc_side = conv_dw_small(ctx, L.g, in, L.grad, B, L.tc_small_part, dW, db, 0, batch_fin ? &later : nullptr);
-          if (!rc_side && batch_fin) finishes.push_back(later);
+          rc_side = conv_dw_small(ctx, L.g, in, L.grad, B, L.tc_part, dW, db, 0);
         } else if (tiled_bwd) {
           int splits = 0;
           rc_side = conv_tiled_dw_partials(ctx, L.g, in, L.grad, B, L.dw_part, &splits);
@@ -367,7 +348,7 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
         if (rc_side) break;
         if (din) {
           if (tc_dx)
-            B200_TRY(conv_tc_dx(ctx, L.g, L.tc_dys, W, din, B, L.tc_wt_dx, L.tc.fwd ? 0 : 1));
+            B200_TRY(conv_gather_dx(ctx, L.g, L.grad, L.tc_wt_dx, din, B));
           else if (tiled_bwd) {
             // the filter copy was made beside the forward pass (same weights: nothing updates
             // them between the two passes of a step)
@@ -380,30 +361,10 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
         break;
       }
       case B200_LAYER_FC:
-        if (can_fork && L.fc_scratch_side) {
-          B200_TRY(fork());
-          rc_side = fc_bwd(ctx, L.fc_in, L.fc_out, in, W, L.grad, nullptr, dW, db, 0, B, L.fc_scratch_side);
-          ctx->stream = main_stream;
-          if (rc_side) break;
-          B200_TRY(fc_bwd(ctx, L.fc_in, L.fc_out, in, W, L.grad, din, nullptr, nullptr, 0, B, L.fc_scratch));
-        } else {
-          B200_TRY(fc_bwd(ctx, L.fc_in, L.fc_out, in, W, L.grad, din, dW, db, 0, B, L.fc_scratch));
-        }
+        B200_TRY(fc_backward(L, false, in, din, W, dW, db, can_fork));
         break;
       case B200_LAYER_MAXPOOL:
-        if (L.grad_to_conv >= 0) {
-          // gradient of this layer (and of the relu before it) written straight into the forms the
-          // tensor-core convolution reads: tall split copy, CHW gradient, bias partials
-          Layer &Cv = net->layers[L.grad_to_conv];
-          // the CHW form of the convolution's dY is written only when one of its backward kernels
-          // reads it (the tensor-core dW and dX passes read the tall copy)
-          const bool cv_din = L.grad_to_conv > 0 || net->input_grad;
-          const bool chw_read = !Cv.tc.dw || (cv_din && !Cv.tc.dx) || net->keep_layer_grads;
-          B200_TRY(conv_tc_tall_dy_unpool(ctx, Cv.g, L.grad, L.argmax,
-                                          L.relu_bwd_fused ? L.out : nullptr,
-                                          chw_read ? Cv.grad : nullptr, B, Cv.tc_dys,
-                                          Cv.tc.dw && Cv.b_len ? Cv.tc_bsum : nullptr));
-        } else if (L.relu_bwd_fused) {
+        if (L.relu_bwd_fused) {
           // the relu before this layer was folded into the producer's epilogue: apply
           // its gradient mask here and write straight into the producer's gradient
           B200_TRY(maxpool_bwd(ctx, L.pd, L.grad, L.argmax, net->layers[i - 2].grad, B, L.out));
@@ -430,7 +391,6 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
       default: B200_REQUIRE(false, "net_backward: unknown layer kind %d", L.kind);
     }
     if (peer_in_step && i == net->peer_early_layer && rc_side == 0 && net->comm) {
-      B200_TRY(flush_finishes());
       // every weight gradient of layers i.. has been issued (main or side stream): send them to
       // the peers now, from a third stream, while the remaining layers still compute
       B200_CUDA(cudaEventRecord(net->ev_comm_main, main_stream));
@@ -453,7 +413,6 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
     }
   }
   ctx->stream = main_stream;
-  if (rc_side == 0) B200_TRY(flush_finishes());
   if (side_used) {  // the optimizer (or the caller's all-reduce) follows on the main stream
     B200_CUDA(cudaEventRecord(net->ev_join, net->side));
     B200_CUDA(cudaStreamWaitEvent(main_stream, net->ev_join, 0));
@@ -547,9 +506,7 @@ int b200_net_create(b200_ctx *ctx, const b200_layer_spec *specs, int n_layers, i
   net->max_batch = max_batch;
   net->layers.resize(n_layers);
   if (const char *e = getenv("B200_NET_NO_FUSE")) net->fuse = !(e[0] == '1');
-  if (const char *e = getenv("B200_NET_BATCH_FINISH")) net->batch_finishes = e[0] == '1';
   if (const char *e = getenv("B200_NET_NO_GRAPH")) net->use_graph = !(e[0] == '1');
-  if (const char *e = getenv("B200_NET_KEEP_GRADS")) net->keep_layer_grads = e[0] == '1';
   if (!getenv("B200_NET_NO_SIDE")) {
     cudaStreamCreateWithFlags(&net->side, cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&net->ev_fork, cudaEventDisableTiming);
@@ -679,31 +636,6 @@ int b200_net_create(b200_ctx *ctx, const b200_layer_spec *specs, int n_layers, i
       if (n_layers >= 3 && net->layers[n_layers - 3].kind == B200_LAYER_RELU) net->head_relu = n_layers - 3;
     }
   }
-  // 2x2 max-pool beside a tensor-core convolution: fuse the tall conversions into the pooling kernels
-  if (net->fuse) {
-    for (int i = 0; i < n_layers; ++i) {
-      Layer &P = net->layers[i];
-      if (P.kind != B200_LAYER_MAXPOOL || !maxpool_can_fuse_relu(P.pd)) continue;
-      if (i + 1 < n_layers) {
-        Layer &N = net->layers[i + 1];
-        if (N.kind == B200_LAYER_CONV && (N.tc.fwd || N.tc.dw) && N.g.C == P.pd.in_c &&
-            N.g.HI == P.pd.out_h && N.g.WI == P.pd.out_w) {
-          P.feeds_conv = i + 1;
-          N.xs_from_pool = true;
-        }
-      }
-      int j = P.relu_bwd_fused ? i - 2 : i - 1;
-      if (j >= 0 && (P.relu_bwd_fused || !net->layers[i - 1].skipped)) {
-        Layer &Cv = net->layers[j];
-        if (Cv.kind == B200_LAYER_CONV && (Cv.tc.dx || Cv.tc.dw) && Cv.g.OC == P.pd.in_c &&
-            Cv.g.OH == P.pd.in_h && Cv.g.OW == P.pd.in_w && (P.relu_bwd_fused || j == i - 1) &&
-            (P.relu_bwd_fused || Cv.fused_act == 0)) {
-          P.grad_to_conv = j;
-          Cv.dys_from_pool = true;
-        }
-      }
-    }
-  }
   // device memory
   size_t f = sizeof(float);
   B200_TRY(net_alloc((void **)&net->params, off * f));
@@ -732,34 +664,24 @@ int b200_net_create(b200_ctx *ctx, const b200_layer_spec *specs, int n_layers, i
     B200_TRY(net_alloc((void **)&L.grad, L.out_dim * max_batch * f));
     if (L.kind == B200_LAYER_MAXPOOL)
       B200_TRY(net_alloc((void **)&L.argmax, L.out_dim * max_batch * sizeof(int32_t)));
-    if (L.kind == B200_LAYER_FC) {
-      B200_TRY(net_alloc((void **)&L.fc_scratch,
-                         fc_scratch_floats(ctx, L.fc_in, L.fc_out, max_batch) * f));
-      if (net->side)
-        B200_TRY(net_alloc((void **)&L.fc_scratch_side,
-                           fc_scratch_floats(ctx, L.fc_in, L.fc_out, max_batch) * f));
+    if (L.kind == B200_LAYER_FC || (L.kind == B200_LAYER_CONV && L.tc.fc)) {
+      const size_t need = fc_scratch_floats(ctx, (int)L.in_dim, (int)L.out_dim, max_batch);
+      B200_TRY(net_alloc((void **)&L.fc_scratch, need * f));
+      if (net->side) B200_TRY(net_alloc((void **)&L.fc_scratch_side, need * f));
     }
-    if (L.kind == B200_LAYER_CONV && L.tiled) {
+    if (L.kind == B200_LAYER_CONV && L.tiled && !L.tc.fc) {
       B200_TRY(net_alloc((void **)&L.wt_fwd, conv_tiled_fwd_scratch(L.g) * f));
       B200_TRY(net_alloc((void **)&L.wt_dx, conv_tiled_dx_scratch(L.g) * f));
       size_t need = conv_tiled_dw_scratch(ctx, L.g, max_batch);
       B200_TRY(net_alloc((void **)&L.dw_part, need * f));
     }
-    if (L.kind == B200_LAYER_CONV && L.tc.dw_small)
-      B200_TRY(net_alloc((void **)&L.tc_small_part, conv_dw_small_floats(ctx, L.g, max_batch) * f));
-    if (L.kind == B200_LAYER_CONV && (L.tc.fwd || L.tiled) && net->side)
-      B200_CUDA(cudaEventCreateWithFlags(&L.ev_prep, cudaEventDisableTiming));
-    if (L.kind == B200_LAYER_CONV && (L.tc.fwd || L.tc.dx || L.tc.dw)) {
-      if (L.tc.fwd || L.tc.dw)
-        B200_TRY(net_alloc((void **)&L.tc_xs, conv_tc_tall_floats(L.g, max_batch, 0) * f));
-      if (L.tc.dx || L.tc.dw)
-        B200_TRY(net_alloc((void **)&L.tc_dys, conv_tc_tall_floats(L.g, max_batch, 1) * f));
-      if (L.tc.fwd) B200_TRY(net_alloc((void **)&L.tc_wt_fwd, conv_tc_filter_floats(ctx, L.g, 0) * f));
-      if (L.tc.dx) B200_TRY(net_alloc((void **)&L.tc_wt_dx, conv_tc_filter_floats(ctx, L.g, 1) * f));
-      if (L.tc.dw) {
-        B200_TRY(net_alloc((void **)&L.tc_part, conv_tc_dw_floats(ctx, L.g, max_batch) * f));
-        B200_TRY(net_alloc((void **)&L.tc_bsum, (size_t)conv_tc_bsum_rows(L.g, max_batch) * L.g.OC * f + 64));
-      }
+    if (L.kind == B200_LAYER_CONV) {
+      if ((L.tc.fwd || L.tc.dx || L.tiled) && net->side)
+        B200_CUDA(cudaEventCreateWithFlags(&L.ev_prep, cudaEventDisableTiming));
+      if (L.tc.fwd) B200_TRY(net_alloc((void **)&L.tc_wt_fwd, conv_gather_filter_floats(ctx, L.g, 0) * f));
+      if (L.tc.dx) B200_TRY(net_alloc((void **)&L.tc_wt_dx, conv_gather_filter_floats(ctx, L.g, 1) * f));
+      if (L.tc.dw) B200_TRY(net_alloc((void **)&L.tc_part, conv_gather_dw_floats(ctx, L.g, max_batch) * f));
+      if (L.tc.dw_small) B200_TRY(net_alloc((void **)&L.tc_part, conv_dw_small_floats(ctx, L.g, max_batch) * f));
     }
   }
   *out = net;
@@ -786,13 +708,9 @@ int b200_net_destroy(b200_net *net) {
     if (L.ev_prep) cudaEventDestroy(L.ev_prep);
     cudaFree(L.dw_part);
     cudaFree(L.fc_scratch_side);
-    cudaFree(L.tc_xs);
-    cudaFree(L.tc_dys);
-    cudaFree(L.tc_bsum);
     cudaFree(L.tc_wt_fwd);
     cudaFree(L.tc_wt_dx);
     cudaFree(L.tc_part);
-    cudaFree(L.tc_small_part);
     cudaFree(L.fc_scratch);
   }
   cudaFree(net->params);
