@@ -1,0 +1,88 @@
+"""The kernels that choose their tiling by size, at the sizes where it can go wrong: edges of tiles, remainders, the
+smallest and the largest of a range.  Convolutions and matrix products against the same sums in double precision,
+whole-network kernels against the layers one by one."""
+import numpy as np
+import pytest
+import torch
+import torch.nn.functional as F
+
+from test_ops_gpu import FWD_TOL, GRAD_TOL, assert_close, host
+from tiny_cnn_b200 import _lib as L
+from tiny_cnn_b200 import network, ops
+
+pytestmark = pytest.mark.gpu
+
+
+# w, h, in, out, k, stride, same, batch
+@pytest.mark.parametrize("case", [
+    (7, 9, 3, 6, 3, 1, True, 1),        # one tile, channels below a vector
+    (13, 11, 17, 130, 3, 1, True, 5),   # two output groups, a channel more than a slab
+    (56, 7, 64, 64, 3, 1, True, 3),     # wide rows, remainder of a pixel set
+    (15, 12, 33, 47, 5, 2, False, 9),   # stride 2, phases of unequal size, odd everything
+    (10, 10, 8, 24, 5, 3, False, 4),    # stride 3: residues without a tap
+    (64, 64, 4, 20, 3, 1, False, 2),    # largest map
+    (8, 8, 256, 256, 3, 1, True, 20),   # most channels
+    (9, 8, 24, 16, 3, 2, True, 300),    # many images in a pixel set
+    (5, 5, 16, 120, 5, 1, False, 16),   # window as large as the input
+])
+def test_conv_tensor_core_edges(ctx, case):
+    w, h, c, oc, k, stride, same, B = case
+    d = ops.conv_params(w, h, c, k, k, oc, same, True, stride, stride)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(B, c * h * w, device="cuda", generator=g)
+    W = torch.randn(oc * c * k * k, device="cuda", generator=g) * 0.1
+    b = torch.randn(oc, device="cuda", generator=g)
+    dy = torch.randn(B, oc * d.out_h * d.out_w, device="cuda", generator=g)
+    y = ops.conv2d_op(ctx, d, x, W, b)
+    dx, dW, db = ops.conv2d_grad_op(ctx, d, x, W, dy)
+    xr = x.double().view(B, c, h, w).requires_grad_()
+    Wr = W.double().view(oc, c, k, k).requires_grad_()
+    br = b.double().requires_grad_()
+    xp = xr
+    if same:
+        xp = F.pad(xr, (k // 2, k - 1 - k // 2, k // 2, k - 1 - k // 2))
+    yr = F.conv2d(xp, Wr, br, stride=stride)[:, :, :d.out_h, :d.out_w]
+    yr.backward(dy.double().view_as(yr))
+    assert_close(host(y), yr.detach().reshape(B, -1).cpu().numpy(), FWD_TOL, "y")
+    for got, want, name in ((dx, xr, "dx"), (dW, Wr, "dW"), (db, br, "db")):
+        assert_close(host(got).reshape(-1), want.grad.reshape(-1).cpu().numpy(), GRAD_TOL, name)
+
+
+def _nets():
+    def odd():
+        n = network.Sequential()
+        n.convolutional_layer(17, 13, 3, 3, 5, pad_same=True).relu_layer().max_pooling_layer(17, 13, 5, 2)
+        n.convolutional_layer(8, 6, 3, 5, 7, w_stride=2, h_stride=2).sigmoid_layer()
+        n.fully_connected_layer(3 * 2 * 7, 37).tanh_layer()
+        return n.fully_connected_layer(37, 10).softmax_layer()
+
+    def one_layer():
+        return network.Sequential().fully_connected_layer(33, 7)
+
+    return {"lenet": network.lenet5, "odd": odd, "mlp": lambda: network.mlp(hidden=65), "one_layer": one_layer}
+
+
+@pytest.mark.parametrize("batch", [1, 5, 19, 40, 150])  # samples of 8, 8, 4, 2 and 1 CTAs
+@pytest.mark.parametrize("name", list(_nets()))
+def test_whole_network_kernels_equal_the_layers(monkeypatch, name, batch):
+    results = []
+    for no_fuse in ("1", "0"):
+        monkeypatch.setenv("B200_NET_NO_FUSE", no_fuse)
+        net = _nets()[name]()
+        net.build(batch)
+        g = torch.Generator(device="cuda").manual_seed(11)
+        params = (torch.rand(net.n_params, device="cuda", generator=g) - 0.5) * 0.4
+        net.set_params(params.cpu().numpy())
+        x = torch.rand(batch, net.in_dim, device="cuda", generator=g)
+        t = torch.zeros(batch, net.out_dim, device="cuda")
+        t[:, 1] = 1.0
+        torch.cuda.synchronize()
+        net.forward(x)
+        net.ctx.sync()
+        out = host(net.output_tensor(batch)).copy()
+        net.train_onebatch(network.momentum(0.1, 0.9), x, t, L.LOSS_MSE)
+        net.ctx.sync()
+        results.append((out, net.get_grads(), net.get_params()))
+        net.close()
+    for a, b, what, tol in zip(results[0], results[1], ("output", "gradients", "weights"), (FWD_TOL, GRAD_TOL, GRAD_TOL)):
+        assert_close(np.asarray(b), np.asarray(a), tol, f"{name} {batch}: {what}")

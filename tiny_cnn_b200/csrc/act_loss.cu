@@ -25,18 +25,6 @@ __global__ void act_fwd_kernel(int kind, float param, const float *__restrict__ 
   for (size_t j = n4 * 4 + i; j < n; j += step) y[j] = apply_act_p(x[j], kind, param);
 }
 
-// relu_layer.h:31-39 dx = dy*(y>0); tanh_layer.h:30-38 dx = dy*(1-y*y)
-// sigmoid_layer.h:32-39 dx = dy*y*(1-y); leaky_relu_layer.h:80-88 dx = dy*(y>0 ? 1 : epsilon);
-// elu_layer.h:44-54 dx = dy*(y>0 ? 1 : alpha+y)
-__device__ __forceinline__ float act_grad(int kind, float param, float y, float dy) {
-  if (kind == B200_ACT_RELU) return dy * (y > 0.f ? 1.f : 0.f);
-  if (kind == B200_ACT_TANH) return __fmul_rn(dy, __fsub_rn(1.f, __fmul_rn(y, y)));
-  if (kind == B200_ACT_SIGMOID) return __fmul_rn(__fmul_rn(dy, y), __fsub_rn(1.f, y));
-  if (kind == B200_ACT_LEAKY_RELU) return __fmul_rn(dy, y > 0.f ? 1.f : param);
-  if (kind == B200_ACT_ELU) return __fmul_rn(dy, y > 0.f ? 1.f : __fadd_rn(param, y));
-  return dy;
-}
-
 __global__ void act_bwd_kernel(int kind, float param, const float *__restrict__ y, const float *__restrict__ dy,
                                float *__restrict__ dx, size_t n4, size_t n) {
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -112,13 +100,6 @@ __global__ void __launch_bounds__(256) softmax_fwd16_kernel(const float *__restr
   float denom = 0.f;
   for (int k = 0; k < dim; ++k) denom += __shfl_sync(0xffffffffu, ej, base + k);
   if (live) y[(size_t)n * dim + j] = ej / denom;
-}
-
-__device__ __forceinline__ float loss_grad_one(int kind, float yi, float ti, float factor) {
-  if (kind == B200_LOSS_MSE) return __fmul_rn(factor, __fsub_rn(yi, ti));
-  if (kind == B200_LOSS_CROSS_ENTROPY)
-    return __fdiv_rn(__fsub_rn(yi, ti), __fmul_rn(yi, __fsub_rn(1.f, yi)));
-  return __fdiv_rn(-ti, yi);
 }
 
 // softmax_layer.h:36-55: dx_j = sum_k dy_k * (k == j ? y_j(1-y_j) : -y_k*y_j)

@@ -253,6 +253,52 @@ int avgpool_fwd(b200_ctx *ctx, const b200_pool_desc &d, const float *in, const f
 int avgpool_bwd(b200_ctx *ctx, const b200_pool_desc &d, const float *in, const float *W,
                 const float *dout, float *din, float *dW, float *db, int accumulate, int B);
 
+// networks that fit one SM (net_small.cu): a step is a layer with the elementwise activation behind it
+enum SmallKind { SN_CONV, SN_FC, SN_AVG, SN_MAX, SN_SOFTMAX, SN_ACT };
+// quotients by a number known on the host; dividend and divisor below 65536
+struct SmallDiv {
+  uint32_t m;
+  void set(int d) { m = d == 1 ? 0 : (uint32_t)(((1ull << 32) + d - 1) / d); }
+#ifdef __CUDACC__
+  __device__ __forceinline__ int of(int a) const { return m ? (int)__umulhi((uint32_t)a, m) : a; }
+#endif
+};
+struct SmallStep {
+  int kind, act, in_n, out_n;
+  float param;
+  int in_off, out_off, arg_off;           // shared memory: input, output, window winners
+  int w_off, b_off, wf_off, wb_off;       // weights, biases, shares of large weights by outputs and by inputs (-1: none)
+  int copy_off, copy_n;                   // parameters copied whole
+  const float *copy;
+  int C, HI, WI, OC, OH, OW, KH, KW, SH, SW, DH, DW, pad_t, pad_l;
+  int has_bias, w_rows;                   // w_rows: fully-connected weights stored [out][in]
+  int slices, span, part_len, w_len, b_len;
+  SmallDiv d_op, d_ow, d_oh, d_onx, d_ip, d_iw, d_ih, d_inx, d_c, d_pairs;  // planes, rows, tiles of four, channels
+  const uint8_t *tbl;
+  const float *W, *b;
+  float *out, *out_pre;                   // value after / before the activation (out_pre: only where a layer owns it)
+  float *grad, *grad_pre;                 // dE/d of the two
+  const float *delta;                     // dE/d of the value before the activation
+  float *part, *dW, *db;
+  int32_t *argmax;
+};
+constexpr int SN_MAX_STEPS = 16;
+struct SmallNet {
+  int n, in_dim, n_act, n_wts;
+  int clusters[4];   // clusters of 1, 2, 4, 8 CTAs that run at once
+  long long fc_floats;
+  int *err;
+  SmallStep step[SN_MAX_STEPS];
+};
+// true when the whole-network kernels run a batch of B faster than the layers one by one
+bool small_net_fits(const b200_ctx *ctx, const SmallNet &n, int B);
+// fills in `clusters`
+int small_net_plan(b200_ctx *ctx, SmallNet *n);
+// forward, and with `backward` the gradients of loss (out, t) too
+int small_net_run(b200_ctx *ctx, const SmallNet &n, const float *x, const float *t, float *in_grad, int B, int backward,
+                  int loss);
+
+
 // `param`: epsilon of leaky relu / alpha of elu (ignored by the other kinds)
 int act_fwd(b200_ctx *ctx, int kind, const float *x, float *y, int dim, int B, float param = 0.f);
 int act_bwd(b200_ctx *ctx, int kind, const float *y, const float *dy, float *dx, int dim, int B,

@@ -29,6 +29,26 @@ __device__ __forceinline__ float apply_act_p(float v, int act, float param) {
   return v;
 }
 
+// relu_layer.h:31-39 dx = dy*(y>0); tanh_layer.h:30-38 dx = dy*(1-y*y)
+// sigmoid_layer.h:32-39 dx = dy*y*(1-y); leaky_relu_layer.h:80-88 dx = dy*(y>0 ? 1 : epsilon);
+// elu_layer.h:44-54 dx = dy*(y>0 ? 1 : alpha+y)
+__device__ __forceinline__ float act_grad(int kind, float param, float y, float dy) {
+  if (kind == B200_ACT_RELU) return dy * (y > 0.f ? 1.f : 0.f);
+  if (kind == B200_ACT_TANH) return __fmul_rn(dy, __fsub_rn(1.f, __fmul_rn(y, y)));
+  if (kind == B200_ACT_SIGMOID) return __fmul_rn(__fmul_rn(dy, y), __fsub_rn(1.f, y));
+  if (kind == B200_ACT_LEAKY_RELU) return __fmul_rn(dy, y > 0.f ? 1.f : param);
+  if (kind == B200_ACT_ELU) return __fmul_rn(dy, y > 0.f ? 1.f : __fadd_rn(param, y));
+  return dy;
+}
+
+// loss_function.h:28-36 (mse; factor = 2 / outputs), :120-128 (cross_entropy), :143-150 (multiclass)
+__device__ __forceinline__ float loss_grad_one(int kind, float yi, float ti, float factor) {
+  if (kind == B200_LOSS_MSE) return __fmul_rn(factor, __fsub_rn(yi, ti));
+  if (kind == B200_LOSS_CROSS_ENTROPY)
+    return __fdiv_rn(__fsub_rn(yi, ti), __fmul_rn(yi, __fsub_rn(1.f, yi)));
+  return __fdiv_rn(-ti, yi);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -106,6 +126,10 @@ __device__ __forceinline__ void mbar_fence_init() {
 }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(smem_u32(bar))
                : "memory");
 }
 __device__ __forceinline__ void bulk_copy_g2s(void *smem_dst, const void *gsrc, uint32_t bytes,

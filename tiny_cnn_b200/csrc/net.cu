@@ -30,12 +30,10 @@ struct Layer {
   float *grad = nullptr;  // dE/d out
   int32_t *argmax = nullptr;
   bool tiled = false;
-  float *wt_fwd = nullptr, *wt_dx = nullptr, *dw_part = nullptr;
-  // tensor-core passes: filter blocks of the forward and dX passes, partial weight gradients
+  float *wt_fwd = nullptr, *wt_dx = nullptr;
+  // tensor-core passes: filter blocks of the forward and dX passes
   ConvTcUse tc = {};
-  float *tc_wt_fwd = nullptr, *tc_wt_dx = nullptr, *tc_part = nullptr;
-  float *fc_scratch = nullptr;  // k-slice partial sums of the small GEMMs
-  float *fc_scratch_side = nullptr;  // the same for the dW GEMM when it runs on the side stream
+  float *tc_wt_fwd = nullptr, *tc_wt_dx = nullptr;
   float act_param = 0.f;  // leaky relu: epsilon; elu: alpha
   // batch normalization: shape, constants, this batch's moments, stddev, moving averages, slice sums
   int bn_c = 0, bn_s = 0;
@@ -59,6 +57,13 @@ struct b200_net {
   // a narrow fully-connected layer + softmax output layer run as one kernel per direction:
   // index of that fully-connected layer (-1: none) and of a relu directly before it (-1: none)
   int head_fc = -1, head_relu = -1;
+  std::vector<void *> mem;  // device memory (net_alloc, net_commit)
+  std::vector<std::pair<void **, size_t>> wanted;
+  // partial sums and split operands of the layer at work on the main / on the side stream
+  float *scratch = nullptr, *scratch_side = nullptr;
+  SmallNet small = {};          // steps of the whole-network kernels (none: the network is not one for them)
+  float *small_part = nullptr;
+  size_t small_part_floats = 0;
   bool train_phase = true;  // net_phase::train (b200_net_set_phase)
   std::vector<OptSegment> segs;  // trainable tensors in update order
   size_t n_params = 0;
@@ -128,9 +133,23 @@ struct b200_net {
 
 namespace {
 
-int net_alloc(void **p, size_t bytes) {
-  B200_CUDA(cudaMalloc(p, bytes ? bytes : 4));
-  B200_CUDA(cudaMemset(*p, 0, bytes ? bytes : 4));
+// Device memory of a network: net_alloc notes who needs how much, net_commit gets it in one block, cleared.  (One
+// allocation and one release in place of sixty.)
+void net_alloc(b200_net *net, void **p, size_t bytes) { net->wanted.push_back({p, align_up(bytes ? bytes : 4, 256)}); }
+
+int net_commit(b200_net *net) {
+  size_t total = 0;
+  for (auto &w : net->wanted) total += w.second;
+  void *block = nullptr;
+  B200_CUDA(cudaMalloc(&block, total));
+  net->mem.push_back(block);
+  B200_CUDA(cudaMemset(block, 0, total));
+  char *next = static_cast<char *>(block);
+  for (auto &w : net->wanted) {
+    *w.first = next;
+    next += w.second;
+  }
+  net->wanted.clear();
   return 0;
 }
 
@@ -145,8 +164,132 @@ int act_of_layer(int kind) {
   return B200_ACT_NONE;
 }
 
+// whether a pass over B samples goes to the whole-network kernels
+bool net_is_small(const b200_net *net, int B) { return small_net_fits(net->ctx, net->small, B); }
+
+// forward and, with t, backward pass in the whole-network kernels
+int net_small_run(b200_net *net, const float *x, const float *t, int B, int loss_kind) {
+  B200_TRY(small_net_run(net->ctx, net->small, x, t, net->input_grad ? net->in_grad : nullptr, B, t != nullptr, loss_kind));
+  net->cur_batch = B;
+  net->cur_x = x;
+  return 0;
+}
+
+// Steps of the whole-network kernels, if every layer is one that they have and the values of a sample fit an SM
+int net_small_plan(b200_net *net) {
+  b200_ctx *ctx = net->ctx;
+  net->small = {};
+  const int n = (int)net->layers.size();
+  if (!net->fuse || ctx->conv_tensor_cores > 1 || ctx->fc_tensor_cores > 1) return 0;
+  SmallNet &S = net->small;
+  S.in_dim = (int)net->layers[0].in_dim;
+  int off = S.in_dim;
+  long long part = 0, part_at[SN_MAX_STEPS];
+  for (int i = 0; i < n; ++i) {
+    Layer &L = net->layers[i];
+    if (S.n == SN_MAX_STEPS || L.in_dim > 50000 || L.out_dim > 50000) return S.n = 0, 0;
+    SmallStep &P = S.step[S.n];
+    P = {};
+    P.in_n = (int)L.in_dim;
+    P.out_n = (int)L.out_dim;
+    P.in_off = S.n ? S.step[S.n - 1].out_off : 0;
+    P.out_off = off;
+    off += P.out_n;
+    P.W = net->params + L.w_off;
+    P.b = net->params + L.b_off;
+    P.dW = net->grads + L.w_off;
+    P.db = net->grads + L.b_off;
+    P.w_len = (int)L.w_len;
+    P.b_len = (int)L.b_len;
+    P.has_bias = L.b_len > 0;
+    P.slices = 1;
+    int last = i;
+    if (L.kind == B200_LAYER_CONV) {
+      if (L.cd.algo != 0) return S.n = 0, 0;
+      P.kind = L.tc.fc ? SN_FC : SN_CONV;
+      P.w_rows = L.tc.fc;
+      P.C = L.g.C, P.HI = L.g.HI, P.WI = L.g.WI, P.OC = L.g.OC, P.OH = L.g.OH, P.OW = L.g.OW;
+      P.KH = L.g.KH, P.KW = L.g.KW, P.SH = L.g.SH, P.SW = L.g.SW, P.DH = L.g.DH, P.DW = L.g.DW;
+      P.pad_t = L.g.pad_t, P.pad_l = L.g.pad_l;
+      P.tbl = L.g.tbl;
+    } else if (L.kind == B200_LAYER_FC) {
+      P.kind = SN_FC;
+    } else if (L.kind == B200_LAYER_AVGPOOL || L.kind == B200_LAYER_MAXPOOL) {
+      P.kind = L.kind == B200_LAYER_AVGPOOL ? SN_AVG : SN_MAX;
+      P.C = P.OC = L.pd.in_c, P.HI = L.pd.in_h, P.WI = L.pd.in_w, P.OH = L.pd.out_h, P.OW = L.pd.out_w;
+      P.KH = L.pd.pool_h, P.KW = L.pd.pool_w, P.SH = L.pd.stride_h, P.SW = L.pd.stride_w;
+      P.argmax = L.argmax;
+      if (P.kind == SN_MAX) {
+        P.arg_off = off;
+        off += P.out_n;
+      }
+    } else if (L.kind == B200_LAYER_SOFTMAX) {
+      if (L.out_dim > 64) return S.n = 0, 0;
+      P.kind = SN_SOFTMAX;
+    } else if (L.kind == B200_LAYER_BATCHNORM) {
+      return S.n = 0, 0;
+    } else {
+      P.kind = SN_ACT;
+      P.act = act_of_layer(L.kind);
+      P.param = L.act_param;
+    }
+    // the activation behind it joins the step
+    if (P.kind != SN_SOFTMAX && P.kind != SN_ACT && i + 1 < n) {
+      const int k = net->layers[i + 1].kind;
+      if (k != B200_LAYER_SOFTMAX && act_of_layer(k) != B200_ACT_NONE) {
+        last = i + 1;
+        P.act = act_of_layer(k);
+        P.param = net->layers[last].act_param;
+        if (!L.fused_act) P.out_pre = L.out;
+        P.grad_pre = L.grad;
+      }
+    }
+    P.out = net->layers[last].out;
+    P.grad = net->layers[last].grad;
+    P.delta = P.grad_pre ? P.grad_pre : P.grad;
+    if (P.kind == SN_CONV) {
+      // pairs of channels, a warp each: enough slices of the output plane for the 128 warps of a cluster
+      P.slices = min(16, max(1, 128 / (P.OC * P.C)));
+      P.part_len = P.w_len + P.OC;
+    } else if (P.kind == SN_AVG) {
+      P.slices = min(8, max(1, 128 / P.C));
+      P.part_len = 2 * P.C;
+    } else if (P.kind == SN_FC) {
+      S.fc_floats += P.w_len;
+    }
+    if (P.C) {
+      P.span = ceil_div(P.OH * P.OW, P.slices);
+      P.d_op.set(P.OH * P.OW);
+      P.d_ow.set(P.OW);
+      P.d_oh.set(P.OH);
+      P.d_onx.set(ceil_div(P.OW, 4));
+      P.d_ip.set(P.HI * P.WI);
+      P.d_iw.set(P.WI);
+      P.d_ih.set(P.HI);
+      P.d_inx.set(ceil_div(P.WI, 4));
+      P.d_c.set(P.C);
+      P.d_pairs.set(P.C * P.OC);
+      if (P.C * P.OC * P.slices > 65535) return S.n = 0, 0;
+    }
+    if (P.part_len) {
+      part_at[S.n] = part;
+      part += (long long)net->max_batch * P.slices * P.part_len;
+    }
+    ++S.n;
+    i = last;
+  }
+  S.n_act = off;
+  S.err = ctx->dev_err;
+  if (!small_net_fits(ctx, S, 1)) return S.n = 0, 0;
+  net->small_part_floats = (size_t)part;
+  for (int i = 0; i < S.n; ++i)
+    if (S.step[i].part_len) S.step[i].part = net->small_part + part_at[i];
+  return 0;
+}
+
 int net_forward_impl(b200_net *net, const float *x, int B) {
   b200_ctx *ctx = net->ctx;
+  if (net_is_small(net, B)) return net_small_run(net, x, nullptr, B, 0);
   const float *in = x;
   size_t n = net->layers.size();
   // The filter matrices of the tensor-core layers depend on the weights only: they are made on the
@@ -205,7 +348,7 @@ int net_forward_impl(b200_net *net, const float *x, int B) {
         if (L.tc.fwd) {
           B200_TRY(conv_gather_fwd(ctx, L.g, in, L.tc_wt_fwd, b, dst, B, L.fused_act));
         } else if (L.tc.fc)
-          B200_TRY(fc_fwd(ctx, (int)L.in_dim, L.g.OC, in, W, b, dst, B, L.fused_act, L.fc_scratch, true));
+          B200_TRY(fc_fwd(ctx, (int)L.in_dim, L.g.OC, in, W, b, dst, B, L.fused_act, net->scratch, true));
         else if (L.tc.fwd_small)
           B200_TRY(conv_fwd_small(ctx, L.g, in, W, b, dst, B, L.fused_act));
         else if (L.tiled)
@@ -218,7 +361,7 @@ int net_forward_impl(b200_net *net, const float *x, int B) {
         if ((int)i == net->head_fc)
           B200_TRY(fc_softmax_fwd(ctx, L.fc_in, L.fc_out, in, W, b, dst, net->layers[n - 1].out, B));
         else
-          B200_TRY(fc_fwd(ctx, L.fc_in, L.fc_out, in, W, b, dst, B, L.fused_act, L.fc_scratch));
+          B200_TRY(fc_fwd(ctx, L.fc_in, L.fc_out, in, W, b, dst, B, L.fused_act, net->scratch));
         break;
       case B200_LAYER_MAXPOOL:
         B200_TRY(maxpool_fwd(ctx, L.pd, in, dst, L.argmax, B));
@@ -257,6 +400,8 @@ int net_forward_impl(b200_net *net, const float *x, int B) {
 int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in_step = false) {
   b200_ctx *ctx = net->ctx;
   int B = net->cur_batch;
+  // called after a forward pass of its own: the values it kept in shared memory are computed again
+  if (net_is_small(net, B)) return net_small_run(net, net->cur_x, t, B, loss_kind);
   int n = (int)net->layers.size();
   Layer &last = net->layers[n - 1];
   // a softmax output layer: loss gradient and softmax gradient in one launch
@@ -295,13 +440,13 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
   auto fc_backward = [&](Layer &L, bool w_rows, const float *in, float *din, const float *W, float *dW, float *db,
                          bool can_fork) -> int {
     const int n_in = (int)L.in_dim, n_out = (int)L.out_dim;
-    if (!can_fork || !L.fc_scratch_side)
-      return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, dW, db, 0, B, L.fc_scratch, w_rows);
+    if (!can_fork)
+      return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, dW, db, 0, B, net->scratch, w_rows);
     B200_TRY(fork());
-    rc_side = fc_bwd(ctx, n_in, n_out, in, W, L.grad, nullptr, dW, db, 0, B, L.fc_scratch_side, w_rows);
+    rc_side = fc_bwd(ctx, n_in, n_out, in, W, L.grad, nullptr, dW, db, 0, B, net->scratch_side, w_rows);
     ctx->stream = main_stream;
     if (rc_side) return 0;
-    return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, nullptr, nullptr, 0, B, L.fc_scratch, w_rows);
+    return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, nullptr, nullptr, 0, B, net->scratch, w_rows);
   };
   for (int i = tail_fused ? n - 2 : n - 1; i >= 0 && rc_side == 0; --i) {
     Layer &L = net->layers[i];
@@ -324,22 +469,24 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
         const bool tc_dx = L.tc.dx && din != nullptr;
         // dW first: its launch precedes the dX launch, so a one-block-per-SM dW kernel is resident
         // when the small blocks of an FFMA dX arrive and both share the SMs
-        if (can_fork && (L.tc.dw || L.tc.dw_small)) B200_TRY(fork());
+        const bool forked = can_fork && (L.tc.dw || L.tc.dw_small);
+        if (forked) B200_TRY(fork());
+        float *part = forked ? net->scratch_side : net->scratch;
         if (L.tc.dw) {
-          rc_side = conv_gather_dw(ctx, L.g, in, L.grad, B, L.tc_part, dW, db, 0);
+          rc_side = conv_gather_dw(ctx, L.g, in, L.grad, B, part, dW, db, 0);
         } else if (L.tc.dw_small) {
-          rc_side = conv_dw_small(ctx, L.g, in, L.grad, B, L.tc_part, dW, db, 0);
+          rc_side = conv_dw_small(ctx, L.g, in, L.grad, B, part, dW, db, 0);
         } else if (tiled_bwd) {
           int splits = 0;
-          rc_side = conv_tiled_dw_partials(ctx, L.g, in, L.grad, B, L.dw_part, &splits);
+          rc_side = conv_tiled_dw_partials(ctx, L.g, in, L.grad, B, part, &splits);
           size_t row = L.w_len + L.g.OC;
           if (!rc_side && db && L.b_off == L.w_off + L.w_len) {
             // [W | b] are neighbours in the bucket as in a partial row: one merge
-            rc_side = merge_rows(ctx, L.dw_part, splits, row, dW, row, 0, &L.g);
+            rc_side = merge_rows(ctx, part, splits, row, dW, row, 0, &L.g);
           } else if (!rc_side) {
-            rc_side = merge_rows(ctx, L.dw_part, splits, row, dW, L.w_len, 0, &L.g);
+            rc_side = merge_rows(ctx, part, splits, row, dW, L.w_len, 0, &L.g);
             if (!rc_side && db)
-              rc_side = merge_rows(ctx, L.dw_part + L.w_len, splits, row, db, L.b_len, 0, nullptr);
+              rc_side = merge_rows(ctx, part + L.w_len, splits, row, db, L.b_len, 0, nullptr);
           }
         } else {
           rc_side = conv_general_dw(ctx, L.g, in, L.grad, dW, db, 0, B);
@@ -476,10 +623,10 @@ int check_net(b200_net *net) {
 
 int step_eager(b200_net *net, const float *x, const float *t, int B, int loss_kind, int opt_kind,
                const b200_opt_hyper *h) {
-  B200_TRY(net_forward_impl(net, x, B));
-  const bool peer = net->peer.world > 1;
-  const bool early = peer && net->comm && net->peer_early_layer >= 0 && net->peer.split < net->peer.n;
-  B200_TRY(net_backward_impl(net, t, loss_kind, early));
+  const bool peer = net->peer.world > 1, small = net_is_small(net, B);
+  if (!small) B200_TRY(net_forward_impl(net, x, B));
+  const bool early = peer && !small && net->comm && net->peer_early_layer >= 0 && net->peer.split < net->peer.n;
+  B200_TRY(small ? net_small_run(net, x, t, B, loss_kind) : net_backward_impl(net, t, loss_kind, early));
   if (peer) {
     if (!early) B200_TRY(peer_reduce_push_early(net->ctx, &net->peer, net->grads));
     B200_TRY(peer_reduce_finish(net->ctx, &net->peer, net->grads, 0, early && net->early_summed));
@@ -638,52 +785,59 @@ int b200_net_create(b200_ctx *ctx, const b200_layer_spec *specs, int n_layers, i
   }
   // device memory
   size_t f = sizeof(float);
-  B200_TRY(net_alloc((void **)&net->params, off * f));
-  B200_TRY(net_alloc((void **)&net->grads, off * f));
-  B200_TRY(net_alloc((void **)&net->state0, off * f));
-  B200_TRY(net_alloc((void **)&net->state1, off * f));
-  B200_TRY(net_alloc((void **)&net->segs_dev, sizeof(OptSegment) * (net->segs.size() + 1)));
-  B200_CUDA(cudaMemcpy(net->segs_dev, net->segs.data(), sizeof(OptSegment) * net->segs.size(),
-                       cudaMemcpyHostToDevice));
-  B200_TRY(net_alloc((void **)&net->pow_tab, f * 2 * (net->segs.size() + 1)));
+  net_alloc(net, (void **)&net->params, off * f);
+  net_alloc(net, (void **)&net->grads, off * f);
+  net_alloc(net, (void **)&net->state0, off * f);
+  net_alloc(net, (void **)&net->state1, off * f);
+  net_alloc(net, (void **)&net->segs_dev, sizeof(OptSegment) * (net->segs.size() + 1));
+  net_alloc(net, (void **)&net->pow_tab, f * 2 * (net->segs.size() + 1));
   size_t in0 = net->layers[0].in_dim;
-  B200_TRY(net_alloc((void **)&net->in_grad, in0 * max_batch * f));
-  B200_TRY(net_alloc((void **)&net->x_dev, in0 * max_batch * f));
-  B200_TRY(net_alloc((void **)&net->t_dev, net->layers[n_layers - 1].out_dim * max_batch * f));
+  net_alloc(net, (void **)&net->in_grad, in0 * max_batch * f);
+  net_alloc(net, (void **)&net->x_dev, in0 * max_batch * f);
+  net_alloc(net, (void **)&net->t_dev, net->layers[n_layers - 1].out_dim * max_batch * f);
+  B200_TRY(net_small_plan(net));
+  const bool all_small = net_is_small(net, max_batch);  // never a layer-by-layer pass
+  if (net->small.n) net_alloc(net, (void **)&net->small_part, net->small_part_floats * f);
+  size_t scratch = 0;
   for (int i = 0; i < n_layers; ++i) {
     Layer &L = net->layers[i];
-    B200_TRY(net_alloc((void **)&L.out, L.out_dim * max_batch * f));
+    net_alloc(net, (void **)&L.out, L.out_dim * max_batch * f);
     if (L.kind == B200_LAYER_BATCHNORM) {
       float **bufs[5] = {&L.bn_mean_cur, &L.bn_var_cur, &L.bn_stddev, &L.bn_mean, &L.bn_var};
-      for (float **b : bufs) {  // the reference's init(): all zeros
-        B200_TRY(net_alloc((void **)b, (size_t)L.bn_c * f));
-        B200_CUDA(cudaMemset(*b, 0, (size_t)L.bn_c * f));
-      }
-      B200_TRY(net_alloc((void **)&L.bn_scratch, batchnorm_scratch_floats(ctx, L.bn_c, max_batch) * f));
+      for (float **b : bufs) net_alloc(net, (void **)b, (size_t)L.bn_c * f);  // the reference's init(): all zeros
+      net_alloc(net, (void **)&L.bn_scratch, batchnorm_scratch_floats(ctx, L.bn_c, max_batch) * f);
     }
-    B200_TRY(net_alloc((void **)&L.grad, L.out_dim * max_batch * f));
+    net_alloc(net, (void **)&L.grad, L.out_dim * max_batch * f);
     if (L.kind == B200_LAYER_MAXPOOL)
-      B200_TRY(net_alloc((void **)&L.argmax, L.out_dim * max_batch * sizeof(int32_t)));
+      net_alloc(net, (void **)&L.argmax, L.out_dim * max_batch * sizeof(int32_t));
+    if (all_small) continue;
+    size_t need = 0;
     if (L.kind == B200_LAYER_FC || (L.kind == B200_LAYER_CONV && L.tc.fc)) {
-      const size_t need = fc_scratch_floats(ctx, (int)L.in_dim, (int)L.out_dim, max_batch);
-      B200_TRY(net_alloc((void **)&L.fc_scratch, need * f));
-      if (net->side) B200_TRY(net_alloc((void **)&L.fc_scratch_side, need * f));
-    }
-    if (L.kind == B200_LAYER_CONV && L.tiled && !L.tc.fc) {
-      B200_TRY(net_alloc((void **)&L.wt_fwd, conv_tiled_fwd_scratch(L.g) * f));
-      B200_TRY(net_alloc((void **)&L.wt_dx, conv_tiled_dx_scratch(L.g) * f));
-      size_t need = conv_tiled_dw_scratch(ctx, L.g, max_batch);
-      B200_TRY(net_alloc((void **)&L.dw_part, need * f));
-    }
-    if (L.kind == B200_LAYER_CONV) {
+      need = fc_scratch_floats(ctx, (int)L.in_dim, (int)L.out_dim, max_batch);
+    } else if (L.kind == B200_LAYER_CONV) {
       if ((L.tc.fwd || L.tc.dx || L.tiled) && net->side)
         B200_CUDA(cudaEventCreateWithFlags(&L.ev_prep, cudaEventDisableTiming));
-      if (L.tc.fwd) B200_TRY(net_alloc((void **)&L.tc_wt_fwd, conv_gather_filter_floats(ctx, L.g, 0) * f));
-      if (L.tc.dx) B200_TRY(net_alloc((void **)&L.tc_wt_dx, conv_gather_filter_floats(ctx, L.g, 1) * f));
-      if (L.tc.dw) B200_TRY(net_alloc((void **)&L.tc_part, conv_gather_dw_floats(ctx, L.g, max_batch) * f));
-      if (L.tc.dw_small) B200_TRY(net_alloc((void **)&L.tc_part, conv_dw_small_floats(ctx, L.g, max_batch) * f));
+      if (L.tc.fwd)
+        net_alloc(net, (void **)&L.tc_wt_fwd, conv_gather_filter_floats(ctx, L.g, 0) * f);
+      else if (L.tiled && !L.tc.fwd_small)
+        net_alloc(net, (void **)&L.wt_fwd, conv_tiled_fwd_scratch(L.g) * f);
+      if (L.tc.dx)
+        net_alloc(net, (void **)&L.tc_wt_dx, conv_gather_filter_floats(ctx, L.g, 1) * f);
+      else if (L.tiled)
+        net_alloc(net, (void **)&L.wt_dx, conv_tiled_dx_scratch(L.g) * f);
+      need = L.tc.dw         ? conv_gather_dw_floats(ctx, L.g, max_batch)
+             : L.tc.dw_small ? conv_dw_small_floats(ctx, L.g, max_batch)
+             : L.tiled       ? conv_tiled_dw_scratch(ctx, L.g, max_batch)
+                             : 0;
     }
+    if (need > scratch) scratch = need;
   }
+  net_alloc(net, (void **)&net->scratch, scratch * f);
+  if (net->side) net_alloc(net, (void **)&net->scratch_side, scratch * f);
+  B200_TRY(net_commit(net));
+  B200_TRY(net_small_plan(net));  // now with the addresses
+  if (net->small.n) B200_TRY(small_net_plan(ctx, &net->small));
+  B200_CUDA(cudaMemcpy(net->segs_dev, net->segs.data(), sizeof(OptSegment) * net->segs.size(), cudaMemcpyHostToDevice));
   *out = net;
   return 0;
 }
@@ -694,40 +848,13 @@ int b200_net_destroy(b200_net *net) {
   cudaStreamSynchronize(net->ctx->stream);
   for (auto &slot : net->slots) slot.clear();
   for (auto &L : net->layers) {
-    cudaFree(L.out);
-    cudaFree(L.grad);
-    cudaFree(L.argmax);
-    cudaFree(L.bn_mean_cur);
-    cudaFree(L.bn_var_cur);
-    cudaFree(L.bn_stddev);
-    cudaFree(L.bn_mean);
-    cudaFree(L.bn_var);
-    cudaFree(L.bn_scratch);
-    cudaFree(L.wt_fwd);
-    cudaFree(L.wt_dx);
     if (L.ev_prep) cudaEventDestroy(L.ev_prep);
-    cudaFree(L.dw_part);
-    cudaFree(L.fc_scratch_side);
-    cudaFree(L.tc_wt_fwd);
-    cudaFree(L.tc_wt_dx);
-    cudaFree(L.tc_part);
-    cudaFree(L.fc_scratch);
   }
-  cudaFree(net->params);
-  cudaFree(net->grads);
-  cudaFree(net->state0);
-  cudaFree(net->state1);
-  cudaFree(net->segs_dev);
-  cudaFree(net->pow_tab);
-  cudaFree(net->in_grad);
   for (int i = 0; i < 2; ++i) {
-    cudaFree(net->x_stage[i]);
-    cudaFree(net->t_stage[i]);
     cudaFree(net->u8_stage[i]);
     cudaFree(net->label_stage[i]);
     if (net->up_done[i]) cudaEventDestroy(net->up_done[i]);
     if (net->stage_free[i]) cudaEventDestroy(net->stage_free[i]);
-    cudaFree(net->out_stage[i]);
     if (net->step_done[i]) cudaEventDestroy(net->step_done[i]);
     if (net->d2h_done[i]) cudaEventDestroy(net->d2h_done[i]);
   }
@@ -741,8 +868,7 @@ int b200_net_destroy(b200_net *net) {
   if (net->side) cudaStreamDestroy(net->side);
   if (net->ev_fork) cudaEventDestroy(net->ev_fork);
   if (net->ev_join) cudaEventDestroy(net->ev_join);
-  cudaFree(net->x_dev);
-  cudaFree(net->t_dev);
+  for (void *q : net->mem) cudaFree(q);
   delete net;
   return 0;
 }
@@ -1097,6 +1223,7 @@ int b200_net_forward_backward(b200_net *net, const float *x, const float *t, int
   B200_REQUIRE(batch >= 1 && batch <= net->max_batch,
                "net_forward_backward: batch %d outside 1..%d", batch, net->max_batch);
   int r = run_captured(net, 1, step_key(net, x, t, batch, loss_kind, -1, nullptr), [&]() {
+    if (net_is_small(net, batch)) return net_small_run(net, x, t, batch, loss_kind);
     B200_TRY(net_forward_impl(net, x, batch));
     return net_backward_impl(net, t, loss_kind);
   });
@@ -1159,19 +1286,21 @@ int b200_net_fit_host_enqueue(b200_net *net, const float *x_host, const float *t
   if (!net->copy_stream) {
     B200_CUDA(cudaStreamCreateWithFlags(&net->copy_stream, cudaStreamNonBlocking));
     for (int i = 0; i < 2; ++i) {
-      B200_TRY(net_alloc((void **)&net->x_stage[i], in_dim * net->max_batch * sizeof(float)));
-      B200_TRY(net_alloc((void **)&net->t_stage[i], out_dim * net->max_batch * sizeof(float)));
+      net_alloc(net, (void **)&net->x_stage[i], in_dim * net->max_batch * sizeof(float));
+      net_alloc(net, (void **)&net->t_stage[i], out_dim * net->max_batch * sizeof(float));
       B200_CUDA(cudaEventCreateWithFlags(&net->up_done[i], cudaEventDisableTiming));
       B200_CUDA(cudaEventCreateWithFlags(&net->stage_free[i], cudaEventDisableTiming));
     }
+    B200_TRY(net_commit(net));
   }
   if (!net->d2h_stream) {
     B200_CUDA(cudaStreamCreateWithFlags(&net->d2h_stream, cudaStreamNonBlocking));
     for (int i = 0; i < 2; ++i) {
-      B200_TRY(net_alloc((void **)&net->out_stage[i], out_dim * net->max_batch * sizeof(float)));
+      net_alloc(net, (void **)&net->out_stage[i], out_dim * net->max_batch * sizeof(float));
       B200_CUDA(cudaEventCreateWithFlags(&net->step_done[i], cudaEventDisableTiming));
       B200_CUDA(cudaEventCreateWithFlags(&net->d2h_done[i], cudaEventDisableTiming));
     }
+    B200_TRY(net_commit(net));
   }
   // A full mini-batch runs where its upload left it (the library keeps one captured step per input
   // address, so two staging buffers mean two graphs) and its output is fetched by a third stream
@@ -1244,11 +1373,12 @@ int b200_net_fit_u8_host(b200_net *net, const b200_image_desc *d, const uint8_t 
   if (!net->copy_stream) {
     B200_CUDA(cudaStreamCreateWithFlags(&net->copy_stream, cudaStreamNonBlocking));
     for (int i = 0; i < 2; ++i) {
-      B200_TRY(net_alloc((void **)&net->x_stage[i], in_dim * net->max_batch * sizeof(float)));
-      B200_TRY(net_alloc((void **)&net->t_stage[i], out_dim * net->max_batch * sizeof(float)));
+      net_alloc(net, (void **)&net->x_stage[i], in_dim * net->max_batch * sizeof(float));
+      net_alloc(net, (void **)&net->t_stage[i], out_dim * net->max_batch * sizeof(float));
       B200_CUDA(cudaEventCreateWithFlags(&net->up_done[i], cudaEventDisableTiming));
       B200_CUDA(cudaEventCreateWithFlags(&net->stage_free[i], cudaEventDisableTiming));
     }
+    B200_TRY(net_commit(net));
   }
   if (net->u8_stage_bytes < img_bytes * net->max_batch) {
     B200_CUDA(cudaStreamSynchronize(st));
@@ -1256,8 +1386,8 @@ int b200_net_fit_u8_host(b200_net *net, const b200_image_desc *d, const uint8_t 
       cudaFree(net->u8_stage[i]);
       cudaFree(net->label_stage[i]);
       net->u8_stage[i] = net->label_stage[i] = nullptr;
-      B200_TRY(net_alloc((void **)&net->u8_stage[i], img_bytes * net->max_batch));
-      B200_TRY(net_alloc((void **)&net->label_stage[i], (size_t)net->max_batch));
+      B200_CUDA(cudaMalloc((void **)&net->u8_stage[i], img_bytes * net->max_batch));
+      B200_CUDA(cudaMalloc((void **)&net->label_stage[i], (size_t)net->max_batch));
     }
     net->u8_stage_bytes = img_bytes * net->max_batch;
   }

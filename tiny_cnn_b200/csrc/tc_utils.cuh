@@ -159,11 +159,6 @@ __host__ __device__ constexpr uint32_t umma_idesc_tf32_major(int M, int N, int a
          ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
 // round to the nearest TF32 (10 explicit mantissa bits, ties away from zero); lo = x - hi is exact
 // in fp32.  Integer form of cvt.rna.tf32.f32 (same bits for every finite input): that instruction
 // issues on the conversion pipe, a quarter-rate unit that a kernel converting an im2col tile in
