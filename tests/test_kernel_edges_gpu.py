@@ -23,6 +23,8 @@ pytestmark = pytest.mark.gpu
     (64, 64, 4, 20, 3, 1, False, 2),    # largest map
     (8, 8, 256, 256, 3, 1, True, 20),   # most channels
     (9, 8, 24, 16, 3, 2, True, 300),    # many images in a pixel set
+    (24, 18, 16, 141, 3, 1, True, 51),  # an odd number of 32-k units a tile, several tiles a block
+    (8, 8, 40, 32, 5, 1, True, 100),    # one pixel set a tile, k's split between two issuers
     (5, 5, 16, 120, 5, 1, False, 16),   # window as large as the input
 ])
 def test_conv_tensor_core_edges(ctx, case):

@@ -169,7 +169,9 @@ int conv_gather_dx(b200_ctx *ctx, const ConvGeom &g, const float *dout, const fl
 bool conv_gather_dw_ok(const b200_ctx *ctx, const ConvGeom &g);
 size_t conv_gather_dw_floats(const b200_ctx *ctx, const ConvGeom &g, int B);
 int conv_gather_dw(b200_ctx *ctx, const ConvGeom &g, const float *in, const float *dout, int B, float *part, float *dW,
-                   float *db, int accumulate);
+                   float *db, int accumulate, bool finish = true);
+// the sums over `part` that a call with finish = false left out
+int conv_gather_dw_finish(b200_ctx *ctx, const ConvGeom &g, int B, const float *part, float *dW, float *db, int accumulate);
 
 // which passes of a layer run on the tensor cores: `algo` 3 = all that can, 1 / 2 = none, 0 = by the
 // context's conv_tensor_cores option

@@ -33,8 +33,9 @@
 // the gather's shared-memory reads.
 // Warp roles: 0-7 epilogue, 8-15 gather (two groups of one warp per TMEM lane quadrant, taking 32-k units
 // in turn), 16-23 loaders, 24 filter producer, 25-26 MMA issuers (each takes every other pixel set: one
-// warp's instruction latency is longer than the MMAs of a narrow unit).  Every wait is bounded; a timeout sets the
-// context's error word, frees tensor memory and returns.
+// warp's instructions take longer, about 900 cycles a unit, than the MMAs of a narrow unit; of a tile of one set
+// each takes every other unit: 8x8, 64 -> 32 channels, 5x5, 256 samples 29.0 us, with the split 21.6 us).
+// Every wait is bounded; a timeout sets the context's error word, frees tensor memory and returns.
 #include <stdio.h>
 #include <stdlib.h>
 
@@ -55,11 +56,7 @@ constexpr int CV_ABUFS = 4;        // 32-k units of A in tensor memory: two per 
 constexpr int CV_A_COLS = 48;      // columns of one: three parts, two k's per column
 constexpr int CV_D_COLS = 256;     // columns of the accumulators; the A units take the other 256
 constexpr int CV_MAX_D = 8;        // accumulators (large and small products) at N = 16
-#ifndef CV_NAP_EPI
-#define CV_NAP_EPI 60
-#define CV_NAP_GATHER 20
-#define CV_NAP_LOAD 150
-#endif
+constexpr int CV_NAP_EPI = 60, CV_NAP_GATHER = 20, CV_NAP_LOAD = 150;  // ns asleep between looks at a barrier
 constexpr int CV_MAX_PHASES = 16;
 constexpr int CV_MAX_F = 12;       // filter ring stages
 
@@ -85,6 +82,7 @@ struct ConvGatherArgs {
   int iys, ixs, oys, oxs, tdy, tdx;
   int CS, nslab, cstr; // channels per slab (a multiple of V), slabs, places per V channels in shared memory
   int S, NP, ngroups, ND, nf;
+  int ks;              // 2: tiles of one pixel set whose k's are split between the issuers, an accumulator each
   int nphases, ntiles, koff_len;
   int resident;        // the whole filter fits the ring: loaded once
   int act;
@@ -183,7 +181,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
     for (int i = 0; i < a.nf; ++i) {
       mbar_init(&filt_full[i], 1);
       mbar_init(&filt_peer[i], 1);
-      mbar_init(&filt_empty[i], min(a.S, CV_ISSUERS));
+      mbar_init(&filt_empty[i], min(a.S * a.ks, CV_ISSUERS));
     }
     mbar_fence_init();
   }
@@ -221,20 +219,22 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
       const int PHW = p.PH * p.PW, total = a.B * PHW;
       const int g0 = ((tile - p.tile0) * CG + (int)rank) * a.S * 128;
       const int n0 = grp * a.NP;
-      for (int s = 0; s < a.S; ++s, ++q) {
-        const uint32_t db = q % a.ND;
+      for (int s = 0; s < a.S; ++s, q += a.ks) {
+        const uint32_t db = q % a.ND, db2 = (q + 1) % a.ND;
         const int g = g0 + s * 128 + quad * 32 + lane;
         const int b = g / PHW, r = g - b * PHW, y = r / p.PW, x = r - y * p.PW;
         float *obase = a.out + ((size_t)b * a.N + n0) * plane_o + (size_t)(y * a.oys + p.oy0) * a.OWf +
                        (x * a.oxs + p.ox0);
         tq = tc_clock();
-        if (!mbar_wait_warp_sleep<CV_NAP_EPI>(&acc_full[db], (q / a.ND) & 1)) {
+        if (!mbar_wait_warp_sleep<CV_NAP_EPI>(&acc_full[db], (q / a.ND) & 1) ||
+            (a.ks == 2 && !mbar_wait_warp_sleep<CV_NAP_EPI>(&acc_full[db2], ((q + 1) / a.ND) & 1))) {
           failed = true;
           break;
         }
         w0 += tc_clock() - tq;
         tc_fence_after();
-        const uint32_t tacc = tmem_base + ((uint32_t)(quad * 32) << 16) + db * 2u * (uint32_t)a.NP;
+        const uint32_t tq0 = tmem_base + ((uint32_t)(quad * 32) << 16), tacc = tq0 + db * 2u * (uint32_t)a.NP,
+                       tacc2 = tq0 + db2 * 2u * (uint32_t)a.NP;
         const int cfirst = (warp >> 2) * 16;
         for (int c = cfirst; c < a.NP || c == cfirst; c += 32) {
           float v[16];
@@ -245,11 +245,21 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(x[j]) + __uint_as_float(y[j]);
+            if (a.ks == 2) {
+              tmem_ld16_nowait(tacc2 + (uint32_t)c, x);
+              tmem_ld16_nowait(tacc2 + (uint32_t)(a.NP + c), y);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(x[j]) + __uint_as_float(y[j]);
+            }
           }
           if (c + 32 >= a.NP) {  // this warp has read its share: the last stores need not hold up the next tile
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_leader<CG>(&acc_empty[db]);
+            if (lane == 0) {
+              mbar_arrive_leader<CG>(&acc_empty[db]);
+              if (a.ks == 2) mbar_arrive_leader<CG>(&acc_empty[db2]);
+            }
           }
           if (g < total && c < a.NP) {
             add_bias_act(v, bias_s + n0 + c, a.act);
@@ -474,16 +484,19 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
     const uint32_t P = PB >> 4;   // one part further, in descriptor units
     const uint64_t f0hi = f0 & 0xffffffff00000000ull;
     uint32_t st = 0, fpar = 0;                 // filter ring: stage, parity of its current use
-    uint32_t v0 = 0, v1 = 0;                   // units taken from each gather group
+    uint32_t v = 0, v1 = 0;                    // units taken (from the two groups, where one issuer serves both)
     uint32_t db0 = 0, dpar0 = 1;               // accumulator of the tile's first pixel set, parity of its last release
     bool first = true, fresh = true;           // first tile of this CTA; accumulators not yet used before
     long long w0 = 0, w1 = 0, w2 = 0, t0 = tc_clock(), tq;
     // No loop ends early on a failed wait: what follows it neither waits nor issues, and the trip counts
-    // depend on the arguments alone, which keeps the loop state in uniform registers.
-    for (int unit = cluster; unit < nunits && me < a.S; unit += nclusters) {
+    // depend on the arguments alone, which keeps the loop state in uniform registers.  An issuer steps through
+    // its own pixel sets only: its instructions, not the tensor pipe, bound layers of 64 outputs and fewer.
+    const int nsets = a.S * a.ks;
+    const bool paired = nsets > 1;             // a gather group and its two buffers belong to one issuer
+    for (int unit = cluster; unit < nunits && me < nsets; unit += nclusters) {
       const ConvPhase &p = phase_of(a, unit / a.ngroups);
-      const int kslab = p.kslab, nfb = (kslab + 63) >> 6, nblk = a.nslab * nfb;
-      uint32_t ulocal = 0;                     // unit of the tile
+      const int kslab = p.kslab, nfb = (kslab + 63) >> 6, nblk = a.nslab * nfb, nku = a.nslab * ((kslab + 31) >> 5);
+      int u0 = 0;                              // units of the tile before this block
       for (int i = 0, fb = 0; i < nblk; ++i, fb = fb + 1 == nfb ? 0 : fb + 1) {
         tq = tc_clock();
         if ((!a.resident || first) && !failed) {
@@ -492,47 +505,45 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
         }
         w0 += tc_clock() - tq;
         const int k16 = min(4, (kslab - fb * 64) >> 4);  // steps of this block, two per unit
-        const uint64_t fst = f0 + (uint64_t)((st * FB) >> 4);
-        for (int h = 0; h * 2 < k16; ++h, ++ulocal) {
-          const bool last = i + 1 == nblk && (h == 1 || k16 <= 2), both = k16 - h * 2 >= 2;
-          uint32_t db = db0, dpar = dpar0;
-          bool unused = fresh;
-          for (int s = 0; s < a.S; ++s) {
-            if ((s & (CV_ISSUERS - 1)) == me) {
-              tq = tc_clock();
-              if ((i | h) == 0 && !unused && !failed) failed = !mbar_wait_warp_cg<CG>(&acc_empty[db], dpar);
-              w1 += tc_clock() - tq;
-              tq = tc_clock();
-              const int grp = a.S > 1 ? me : (int)(ulocal & 1);
-              const uint32_t vv = grp ? v1 : v0, ab = grp * 2 + (vv & 1);
-              if (!failed) failed = !mbar_wait_warp_cg<CG>(&a_full[ab], (vv >> 1) & 1);
-              if (grp)
-                ++v1;
-              else
-                ++v0;
-              w2 += tc_clock() - tq;
-              tc_fence_after();
-              const uint32_t dm = uni(tmem_base + db * 2u * (uint32_t)a.NP), dl = dm + (uint32_t)a.NP;
-              const uint32_t a1 = uni(tmem_a + ab * CV_A_COLS);
-              const uint64_t b1 = f0hi | uni((uint32_t)fst + (uint32_t)(h * 4));
-              const uint32_t more = (uint32_t)(i | h) != 0;
-              if (!failed && elect_one()) {
-                umma_6<CG>(dm, dl, a1, b1, P, idesc, more);
-                if (both) umma_6<CG>(dm, dl, a1 + 8, b1 + 2, P, idesc, 1);
-                umma_commit_cg<CG>(&a_empty[ab]);
-                if (last) umma_commit_cg<CG>(&acc_full[db]);
-              }
-              __syncwarp();
+        const uint32_t fst = (uint32_t)f0 + ((st * FB) >> 4);
+        const int nh = (k16 + 1) >> 1;
+        for (int h = a.ks == 2 ? (u0 ^ me) & 1 : 0; h < nh; h += a.ks) {
+          const bool last = u0 + h + a.ks >= nku, both = k16 - h * 2 >= 2;
+          const uint32_t more = u0 + h >= a.ks;
+          const uint64_t b1 = f0hi | uni(fst + (uint32_t)(h * 4));
+          for (int s = me; s < nsets; s += CV_ISSUERS) {
+            uint32_t db = db0 + s;
+            const bool wrapped = db >= (uint32_t)a.ND;
+            if (wrapped) db -= a.ND;
+            tq = tc_clock();
+            if (more == 0 && !(fresh && !wrapped) && !failed)
+              failed = !mbar_wait_warp_cg<CG>(&acc_empty[db], dpar0 ^ (uint32_t)wrapped);
+            w1 += tc_clock() - tq;
+            tq = tc_clock();
+            // one issuer alone takes the groups in turn, from group 0 in every tile
+            const bool second = !paired && ((u0 + h) & 1);
+            const uint32_t turn = second ? v1++ : v++, ab = (paired ? me : (int)second) * 2 + (turn & 1);
+            if (!failed) failed = !mbar_wait_warp_cg<CG>(&a_full[ab], (turn >> 1) & 1);
+            w2 += tc_clock() - tq;
+            tc_fence_after();
+            const uint32_t dm = uni(tmem_base + db * 2u * (uint32_t)a.NP), dl = dm + (uint32_t)a.NP;
+            const uint32_t a1 = uni(tmem_a + ab * CV_A_COLS);
+            if (!failed && elect_one()) {
+              umma_6<CG>(dm, dl, a1, b1, P, idesc, more);
+              if (both) umma_6<CG>(dm, dl, a1 + 8, b1 + 2, P, idesc, 1);
+              umma_commit_cg<CG>(&a_empty[ab]);
+              if (last) umma_commit_cg<CG>(&acc_full[db]);
             }
-            if (++db == (uint32_t)a.ND) db = 0, dpar ^= 1, unused = false;
+            __syncwarp();
           }
         }
+        u0 += nh;
         if (!failed && !a.resident && elect_one()) umma_commit_cg<CG>(&filt_empty[st]);
         __syncwarp();
         if (++st == (uint32_t)a.nf) st = 0, fpar ^= 1;
       }
       first = false;
-      db0 += a.S;
+      db0 += nsets;
       if (db0 >= (uint32_t)a.ND) db0 -= a.ND, dpar0 ^= 1, fresh = false;
     }
     CV_TIMING(3, warp == CV_W_MMA)
@@ -759,6 +770,16 @@ FilterSet filter_set(const GatherPlan &p, const ConvGeom &g, int for_dx, float *
   return s;
 }
 
+// 32-k units of the phase with the fewest
+int least_units(const GatherPlan &p) {
+  int n = 1 << 30;
+  for (int i = 0; i < p.nphases; ++i) {
+    const int u = p.nslab * ((p.ph[i].kslab + 31) / 32);
+    if (u < n) n = u;
+  }
+  return n;
+}
+
 int launch_conv_gather(b200_ctx *ctx, const GatherPlan &p, const ConvGeom &g, int for_dx, const float *in, const float *filt,
                        const float *bias, float *out, int B, int act) {
   ConvGatherArgs a = {};
@@ -792,19 +813,20 @@ int launch_conv_gather(b200_ctx *ctx, const GatherPlan &p, const ConvGeom &g, in
   // CTA pair or single CTAs, and S: the least time of the busiest SM, tile after tile, a tile taking the
   // longer of its MMAs (N / 2 cycles each, with a floor; pairs measured 1.2 x as fast) and its loads (about
   // 40 cycles for 32 places of a channel pair).
-  static const int force_cg = getenv("B200_CONV_CG") ? atoi(getenv("B200_CONV_CG")) : 0;
   long long best = -1;
   int CG = 1;
   for (int cg = 2; cg >= 1; --cg) {
-    if (force_cg && cg != force_cg) continue;
     for (int S = p.S; S >= 1; S /= 2) {
+      const int ks = S == 1 && p.ND >= 2 && least_units(p) >= 2 ? 2 : 1;
       const long long slots = ctx->sm_count / cg;
       long long tiles = 0, tile_cost = 0;
       for (int i = 0; i < p.nphases; ++i) {
         const ConvPhase &q = p.ph[i];
         tiles += ((long long)B * q.PH * q.PW + cg * S * 128 - 1) / (cg * S * 128);
         const long long units = (long long)p.nslab * ((q.kslab + 31) / 32) * S;
-        const long long mma = units * (p.NP > 64 ? p.NP * 6 : 450) * (cg == 2 ? 5 : 6) / 5;
+        // about 900 cycles of an issuer's instructions a unit
+        const long long issue = S * ks > 1 ? 450 : 900;
+        const long long mma = units * (p.NP * 6 > issue ? p.NP * 6 : issue) * (cg == 2 ? 5 : 6) / 5;
         const long long load = (long long)p.nslab * ((p.CS + 1) / 2) * ((rows_needed(q, p, S * 128) * q.pitch + 31) / 32) * 40;
         tile_cost += mma > load ? mma : load;
       }
@@ -813,6 +835,7 @@ int launch_conv_gather(b200_ctx *ctx, const GatherPlan &p, const ConvGeom &g, in
         best = cost;
         CG = cg;
         a.S = S;
+        a.ks = ks;
       }
     }
   }

@@ -649,7 +649,7 @@ size_t conv_gather_dw_floats(const b200_ctx *ctx, const ConvGeom &g, int B) {
 }
 
 int conv_gather_dw(b200_ctx *ctx, const ConvGeom &g, const float *in, const float *dout, int B, float *part, float *dW,
-                   float *db, int accumulate) {
+                   float *db, int accumulate, bool finish) {
   ConvDwArgs a;
   size_t smem;
   B200_REQUIRE(dw_plan(ctx, g, &a, &smem), "tensor-core dW: the tiles do not fit");
@@ -687,6 +687,16 @@ int conv_gather_dw(b200_ctx *ctx, const ConvGeom &g, const float *in, const floa
             s[1], s[2], s[3], s[4], s[5], s[6], s[8], s[9], s[10]);
   }
 #endif
+  return finish ? conv_gather_dw_finish(ctx, g, B, part, dW, db, accumulate) : 0;
+}
+
+int conv_gather_dw_finish(b200_ctx *ctx, const ConvGeom &g, int B, const float *part, float *dW, float *db, int accumulate) {
+  ConvDwArgs a;
+  size_t smem;
+  B200_REQUIRE(dw_plan(ctx, g, &a, &smem), "tensor-core dW: the tiles do not fit");
+  const size_t n = dw_splits(ctx, &a, B);
+  a.part = const_cast<float *>(part);
+  a.bpart = db != nullptr && g.has_bias ? a.part + n : nullptr;
   int rows = 0, most = 0;
   for (int i = 0; i < a.nkg; ++i) {
     rows += a.ocb * a.ccb * a.kg[i].nky * a.NB * a.kg[i].nkx * a.CB;

@@ -31,9 +31,9 @@ struct Layer {
   int32_t *argmax = nullptr;
   bool tiled = false;
   float *wt_fwd = nullptr, *wt_dx = nullptr;
-  // tensor-core passes: filter blocks of the forward and dX passes
+  // tensor-core passes: filter blocks of the forward and dX passes, partial weight gradients
   ConvTcUse tc = {};
-  float *tc_wt_fwd = nullptr, *tc_wt_dx = nullptr;
+  float *tc_wt_fwd = nullptr, *tc_wt_dx = nullptr, *tc_part = nullptr;
   float act_param = 0.f;  // leaky relu: epsilon; elu: alpha
   // batch normalization: shape, constants, this batch's moments, stddev, moving averages, slice sums
   int bn_c = 0, bn_s = 0;
@@ -77,8 +77,8 @@ struct b200_net {
   float *x_dev = nullptr, *t_dev = nullptr;  // staging for the HOST step
   // side stream for independent work of one layer's backward pass (a tensor-core dW beside an
   // FFMA dX use different units of the SM and share it)
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t side = nullptr, sums = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_dw = nullptr;
   // b200_net_fit_host: uploads of the next mini-batch overlap the step of the current one
   cudaStream_t copy_stream = nullptr;
   float *x_stage[2] = {nullptr, nullptr}, *t_stage[2] = {nullptr, nullptr};
@@ -436,6 +436,9 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
     side_used = true;
     return 0;
   };
+  // The sums over a tensor-core dW kernel's partial results go to a third stream: behind their kernel they would hold
+  // up the next layer's dW on the side branch.  With peers they stay there, since the gradients leave early.
+  bool sums_used = false;
   // a fully-connected layer, or a convolution that is one (w_rows)
   auto fc_backward = [&](Layer &L, bool w_rows, const float *in, float *din, const float *W, float *dW, float *db,
                          bool can_fork) -> int {
@@ -473,7 +476,15 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
         if (forked) B200_TRY(fork());
         float *part = forked ? net->scratch_side : net->scratch;
         if (L.tc.dw) {
-          rc_side = conv_gather_dw(ctx, L.g, in, L.grad, B, part, dW, db, 0);
+          const bool later = forked && !peer_in_step;
+          rc_side = conv_gather_dw(ctx, L.g, in, L.grad, B, L.tc_part, dW, db, 0, !later);
+          if (!rc_side && later) {
+            B200_CUDA(cudaEventRecord(net->ev_dw, net->side));
+            B200_CUDA(cudaStreamWaitEvent(net->sums, net->ev_dw, 0));
+            ctx->stream = net->sums;
+            rc_side = conv_gather_dw_finish(ctx, L.g, B, L.tc_part, dW, db, 0);
+            sums_used = true;
+          }
         } else if (L.tc.dw_small) {
           rc_side = conv_dw_small(ctx, L.g, in, L.grad, B, part, dW, db, 0);
         } else if (tiled_bwd) {
@@ -560,6 +571,10 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
     }
   }
   ctx->stream = main_stream;
+  if (sums_used) {
+    B200_CUDA(cudaEventRecord(net->ev_dw, net->sums));
+    B200_CUDA(cudaStreamWaitEvent(main_stream, net->ev_dw, 0));
+  }
   if (side_used) {  // the optimizer (or the caller's all-reduce) follows on the main stream
     B200_CUDA(cudaEventRecord(net->ev_join, net->side));
     B200_CUDA(cudaStreamWaitEvent(main_stream, net->ev_join, 0));
@@ -656,8 +671,10 @@ int b200_net_create(b200_ctx *ctx, const b200_layer_spec *specs, int n_layers, i
   if (const char *e = getenv("B200_NET_NO_GRAPH")) net->use_graph = !(e[0] == '1');
   if (!getenv("B200_NET_NO_SIDE")) {
     cudaStreamCreateWithFlags(&net->side, cudaStreamNonBlocking);
+    cudaStreamCreateWithFlags(&net->sums, cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&net->ev_fork, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&net->ev_join, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&net->ev_dw, cudaEventDisableTiming);
   }
   size_t off = 0;
   size_t prev_out = 0;
@@ -825,7 +842,8 @@ int b200_net_create(b200_ctx *ctx, const b200_layer_spec *specs, int n_layers, i
         net_alloc(net, (void **)&L.tc_wt_dx, conv_gather_filter_floats(ctx, L.g, 1) * f);
       else if (L.tiled)
         net_alloc(net, (void **)&L.wt_dx, conv_tiled_dx_scratch(L.g) * f);
-      need = L.tc.dw         ? conv_gather_dw_floats(ctx, L.g, max_batch)
+      if (L.tc.dw) net_alloc(net, (void **)&L.tc_part, conv_gather_dw_floats(ctx, L.g, max_batch) * f);
+      need = L.tc.dw         ? 0
              : L.tc.dw_small ? conv_dw_small_floats(ctx, L.g, max_batch)
              : L.tiled       ? conv_tiled_dw_scratch(ctx, L.g, max_batch)
                              : 0;
@@ -866,8 +884,10 @@ int b200_net_destroy(b200_net *net) {
   if (net->ev_comm_side) cudaEventDestroy(net->ev_comm_side);
   if (net->ev_comm_done) cudaEventDestroy(net->ev_comm_done);
   if (net->side) cudaStreamDestroy(net->side);
+  if (net->sums) cudaStreamDestroy(net->sums);
   if (net->ev_fork) cudaEventDestroy(net->ev_fork);
   if (net->ev_join) cudaEventDestroy(net->ev_join);
+  if (net->ev_dw) cudaEventDestroy(net->ev_dw);
   for (void *q : net->mem) cudaFree(q);
   delete net;
   return 0;
