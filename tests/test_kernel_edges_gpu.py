@@ -25,6 +25,9 @@ pytestmark = pytest.mark.gpu
     (9, 8, 24, 16, 3, 2, True, 300),    # many images in a pixel set
     (24, 18, 16, 141, 3, 1, True, 51),  # an odd number of 32-k units a tile, several tiles a block
     (8, 8, 40, 32, 5, 1, True, 100),    # one pixel set a tile, k's split between two issuers
+    (32, 32, 3, 40, 5, 1, True, 7),     # few input channels: dW with the window's columns as channels
+    (100, 9, 8, 64, 3, 1, False, 3),    # the same, wide rows
+    (11, 30, 2, 200, 5, 1, True, 70),   # the same, two groups of output channels
     (5, 5, 16, 120, 5, 1, False, 16),   # window as large as the input
 ])
 def test_conv_tensor_core_edges(ctx, case):
