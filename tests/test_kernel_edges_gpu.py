@@ -1,12 +1,15 @@
 """The kernels that choose their tiling by size, at the sizes where it can go wrong: edges of tiles, remainders, the
 smallest and the largest of a range.  Convolutions and matrix products against the same sums in double precision,
 whole-network kernels against the layers one by one."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 import torch.nn.functional as F
 
-from test_ops_gpu import FWD_TOL, GRAD_TOL, assert_close, host
+import oracle_lib as o
+from test_ops_gpu import FWD_TOL, GRAD_TOL, assert_close, dev, host
 from tiny_cnn_b200 import _lib as L
 from tiny_cnn_b200 import network, ops
 
@@ -91,3 +94,31 @@ def test_whole_network_kernels_equal_the_layers(monkeypatch, name, batch):
         net.close()
     for a, b, what, tol in zip(results[0], results[1], ("output", "gradients", "weights"), (FWD_TOL, GRAD_TOL, GRAD_TOL)):
         assert_close(np.asarray(b), np.asarray(a), tol, f"{name} {batch}: {what}")
+
+
+# w, h, in, out, k, stride, batch: blocks of a sample 8 to 1, pixels and channels off every tile
+@pytest.mark.parametrize("case", [(8, 8, 3, 6, 3, 1, 1), (28, 28, 32, 64, 5, 1, 3), (28, 23, 31, 63, 5, 1, 30), (13, 11, 9, 17, 3, 2, 70),
+                                  (28, 28, 32, 64, 5, 1, 75)])  # the last: accumulators wait in the output's place
+def test_quantized_conv_edges(ctx, oracle, case):
+    w, h, c, oc, k, stride, B = case
+    d = ops.conv_params(w, h, c, k, k, oc, False, True, stride, stride)
+    rng = np.random.default_rng(5)
+    x = rng.uniform(-1, 1, (B, c * w * h)).astype(np.float32)
+    W = rng.uniform(-0.5, 0.5, oc * c * k * k).astype(np.float32)
+    b = rng.uniform(-0.1, 0.1, oc).astype(np.float32)
+    y = o.f32(B, oc * d.out_h * d.out_w)
+    assert oracle.orc_qconv2d_fwd(C.byref(d), o.p(x), o.p(W), o.p(b), o.p(y), B, None, None) == 0
+    got = host(ops.quantized_conv2d(ctx, d, dev(x), dev(W), dev(b)))
+    assert np.array_equal(got.view(np.uint32), y.view(np.uint32))
+
+
+@pytest.mark.parametrize("n_in,n_out,B", [(64, 10, 1), (9216, 256, 3), (1031, 65, 128), (33, 257, 66)])
+def test_quantized_fc_edges(ctx, oracle, n_in, n_out, B):
+    rng = np.random.default_rng(6)
+    x = rng.uniform(-1, 1, (B, n_in)).astype(np.float32)
+    W = rng.uniform(-0.5, 0.5, n_in * n_out).astype(np.float32)
+    b = rng.uniform(-0.1, 0.1, n_out).astype(np.float32)
+    y = o.f32(B, n_out)
+    assert oracle.orc_qfc_fwd(n_in, n_out, o.p(x), o.p(W), o.p(b), o.p(y), B) == 0
+    got = host(ops.quantized_fully_connected(ctx, n_in, n_out, dev(x), dev(W), dev(b)))
+    assert np.array_equal(got.view(np.uint32), y.view(np.uint32))

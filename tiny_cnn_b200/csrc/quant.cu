@@ -78,7 +78,7 @@ struct QSample {
   int off_in;              // quantized 0.0 of the input
   int zero_total;          // quantized 0.0 of the accumulator space
   int acc_min, acc_max;    // observed accumulator extremes
-  int sum_in;              // sum of the quantized input bytes (dp4a path)
+  int sum_in;              // sum of the quantized input bytes (fully connected)
   // requantize_many_in_new_range<int32,uint8> constants (:159-171)
   long long range_scale_fp, input_offset_fp, output_offset_fp;
   float min_new, max_new;  // shrunk output range
@@ -132,12 +132,12 @@ __global__ void q_input_range_kernel(const float *__restrict__ in, size_t row_le
 
 // ---- 2. filter / bias ranges ---------------------------------------------------
 
-// Single block.  Filter: `nseg` segments of `seg_len` elements every
+// By a whole block.  Filter: `nseg` segments of `seg_len` elements every
 // `seg_stride`, seeded with W[0]; equal min/max widen to W[0] -+ 1e-3.
 // Bias: all `nbias` elements, seeded with 0; equal min/max widen to b[0] -+ 1e-3.
-__global__ void q_filter_range_kernel(const float *__restrict__ W, int nseg, size_t seg_stride,
-                                      size_t seg_len, const float *__restrict__ bias, int nbias,
-                                      QGlobal *qg) {
+// `qg` lies in shared memory; every thread may read it afterwards.
+__device__ __forceinline__ void filter_range(const float *__restrict__ W, int nseg, size_t seg_stride, size_t seg_len,
+                                             const float *__restrict__ bias, int nbias, QGlobal &qg) {
   float mn = W[0], mx = W[0];
   size_t total = (size_t)nseg * seg_len;
   for (size_t t = threadIdx.x; t < total; t += blockDim.x) {
@@ -179,13 +179,22 @@ __global__ void q_filter_range_kernel(const float *__restrict__ W, int nseg, siz
         bmx = __fadd_rn(bias[0], 1e-3f);
         bmn = __fsub_rn(bias[0], 1e-3f);
       }
-      qg->min_f = mn;
-      qg->max_f = mx;
-      qg->min_b = bmn;
-      qg->max_b = bmx;
-      qg->off_f = (int)f2q_unclamped<8>(0.0f, mn, mx);
+      qg.min_f = mn;
+      qg.max_f = mx;
+      qg.min_b = bmn;
+      qg.max_b = bmx;
+      qg.off_f = (int)f2q_unclamped<8>(0.0f, mn, mx);
     }
   }
+  __syncthreads();
+}
+
+__global__ void q_filter_range_kernel(const float *__restrict__ W, int nseg, size_t seg_stride,
+                                      size_t seg_len, const float *__restrict__ bias, int nbias,
+                                      QGlobal *out) {
+  __shared__ QGlobal qg;
+  filter_range(W, nseg, seg_stride, seg_len, bias, nbias, qg);
+  if (threadIdx.x == 0) *out = qg;
 }
 
 // ---- 3. quantize --------------------------------------------------------------
@@ -217,19 +226,15 @@ __global__ void q_quantize_input_kernel(const float *__restrict__ in, size_t row
 
 // quantization_range_for_multiplication<u8,u8,i32> (:95-114); the fc kernel
 // then adds the bias range to it (fc :67-68).
-__global__ void q_sample_params_kernel(QSample *qs, const QGlobal *__restrict__ qg, int B,
-                                       int add_bias_range) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= B) return;
-  QSample s = qs[n];
+__device__ __forceinline__ void sample_params(QSample &s, const QGlobal &qg, int add_bias_range) {
   float a_level = one_level_u8(s.min_in, s.max_in);
-  float b_level = one_level_u8(qg->min_f, qg->max_f);
+  float b_level = one_level_u8(qg.min_f, qg.max_f);
   float c_level = __fmul_rn(a_level, b_level);
   float mn = __fmul_rn(c_level, (float)(-(1LL << 31)));
   float mx = __fmul_rn(c_level, (float)((1LL << 31) - 1));
   if (add_bias_range) {
-    mn = __fadd_rn(mn, qg->min_b);
-    mx = __fadd_rn(mx, qg->max_b);
+    mn = __fadd_rn(mn, qg.min_b);
+    mx = __fadd_rn(mx, qg.max_b);
   }
   s.min_out = mn;
   s.max_out = mx;
@@ -238,6 +243,14 @@ __global__ void q_sample_params_kernel(QSample *qs, const QGlobal *__restrict__ 
   s.acc_min = INT_MAX;
   s.acc_max = INT_MIN;
   s.sum_in = 0;
+}
+
+__global__ void q_sample_params_kernel(QSample *qs, const QGlobal *__restrict__ qg, int B,
+                                       int add_bias_range) {
+  int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= B) return;
+  QSample s = qs[n];
+  sample_params(s, *qg, add_bias_range);
   qs[n] = s;
 }
 
@@ -303,321 +316,11 @@ __global__ void q_conv_acc_kernel(ConvGeom g, const uint8_t *__restrict__ inq,
   block_minmax_atomic(mn, mx, &qs[n].acc_min, &qs[n].acc_max);
 }
 
-// ---- 5b. the same accumulators through dp4a --------------------------------------------
-//
-// sum (w - off_w)(x - off_x) = sum w*x - off_x * sum w - off_w * sum x + n * off_w * off_x is exact
-// in integers, so the products can be taken four bytes at a time (dp4a on unsigned bytes) from
-// operands laid out with the contracted index fastest.  All arithmetic is modulo 2^32 and the
-// true value fits an int32, so intermediate wrap-around is harmless.
-
-// min / max of a long vector, many blocks: per-block results, reduced by q_filter_range_kernel
-__global__ void q_minmax_partial_kernel(const float *__restrict__ v, size_t n, float *__restrict__ part) {
-  float mn = v[0], mx = v[0];
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    mn = fminf(mn, v[i]);
-    mx = fmaxf(mx, v[i]);
-  }
-  __shared__ float s2[2][32];
-  mn = warp_min(mn);
-  mx = warp_max(mx);
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) {
-    s2[0][wid] = mn;
-    s2[1][wid] = mx;
-  }
-  __syncthreads();
-  if (wid == 0) {
-    int nw = blockDim.x >> 5;
-    mn = warp_min(lane < nw ? s2[0][lane] : s2[0][0]);
-    mx = warp_max(lane < nw ? s2[1][lane] : s2[1][0]);
-    if (lane == 0) {
-      part[2 * blockIdx.x] = mn;
-      part[2 * blockIdx.x + 1] = mx;
-    }
-  }
-}
-
-// fully-connected filter, quantized and transposed: Wt[i][c] (row pitch `pitch` bytes, zero padded)
-// from W[c*out + i]; 32 x 32 tiles through shared memory
-__global__ void q_quantize_filter_t_kernel(const float *__restrict__ W, int in_size, int out_size, int pitch,
-                                           const float *__restrict__ bias, int nbias,
-                                           const QGlobal *__restrict__ qg, uint8_t *__restrict__ Wt,
-                                           uint8_t *__restrict__ bq) {
-  __shared__ uint8_t tile[32][33];
-  const float mn = qg->min_f, mx = qg->max_f;
-  if (blockIdx.x == 0 && blockIdx.y == 0) {
-    const float bmn = qg->min_b, bmx = qg->max_b;
-    for (int j = threadIdx.y * 32 + threadIdx.x; j < nbias; j += 256) bq[j] = (uint8_t)f2q<8>(bias[j], bmn, bmx);
-  }
-  const int c0 = blockIdx.y * 32, i0 = blockIdx.x * 32;
-  for (int j = threadIdx.y; j < 32; j += 8) {
-    int c = c0 + j, i = i0 + threadIdx.x;
-    tile[j][threadIdx.x] = (c < in_size && i < out_size) ? (uint8_t)f2q<8>(W[(size_t)c * out_size + i], mn, mx) : 0;
-  }
-  __syncthreads();
-  for (int j = threadIdx.y; j < 32; j += 8) {
-    int i = i0 + j, c = c0 + threadIdx.x;
-    if (i < out_size && c < pitch) Wt[(size_t)i * pitch + c] = tile[threadIdx.x][j];
-  }
-}
-
-// input rows quantized with a row pitch (zero padded) and their byte sums (sum_in starts at 0:
-// q_sample_params_kernel); grid = (slices of 1024 bytes, B)
-__global__ void __launch_bounds__(256) q_quantize_input_pitch_kernel(const float *__restrict__ in, int row_len,
-                                                                    int pitch, QSample *qs,
-                                                                    uint8_t *__restrict__ inq) {
-  const int n = blockIdx.y;
-  const float mn = qs[n].min_in, mx = qs[n].max_in;
-  const float *r = in + (size_t)n * row_len;
-  const int j0 = blockIdx.x * 1024 + threadIdx.x * 4;
-  int sum = 0;
-  if (j0 < pitch) {  // pitch is a multiple of 4
-    unsigned w = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      unsigned v = j0 + k < row_len ? (unsigned)f2q<8>(r[j0 + k], mn, mx) : 0u;
-      w |= v << (8 * k);
-      sum += (int)v;
-    }
-    *reinterpret_cast<unsigned *>(inq + (size_t)n * pitch + j0) = w;
-  }
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&qs[n].sum_in, sum);
-}
-
-// fc :100-112.  One warp per pair of outputs and group of 8 samples; lanes split the contraction
-// in 16-byte pieces (pitch is a multiple of 16).
-constexpr int QFC_SAMPLES = 8, QFC_OUTS = 2;
-__device__ __forceinline__ unsigned dp4a4(const uint4 &a, const uint4 &b, unsigned c) {
-  c = __dp4a(a.x, b.x, c);
-  c = __dp4a(a.y, b.y, c);
-  c = __dp4a(a.z, b.z, c);
-  return __dp4a(a.w, b.w, c);
-}
-__global__ void __launch_bounds__(128) q_fc_acc_dp4a_kernel(int in_size, int out_size, int pitch, int has_bias,
-                                                           int B, const uint8_t *__restrict__ inq,
-                                                           const uint8_t *__restrict__ Wt,
-                                                           const uint8_t *__restrict__ bq,
-                                                           const QGlobal *__restrict__ qg, QSample *qs,
-                                                           int *__restrict__ acc) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int i0 = (blockIdx.x * 4 + warp) * QFC_OUTS, n0 = blockIdx.y * QFC_SAMPLES;
-  if (i0 >= out_size) return;
-  const int vecs = pitch >> 4;
-  const uint4 ones = make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
-  const uint4 *wrow[QFC_OUTS];
-#pragma unroll
-  for (int k = 0; k < QFC_OUTS; ++k)
-    wrow[k] = reinterpret_cast<const uint4 *>(Wt + (size_t)min(i0 + k, out_size - 1) * pitch);
-  const uint4 *xrow[QFC_SAMPLES];
-#pragma unroll
-  for (int s = 0; s < QFC_SAMPLES; ++s)
-    xrow[s] = reinterpret_cast<const uint4 *>(inq + (size_t)min(n0 + s, B - 1) * pitch);
-  unsigned a[QFC_OUTS][QFC_SAMPLES], sw[QFC_OUTS];
-#pragma unroll
-  for (int k = 0; k < QFC_OUTS; ++k) {
-    sw[k] = 0;
-#pragma unroll
-    for (int s = 0; s < QFC_SAMPLES; ++s) a[k][s] = 0;
-  }
-  for (int q = lane; q < vecs; q += 32) {
-    uint4 w[QFC_OUTS];
-#pragma unroll
-    for (int k = 0; k < QFC_OUTS; ++k) {
-      w[k] = __ldg(wrow[k] + q);
-      sw[k] = dp4a4(w[k], ones, sw[k]);
-    }
-#pragma unroll
-    for (int s = 0; s < QFC_SAMPLES; ++s) {
-      const uint4 x = __ldg(xrow[s] + q);
-#pragma unroll
-      for (int k = 0; k < QFC_OUTS; ++k) a[k][s] = dp4a4(w[k], x, a[k][s]);
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int k = 0; k < QFC_OUTS; ++k) {
-      sw[k] += __shfl_xor_sync(0xffffffffu, sw[k], o);
-#pragma unroll
-      for (int s = 0; s < QFC_SAMPLES; ++s) a[k][s] += __shfl_xor_sync(0xffffffffu, a[k][s], o);
-    }
-  // lanes 0..15 each finish one (output, sample) pair
-  const int k = lane >> 3, sl = lane & 7;
-  unsigned mine = 0, msw = 0;
-#pragma unroll
-  for (int kk = 0; kk < QFC_OUTS; ++kk)
-#pragma unroll
-    for (int s = 0; s < QFC_SAMPLES; ++s)
-      if (kk == k && s == sl) {
-        mine = a[kk][s];
-        msw = sw[kk];
-      }
-  if (k < QFC_OUTS && i0 + k < out_size && n0 + sl < B) {
-    const int n = n0 + sl, i = i0 + k;
-    const unsigned off_f = (unsigned)qg->off_f, off_in = (unsigned)qs[n].off_in;
-    unsigned v = mine - off_in * msw - off_f * (unsigned)qs[n].sum_in + (unsigned)in_size * off_f * off_in;
-    int sum = (int)v;
-    if (has_bias) sum += (int)bq[i] - qs[n].zero_total;
-    acc[(size_t)n * out_size + i] = sum;
-    atomicMin(&qs[n].acc_min, sum);
-    atomicMax(&qs[n].acc_max, sum);
-  }
-}
-
-// convolution operands with the channel index fastest: input [n][y][x][c], filter [o][tap][c]
-__global__ void q_quantize_input_nhwc_kernel(const float *__restrict__ in, int C, int HW, const QSample *__restrict__ qs,
-                                             uint8_t *__restrict__ inq) {
-  const int n = blockIdx.y;
-  const float mn = qs[n].min_in, mx = qs[n].max_in;
-  const float *r = in + (size_t)n * C * HW;
-  unsigned *q = reinterpret_cast<unsigned *>(inq + (size_t)n * C * HW);
-  const int Cw = C >> 2, total = HW * Cw;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x) {
-    const int p = j % HW, cw = j / HW;  // pixel fastest: the four plane reads are coalesced
-    unsigned w = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) w |= (unsigned)f2q<8>(r[(size_t)(cw * 4 + k) * HW + p], mn, mx) << (8 * k);
-    q[(size_t)p * Cw + cw] = w;
-  }
-}
-
-__global__ void q_quantize_filter_otc_kernel(const float *__restrict__ W, int C, int OC, int KK,
-                                             const float *__restrict__ bias, int nbias,
-                                             const QGlobal *__restrict__ qg, uint8_t *__restrict__ Wq,
-                                             uint8_t *__restrict__ bq) {
-  const float mn = qg->min_f, mx = qg->max_f;
-  const int total = OC * KK * C;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x) {
-    const int c = j % C, r = j / C, tap = r % KK, o = r / KK;
-    Wq[j] = (uint8_t)f2q<8>(W[((size_t)o * C + c) * KK + tap], mn, mx);
-  }
-  const float bmn = qg->min_b, bmx = qg->max_b;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nbias; j += gridDim.x * blockDim.x)
-    bq[j] = (uint8_t)f2q<8>(bias[j], bmn, bmx);
-}
-
-// conv :89-133.  Block = one sample, 128 output pixels, all output channels; thread = 4 pixels x 8
-// output channels (a warp shares the channels, so its filter loads are broadcasts); the whole
-// quantized filter sits in shared memory.
-constexpr int QCV_PPT = 4, QCV_OPT = 8, QCV_PIX = 32 * QCV_PPT, QCV_WARPS = 8;
-template <bool VEC>
-__global__ void __launch_bounds__(256) q_conv_acc_dp4a_kernel(ConvGeom g, const uint8_t *__restrict__ inq,
-                                                             const uint8_t *__restrict__ Wq,
-                                                             const uint8_t *__restrict__ bq,
-                                                             const QGlobal *__restrict__ qg, QSample *qs,
-                                                             int *__restrict__ acc) {
-  extern __shared__ __align__(16) uint8_t qsm[];
-  const int KK = g.KH * g.KW, Cw = g.C >> 2;
-  const int wlen = g.OC * KK * g.C;                         // bytes of the filter
-  unsigned *wsm = reinterpret_cast<unsigned *>(qsm);         // [o][tap][Cw] words
-  unsigned *wsum = wsm + ((wlen >> 2) + 3) / 4 * 4;         // [OC]
-  const int n = blockIdx.y, tid = threadIdx.x;
-  for (int j = tid; j < (wlen >> 2); j += 256) wsm[j] = reinterpret_cast<const unsigned *>(Wq)[j];
-  __syncthreads();
-  for (int o = tid; o < g.OC; o += 256) {
-    unsigned t = 0;
-    for (int j = 0; j < KK * Cw; ++j) t = __dp4a(wsm[o * KK * Cw + j], 0x01010101u, t);
-    wsum[o] = t;
-  }
-  __syncthreads();
-  const int npix = g.OH * g.OW;
-  const int p0 = blockIdx.x * QCV_PIX + (tid & 31) * QCV_PPT, og = tid >> 5;
-  const unsigned off_f = (unsigned)qg->off_f, off_in = (unsigned)qs[n].off_in;
-  const int zero_total = qs[n].zero_total;
-  const unsigned *ib = reinterpret_cast<const unsigned *>(inq + (size_t)n * g.C * g.HI * g.WI);
-  int pbase[QCV_PPT];  // word offset of the window origin of each pixel (pixels past the end repeat the last)
-#pragma unroll
-  for (int k = 0; k < QCV_PPT; ++k) {
-    const int p = min(p0 + k, npix - 1);
-    const int y = p / g.OW, x = p - y * g.OW;
-    pbase[k] = (y * g.SH * g.WI + x * g.SW) * Cw;
-  }
-  int mn = INT_MAX, mx = INT_MIN;
-  for (int o0 = og * QCV_OPT; o0 < g.OC; o0 += QCV_WARPS * QCV_OPT) {
-    unsigned a[QCV_PPT][QCV_OPT], sx[QCV_PPT];
-#pragma unroll
-    for (int k = 0; k < QCV_PPT; ++k) {
-      sx[k] = 0;
-#pragma unroll
-      for (int j = 0; j < QCV_OPT; ++j) a[k][j] = 0;
-    }
-    for (int wy = 0; wy < g.KH; ++wy)
-      for (int wx = 0; wx < g.KW; ++wx) {
-        const int ioff = (wy * g.WI + wx) * Cw;
-        const unsigned *wp = wsm + (size_t)(o0 * KK + wy * g.KW + wx) * Cw;
-        if (VEC) {  // 16 channels per load
-          for (int cw = 0; cw < Cw; cw += 4) {
-            uint4 xv[QCV_PPT];
-#pragma unroll
-            for (int k = 0; k < QCV_PPT; ++k) {
-              xv[k] = *reinterpret_cast<const uint4 *>(ib + pbase[k] + ioff + cw);
-              sx[k] = dp4a4(xv[k], make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u), sx[k]);
-            }
-#pragma unroll
-            for (int j = 0; j < QCV_OPT; ++j) {
-              const int o = min(o0 + j, g.OC - 1);
-              const uint4 wv = *reinterpret_cast<const uint4 *>(wp + (o - o0) * KK * Cw + cw);
-#pragma unroll
-              for (int k = 0; k < QCV_PPT; ++k) a[k][j] = dp4a4(wv, xv[k], a[k][j]);
-            }
-          }
-        } else {
-          for (int cw = 0; cw < Cw; ++cw) {
-            unsigned xv[QCV_PPT];
-#pragma unroll
-            for (int k = 0; k < QCV_PPT; ++k) {
-              xv[k] = ib[pbase[k] + ioff + cw];
-              sx[k] = __dp4a(xv[k], 0x01010101u, sx[k]);
-            }
-#pragma unroll
-            for (int j = 0; j < QCV_OPT; ++j) {
-              const int o = min(o0 + j, g.OC - 1);
-              const unsigned wv = wp[(o - o0) * KK * Cw + cw];
-#pragma unroll
-              for (int k = 0; k < QCV_PPT; ++k) a[k][j] = __dp4a(wv, xv[k], a[k][j]);
-            }
-          }
-        }
-      }
-#pragma unroll
-    for (int j = 0; j < QCV_OPT; ++j) {
-      const int o = o0 + j;
-      if (o < g.OC) {
-        int sums[QCV_PPT];
-#pragma unroll
-        for (int k = 0; k < QCV_PPT; ++k) {
-          unsigned v = a[k][j] - off_in * wsum[o] - off_f * sx[k] + (unsigned)(KK * g.C) * off_f * off_in;
-          int sum = (int)v;
-          if (g.has_bias) sum += (int)bq[o] - zero_total;
-          sums[k] = sum;
-          if (p0 + k < npix) {
-            mn = min(mn, sum);
-            mx = max(mx, sum);
-          }
-        }
-        int *dst = acc + (size_t)n * g.OC * npix + (size_t)o * npix + p0;
-        if (p0 + QCV_PPT <= npix && (npix & 3) == 0) {
-          *reinterpret_cast<int4 *>(dst) = make_int4(sums[0], sums[1], sums[2], sums[3]);
-        } else {
-#pragma unroll
-          for (int k = 0; k < QCV_PPT; ++k)
-            if (p0 + k < npix) dst[k] = sums[k];
-        }
-      }
-    }
-  }
-  block_minmax_atomic(mn, mx, &qs[n].acc_min, &qs[n].acc_max);
-}
-
 // ---- 6. shrink range, requantize, dequantize ---------------------------------------
 
 // quantize_down_and_shrink_range (:230-254) and the constants of
 // requantize_many_in_new_range<int32,uint8> (:159-171), once per sample.
-__global__ void q_requant_params_kernel(QSample *qs, int B) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= B) return;
-  QSample s = qs[n];
+__device__ __forceinline__ void requant_params(QSample &s) {
   float min_new = fminf(0.0f, q2f<32>((long long)s.acc_min, s.min_out, s.max_out));
   float max_new = q2f<32>((long long)s.acc_max, s.min_out, s.max_out);
   const float input_range = __fsub_rn(s.max_out, s.min_out);
@@ -633,7 +336,23 @@ __global__ void q_requant_params_kernel(QSample *qs, int B) {
   s.output_offset_fp = (long long)roundf(__fdiv_rn(__fmul_rn(min_new, 255.0f), output_range));
   s.min_new = min_new;
   s.max_new = max_new;
+}
+
+__global__ void q_requant_params_kernel(QSample *qs, int B) {
+  int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= B) return;
+  QSample s = qs[n];
+  requant_params(s);
   qs[n] = s;
+}
+
+// inner loop of requantize_many_in_new_range<int32,uint8> (:172-185): the quantized value of one accumulator
+__device__ __forceinline__ int requant_one(int acc, const QSample &s) {
+  const long long rounding_delta = 1LL << 15;
+  const long long fp_value = (((long long)acc * s.range_scale_fp) >> 32) + s.input_offset_fp;
+  const long long ri = ((fp_value >= 0) ? (fp_value + rounding_delta) : (fp_value - rounding_delta)) >> 16;
+  const long long q = ri - s.output_offset_fp;
+  return q > 0 ? (q < 255 ? (int)q : 255) : 0;
 }
 
 // inner loop of requantize_many_in_new_range<int32,uint8> (:172-185) followed
@@ -644,17 +363,503 @@ __global__ void q_requant_dequant_kernel(const int *__restrict__ acc, size_t out
   const QSample s = qs[n];
   const int *a = acc + (size_t)n * out_len;
   float *o = out + (size_t)n * out_len;
-  const long long rounding_delta = 1LL << 15;
   size_t step = (size_t)gridDim.x * blockDim.x;
-  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < out_len; j += step) {
-    long long v = (long long)a[j];
-    long long fp_value = ((v * s.range_scale_fp) >> 32) + s.input_offset_fp;
-    long long ri = ((fp_value >= 0) ? (fp_value + rounding_delta) : (fp_value - rounding_delta)) >> 16;
-    long long q = ri - s.output_offset_fp;
-    q = q > 0 ? q : 0;
-    q = q < 255 ? q : 255;
-    o[j] = q2f<8>(q, s.min_new, s.max_new);
+  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < out_len; j += step)
+    o[j] = q2f<8>(requant_one(a[j], s), s.min_new, s.max_new);
+}
+
+// ---- 5b. convolution of a whole sample in one kernel ------------------------------------------------
+//
+// sum (w - off_w)(x - off_x) = sum w*x - off_x * sum w - off_w * sum x + n * off_w * off_x is exact
+// in integers, so the products are taken on bytes by the tensor cores (mma.m16n8k32, unsigned bytes, 32-bit
+// sums).  All arithmetic is modulo 2^32 and the true value fits an int32, so intermediate wrap-around is harmless.
+//
+// A cluster of 1 to 8 blocks takes a sample, each block a run of output pixels: it finds the sample's range
+// (blocks exchange theirs), quantizes the input rows that it needs into shared memory with the channels fastest,
+// takes the products, exchanges the accumulators' extremes and requantizes.  In eight launches each step read and
+// wrote memory (28x28x32 -> 64, 5x5, 128 samples: 247 us, of which the dp4a products 174 us and the requantizing
+// 20 us; this 65 us).  What bounds it: the products' shared-memory reads, 8 bytes a lane for every two
+// 16 x 8 x 32 products of a fragment, and then the requantizing's 64-bit integer multiplications.
+// A k step is 32 bytes: four groups of 8 channels, wherever in the window they lie (`tab`); channels are
+// padded to 8, the filter's rows to 32 bytes with zeros.
+struct QScale {  // f2q<8> of one range: the same operations, the ones that do not depend on the value done once
+  double scale, low;
+  bool flat;
+  __device__ __forceinline__ void set(float rmin, float rmax) {
+    flat = rmin == rmax;
+    const double range_adjust = __ddiv_rn(256.0, __dsub_rn(256.0, 1.0));
+    const double range = __dmul_rn((double)__fsub_rn(rmax, rmin), range_adjust);
+    scale = __ddiv_rn(256.0, range);
+    low = round(__dmul_rn((double)rmin, scale));
   }
+  __device__ __forceinline__ unsigned of(float v) const {
+    if (flat) return 0u;
+    const long long q = (long long)__dsub_rn(round(__dmul_rn((double)v, scale)), low);
+    return (unsigned)(q > 0 ? (q < 255 ? q : 255) : 0);
+  }
+};
+
+__device__ __forceinline__ void mma_u8(unsigned *c, const uint2 &a0, const uint2 &a1, const uint2 &b) {
+  // lane (g, q) holds bytes 8 q .. 8 q + 7 of rows g and g + 8 and of column g: the order of the k's is free as long
+  // as both operands have the same
+  asm volatile(
+    "mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+    : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+    : "r"(a0.x), "r"(a1.x), "r"(a0.y), "r"(a1.y), "r"(b.x), "r"(b.y));
+}
+
+struct QConvArgs {
+  const float *in;
+  float *out;
+  const uint8_t *Wq, *bq;
+  const unsigned *wsum;
+  const QGlobal *qg;
+  int C, HI, WI, OC, OH, OW, KH, KW, SH, SW, has_bias;
+  int Cp, ksteps, pitch, ntiles;  // channels padded to 8; k steps; bytes of a filter row; 8-channel tiles of the outputs
+  int per, rows;                  // output pixels of a block (a multiple of 16), most input rows it needs
+  int acc_smem;                   // the accumulators wait in shared memory, not in the output's place
+};
+
+constexpr int QC_THREADS = 512, QC_WARPS = QC_THREADS / 32;
+
+// bytes of a filter row in shared memory: 32 or 96 more than a multiple of 128, so that rows fall on different banks
+__host__ __device__ __forceinline__ int qc_pitch(int ksteps) { return ksteps * 32 + (ksteps % 2 == 0 ? 32 : 0); }
+
+// filter rows quantized as [o][tap][Cp], their byte sums, the quantized biases and the ranges; a block a row
+__global__ void __launch_bounds__(256) q_conv_filter_kernel(const float *__restrict__ W, int nseg, size_t seg_stride,
+                                                            size_t seg_len, int C, int Cp, int OC, int KK, int pitch,
+                                                            const float *__restrict__ bias, int nbias, QGlobal *out_qg,
+                                                            uint8_t *__restrict__ Wq, uint8_t *__restrict__ bq,
+                                                            unsigned *__restrict__ wsum) {
+  __shared__ QGlobal qg;
+  __shared__ unsigned part[8];
+  filter_range(W, nseg, seg_stride, seg_len, bias, nbias, qg);
+  const int o = blockIdx.x;
+  QScale q;
+  q.set(qg.min_f, qg.max_f);
+  unsigned sum = 0;
+  for (int k = threadIdx.x; k < pitch; k += 256) {
+    const int tap = k / Cp, c = k - tap * Cp;
+    const unsigned v = tap < KK && c < C && o < OC ? q.of(W[((size_t)o * C + c) * KK + tap]) : 0u;
+    Wq[(size_t)o * pitch + k] = (uint8_t)v;
+    sum += v;
+  }
+  for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) sum += part[k];
+    wsum[o] = sum;
+    if (o < nbias) bq[o] = (uint8_t)f2q<8>(bias[o], qg.min_b, qg.max_b);
+    if (o == 0) *out_qg = qg;
+  }
+}
+
+__device__ __forceinline__ void q_cluster_sync(int n) {
+  if (n == 1)
+    __syncthreads();
+  else
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ unsigned q_remote(const void *p, int rank) {  // a word of another block's shared memory
+  unsigned at, v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];\n" : "=r"(v) : "r"(at) : "memory");
+  return v;
+}
+
+__global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __grid_constant__ QConvArgs a) {
+  extern __shared__ __align__(16) uint8_t qsm[];
+  __shared__ float rmin[QC_WARPS], rmax[QC_WARPS], range[2];
+  __shared__ int amin[QC_WARPS], amax[QC_WARPS], extremes[2];
+  __shared__ QSample smp;
+  __shared__ float lut[256];
+  int nc, rank;
+  asm("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(nc));
+  asm("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+  const int n = blockIdx.x / nc, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int npix = a.OH * a.OW, p0 = min(npix, rank * a.per), p1 = min(npix, p0 + a.per), plane = a.HI * a.WI;
+  const int iy0 = p1 > p0 ? p0 / a.OW * a.SH : 0, iy1 = p1 > p0 ? (p1 - 1) / a.OW * a.SH + a.KH : 0;
+  const int places = (iy1 - iy0) * a.WI, KK = a.KH * a.KW;
+  uint8_t *ws = qsm, *xs = ws + (size_t)a.ntiles * 8 * a.pitch;                      // filter, input
+  int *tab = reinterpret_cast<int *>(xs + (size_t)a.rows * a.WI * a.Cp);             // [ksteps * 4]
+  unsigned *psum = reinterpret_cast<unsigned *>(tab + a.ksteps * 4);                 // [places] byte sums over the channels
+  unsigned *xsum = psum + a.rows * a.WI;                                             // [per] over the window
+  int *acc = a.acc_smem ? reinterpret_cast<int *>(xsum + a.per) : reinterpret_cast<int *>(a.out) + (size_t)n * a.OC * npix + p0;
+  const int acc_step = a.acc_smem ? a.per : npix;                                    // from output channel to output channel
+  for (int i = tid; i < a.ntiles * 8 * a.pitch / 16; i += QC_THREADS) cp_async16(ws + 16 * i, a.Wq + 16 * i, true);
+  cp_async_commit();
+  for (int i = tid; i < a.ksteps * 4; i += QC_THREADS) {
+    const int k = i * 8, tap = min(k / a.Cp, KK - 1), c = k % a.Cp;  // groups behind the window meet zeros of the filter
+    tab[i] = (tap / a.KW * a.WI + tap % a.KW) * a.Cp + c;
+  }
+  const float *in = a.in + (size_t)n * a.C * plane;
+  // the range: the reference scans the first HI * HI values of every plane, starting from the first value
+  {
+    float mn = in[0], mx = in[0];
+    const int scan = a.HI * a.HI, parts = max(1, QC_WARPS * nc / a.C), span = (scan + parts - 1) / parts;
+    for (int u = rank * QC_WARPS + warp; u < a.C * parts; u += nc * QC_WARPS) {
+      const int c = u / parts, b = (u - c * parts) * span;
+#pragma unroll 8
+      for (int e = b + lane; e < min(scan, b + span); e += 32) {
+        const float v = in[(size_t)c * plane + e];
+        mn = fminf(mn, v);
+        mx = fmaxf(mx, v);
+      }
+    }
+    mn = warp_min(mn);
+    mx = warp_max(mx);
+    if (lane == 0) {
+      rmin[warp] = mn;
+      rmax[warp] = mx;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      mn = warp_min(rmin[lane & (QC_WARPS - 1)]);
+      mx = warp_max(rmax[lane & (QC_WARPS - 1)]);
+      if (lane == 0) {
+        range[0] = mn;
+        range[1] = mx;
+      }
+    }
+    q_cluster_sync(nc);
+    if (tid == 0) {
+      for (int r = 0; r < nc && nc > 1; ++r) {
+        mn = fminf(mn, __uint_as_float(q_remote(&range[0], r)));
+        mx = fmaxf(mx, __uint_as_float(q_remote(&range[1], r)));
+      }
+      smp.min_in = mn;
+      smp.max_in = mx;
+      sample_params(smp, *a.qg, 0);
+    }
+    __syncthreads();
+  }
+  {
+    QScale q;
+    q.set(smp.min_in, smp.max_in);
+    const int groups = a.Cp / 4;
+#pragma unroll 2
+    for (int j = tid; j < places * groups; j += QC_THREADS) {
+      const int cg = j / places, p = j - cg * places;
+      const float *src = in + (size_t)cg * 4 * plane + iy0 * a.WI + p;
+      unsigned w = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (cg * 4 + k < a.C) w |= q.of(src[(size_t)k * plane]) << (8 * k);
+      *reinterpret_cast<unsigned *>(xs + (size_t)p * a.Cp + cg * 4) = w;
+    }
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  for (int p = tid; p < places; p += QC_THREADS) {
+    unsigned s = 0;
+    for (int k = 0; k < a.Cp; k += 8) {
+      const uint2 x = *reinterpret_cast<const uint2 *>(xs + (size_t)p * a.Cp + k);
+      s = __dp4a(x.y, 0x01010101u, __dp4a(x.x, 0x01010101u, s));
+    }
+    psum[p] = s;
+  }
+  __syncthreads();
+  for (int p = tid; p < p1 - p0; p += QC_THREADS) {
+    const int y = (p0 + p) / a.OW, x = p0 + p - y * a.OW;
+    const unsigned *s = psum + (y * a.SH - iy0) * a.WI + x * a.SW;
+    unsigned t = 0;
+    for (int ky = 0; ky < a.KH; ++ky)
+      for (int kx = 0; kx < a.KW; ++kx) t += s[ky * a.WI + kx];
+    xsum[p] = t;
+  }
+  __syncthreads();
+  // products: units of 16 pixels x 4 tiles of 8 outputs
+  const unsigned off_f = (unsigned)a.qg->off_f, off_in = (unsigned)smp.off_in, both = (unsigned)(KK * a.C) * off_f * off_in;
+  const int mtiles = (p1 - p0 + 15) / 16, ngroups = (a.ntiles + 3) / 4, g = lane >> 2, q = lane & 3;
+  int mn = INT_MAX, mx = INT_MIN;
+  for (int u = warp; u < mtiles * ngroups; u += QC_WARPS) {
+    const int ng = u / mtiles, m = u - ng * mtiles, nt = min(4, a.ntiles - ng * 4);
+    const uint8_t *x[2];
+    int pix[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      pix[e] = m * 16 + g + 8 * e;
+      const int p = min(p0 + pix[e], p1 - 1), y = p / a.OW;
+      x[e] = xs + ((size_t)(y * a.SH - iy0) * a.WI + (p - y * a.OW) * a.SW) * a.Cp;
+    }
+    const uint8_t *w = ws + (size_t)(ng * 32 + g) * a.pitch + q * 8;
+    unsigned c[4][4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) c[t][k] = 0;
+#pragma unroll 2
+    for (int ks = 0; ks < a.ksteps; ++ks) {
+      const int off = tab[ks * 4 + q];
+      const uint2 a0 = *reinterpret_cast<const uint2 *>(x[0] + off), a1 = *reinterpret_cast<const uint2 *>(x[1] + off);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const uint2 b = *reinterpret_cast<const uint2 *>(w + (size_t)(t < nt ? t : 0) * 8 * a.pitch + ks * 32);
+        mma_u8(c[t], a0, a1, b);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int o = (ng * 4 + t) * 8 + q * 2 + (k & 1), p = pix[k >> 1];
+        if (t >= nt || o >= a.OC || p >= p1 - p0) continue;
+        int v = (int)(c[t][k] - off_in * a.wsum[o] - off_f * xsum[p] + both);
+        if (a.has_bias) v += (int)a.bq[o] - smp.zero_total;
+        acc[(size_t)o * acc_step + p] = v;
+        mn = min(mn, v);
+        mx = max(mx, v);
+      }
+  }
+  mn = warp_min_i(mn);
+  mx = warp_max_i(mx);
+  if (lane == 0) {
+    amin[warp] = mn;
+    amax[warp] = mx;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    mn = warp_min_i(amin[lane & (QC_WARPS - 1)]);
+    mx = warp_max_i(amax[lane & (QC_WARPS - 1)]);
+    if (lane == 0) {
+      extremes[0] = mn;
+      extremes[1] = mx;
+    }
+  }
+  q_cluster_sync(nc);
+  if (tid == 0) {
+    for (int r = 0; r < nc && nc > 1; ++r) {
+      mn = min(mn, (int)q_remote(&extremes[0], r));
+      mx = max(mx, (int)q_remote(&extremes[1], r));
+    }
+    smp.acc_min = mn;
+    smp.acc_max = mx;
+    requant_params(smp);
+  }
+  q_cluster_sync(nc);  // nobody leaves while others may read its extremes
+  const QSample s = smp;
+  if (tid < 256) lut[tid] = q2f<8>(tid, s.min_new, s.max_new);
+  __syncthreads();
+  float *out = a.out + (size_t)n * a.OC * npix + p0;
+  const int count = p1 - p0;
+  for (int i = tid; i < a.OC * count; i += QC_THREADS) {
+    const int o = i / count, p = i - o * count;
+    out[(size_t)o * npix + p] = lut[requant_one(acc[(size_t)o * acc_step + p], s)];
+  }
+}
+
+// ---- 5c. fully connected ----------------------------------------------------------------------------
+//
+// Four launches: ranges of the samples and of the filter (B + `wblocks` blocks), quantizing (the filter transposed to
+// [out][in]), the byte products (tensor cores as above; tiles of 64 samples x 64 outputs, the inputs dealt to
+// enough blocks to fill the chip, whole-number sums added in any order), and a sample's requantizing by one block.
+// In nine launches 9216 -> 256 of 128 samples took 64 us, now 39 us; what is left is reading the filter twice
+// and the gaps between the launches.
+__global__ void __launch_bounds__(256) q_fc_range_kernel(const float *__restrict__ in, int in_size, int B,
+                                                         const float *__restrict__ W, size_t lenW, int out_size, QSample *qs,
+                                                         float *__restrict__ part, int *__restrict__ acc,
+                                                         unsigned *__restrict__ wsum) {
+  const bool row = (int)blockIdx.x < B;
+  const int w = blockIdx.x - B, nw = gridDim.x - B;
+  const float *v = row ? in + (size_t)blockIdx.x * in_size : W;
+  const size_t len = row ? (size_t)in_size : lenW;
+  const size_t first = row ? threadIdx.x : (size_t)w * 256 + threadIdx.x, step = row ? 256 : (size_t)nw * 256;
+  float mn = v[0], mx = v[0];
+  if (((uintptr_t)v & 15) == 0) {
+    const float4 *v4 = reinterpret_cast<const float4 *>(v);
+#pragma unroll 4
+    for (size_t i = first; i < len / 4; i += step) {
+      const float4 x = v4[i];
+      mn = fminf(fminf(fminf(mn, x.x), fminf(x.y, x.z)), x.w);
+      mx = fmaxf(fmaxf(fmaxf(mx, x.x), fmaxf(x.y, x.z)), x.w);
+    }
+    for (size_t i = len / 4 * 4 + first; i < len; i += step) {
+      mn = fminf(mn, v[i]);
+      mx = fmaxf(mx, v[i]);
+    }
+  } else {
+#pragma unroll 4
+    for (size_t i = first; i < len; i += step) {
+      mn = fminf(mn, v[i]);
+      mx = fmaxf(mx, v[i]);
+    }
+  }
+  __shared__ float smn[8], smx[8];
+  mn = warp_min(mn);
+  mx = warp_max(mx);
+  if ((threadIdx.x & 31) == 0) {
+    smn[threadIdx.x >> 5] = mn;
+    smx[threadIdx.x >> 5] = mx;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    mn = warp_min(smn[threadIdx.x & 7]);
+    mx = warp_max(smx[threadIdx.x & 7]);
+    if (threadIdx.x == 0) {
+      if (row) {
+        qs[blockIdx.x].min_in = mn;
+        qs[blockIdx.x].max_in = mx;
+        qs[blockIdx.x].sum_in = 0;
+      } else {
+        part[2 * w] = mn;
+        part[2 * w + 1] = mx;
+      }
+    }
+  }
+  if (row)
+    for (int i = threadIdx.x; i < out_size; i += 256) acc[(size_t)blockIdx.x * out_size + i] = 0;
+  else if (w == 0)
+    for (int i = threadIdx.x; i < out_size; i += 256) wsum[i] = 0u;
+}
+
+// blocks [0, B * rblocks): 1024 bytes of a sample's row; behind them 32 outputs x 256 inputs of the filter each
+__global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restrict__ in, int in_size, int B, int pitch,
+                                                            int rblocks, const float *__restrict__ W, int out_size,
+                                                            const float *__restrict__ bias, int nbias,
+                                                            const float *__restrict__ part, int nparts, QSample *qs,
+                                                            QGlobal *out_qg, uint8_t *__restrict__ inq,
+                                                            uint8_t *__restrict__ Wt, uint8_t *__restrict__ bq,
+                                                            unsigned *__restrict__ wsum) {
+  if ((int)blockIdx.x < B * rblocks) {
+    const int n = blockIdx.x / rblocks, j0 = (blockIdx.x - n * rblocks) * 1024 + threadIdx.x * 4;
+    const float *r = in + (size_t)n * in_size;
+    QScale q;
+    q.set(qs[n].min_in, qs[n].max_in);
+    int sum = 0;
+    if (j0 < pitch) {  // pitch is a multiple of 4
+      unsigned w = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const unsigned v = j0 + k < in_size ? q.of(r[j0 + k]) : 0u;
+        w |= v << (8 * k);
+        sum += (int)v;
+      }
+      *reinterpret_cast<unsigned *>(inq + (size_t)n * pitch + j0) = w;
+    }
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&qs[n].sum_in, sum);
+    return;
+  }
+  __shared__ QGlobal qg;
+  __shared__ uint8_t tile[256][36];
+  // the partial results stand in for the filter: same extremes, and when all are equal so is W[0]
+  filter_range(part, 1, 0, (size_t)2 * nparts, bias, nbias, qg);
+  const int b = blockIdx.x - B * rblocks, oblocks = (out_size + 31) / 32;
+  const int i0 = b % oblocks * 32, c0 = b / oblocks * 256, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (b == 0) {
+    if (threadIdx.x == 0) *out_qg = qg;
+    for (int j = threadIdx.x; j < nbias; j += 256) bq[j] = (uint8_t)f2q<8>(bias[j], qg.min_b, qg.max_b);
+  }
+  QScale q;
+  q.set(qg.min_f, qg.max_f);
+  unsigned sum = 0;
+#pragma unroll 8
+  for (int j = warp; j < 256; j += 8) {
+    const int c = c0 + j, i = i0 + lane;
+    const unsigned v = c < in_size && i < out_size ? q.of(W[(size_t)c * out_size + i]) : 0u;
+    tile[j][lane] = (uint8_t)v;
+    sum += v;
+  }
+  if (i0 + lane < out_size && sum) atomicAdd(&wsum[i0 + lane], sum);
+  __syncthreads();
+  // a warp writes rows of 256 bytes, a lane 8 bytes of each
+  for (int r = warp; r < 32; r += 8) {
+    if (i0 + r >= out_size) break;
+    uint2 v;
+    unsigned char *d = reinterpret_cast<unsigned char *>(&v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) d[k] = tile[lane * 8 + k][r];
+    if (c0 + lane * 8 < pitch) *reinterpret_cast<uint2 *>(Wt + (size_t)(i0 + r) * pitch + c0 + lane * 8) = v;
+  }
+}
+
+constexpr int QF_K = 512;  // bytes of a row in shared memory at a time; pitch 544: rows on different banks
+__global__ void __launch_bounds__(256) q_fc_gemm_kernel(int B, int out_size, int pitch, int per,
+                                                        const uint8_t *__restrict__ inq, const uint8_t *__restrict__ Wt,
+                                                        int *__restrict__ acc) {
+  extern __shared__ __align__(16) uint8_t qsm[];
+  constexpr int ROW = QF_K + 32;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64, k0 = blockIdx.z * per, k1 = min(pitch, k0 + per);
+  uint8_t *xs = qsm, *ws = xs + 64 * ROW;
+  unsigned c[4][4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[t][k] = 0;
+  const uint8_t *xa = xs + ((warp >> 1) * 16 + g) * ROW + q * 8, *wb = ws + ((warp & 1) * 32 + g) * ROW + q * 8;
+  for (int kb = k0; kb < k1; kb += QF_K) {
+    for (int i = tid; i < 128 * (QF_K / 16); i += 256) {
+      const int r = i / (QF_K / 16), at = i % (QF_K / 16) * 16, k = kb + at;
+      const bool x = r < 64;
+      const int row = x ? m0 + r : n0 + r - 64;
+      const bool ok = row < (x ? B : out_size) && k < k1;
+      cp_async16((x ? xs : ws) + (size_t)(r & 63) * ROW + at, (x ? inq : Wt) + (ok ? (size_t)row * pitch + k : 0), ok);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    const int steps = (min(k1 - kb, QF_K) + 31) / 32;
+#pragma unroll 4
+    for (int ks = 0; ks < steps; ++ks) {
+      const uint2 a0 = *reinterpret_cast<const uint2 *>(xa + ks * 32), a1 = *reinterpret_cast<const uint2 *>(xa + 8 * ROW + ks * 32);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) mma_u8(c[t], a0, a1, *reinterpret_cast<const uint2 *>(wb + t * 8 * ROW + ks * 32));
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int n = m0 + (warp >> 1) * 16 + g + (k >> 1) * 8, o = n0 + (warp & 1) * 32 + t * 8 + q * 2 + (k & 1);
+      if (n < B && o < out_size) atomicAdd(&acc[(size_t)n * out_size + o], (int)c[t][k]);
+    }
+}
+
+__global__ void __launch_bounds__(256) q_fc_requant_kernel(int in_size, int out_size, int has_bias,
+                                                           const int *__restrict__ acc, const QSample *__restrict__ qs,
+                                                           const QGlobal *__restrict__ qg, const unsigned *__restrict__ wsum,
+                                                           const uint8_t *__restrict__ bq, float *__restrict__ out) {
+  __shared__ QSample s;
+  __shared__ int smn[8], smx[8];
+  const int n = blockIdx.x, tid = threadIdx.x;
+  const unsigned sum_in = (unsigned)qs[n].sum_in;
+  if (tid == 0) {
+    s = qs[n];
+    sample_params(s, *qg, 1);
+  }
+  __syncthreads();
+  const unsigned off_f = (unsigned)qg->off_f, off_in = (unsigned)s.off_in;
+  const unsigned both = (unsigned)in_size * off_f * off_in - off_f * sum_in;
+  const int zero = s.zero_total;
+  auto value = [&](int i) {
+    int v = (int)((unsigned)acc[(size_t)n * out_size + i] - off_in * wsum[i] + both);
+    return has_bias ? v + (int)bq[i] - zero : v;
+  };
+  int mn = INT_MAX, mx = INT_MIN;
+  for (int i = tid; i < out_size; i += 256) {
+    const int v = value(i);
+    mn = min(mn, v);
+    mx = max(mx, v);
+  }
+  mn = warp_min_i(mn);
+  mx = warp_max_i(mx);
+  if ((tid & 31) == 0) {
+    smn[tid >> 5] = mn;
+    smx[tid >> 5] = mx;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    for (int k = 1; k < 8; ++k) mn = min(mn, smn[k]), mx = max(mx, smx[k]);
+    s.acc_min = mn;
+    s.acc_max = mx;
+    requant_params(s);
+  }
+  __syncthreads();
+  const QSample t = s;
+  for (int i = tid; i < out_size; i += 256) out[(size_t)n * out_size + i] = q2f<8>(requant_one(value(i), t), t.min_new, t.max_new);
 }
 
 // ---- 7. the forms for chained quantized layers ("eq") -----------------------------------------
@@ -741,17 +946,9 @@ __global__ void q_requant_u8_kernel(const int *__restrict__ acc, size_t out_len,
   const QSample s = qs[n];
   const int *a = acc + (size_t)n * out_len;
   float *o = out + (size_t)n * out_len;
-  const long long rounding_delta = 1LL << 15;
   size_t step = (size_t)gridDim.x * blockDim.x;
-  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < out_len; j += step) {
-    long long v = (long long)a[j];
-    long long fp_value = ((v * s.range_scale_fp) >> 32) + s.input_offset_fp;
-    long long ri = ((fp_value >= 0) ? (fp_value + rounding_delta) : (fp_value - rounding_delta)) >> 16;
-    long long q = ri - s.output_offset_fp;
-    q = q > 0 ? q : 0;
-    q = q < 255 ? q : 255;
-    o[j] = (float)q;
-  }
+  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < out_len; j += step)
+    o[j] = (float)requant_one(a[j], s);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     out_r[2 * n] = s.min_new;
     out_r[2 * n + 1] = s.max_new;
@@ -800,12 +997,6 @@ static int q_carve(b200_ctx *ctx, int B, size_t in_len, size_t lenW, size_t nbia
   return 0;
 }
 
-// shared memory of q_conv_acc_dp4a_kernel: the quantized filter and one byte sum per output channel
-static size_t qconv_dp4a_smem(const ConvGeom &g) {
-  size_t words = (size_t)g.OC * g.KH * g.KW * g.C / 4;
-  return ((words + 3) / 4 * 4 + g.OC) * 4;
-}
-
 int qconv_fwd(b200_ctx *ctx, const b200_conv_desc *d, const float *in, const float *W,
               const float *bias, float *out, int B) {
   b200_conv_desc dd = *d;
@@ -827,56 +1018,76 @@ int qconv_fwd(b200_ctx *ctx, const b200_conv_desc *d, const float *in, const flo
   B200_REQUIRE((size_t)(g.C - 1) * plane + (size_t)g.KH * g.KH <= lenW,
                "quantized convolution: the reference's filter range scan leaves the filter "
                "tensor for this shape");
+  cudaStream_t st = ctx->stream;
+  const int nbias = g.has_bias ? g.OC : 0;
+  if (!g.tbl) {
+    QConvArgs a = {};
+    a.in = in, a.out = out;
+    a.C = g.C, a.HI = g.HI, a.WI = g.WI, a.OC = g.OC, a.OH = g.OH, a.OW = g.OW;
+    a.KH = g.KH, a.KW = g.KW, a.SH = g.SH, a.SW = g.SW, a.has_bias = g.has_bias;
+    a.Cp = (g.C + 7) / 8 * 8;
+    a.ksteps = (g.KH * g.KW * a.Cp + 31) / 32;
+    a.pitch = qc_pitch(a.ksteps);
+    a.ntiles = (g.OC + 7) / 8;
+    const int npix = g.OH * g.OW;
+    // blocks of a sample: as many as leave every sample a place; more where the rows of one do not fit
+    int nc = 8;
+    while (nc > 1 && (long long)B * nc > ctx->sm_count) nc /= 2;
+    size_t smem = 0;
+    for (; nc <= 8; nc *= 2) {
+      a.per = (ceil_div(npix, nc) + 15) / 16 * 16;
+      const int rows = (a.per + g.OW - 2) / g.OW * g.SH + g.KH;  // a run of `per` pixels needs at most that many
+      a.rows = rows < g.HI ? rows : g.HI;
+      smem = (size_t)a.ntiles * 8 * a.pitch + (size_t)a.rows * g.WI * a.Cp +
+             4 * ((size_t)a.ksteps * 4 + (size_t)a.rows * g.WI + a.per);
+      const size_t with_acc = smem + 4 * (size_t)g.OC * a.per;
+      a.acc_smem = with_acc + 4096 <= ctx->smem_optin;  // beside the kernel's own shared variables
+      if (a.acc_smem) smem = with_acc;
+      if (smem + 4096 <= ctx->smem_optin) break;
+    }
+    if (nc <= 8) {
+      QScratch s;
+      B200_TRY(q_carve(ctx, 1, 0, (size_t)a.ntiles * 8 * a.pitch, g.OC, (size_t)a.ntiles * 8, &s));
+      unsigned *wsum = reinterpret_cast<unsigned *>(s.acc);
+      q_conv_filter_kernel<<<a.ntiles * 8, 256, 0, st>>>(W, g.C, plane, (size_t)g.KH * g.KH, g.C, a.Cp, g.OC, g.KH * g.KW,
+                                                        a.pitch, bias, nbias, s.qg, s.Wq, s.bq, wsum);
+      B200_LAUNCHED();
+      a.Wq = s.Wq, a.bq = s.bq, a.wsum = wsum, a.qg = s.qg;
+      B200_CUDA(cudaFuncSetAttribute(q_conv_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      cudaLaunchConfig_t c = {};
+      c.gridDim = dim3((unsigned)(B * nc));
+      c.blockDim = dim3(QC_THREADS);
+      c.dynamicSmemBytes = smem;
+      c.stream = st;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = (unsigned)nc;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      c.attrs = at;
+      c.numAttrs = 1;
+      B200_CUDA(cudaLaunchKernelEx(&c, q_conv_fused_kernel, a));
+      B200_LAUNCHED();
+      return 0;
+    }
+  }
+  // with a connection table, or a filter that does not fit shared memory
   QScratch s;
   B200_TRY(q_carve(ctx, B, in_len, lenW, g.OC, out_len, &s));
-  cudaStream_t st = ctx->stream;
-  // channel-fastest operands and dp4a when every window position is connected
-  const size_t smem = qconv_dp4a_smem(g);
-  const bool fast = !g.tbl && g.C % 4 == 0 && smem <= 200 * 1024;
   q_input_range_kernel<<<B, 1024, 0, st>>>(in, in_len, g.C, plane, (size_t)g.HI * g.HI, s.qs);
   B200_LAUNCHED();
-  q_filter_range_kernel<<<1, 256, 0, st>>>(W, g.C, plane, (size_t)g.KH * g.KH, bias,
-                                          g.has_bias ? g.OC : 0, s.qg);
+  q_filter_range_kernel<<<1, 256, 0, st>>>(W, g.C, plane, (size_t)g.KH * g.KH, bias, nbias, s.qg);
   B200_LAUNCHED();
-  if (fast)
-    q_quantize_filter_otc_kernel<<<blocks_for(lenW, 256), 256, 0, st>>>(
-      W, g.C, g.OC, g.KH * g.KW, bias, g.has_bias ? g.OC : 0, s.qg, s.Wq, s.bq);
-  else
-    q_quantize_filter_kernel<<<blocks_for(lenW, 256), 256, 0, st>>>(W, lenW, bias,
-                                                                    g.has_bias ? g.OC : 0, s.qg,
-                                                                    s.Wq, s.bq);
+  q_quantize_filter_kernel<<<blocks_for(lenW, 256), 256, 0, st>>>(W, lenW, bias, nbias, s.qg, s.Wq, s.bq);
   B200_LAUNCHED();
   q_sample_params_kernel<<<ceil_div(B, 128), 128, 0, st>>>(s.qs, s.qg, B, 0);
   B200_LAUNCHED();
-  if (fast) {
-    q_quantize_input_nhwc_kernel<<<dim3(blocks_for(in_len / 4, 256), B), 256, 0, st>>>(
-      in, g.C, (int)plane, s.qs, s.inq);
-    B200_LAUNCHED();
-    static bool attr_set = false;
-    if (!attr_set) {
-      B200_CUDA(cudaFuncSetAttribute(q_conv_acc_dp4a_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     200 * 1024));
-      B200_CUDA(cudaFuncSetAttribute(q_conv_acc_dp4a_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     200 * 1024));
-      attr_set = true;
-    }
-    dim3 grid(ceil_div(g.OH * g.OW, QCV_PIX), B);
-    if (g.C % 16 == 0)
-      q_conv_acc_dp4a_kernel<true><<<grid, 256, smem, st>>>(g, s.inq, s.Wq, s.bq, s.qg, s.qs, s.acc);
-    else
-      q_conv_acc_dp4a_kernel<false><<<grid, 256, smem, st>>>(g, s.inq, s.Wq, s.bq, s.qg, s.qs, s.acc);
-  } else {
-    q_quantize_input_kernel<<<dim3(blocks_for(in_len, 256), B), 256, 0, st>>>(in, in_len, s.qs,
-                                                                             s.inq);
-    B200_LAUNCHED();
-    q_conv_acc_kernel<<<dim3(blocks_for(out_len, 256), B), 256, 0, st>>>(g, s.inq, s.Wq, s.bq,
-                                                                        s.qg, s.qs, s.acc, nullptr);
-  }
+  q_quantize_input_kernel<<<dim3(blocks_for(in_len, 256), B), 256, 0, st>>>(in, in_len, s.qs, s.inq);
+  B200_LAUNCHED();
+  q_conv_acc_kernel<<<dim3(blocks_for(out_len, 256), B), 256, 0, st>>>(g, s.inq, s.Wq, s.bq, s.qg, s.qs, s.acc, nullptr);
   B200_LAUNCHED();
   q_requant_params_kernel<<<ceil_div(B, 128), 128, 0, st>>>(s.qs, B);
   B200_LAUNCHED();
-  q_requant_dequant_kernel<<<dim3(blocks_for(out_len, 256), B), 256, 0, st>>>(s.acc, out_len, s.qs,
-                                                                             out);
+  q_requant_dequant_kernel<<<dim3(blocks_for(out_len, 256), B), 256, 0, st>>>(s.acc, out_len, s.qs, out);
   B200_LAUNCHED();
   return 0;
 }
@@ -887,33 +1098,30 @@ int qfc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const flo
   if (B == 0) return 0;
   const size_t lenW = (size_t)in_size * out_size;
   const int nbias = bias ? out_size : 0;
-  const int pitch = (in_size + 15) / 16 * 16;  // bytes per quantized row, zero padded
+  const int pitch = (in_size + 31) / 32 * 32;  // bytes per quantized row, zero padded
   QScratch s;
-  B200_TRY(q_carve(ctx, B, pitch, (size_t)pitch * out_size, out_size, out_size, &s));
+  B200_TRY(q_carve(ctx, B, pitch, (size_t)pitch * out_size, out_size, (size_t)out_size + ceil_div(out_size, B), &s));
+  unsigned *wsum = reinterpret_cast<unsigned *>(s.acc + (size_t)B * out_size);
   cudaStream_t st = ctx->stream;
-  q_input_range_kernel<<<B, 1024, 0, st>>>(in, in_size, 1, 0, in_size, s.qs);
+  int wblocks = blocks_for(lenW, 4096);
+  if (wblocks > Q_PART_BLOCKS) wblocks = Q_PART_BLOCKS;
+  q_fc_range_kernel<<<B + wblocks, 256, 0, st>>>(in, in_size, B, W, lenW, out_size, s.qs, s.part, s.acc, wsum);
   B200_LAUNCHED();
-  int pblocks = blocks_for(lenW, 1024);
-  if (pblocks > Q_PART_BLOCKS) pblocks = Q_PART_BLOCKS;
-  q_minmax_partial_kernel<<<pblocks, 1024, 0, st>>>(W, lenW, s.part);
+  const int rblocks = ceil_div(pitch, 1024), fblocks = ceil_div(out_size, 32) * ceil_div(pitch, 256);
+  q_fc_quantize_kernel<<<B * rblocks + fblocks, 256, 0, st>>>(in, in_size, B, pitch, rblocks, W, out_size, bias, nbias, s.part,
+                                                             wblocks, s.qs, s.qg, s.inq, s.Wq, s.bq, wsum);
   B200_LAUNCHED();
-  // the partial results stand in for the filter: same extremes, and when all are equal so is W[0]
-  q_filter_range_kernel<<<1, 1024, 0, st>>>(s.part, 1, 0, (size_t)2 * pblocks, bias, nbias, s.qg);
+  // the inputs dealt out so that two blocks an SM have work, 128 bytes at least
+  const int tiles = ceil_div(out_size, 64) * ceil_div(B, 64);
+  int splits = ceil_div(2 * ctx->sm_count, tiles);
+  if (splits > ceil_div(pitch, 128)) splits = ceil_div(pitch, 128);
+  const int per = (ceil_div(pitch, splits) + 31) / 32 * 32;
+  constexpr int gemm_smem = 128 * (QF_K + 32);
+  B200_CUDA(cudaFuncSetAttribute(q_fc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem));
+  q_fc_gemm_kernel<<<dim3(ceil_div(out_size, 64), ceil_div(B, 64), ceil_div(pitch, per)), 256, gemm_smem, st>>>(
+    B, out_size, pitch, per, s.inq, s.Wq, s.acc);
   B200_LAUNCHED();
-  q_quantize_filter_t_kernel<<<dim3(ceil_div(out_size, 32), ceil_div(pitch, 32)), dim3(32, 8), 0, st>>>(
-    W, in_size, out_size, pitch, bias, nbias, s.qg, s.Wq, s.bq);
-  B200_LAUNCHED();
-  q_sample_params_kernel<<<ceil_div(B, 128), 128, 0, st>>>(s.qs, s.qg, B, 1);
-  B200_LAUNCHED();
-  q_quantize_input_pitch_kernel<<<dim3(ceil_div(pitch, 1024), B), 256, 0, st>>>(in, in_size, pitch, s.qs, s.inq);
-  B200_LAUNCHED();
-  q_fc_acc_dp4a_kernel<<<dim3(ceil_div(out_size, 4 * QFC_OUTS), ceil_div(B, QFC_SAMPLES)), 128, 0, st>>>(
-    in_size, out_size, pitch, nbias > 0, B, s.inq, s.Wq, s.bq, s.qg, s.qs, s.acc);
-  B200_LAUNCHED();
-  q_requant_params_kernel<<<ceil_div(B, 128), 128, 0, st>>>(s.qs, B);
-  B200_LAUNCHED();
-  q_requant_dequant_kernel<<<dim3(blocks_for(out_size, 256), B), 256, 0, st>>>(s.acc, out_size,
-                                                                              s.qs, out);
+  q_fc_requant_kernel<<<B, 256, 0, st>>>(in_size, out_size, nbias > 0, s.acc, s.qs, s.qg, wsum, s.bq, out);
   B200_LAUNCHED();
   return 0;
 }
