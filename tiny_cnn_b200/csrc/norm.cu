@@ -32,15 +32,111 @@ __device__ __forceinline__ float block_sum_all(float v) {
   return v;
 }
 
-// the slices of channel c added in slice order (every block gets the same bits)
-__device__ __forceinline__ float add_slices(const float *part, int c, int slices) {
+// the slices' results of channel c, fetched side by side (one after the other they cost a block 6 us)
+struct Slices {
+  float a[64], b[64];
+  __device__ __forceinline__ void fetch(const float *pa, const float *pb, int c, int C, int slices) {
+    if ((int)threadIdx.x < slices) {
+      a[threadIdx.x] = pa[(size_t)threadIdx.x * C + c];
+      b[threadIdx.x] = pb[(size_t)threadIdx.x * C + c];
+    }
+    __syncthreads();
+  }
+};
+// added in slice order (every block gets the same bits)
+__device__ __forceinline__ float add_slices(const float *part, int slices) {
   float s = 0.f;
-  for (int z = 0; z < slices; ++z) s += part[(size_t)z * gridDim.x + c];
+  for (int z = 0; z < slices; ++z) s += part[z];
   return s;
 }
 
-// pass 1 of moments() (tiny_dnn/util/math_functions.h:25-37): per (channel, batch slice) the sum of x
-// (two inputs: also the sum of x*y, for the backward pass)
+// Every value, or 16-byte piece (S4 of them a map), of channel c in the samples n0 .. n1 - 1: f(its index).  One loop over all of them, so
+// that a thread has several loads on the way; a loop per sample had one (256 samples of 64 maps of 32x32: 29 us for
+// the 67 MB of a forward sum).
+template <typename F>
+__device__ __forceinline__ void pieces_of(int c, int C, int S4, int n0, int n1, F f) {
+  const unsigned total = (unsigned)(n1 - n0) * (unsigned)S4;
+  const size_t base = ((size_t)n0 * C + c) * S4, skip = (size_t)(C - 1) * S4;
+#pragma unroll 8
+  for (unsigned i = threadIdx.x; i < total; i += BN_THREADS) f(base + i + (i / (unsigned)S4) * skip);
+}
+
+// The same for a pass that also stores: `load` fetches the operands of four pieces before `store` writes the first,
+// because the compiler may not move a load past a store on its own.
+template <typename V, typename Load, typename Store>
+__device__ __forceinline__ void pieces_map(int c, int C, int S4, int n0, int n1, Load load, Store store) {
+  const unsigned total = (unsigned)(n1 - n0) * (unsigned)S4;
+  const size_t base = ((size_t)n0 * C + c) * S4, skip = (size_t)(C - 1) * S4;
+  for (unsigned i = threadIdx.x; i < total; i += 4 * BN_THREADS) {
+    V v[4];
+    size_t at[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const unsigned k = min(i + u * BN_THREADS, total - 1);
+      at[u] = base + k + (k / (unsigned)S4) * skip;
+      v[u] = load(at[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * BN_THREADS < total) store(at[u], v[u]);
+  }
+}
+
+// moments() (tiny_dnn/util/math_functions.h:25-61) in one pass: per (channel, batch slice) the mean and the sum of
+// (x - mean)^2.  Values are taken relative to a rough mean (of four of the slice's first map), and each thread's sum
+// of squares is reduced to its own mean before it is combined, so nothing large is subtracted.
+__global__ void __launch_bounds__(BN_THREADS) bn_moments_kernel(const float *__restrict__ x, int S, int B,
+                                                                float *__restrict__ part_m, float *__restrict__ part_v,
+                                                                int vec4) {
+  const int c = blockIdx.x, C = gridDim.x, z = blockIdx.y, Z = gridDim.y;
+  const int n0 = (int)((long long)B * z / Z), n1 = (int)((long long)B * (z + 1) / Z);
+  const float *head = x + ((size_t)n0 * C + c) * S;
+  const float rough = 0.25f * ((head[0] + head[S / 4]) + (head[S / 2] + head[S - 1]));
+  float s1 = 0.f, s2 = 0.f;
+  int count;  // values of this thread
+  const unsigned pieces = (unsigned)(n1 - n0) * (unsigned)(vec4 ? S / 4 : S);
+  count = pieces > threadIdx.x ? (int)((pieces - threadIdx.x + BN_THREADS - 1) / BN_THREADS) * (vec4 ? 4 : 1) : 0;
+  if (vec4) {
+    const float4 *x4 = reinterpret_cast<const float4 *>(x);
+    pieces_of(c, C, S / 4, n0, n1, [&](size_t i) {
+      const float4 v = x4[i];
+      const float a = v.x - rough, b = v.y - rough, e = v.z - rough, f = v.w - rough;
+      s1 += (a + b) + (e + f);
+      s2 += (a * a + b * b) + (e * e + f * f);
+    });
+  } else {
+    pieces_of(c, C, S, n0, n1, [&](size_t i) {
+      const float d = x[i] - rough;
+      s1 += d;
+      s2 += d * d;
+    });
+  }
+  const float mine = count ? s1 / (float)count : 0.f, m2 = count ? fmaxf(0.f, s2 - s1 * mine) : 0.f;
+  const float mean = block_sum_all(s1) / ((float)(n1 - n0) * (float)S), off = mine - mean;
+  const float var = block_sum_all(m2 + (float)count * off * off);
+  if (threadIdx.x == 0) {
+    part_m[(size_t)z * C + c] = rough + mean;
+    part_v[(size_t)z * C + c] = var;
+  }
+}
+
+// mean and sum of (x - mean)^2 of channel c over all slices, in slice order (every block gets the same bits)
+__device__ __forceinline__ void merge_slices(const Slices &p, int S, int B, int slices, float *mean_out, float *sq_out) {
+  auto samples = [&](int z) { return (float)((int)((long long)B * (z + 1) / slices) - (int)((long long)B * z / slices)); };
+  const float base = p.a[0];
+  float s = 0.f;
+  for (int z = 1; z < slices; ++z) s += samples(z) * (p.a[z] - base);
+  const float mean = base + s / (float)B;
+  float v = 0.f;
+  for (int z = 0; z < slices; ++z) {
+    const float off = p.a[z] - mean;
+    v += p.b[z] + samples(z) * (float)S * off * off;
+  }
+  *mean_out = mean;
+  *sq_out = v;
+}
+
+// backward: per (channel, batch slice) the sums of dy and of dy * y
 __global__ void __launch_bounds__(BN_THREADS) bn_sum_kernel(const float *__restrict__ x, const float *__restrict__ y,
                                                             int S, int B, float *__restrict__ part_x,
                                                             float *__restrict__ part_xy, int vec4) {
@@ -48,65 +144,25 @@ __global__ void __launch_bounds__(BN_THREADS) bn_sum_kernel(const float *__restr
   const int n0 = (int)((long long)B * z / Z), n1 = (int)((long long)B * (z + 1) / Z);
   float sx = 0.f, sxy = 0.f;
   if (vec4) {  // 16-byte loads: S a multiple of 4 and the tensors 16-byte aligned (checked by the launcher)
-    for (int n = n0; n < n1; ++n) {
-      const size_t base = ((size_t)n * C + c) * S;
-      const float4 *x4 = reinterpret_cast<const float4 *>(x + base);
-      const float4 *y4 = y != nullptr ? reinterpret_cast<const float4 *>(y + base) : nullptr;
-      for (int k = threadIdx.x; k < S / 4; k += BN_THREADS) {
-        const float4 v = x4[k];
-        sx += (v.x + v.y) + (v.z + v.w);
-        if (y4 != nullptr) {
-          const float4 w = y4[k];
-          sxy += (v.x * w.x + v.y * w.y) + (v.z * w.z + v.w * w.w);
-        }
-      }
-    }
+    const float4 *x4 = reinterpret_cast<const float4 *>(x), *y4 = reinterpret_cast<const float4 *>(y);
+    pieces_of(c, C, S / 4, n0, n1, [&](size_t i) {
+      const float4 v = x4[i], w = y4[i];
+      sx += (v.x + v.y) + (v.z + v.w);
+      sxy += (v.x * w.x + v.y * w.y) + (v.z * w.z + v.w * w.w);
+    });
   } else {
-    for (int n = n0; n < n1; ++n) {
-      const size_t base = ((size_t)n * C + c) * S;
-      for (int k = threadIdx.x; k < S; k += BN_THREADS) {
-        const float v = x[base + k];
-        sx += v;
-        if (y != nullptr) sxy += v * y[base + k];
-      }
-    }
+    pieces_of(c, C, S, n0, n1, [&](size_t i) {
+      const float v = x[i];
+      sx += v;
+      sxy += v * y[i];
+    });
   }
   sx = block_sum_all(sx);
-  if (y != nullptr) sxy = block_sum_all(sxy);
+  sxy = block_sum_all(sxy);
   if (threadIdx.x == 0) {
     part_x[(size_t)z * C + c] = sx;
-    if (y != nullptr) part_xy[(size_t)z * C + c] = sxy;
+    part_xy[(size_t)z * C + c] = sxy;
   }
-}
-
-// pass 2 (math_functions.h:39-61): per (channel, batch slice) the sum of (x - mean)^2
-__global__ void __launch_bounds__(BN_THREADS) bn_var_kernel(const float *__restrict__ x, int S, int B, int slices,
-                                                            const float *__restrict__ part_x,
-                                                            float *__restrict__ part_v, int vec4) {
-  const int c = blockIdx.x, C = gridDim.x, z = blockIdx.y, Z = gridDim.y;
-  const float mean = __fdiv_rn(add_slices(part_x, c, slices), (float)B * (float)S);
-  const int n0 = (int)((long long)B * z / Z), n1 = (int)((long long)B * (z + 1) / Z);
-  float sv = 0.f;
-  if (vec4) {
-    for (int n = n0; n < n1; ++n) {
-      const float4 *x4 = reinterpret_cast<const float4 *>(x + ((size_t)n * C + c) * S);
-      for (int k = threadIdx.x; k < S / 4; k += BN_THREADS) {
-        const float4 v = x4[k];
-        const float a = v.x - mean, b = v.y - mean, e = v.z - mean, f = v.w - mean;
-        sv += (a * a + b * b) + (e * e + f * f);
-      }
-    }
-  } else {
-    for (int n = n0; n < n1; ++n) {
-      const size_t base = ((size_t)n * C + c) * S;
-      for (int k = threadIdx.x; k < S; k += BN_THREADS) {
-        const float d = __fsub_rn(x[base + k], mean);
-        sv += __fmul_rn(d, d);
-      }
-    }
-  }
-  sv = block_sum_all(sv);
-  if (threadIdx.x == 0) part_v[(size_t)z * C + c] = sv;
 }
 
 // y = (x - mean) / sqrt(variance + eps) (batch_normalization_layer.h:136-168).  Train phase
@@ -120,8 +176,14 @@ __global__ void __launch_bounds__(BN_THREADS) bn_apply_kernel(const float *__res
   const int c = blockIdx.x, C = gridDim.x, z = blockIdx.y, Z = gridDim.y;
   float mean, var;
   if (part_x != nullptr) {
-    mean = __fdiv_rn(add_slices(part_x, c, slices), (float)B * (float)S);
-    var = __fdiv_rn(add_slices(part_v, c, slices), fmaxf(1.0f, __fsub_rn((float)((long long)B * S), 1.0f)));
+    __shared__ Slices p;
+    __shared__ float both[2];
+    p.fetch(part_x, part_v, c, C, slices);
+    if (threadIdx.x == 0) merge_slices(p, S, B, slices, &both[0], &both[1]);
+    __syncthreads();
+    mean = both[0];
+    const float sq = both[1];
+    var = __fdiv_rn(sq, fmaxf(1.0f, __fsub_rn((float)((long long)B * S), 1.0f)));
   } else {
     mean = mean_io[c];
     var = var_io[c];
@@ -136,25 +198,19 @@ __global__ void __launch_bounds__(BN_THREADS) bn_apply_kernel(const float *__res
   }
   const int n0 = (int)((long long)B * z / Z), n1 = (int)((long long)B * (z + 1) / Z);
   if (vec4) {
-    for (int n = n0; n < n1; ++n) {
-      const size_t base = ((size_t)n * C + c) * S;
-      const float4 *x4 = reinterpret_cast<const float4 *>(x + base);
-      float4 *y4 = reinterpret_cast<float4 *>(y + base);
-      for (int k = threadIdx.x; k < S / 4; k += BN_THREADS) {
-        float4 v = x4[k];
-        v.x = __fdiv_rn(__fsub_rn(v.x, mean), sd);
-        v.y = __fdiv_rn(__fsub_rn(v.y, mean), sd);
-        v.z = __fdiv_rn(__fsub_rn(v.z, mean), sd);
-        v.w = __fdiv_rn(__fsub_rn(v.w, mean), sd);
-        y4[k] = v;
-      }
-    }
+    const float4 *x4 = reinterpret_cast<const float4 *>(x);
+    float4 *y4 = reinterpret_cast<float4 *>(y);
+    pieces_map<float4>(c, C, S / 4, n0, n1, [&](size_t i) { return x4[i]; }, [&](size_t i, float4 v) {
+      v.x = __fdiv_rn(__fsub_rn(v.x, mean), sd);
+      v.y = __fdiv_rn(__fsub_rn(v.y, mean), sd);
+      v.z = __fdiv_rn(__fsub_rn(v.z, mean), sd);
+      v.w = __fdiv_rn(__fsub_rn(v.w, mean), sd);
+      y4[i] = v;
+    });
     return;
   }
-  for (int n = n0; n < n1; ++n) {
-    const size_t base = ((size_t)n * C + c) * S;
-    for (int k = threadIdx.x; k < S; k += BN_THREADS) y[base + k] = __fdiv_rn(__fsub_rn(x[base + k], mean), sd);
-  }
+  pieces_map<float>(c, C, S, n0, n1, [&](size_t i) { return x[i]; },
+                    [&](size_t i, float v) { y[i] = __fdiv_rn(__fsub_rn(v, mean), sd); });
 }
 
 // dx = (dy - mean(dy) - mean(dy*y) * y) / stddev (batch_normalization_layer.h:94-134)
@@ -165,34 +221,32 @@ __global__ void __launch_bounds__(BN_THREADS) bn_bwd_kernel(const float *__restr
                                                             const float *__restrict__ stddev, int vec4) {
   const int c = blockIdx.x, C = gridDim.x, z = blockIdx.y, Z = gridDim.y;
   const float count = (float)B * (float)S;
-  const float mean_d = __fdiv_rn(add_slices(part_d, c, slices), count);
-  const float mean_dy = __fdiv_rn(add_slices(part_dy, c, slices), count);
+  __shared__ Slices p;
+  p.fetch(part_d, part_dy, c, C, slices);
+  const float mean_d = __fdiv_rn(add_slices(p.a, slices), count);
+  const float mean_dy = __fdiv_rn(add_slices(p.b, slices), count);
   const float sd = stddev[c];
   const int n0 = (int)((long long)B * z / Z), n1 = (int)((long long)B * (z + 1) / Z);
   if (vec4) {
-    for (int n = n0; n < n1; ++n) {
-      const size_t base = ((size_t)n * C + c) * S;
-      const float4 *y4 = reinterpret_cast<const float4 *>(y + base), *g4 = reinterpret_cast<const float4 *>(dy + base);
-      float4 *d4 = reinterpret_cast<float4 *>(dx + base);
-      for (int k = threadIdx.x; k < S / 4; k += BN_THREADS) {
-        const float4 a = y4[k], g = g4[k];
-        float4 o;
-        o.x = __fdiv_rn(__fsub_rn(__fsub_rn(g.x, mean_d), __fmul_rn(mean_dy, a.x)), sd);
-        o.y = __fdiv_rn(__fsub_rn(__fsub_rn(g.y, mean_d), __fmul_rn(mean_dy, a.y)), sd);
-        o.z = __fdiv_rn(__fsub_rn(__fsub_rn(g.z, mean_d), __fmul_rn(mean_dy, a.z)), sd);
-        o.w = __fdiv_rn(__fsub_rn(__fsub_rn(g.w, mean_d), __fmul_rn(mean_dy, a.w)), sd);
-        d4[k] = o;
-      }
-    }
+    const float4 *y4 = reinterpret_cast<const float4 *>(y), *g4 = reinterpret_cast<const float4 *>(dy);
+    float4 *d4 = reinterpret_cast<float4 *>(dx);
+    struct Pair {
+      float4 a, g;
+    };
+    pieces_map<Pair>(c, C, S / 4, n0, n1, [&](size_t i) { return Pair{y4[i], g4[i]}; }, [&](size_t i, const Pair &p) {
+      const float4 a = p.a, g = p.g;
+      float4 o;
+      o.x = __fdiv_rn(__fsub_rn(__fsub_rn(g.x, mean_d), __fmul_rn(mean_dy, a.x)), sd);
+      o.y = __fdiv_rn(__fsub_rn(__fsub_rn(g.y, mean_d), __fmul_rn(mean_dy, a.y)), sd);
+      o.z = __fdiv_rn(__fsub_rn(__fsub_rn(g.z, mean_d), __fmul_rn(mean_dy, a.z)), sd);
+      o.w = __fdiv_rn(__fsub_rn(__fsub_rn(g.w, mean_d), __fmul_rn(mean_dy, a.w)), sd);
+      d4[i] = o;
+    });
     return;
   }
-  for (int n = n0; n < n1; ++n) {
-    const size_t base = ((size_t)n * C + c) * S;
-    for (int k = threadIdx.x; k < S; k += BN_THREADS) {
-      const float v = __fsub_rn(__fsub_rn(dy[base + k], mean_d), __fmul_rn(mean_dy, y[base + k]));
-      dx[base + k] = __fdiv_rn(v, sd);
-    }
-  }
+  pieces_map<float2>(c, C, S, n0, n1, [&](size_t i) { return make_float2(y[i], dy[i]); }, [&](size_t i, float2 v) {
+    dx[i] = __fdiv_rn(__fsub_rn(__fsub_rn(v.y, mean_d), __fmul_rn(mean_dy, v.x)), sd);
+  });
 }
 
 // running = momentum * running + (1 - momentum) * current (batch_normalization_layer.h:174-180)
@@ -273,9 +327,7 @@ int batchnorm_fwd(b200_ctx *ctx, int channels, int spatial, float eps, const flo
   float *part_x = scratch, *part_v = scratch + (size_t)Z * channels;
   const int vec4 = spatial % 4 == 0 && aligned16(x) && aligned16(y);
   if (train) {
-    bn_sum_kernel<<<grid, BN_THREADS, 0, ctx->stream>>>(x, nullptr, spatial, B, part_x, nullptr, vec4);
-    B200_LAUNCHED();
-    bn_var_kernel<<<grid, BN_THREADS, 0, ctx->stream>>>(x, spatial, B, Z, part_x, part_v, vec4);
+    bn_moments_kernel<<<grid, BN_THREADS, 0, ctx->stream>>>(x, spatial, B, part_x, part_v, vec4);
     B200_LAUNCHED();
   }
   bn_apply_kernel<<<grid, BN_THREADS, 0, ctx->stream>>>(x, y, spatial, B, eps, Z, train ? part_x : nullptr,
