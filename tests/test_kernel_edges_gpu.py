@@ -122,3 +122,17 @@ def test_quantized_fc_edges(ctx, oracle, n_in, n_out, B):
     assert oracle.orc_qfc_fwd(n_in, n_out, o.p(x), o.p(W), o.p(b), o.p(y), B) == 0
     got = host(ops.quantized_fully_connected(ctx, n_in, n_out, dev(x), dev(W), dev(b)))
     assert np.array_equal(got.view(np.uint32), y.view(np.uint32))
+
+
+# inputs, outputs, batch of products that go to the tensor cores: tiles of every shape, no size a multiple of one
+@pytest.mark.parametrize("n_in,n_out,B", [(1031, 515, 130), (784, 1000, 1024), (70, 8200, 257), (4096, 130, 129), (1500, 2000, 700)])
+def test_fully_connected_tensor_core_edges(ctx, n_in, n_out, B):
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x, dy = torch.randn(B, n_in, device="cuda", generator=g), torch.randn(B, n_out, device="cuda", generator=g)
+    W, b = torch.randn(n_in, n_out, device="cuda", generator=g), torch.randn(n_out, device="cuda", generator=g)
+    y = ops.fully_connected_op(ctx, n_in, n_out, x, W.view(-1), b)
+    dx, dW, db = ops.fully_connected_grad_op(ctx, n_in, n_out, x, W.view(-1), dy)
+    xd, Wd, dd = x.double(), W.double(), dy.double()
+    for got, want, name in ((y, xd @ Wd + b.double(), "y"), (dx, dd @ Wd.T, "dx"), (dW.view(n_in, n_out), xd.T @ dd, "dW"),
+                            (db, dd.sum(0), "db")):
+        assert float((got.double() - want).norm() / want.norm()) < 2e-5, name

@@ -205,8 +205,8 @@ int merge_rows(b200_ctx *ctx, const float *src, int rows, size_t stride, float *
 // ----------------------------------------------------------------------------
 // other ops
 // ----------------------------------------------------------------------------
-// tensor-core GEMM (gemm_tc.cu): D[M][N] (+)= A * Bt^T, operands split into TF32 hi/lo
-// pairs in `scratch` (gemm_tc_scratch_floats floats)
+// tensor-core GEMM (gemm_tc.cu): D[M][N] (+)= A * Bt^T, operands split into three bf16
+// parts in `scratch` (gemm_tc_scratch_floats floats)
 size_t gemm_tc_scratch_floats(int M, int N, int K);
 int gemm_tc(b200_ctx *ctx, int M, int N, int K, const float *src_a, long long lda, bool a_transposed,
             const float *src_b, long long ldb, bool b_transposed, float *D, const float *bias,

@@ -1,69 +1,64 @@
-// FP32-accurate GEMM on the 5th-generation tensor cores (tcgen05) by the 3xTF32
-// split: every fp32 operand x is written as hi + lo with hi = x truncated to
-// TF32 and lo = x - hi (exact), and
-//     A*B ~= A_lo*B_hi + A_hi*B_lo + A_hi*B_hi      (the lo*lo term, ~2^-22 relative, is dropped)
-// is accumulated in fp32 in tensor memory.  Used for the large fully-connected
+// FP32-accurate GEMM on the 5th-generation tensor cores (tcgen05).  Used for the large fully-connected
 // GEMMs (the MLP configuration); the reference computes them with scalar
 // loops (tiny_dnn/core/kernels/fully_connected_op_internal.h:15-71).
 //
-//   D[M][N] (+)= sum_k A[M][k] * Bt[N][k]         both operands K-major
+//   D[M][N] (+)= sum_k A(m, k) * B(n, k)
 //
-// One block computes a 128 x BN tile of D:
-//   warp 4 (one thread)  TMA producer: cp.async.bulk.tensor 2D loads of the
-//                        A_hi/A_lo/B_hi/B_lo tiles of a 32-float k-block into a
-//                        3-stage ring (128-byte swizzle), signalled on mbarriers
-//   warp 5 (one thread)  tcgen05.mma issuer: 4 k-steps x 3 products per k-block
-//                        into a 128 x BN fp32 accumulator in TMEM; tcgen05.commit
-//                        frees the stage / publishes the accumulator
-//   warps 0-3            epilogue: tcgen05.ld of their 32 TMEM lanes, bias /
-//                        activation / accumulate, stores to D
-// Every load is CTA-local; every wait is bounded and a timeout sets the
-// context's error word, releases TMEM and returns.
+// Arithmetic as in conv_gather.cu: every operand is split into three bf16 numbers, six products per 16 k's, the
+// large one to an accumulator of its own.  A kernel splits each operand once, as it lies in memory, into three bf16
+// matrices; an operand whose rows run along k is read as K-major tiles, one whose rows run along m or n as MN-major
+// tiles, so nothing is transposed.
+//
+// A CTA pair computes a 256 x BN tile (a single CTA 128 x BN): each CTA holds its 128 rows of A and its half of B's
+// rows, one TMA load a part of 64 columns or all three parts of a K-major block, 32 k's a stage.
+//   warps 0-7  epilogue: two warps per TMEM lane quadrant, bias / activation / accumulate, stores to D
+//   warp 8     TMA producer (every load is CTA-local), TMEM allocation
+//   warp 9     MMA issuer of the pair's first CTA; in the second it passes on that its stage has arrived
+// What bounds it: the loads from the L2 cache.  A stage of a pair is 96 KB for 12 MMAs of 128 cycles; 128 x 128 tiles
+// of two TF32 halves asked for twice that a product (784-4096-4096-10, 1024 samples: products 997 us and splits
+// 266 us a step, now 726 and 159 us).  Tiles are taken row block by row block, so that the pairs at work share B.
+// Every wait is bounded and a timeout sets the context's error word, releases TMEM and returns.
 #include "tc_utils.cuh"
 
 namespace b200 {
 
-constexpr int TC_BM = 128;
-constexpr int TC_BK = 32;       // floats per k-block = 128 bytes = one swizzle row
-constexpr int TC_STAGES = 3;
-constexpr int TC_THREADS = 192;
+namespace {
 
-// ---- operand preparation -----------------------------------------------------
+constexpr int TC_BK = 32, TC_MAX_STAGES = 8;
+constexpr int TC_EPI = 8, TC_W_TMA = TC_EPI, TC_W_MMA = TC_EPI + 1, TC_THREADS = (TC_EPI + 2) * 32;
 
-// hi/lo[r][c] = split(src[r*ld + c]) for c < cols, 0 for cols <= c < pitch
-__global__ void tc_split_kernel(const float *__restrict__ src, int rows, int cols, long long ld,
-                                float *__restrict__ hi, float *__restrict__ lo, int pitch) {
-  long long total = (long long)rows * pitch;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    int c = (int)(i % pitch);
-    long long r = i / pitch;
-    float h = 0.f, l = 0.f;
-    if (c < cols) split_tf32(src[r * ld + c], h, l);
-    hi[i] = h;
-    lo[i] = l;
-  }
-}
-
-// hi/lo[c][r] = split(src[r*ld + c]): the transposed operand, rows of length
-// `pitch` (r < rows, zero beyond); 32x32 tiles through shared memory
-__global__ void tc_split_transpose_kernel(const float *__restrict__ src, int rows, int cols,
-                                          long long ld, float *__restrict__ hi,
-                                          float *__restrict__ lo, int pitch) {
-  __shared__ float tile[32][33];
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
-  for (int j = threadIdx.y; j < 32; j += 8) {
-    int r = r0 + j, c = c0 + threadIdx.x;
-    tile[j][threadIdx.x] = (r < rows && c < cols) ? src[(long long)r * ld + c] : 0.f;
-  }
-  __syncthreads();
-  for (int j = threadIdx.y; j < 32; j += 8) {
-    int c = c0 + j, r = r0 + threadIdx.x;  // output row c, column r
-    if (c < cols && r < pitch) {
-      float h, l;
-      split_tf32(tile[threadIdx.x][j], h, l);
-      hi[(long long)c * pitch + r] = h;
-      lo[(long long)c * pitch + r] = l;
+// dst[part][r][c] = the three bf16 parts of src[r*ld + c] for c < cols, 0 for cols <= c < pitch (a multiple of 8)
+template <bool VEC>
+__global__ void __launch_bounds__(256) tc_split_kernel(const float *__restrict__ src, int rows, int cols, long long ld, int pitch,
+                                                       uint32_t *__restrict__ dst) {
+  const int quads = pitch / 4;
+  const long long total = (long long)rows * quads, plane = (long long)rows * pitch / 2;
+  for (long long i0 = blockIdx.x * 1024ll + threadIdx.x; i0 < total; i0 += gridDim.x * 1024ll) {
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long i = i0 + u * 256;
+      const int r = (int)(i / quads), c = (int)(i - (long long)r * quads) * 4;
+      const float *p = src + r * ld + c;
+      const bool live = i < total;
+      if (VEC) {
+        v[u] = live && c < cols ? *reinterpret_cast<const float4 *>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+        v[u].x = live && c < cols ? p[0] : 0.f;
+        v[u].y = live && c + 1 < cols ? p[1] : 0.f;
+        v[u].z = live && c + 2 < cols ? p[2] : 0.f;
+        v[u].w = live && c + 3 < cols ? p[3] : 0.f;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long i = i0 + u * 256;
+      if (i >= total) break;
+      uint2 p[3];
+      split_bf16x3(__float_as_uint(v[u].x), __float_as_uint(v[u].y), p[0].x, p[1].x, p[2].x);
+      split_bf16x3(__float_as_uint(v[u].z), __float_as_uint(v[u].w), p[0].y, p[1].y, p[2].y);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2 *>(dst + q * plane + i * 2) = p[q];
     }
   }
 }
@@ -72,216 +67,317 @@ struct TcArgs {
   float *D;
   const float *bias;
   int *err;
-  int M, N, K;  // K = padded contraction length (multiple of 4)
+  int M, N, nkb;      // nkb: 32-k blocks
+  int a_mn, b_mn;     // the operand's rows run along m / n
+  int mtiles, ntiles, nst;
   int accumulate, act;
 };
 
-template <int BN>
+template <int CG>
+__device__ __forceinline__ void umma_bf16_cg(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (CG == 1)
+    asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+  else
+    asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// One operand of ROWS rows in a stage, all parts:
+//   K-major   [part][row][32 k], 64-byte rows, 64-byte swizzle
+//   MN-major  [64 rows][part][32 k][64 rows as 128 bytes], 128-byte swizzle
+constexpr uint32_t TC_MN_PART = TC_BK * 128, TC_MN_BLOCK = 3 * TC_MN_PART;
+__device__ __forceinline__ uint64_t operand_desc(uint32_t at, int mn) {
+  return mn ? umma_desc(at, TC_MN_BLOCK, 1024, 2) : umma_desc(at, 16, 512, 4);
+}
+
+template <int CG, int BN>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-  gemm3x_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_constant__ CUtensorMap mapAlo,
-                const __grid_constant__ CUtensorMap mapBhi, const __grid_constant__ CUtensorMap mapBlo,
-                const TcArgs a) {
-  constexpr uint32_t A_BYTES = TC_BM * TC_BK * 4;  // 16 KiB
-  constexpr uint32_t B_BYTES = BN * TC_BK * 4;
-  constexpr uint32_t STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
+  gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ TcArgs a) {
+  constexpr int BROWS = BN / CG;                                       // rows of B that this CTA holds
+  constexpr uint32_t A_BYTES = 128 * TC_BK * 6, B_BYTES = BROWS * TC_BK * 6, STAGE = A_BYTES + B_BYTES;
+  constexpr uint32_t COLS = BN == 256 ? 512 : 2 * BN;                  // the large and the small products' accumulators
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  // tiles need 1024-byte alignment (in the shared address space) for the 128-byte swizzle
   uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + TC_STAGES * STAGE_BYTES);
-  uint64_t *empty = full + TC_STAGES;
-  uint64_t *accum = empty + TC_STAGES;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accum + 1);
-
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)a.nst * STAGE);
+  uint64_t *peer = full + TC_MAX_STAGES, *empty = peer + TC_MAX_STAGES, *acc_full = empty + TC_MAX_STAGES, *acc_empty = acc_full + 1;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 1);
   const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
-  const int m0 = blockIdx.y * TC_BM, n0 = blockIdx.x * BN;
-  const int nkb = (a.K + TC_BK - 1) / TC_BK;
-
+  const uint32_t rank = CG == 2 ? cluster_rank() : 0;
+  const int cluster = blockIdx.x / CG, nclusters = gridDim.x / CG, tiles = a.mtiles * a.ntiles;
   if (tid == 0) {
-    for (int s = 0; s < TC_STAGES; ++s) {
+    for (int s = 0; s < a.nst; ++s) {
       mbar_init(&full[s], 1);
+      mbar_init(&peer[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(accum, 1);
+    mbar_init(acc_full, 1);
+    mbar_init(acc_empty, TC_EPI * CG);
     mbar_fence_init();
   }
-  if (warp == 4) {  // one warp allocates the accumulator columns
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
-                   smem_u32(tmem_slot)),
-                 "r"((uint32_t)BN)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-  }
+  if (warp == TC_W_TMA) tmem_alloc_cg<CG>(tmem_slot, COLS);
   tc_fence_before();
   __syncthreads();
+  if (CG == 2) cluster_sync();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem = uni(*tmem_slot);
   bool failed = false;
-
-  if (warp == 4 && lane == 0) {
-    // ---- producer -------------------------------------------------------------
-    for (int kb = 0; kb < nkb && !failed; ++kb) {
-      const int s = kb % TC_STAGES;
-      const uint32_t use = kb / TC_STAGES;
-      if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1) & 1)) {
-        failed = true;
-        break;
-      }
-      uint8_t *st = smem + s * STAGE_BYTES;
-      mbar_expect_tx(&full[s], STAGE_BYTES);
-      tma_load_2d(st, &mapAhi, kb * TC_BK, m0, &full[s]);
-      tma_load_2d(st + A_BYTES, &mapAlo, kb * TC_BK, m0, &full[s]);
-      tma_load_2d(st + 2 * A_BYTES, &mapBhi, kb * TC_BK, n0, &full[s]);
-      tma_load_2d(st + 2 * A_BYTES + B_BYTES, &mapBlo, kb * TC_BK, n0, &full[s]);
-    }
-  } else if (warp == 5) {
-    // ---- MMA issuer (the whole warp stays converged: see elect_one) ---
-    constexpr uint32_t idesc = umma_idesc_tf32(TC_BM, BN);
-    for (int kb = 0; kb < nkb; ++kb) {
-      const int s = kb % TC_STAGES;
-      if (!mbar_wait_warp(&full[s], (kb / TC_STAGES) & 1)) {
-        failed = true;
-        break;
-      }
+  // a failed wait ends no loop: what follows it neither waits nor issues
+  if (warp < TC_EPI) {
+    const int quad = warp & 3;
+    uint32_t it = 0;
+    for (int tile = cluster; tile < tiles; tile += nclusters, ++it) {
+      const int nt = tile / a.mtiles, mt = tile - nt * a.mtiles;
+      const int row = (mt * CG + (int)rank) * 128 + quad * 32 + lane, n0 = nt * BN;
+      if (!failed) failed = !mbar_wait_warp_sleep<100>(acc_full, it & 1);
       tc_fence_after();
-      const uint64_t a0 = umma_desc_k128(smem_u32(smem + s * STAGE_BYTES));
-      const uint64_t b0 = a0 + (2 * A_BYTES >> 4);
-      if (elect_one()) {
-#pragma unroll
-        for (int k4 = 0; k4 < TC_BK / 8; ++k4) {
-          // one instruction consumes 8 floats (32 bytes) of k: advance inside the swizzle row
-          const uint64_t ahi = a0 + k4 * 2, alo = ahi + (A_BYTES >> 4);
-          const uint64_t bhi = b0 + k4 * 2, blo = bhi + (B_BYTES >> 4);
-          umma_tf32(tmem_base, alo, bhi, idesc, (kb | k4) != 0);
-          umma_tf32(tmem_base, ahi, blo, idesc, 1);
-          umma_tf32(tmem_base, ahi, bhi, idesc, 1);
+      const uint32_t t = tmem + ((uint32_t)(quad * 32) << 16);
+      float *drow = a.D + (size_t)row * a.N + n0;
+      const bool vec = a.N % 4 == 0 && ((uintptr_t)a.D & 15) == 0;
+      for (int c = (warp >> 2) * 16; c < BN; c += 32) {
+        uint32_t x[16], y[16];
+        tmem_ld16_nowait(t + (uint32_t)c, x);
+        tmem_ld16_nowait(t + (uint32_t)(BN + c), y);
+        tmem_ld_wait();
+        if (c + 32 >= BN) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_leader<CG>(acc_empty);
         }
-        umma_commit(&empty[s]);  // the stage may be refilled once these MMAs have read it
-      }
-      __syncwarp();
-    }
-    if (!failed && elect_one()) umma_commit(accum);  // accumulator complete
-  } else if (warp < 4) {
-    // ---- epilogue ------------------------------------------------------------------
-    if (!mbar_wait_bounded(accum, 0)) failed = true;
-    tc_fence_after();
-    if (!failed) {
-      const int row = m0 + warp * 32 + lane;
-#pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
-        float v[32];
-        tmem_ld32(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-        if (row < a.M) {
-          float *drow = a.D + (size_t)row * a.N + n0 + c0;
-          // all loads before the stores: interleaved, every load would wait for the store before it
+        if (row >= a.M || failed) continue;
+        float v[16];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            int col = n0 + c0 + j;
-            if (col < a.N) {
-              if (a.bias) v[j] += __ldg(a.bias + col);
-              if (a.accumulate) v[j] += drow[j];
+        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(x[j]) + __uint_as_float(y[j]);
+        const int left = a.N - n0 - c;
+        if (vec && left >= 16) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 4) {
+            float4 *d = reinterpret_cast<float4 *>(drow + c + j);
+            float4 o = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            if (a.bias) {
+              const float *b = a.bias + n0 + c + j;
+              o.x += b[0], o.y += b[1], o.z += b[2], o.w += b[3];
             }
+            if (a.accumulate) {
+              const float4 e = *d;
+              o.x += e.x, o.y += e.y, o.z += e.z, o.w += e.w;
+            }
+            o.x = apply_act(o.x, a.act), o.y = apply_act(o.y, a.act), o.z = apply_act(o.z, a.act), o.w = apply_act(o.w, a.act);
+            *d = o;
           }
+        } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (n0 + c0 + j < a.N) drow[j] = apply_act(v[j], a.act);
+          for (int j = 0; j < 16; ++j)
+            if (j < left) {
+              float o = v[j];
+              if (a.bias) o += a.bias[n0 + c + j];
+              if (a.accumulate) o += drow[c + j];
+              drow[c + j] = apply_act(o, a.act);
+            }
         }
+      }
+    }
+  } else if (warp == TC_W_TMA) {
+    uint32_t s = 0, par = 1;
+    bool first = true;
+    for (int tile = cluster; tile < tiles; tile += nclusters) {
+      const int nt = tile / a.mtiles, mt = tile - nt * a.mtiles;
+      const int m0 = (mt * CG + (int)rank) * 128, n0 = nt * BN + (int)rank * BROWS;
+      for (int kb = 0; kb < a.nkb; ++kb) {
+        if (!first && !failed) failed = !mbar_wait_warp_sleep<20>(&empty[s], par);
+        if (!failed && elect_one()) {
+          uint8_t *st = smem + (size_t)s * STAGE;
+          mbar_expect_tx(&full[s], STAGE);
+          if (a.a_mn)
+            for (int q = 0; q < 2; ++q) tma_load_3d(st + q * TC_MN_BLOCK, &map_a, m0 + q * 64, kb * TC_BK, 0, &full[s]);
+          else
+            tma_load_3d(st, &map_a, kb * TC_BK, m0, 0, &full[s]);
+          st += A_BYTES;
+          if (a.b_mn)
+            for (int q = 0; q < BROWS / 64; ++q) tma_load_3d(st + q * TC_MN_BLOCK, &map_b, n0 + q * 64, kb * TC_BK, 0, &full[s]);
+          else
+            tma_load_3d(st, &map_b, kb * TC_BK, n0, 0, &full[s]);
+        }
+        __syncwarp();
+        if (++s == (uint32_t)a.nst) s = 0, par ^= 1, first = false;
+      }
+    }
+  } else if (rank != 0) {
+    uint32_t s = 0, par = 0;
+    for (int tile = cluster; tile < tiles; tile += nclusters)
+      for (int kb = 0; kb < a.nkb; ++kb) {
+        if (!failed) failed = !mbar_wait_warp(&full[s], par);
+        if (!failed && elect_one()) mbar_arrive_leader<CG>(&peer[s]);
+        __syncwarp();
+        if (++s == (uint32_t)a.nst) s = 0, par ^= 1;
+      }
+  } else {
+    const uint32_t idesc = umma_idesc_bf16(128 * CG, BN) | ((uint32_t)a.a_mn << 15) | ((uint32_t)a.b_mn << 16);
+    const uint64_t a0 = operand_desc(smem_u32(smem), a.a_mn), b0 = operand_desc(smem_u32(smem) + A_BYTES, a.b_mn);
+    const uint64_t ahi = a0 & 0xffffffff00000000ull, bhi = b0 & 0xffffffff00000000ull;
+    // descriptor units: from part to part, from 16 k's to the next
+    const uint32_t ap = (a.a_mn ? TC_MN_PART : 128 * TC_BK * 2) >> 4, ak = (a.a_mn ? 2048 : 32) >> 4;
+    const uint32_t bp = (a.b_mn ? TC_MN_PART : BROWS * TC_BK * 2) >> 4, bk = (a.b_mn ? 2048 : 32) >> 4;
+    uint32_t s = 0, par = 0, it = 0;
+    for (int tile = cluster; tile < tiles; tile += nclusters, ++it) {
+      if (it > 0 && !failed) failed = !mbar_wait_warp_cg<CG>(acc_empty, (it - 1) & 1);
+      for (int kb = 0; kb < a.nkb; ++kb) {
+        if (!failed) failed = !mbar_wait_warp(&full[s], par);
+        if (CG == 2 && !failed) failed = !mbar_wait_warp_cluster(&peer[s], par);
+        tc_fence_after();
+        const uint32_t sa = uni((uint32_t)a0 + ((s * STAGE) >> 4)), sb = uni((uint32_t)b0 + ((s * STAGE) >> 4));
+        if (!failed && elect_one()) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint64_t x1 = ahi | (sa + h * ak), x2 = ahi | (sa + h * ak + ap), x3 = ahi | (sa + h * ak + 2 * ap);
+            const uint64_t y1 = bhi | (sb + h * bk), y2 = bhi | (sb + h * bk + bp), y3 = bhi | (sb + h * bk + 2 * bp);
+            const uint32_t more = (uint32_t)(kb | h);
+            umma_bf16_cg<CG>(tmem + BN, x3, y1, idesc, more);
+            umma_bf16_cg<CG>(tmem + BN, x1, y3, idesc, 1);
+            umma_bf16_cg<CG>(tmem + BN, x2, y2, idesc, 1);
+            umma_bf16_cg<CG>(tmem + BN, x2, y1, idesc, 1);
+            umma_bf16_cg<CG>(tmem + BN, x1, y2, idesc, 1);
+            umma_bf16_cg<CG>(tmem, x1, y1, idesc, more);
+          }
+          umma_commit_cg<CG>(&empty[s]);
+          if (kb + 1 == a.nkb) umma_commit_cg<CG>(acc_full);
+        }
+        __syncwarp();
+        if (++s == (uint32_t)a.nst) s = 0, par ^= 1;
       }
     }
   }
   if (failed && a.err) atomicExch(a.err, 2);
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base),
-                 "r"((uint32_t)BN)
-                 : "memory");
-  }
+  if (CG == 2) cluster_sync();
+  if (warp == TC_W_TMA) tmem_dealloc_cg<CG>(tmem, COLS);
 }
 
 // ---- host side ---------------------------------------------------------------------
 
-// 2D fp32 tensor [rows][pitch]; box = 32 floats x box_rows, 128-byte swizzle, zero fill
-static int make_map(CUtensorMap *m, const float *base, int rows, int cols, int pitch, int box_rows) {
+int tc_pitch(int n) { return (n + 7) / 8 * 8; }
+
+// the three parts of an operand with `rows` x `cols` values as they lie in memory; box: what one load takes
+int make_map(CUtensorMap *m, const void *base, int rows, int cols, int box_cols, int box_rows) {
   EncodeTiledFn fn = encode_fn();
   B200_REQUIRE(fn != nullptr, "cuTensorMapEncodeTiled is not available from the driver");
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)pitch * sizeof(float)};
-  cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box,
-                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  const cuuint64_t pitch = (cuuint64_t)tc_pitch(cols) * 2;
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 3};
+  cuuint64_t strides[2] = {pitch, pitch * (cuuint64_t)rows};
+  cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 3};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  B200_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed (%d) for a %d x %d tensor, pitch %d",
-               (int)r, rows, cols, pitch);
+  B200_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed (%d) for a %d x %d operand", (int)r, rows, cols);
   return 0;
 }
 
-static int tc_pitch(int k) { return (k + 3) / 4 * 4; }
-
-// floats of scratch for the split operands of a GEMM with these extents
-size_t gemm_tc_scratch_floats(int M, int N, int K) {
-  return (size_t)2 * ((size_t)M + N) * tc_pitch(K) + 64;
-}
-
-template <int BN>
-static int launch_tc(b200_ctx *ctx, const CUtensorMap maps[4], const TcArgs &a) {
-  constexpr size_t smem = TC_STAGES * (2 * TC_BM * TC_BK * 4 + 2 * BN * TC_BK * 4) + 1024 + 128;
-  B200_CUDA(cudaFuncSetAttribute(gemm3x_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-  dim3 grid(ceil_div(a.N, BN), ceil_div(a.M, TC_BM));
-  gemm3x_kernel<BN><<<grid, TC_THREADS, smem, ctx->stream>>>(maps[0], maps[1], maps[2], maps[3], a);
+template <int CG, int BN>
+int launch_gemm(b200_ctx *ctx, const CUtensorMap &ma, const CUtensorMap &mb, TcArgs a) {
+  constexpr size_t stage = (size_t)(128 + BN / CG) * TC_BK * 6, fixed = 1024 + (3 * TC_MAX_STAGES + 2) * 8 + 16;
+  a.mtiles = ceil_div(a.M, 128 * CG);
+  a.ntiles = ceil_div(a.N, BN);
+  a.nst = (int)((ctx->smem_optin - fixed) / stage);
+  if (a.nst > TC_MAX_STAGES) a.nst = TC_MAX_STAGES;
+  const size_t smem = fixed + a.nst * stage;
+  B200_CUDA(cudaFuncSetAttribute(gemm_kernel<CG, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int tiles = a.mtiles * a.ntiles, slots = ctx->sm_count / CG;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)((tiles < slots ? tiles : slots) * CG));
+  c.blockDim = dim3(TC_THREADS);
+  c.dynamicSmemBytes = smem;
+  c.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CG;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  c.attrs = at;
+  c.numAttrs = 1;
+  B200_CUDA(cudaLaunchKernelEx(&c, gemm_kernel<CG, BN>, ma, mb, a));
   B200_LAUNCHED();
   return 0;
 }
 
-// D[M][N] (+)= A * Bt^T with A given as src_a (M x K when !a_transposed, else K x M
-// to be transposed) and Bt as src_b (N x K when !b_transposed, else K x N).
+}  // namespace
+
+// floats of scratch for the split operands of a GEMM with these extents, whichever way they lie
+size_t gemm_tc_scratch_floats(int M, int N, int K) {
+  auto words = [](int r, int c) { return (size_t)r * tc_pitch(c) > (size_t)c * tc_pitch(r) ? (size_t)r * tc_pitch(c) : (size_t)c * tc_pitch(r); };
+  return (words(M, K) + words(N, K)) * 3 / 2 + 128;
+}
+
+// D[M][N] (+)= A * Bt^T with A given as src_a (M x K when !a_transposed, else K x M)
+// and Bt as src_b (N x K when !b_transposed, else K x N).
 int gemm_tc(b200_ctx *ctx, int M, int N, int K, const float *src_a, long long lda, bool a_transposed,
             const float *src_b, long long ldb, bool b_transposed, float *D, const float *bias,
             int accumulate, int act, float *scratch) {
   if (M == 0 || N == 0) return 0;
-  const int Kp = tc_pitch(K);
-  float *a_hi = scratch, *a_lo = a_hi + (size_t)M * Kp;
-  float *b_hi = a_lo + (size_t)M * Kp, *b_lo = b_hi + (size_t)N * Kp;
-  cudaStream_t st = ctx->stream;
-  auto split = [&](const float *src, long long ld, bool transposed, int rows, float *hi, float *lo) {
-    // result: rows x Kp (K-major)
-    if (!transposed) {
-      long long total = (long long)rows * Kp;
-      int blocks = (int)((total + 255) / 256 < (long long)ctx->sm_count * 16 ? (total + 255) / 256
-                                                                              : ctx->sm_count * 16);
-      tc_split_kernel<<<blocks, 256, 0, st>>>(src, rows, K, ld, hi, lo, Kp);
-    } else {
-      // src is K x rows; zero the padding columns first when K is not a multiple of 4
-      if (Kp != K) {
-        cudaMemsetAsync(hi, 0, sizeof(float) * (size_t)rows * Kp, st);
-        cudaMemsetAsync(lo, 0, sizeof(float) * (size_t)rows * Kp, st);
-      }
-      dim3 grid(ceil_div(rows, 32), ceil_div(K, 32));
-      tc_split_transpose_kernel<<<grid, dim3(32, 8), 0, st>>>(src, K, rows, ld, hi, lo, Kp);
-    }
+  char *next = reinterpret_cast<char *>(align_up((size_t)reinterpret_cast<uintptr_t>(scratch), 128));
+  auto split = [&](const float *src, long long ld, int rows, int cols) -> void * {
+    const int pitch = tc_pitch(cols);
+    const long long quads = (long long)rows * pitch / 4;
+    const long long want = (quads + 1023) / 1024, cap = (long long)ctx->sm_count * 8;
+    const int blocks = (int)(want < cap ? want : cap);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(next);
+    next += align_up((size_t)rows * pitch * 6, 128);
+    if (cols % 4 == 0 && ld % 4 == 0 && ((uintptr_t)src & 15) == 0)
+      tc_split_kernel<true><<<blocks, 256, 0, ctx->stream>>>(src, rows, cols, ld, pitch, dst);
+    else
+      tc_split_kernel<false><<<blocks, 256, 0, ctx->stream>>>(src, rows, cols, ld, pitch, dst);
+    return dst;
   };
-  split(src_a, lda, a_transposed, M, a_hi, a_lo);
+  const int ar = a_transposed ? K : M, ac = a_transposed ? M : K, br = b_transposed ? K : N, bc = b_transposed ? N : K;
+  const void *pa = split(src_a, lda, ar, ac);
   B200_LAUNCHED();
-  split(src_b, ldb, b_transposed, N, b_hi, b_lo);
+  const void *pb = split(src_b, ldb, br, bc);
   B200_LAUNCHED();
-  const int BN = N >= 128 ? 128 : 64;
-  CUtensorMap maps[4];
-  B200_TRY(make_map(&maps[0], a_hi, M, Kp, Kp, TC_BM));
-  B200_TRY(make_map(&maps[1], a_lo, M, Kp, Kp, TC_BM));
-  B200_TRY(make_map(&maps[2], b_hi, N, Kp, Kp, BN));
-  B200_TRY(make_map(&maps[3], b_lo, N, Kp, Kp, BN));
-  TcArgs a;
+  // The tile: turns that the busiest SM takes times the cycles of a stage, MMAs (N / 2 cycles each, a pair's M
+  // counts double) or loads (about 35 bytes a cycle and SM), whichever is longer.
+  struct Shape {
+    int cg, bn;
+  };
+  const Shape shapes[4] = {{2, 256}, {2, 128}, {1, 128}, {1, 64}};
+  int pick = 0;
+  double best = -1;
+  for (int i = 0; i < 4; ++i) {
+    const int cg = shapes[i].cg, bn = shapes[i].bn;
+    const long long tiles = (long long)ceil_div(M, 128 * cg) * ceil_div(N, bn), slots = ctx->sm_count / cg;
+    const double mma = 12 * (bn / 2 > 48 ? bn / 2 : 48), load = (128 + bn / cg) * TC_BK * 6 / 35.0;
+    const double cost = (double)((tiles + slots - 1) / slots) * ((mma > load ? mma : load) * ceil_div(K, TC_BK) + 20 * bn + 2000);
+    if (best < 0 || cost < best) {
+      best = cost;
+      pick = i;
+    }
+  }
+  const int brows = shapes[pick].bn / shapes[pick].cg;
+  CUtensorMap ma, mb;
+  B200_TRY(make_map(&ma, pa, ar, ac, a_transposed ? 64 : TC_BK, a_transposed ? TC_BK : 128));
+  B200_TRY(make_map(&mb, pb, br, bc, b_transposed ? 64 : TC_BK, b_transposed ? TC_BK : brows));
+  TcArgs a = {};
   a.D = D;
   a.bias = bias;
   a.err = ctx->dev_err;
   a.M = M;
   a.N = N;
-  a.K = Kp;
+  a.nkb = ceil_div(K, TC_BK);
+  a.a_mn = a_transposed;
+  a.b_mn = b_transposed;
   a.accumulate = accumulate;
   a.act = act;
-  if (BN == 128) return launch_tc<128>(ctx, maps, a);
-  return launch_tc<64>(ctx, maps, a);
+  switch (pick) {
+    case 0: return launch_gemm<2, 256>(ctx, ma, mb, a);
+    case 1: return launch_gemm<2, 128>(ctx, ma, mb, a);
+    case 2: return launch_gemm<1, 128>(ctx, ma, mb, a);
+    default: return launch_gemm<1, 64>(ctx, ma, mb, a);
+  }
 }
 
 }  // namespace b200
