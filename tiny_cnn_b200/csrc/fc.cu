@@ -134,6 +134,7 @@ __global__ void col_sum_kernel(const float *__restrict__ d, float *__restrict__ 
   int col = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
   if (col < N)
+#pragma unroll 8
     for (int r = threadIdx.y; r < rows; r += 8) s += d[(size_t)r * N + col];
   part[threadIdx.y][threadIdx.x] = s;
   __syncthreads();

@@ -25,6 +25,7 @@ namespace b200 {
 namespace {
 
 constexpr int TC_BK = 32, TC_MAX_STAGES = 8;
+constexpr size_t TC_PART_FLOATS = 80 * 65536;  // room for partial sums: a tile for every pair of SMs
 constexpr int TC_EPI = 8, TC_W_TMA = TC_EPI, TC_W_MMA = TC_EPI + 1, TC_THREADS = (TC_EPI + 2) * 32;
 
 // dst[part][r][c] = the three bf16 parts of src[r*ld + c] for c < cols, 0 for cols <= c < pitch (a multiple of 8)
@@ -70,6 +71,7 @@ struct TcArgs {
   int M, N, nkb;      // nkb: 32-k blocks
   int a_mn, b_mn;     // the operand's rows run along m / n
   int mtiles, ntiles, nst;
+  int splits, kper;   // k blocks dealt to `splits` tiles; with more than one, D is [splits][M][N] of partial sums
   int accumulate, act;
 };
 
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 1);
   const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const uint32_t rank = CG == 2 ? cluster_rank() : 0;
-  const int cluster = blockIdx.x / CG, nclusters = gridDim.x / CG, tiles = a.mtiles * a.ntiles;
+  const int cluster = blockIdx.x / CG, nclusters = gridDim.x / CG, tiles = a.mtiles * a.ntiles * a.splits;
   if (tid == 0) {
     for (int s = 0; s < a.nst; ++s) {
       mbar_init(&full[s], 1);
@@ -133,12 +135,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int quad = warp & 3;
     uint32_t it = 0;
     for (int tile = cluster; tile < tiles; tile += nclusters, ++it) {
-      const int nt = tile / a.mtiles, mt = tile - nt * a.mtiles;
+      const int sp = tile / (a.mtiles * a.ntiles), rest = tile - sp * a.mtiles * a.ntiles, nt = rest / a.mtiles, mt = rest - nt * a.mtiles;
       const int row = (mt * CG + (int)rank) * 128 + quad * 32 + lane, n0 = nt * BN;
       if (!failed) failed = !mbar_wait_warp_sleep<100>(acc_full, it & 1);
       tc_fence_after();
       const uint32_t t = tmem + ((uint32_t)(quad * 32) << 16);
-      float *drow = a.D + (size_t)row * a.N + n0;
+      float *drow = a.D + ((size_t)sp * a.M + row) * a.N + n0;
       const bool vec = a.N % 4 == 0 && ((uintptr_t)a.D & 15) == 0;
       for (int c = (warp >> 2) * 16; c < BN; c += 32) {
         uint32_t x[16], y[16];
@@ -187,9 +189,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     uint32_t s = 0, par = 1;
     bool first = true;
     for (int tile = cluster; tile < tiles; tile += nclusters) {
-      const int nt = tile / a.mtiles, mt = tile - nt * a.mtiles;
-      const int m0 = (mt * CG + (int)rank) * 128, n0 = nt * BN + (int)rank * BROWS;
-      for (int kb = 0; kb < a.nkb; ++kb) {
+      const int sp = tile / (a.mtiles * a.ntiles), rest = tile - sp * a.mtiles * a.ntiles, nt = rest / a.mtiles, mt = rest - nt * a.mtiles;
+      const int m0 = (mt * CG + (int)rank) * 128, n0 = nt * BN + (int)rank * BROWS, kend = min(a.nkb, (sp + 1) * a.kper);
+      for (int kb = sp * a.kper; kb < kend; ++kb) {
         if (!first && !failed) failed = !mbar_wait_warp_sleep<20>(&empty[s], par);
         if (!failed && elect_one()) {
           uint8_t *st = smem + (size_t)s * STAGE;
@@ -210,13 +212,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     }
   } else if (rank != 0) {
     uint32_t s = 0, par = 0;
-    for (int tile = cluster; tile < tiles; tile += nclusters)
-      for (int kb = 0; kb < a.nkb; ++kb) {
+    for (int tile = cluster; tile < tiles; tile += nclusters) {
+      const int sp = tile / (a.mtiles * a.ntiles), kend = min(a.nkb, (sp + 1) * a.kper);
+      for (int kb = sp * a.kper; kb < kend; ++kb) {
         if (!failed) failed = !mbar_wait_warp(&full[s], par);
         if (!failed && elect_one()) mbar_arrive_leader<CG>(&peer[s]);
         __syncwarp();
         if (++s == (uint32_t)a.nst) s = 0, par ^= 1;
       }
+    }
   } else {
     const uint32_t idesc = umma_idesc_bf16(128 * CG, BN) | ((uint32_t)a.a_mn << 15) | ((uint32_t)a.b_mn << 16);
     const uint64_t a0 = operand_desc(smem_u32(smem), a.a_mn), b0 = operand_desc(smem_u32(smem) + A_BYTES, a.b_mn);
@@ -227,7 +231,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     uint32_t s = 0, par = 0, it = 0;
     for (int tile = cluster; tile < tiles; tile += nclusters, ++it) {
       if (it > 0 && !failed) failed = !mbar_wait_warp_cg<CG>(acc_empty, (it - 1) & 1);
-      for (int kb = 0; kb < a.nkb; ++kb) {
+      const int sp = tile / (a.mtiles * a.ntiles), kbeg = sp * a.kper, kend = min(a.nkb, kbeg + a.kper);
+      for (int kb = kbeg; kb < kend; ++kb) {
         if (!failed) failed = !mbar_wait_warp(&full[s], par);
         if (CG == 2 && !failed) failed = !mbar_wait_warp_cluster(&peer[s], par);
         tc_fence_after();
@@ -237,7 +242,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           for (int h = 0; h < 2; ++h) {
             const uint64_t x1 = ahi | (sa + h * ak), x2 = ahi | (sa + h * ak + ap), x3 = ahi | (sa + h * ak + 2 * ap);
             const uint64_t y1 = bhi | (sb + h * bk), y2 = bhi | (sb + h * bk + bp), y3 = bhi | (sb + h * bk + 2 * bp);
-            const uint32_t more = (uint32_t)(kb | h);
+            const uint32_t more = (uint32_t)((kb - kbeg) | h);
             umma_bf16_cg<CG>(tmem + BN, x3, y1, idesc, more);
             umma_bf16_cg<CG>(tmem + BN, x1, y3, idesc, 1);
             umma_bf16_cg<CG>(tmem + BN, x2, y2, idesc, 1);
@@ -246,7 +251,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             umma_bf16_cg<CG>(tmem, x1, y1, idesc, more);
           }
           umma_commit_cg<CG>(&empty[s]);
-          if (kb + 1 == a.nkb) umma_commit_cg<CG>(acc_full);
+          if (kb + 1 == kend) umma_commit_cg<CG>(acc_full);
         }
         __syncwarp();
         if (++s == (uint32_t)a.nst) s = 0, par ^= 1;
@@ -258,6 +263,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __syncthreads();
   if (CG == 2) cluster_sync();
   if (warp == TC_W_TMA) tmem_dealloc_cg<CG>(tmem, COLS);
+}
+
+// D = act((accumulate ? D : 0) + bias + the partial sums in order)
+__global__ void __launch_bounds__(256) gemm_sum_kernel(const float *__restrict__ part, int splits, size_t MN, int N,
+                                                       float *__restrict__ D, const float *__restrict__ bias, int accumulate,
+                                                       int act) {
+  for (size_t i = blockIdx.x * 256 + threadIdx.x; i < MN; i += (size_t)gridDim.x * 256) {
+    float v = part[i];
+#pragma unroll 4
+    for (int z = 1; z < splits; ++z) v += part[z * MN + i];
+    if (bias) v += bias[i % N];
+    if (accumulate) v += D[i];
+    D[i] = apply_act(v, act);
+  }
 }
 
 // ---- host side ---------------------------------------------------------------------
@@ -289,7 +308,7 @@ int launch_gemm(b200_ctx *ctx, const CUtensorMap &ma, const CUtensorMap &mb, TcA
   if (a.nst > TC_MAX_STAGES) a.nst = TC_MAX_STAGES;
   const size_t smem = fixed + a.nst * stage;
   B200_CUDA(cudaFuncSetAttribute(gemm_kernel<CG, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int tiles = a.mtiles * a.ntiles, slots = ctx->sm_count / CG;
+  const int tiles = a.mtiles * a.ntiles * a.splits, slots = ctx->sm_count / CG;
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3((unsigned)((tiles < slots ? tiles : slots) * CG));
   c.blockDim = dim3(TC_THREADS);
@@ -311,7 +330,7 @@ int launch_gemm(b200_ctx *ctx, const CUtensorMap &ma, const CUtensorMap &mb, TcA
 // floats of scratch for the split operands of a GEMM with these extents, whichever way they lie
 size_t gemm_tc_scratch_floats(int M, int N, int K) {
   auto words = [](int r, int c) { return (size_t)r * tc_pitch(c) > (size_t)c * tc_pitch(r) ? (size_t)r * tc_pitch(c) : (size_t)c * tc_pitch(r); };
-  return (words(M, K) + words(N, K)) * 3 / 2 + 128;
+  return (words(M, K) + words(N, K)) * 3 / 2 + TC_PART_FLOATS + 128;
 }
 
 // D[M][N] (+)= A * Bt^T with A given as src_a (M x K when !a_transposed, else K x M)
@@ -339,22 +358,31 @@ int gemm_tc(b200_ctx *ctx, int M, int N, int K, const float *src_a, long long ld
   B200_LAUNCHED();
   const void *pb = split(src_b, ldb, br, bc);
   B200_LAUNCHED();
-  // The tile: turns that the busiest SM takes times the cycles of a stage, MMAs (N / 2 cycles each, a pair's M
-  // counts double) or loads (about 35 bytes a cycle and SM), whichever is longer.
+  // The tile and the split of k: turns that the busiest SM takes times the cycles of a turn: stages of MMAs (N / 2
+  // cycles each, a pair's M counts double) or loads (about 22 bytes a cycle and SM), whichever is longer, the
+  // epilogue, and for a split k the pass that adds up the partial sums.  (1024 x 784, k = 4096: 118 us in 104 tiles
+  // of 128 x 64, KSPLIT us in 16 tiles of 256 x 256 of four splits.)
   struct Shape {
     int cg, bn;
   };
   const Shape shapes[4] = {{2, 256}, {2, 128}, {1, 128}, {1, 64}};
-  int pick = 0;
+  const int nkb = ceil_div(K, TC_BK);
+  int pick = 0, splits = 1;
   double best = -1;
   for (int i = 0; i < 4; ++i) {
     const int cg = shapes[i].cg, bn = shapes[i].bn;
     const long long tiles = (long long)ceil_div(M, 128 * cg) * ceil_div(N, bn), slots = ctx->sm_count / cg;
-    const double mma = 12 * (bn / 2 > 48 ? bn / 2 : 48), load = (128 + bn / cg) * TC_BK * 6 / 35.0;
-    const double cost = (double)((tiles + slots - 1) / slots) * ((mma > load ? mma : load) * ceil_div(K, TC_BK) + 20 * bn + 2000);
-    if (best < 0 || cost < best) {
-      best = cost;
-      pick = i;
+    const double mma = 12 * (bn / 2 > 48 ? bn / 2 : 48), load = (128 + bn / cg) * TC_BK * 6 / 22.0;
+    for (int sp = 1; sp <= 16 && sp * 8 <= nkb + 7; ++sp) {
+      if (sp > 1 && (tiles * sp > slots || (size_t)sp * M * N > TC_PART_FLOATS)) break;
+      const double turn = (mma > load ? mma : load) * ceil_div(nkb, sp) + 20 * bn + 2000;
+      const double cost = (double)((tiles * sp + slots - 1) / slots) * turn +
+                          (sp > 1 ? 6000 + (sp + 1) * (double)M * N * 4 / (ctx->sm_count * 16) : 0);
+      if (best < 0 || cost < best) {
+        best = cost;
+        pick = i;
+        splits = sp;
+      }
     }
   }
   const int brows = shapes[pick].bn / shapes[pick].cg;
@@ -367,17 +395,28 @@ int gemm_tc(b200_ctx *ctx, int M, int N, int K, const float *src_a, long long ld
   a.err = ctx->dev_err;
   a.M = M;
   a.N = N;
-  a.nkb = ceil_div(K, TC_BK);
+  a.nkb = nkb;
+  a.kper = ceil_div(nkb, splits);
+  a.splits = ceil_div(nkb, a.kper);
   a.a_mn = a_transposed;
   a.b_mn = b_transposed;
   a.accumulate = accumulate;
   a.act = act;
-  switch (pick) {
-    case 0: return launch_gemm<2, 256>(ctx, ma, mb, a);
-    case 1: return launch_gemm<2, 128>(ctx, ma, mb, a);
-    case 2: return launch_gemm<1, 128>(ctx, ma, mb, a);
-    default: return launch_gemm<1, 64>(ctx, ma, mb, a);
+  if (a.splits > 1) {  // plain sums first
+    a.D = reinterpret_cast<float *>(next);
+    a.bias = nullptr;
+    a.accumulate = 0;
+    a.act = B200_ACT_NONE;
   }
+  B200_TRY((pick == 0   ? launch_gemm<2, 256>(ctx, ma, mb, a)
+            : pick == 1 ? launch_gemm<2, 128>(ctx, ma, mb, a)
+            : pick == 2 ? launch_gemm<1, 128>(ctx, ma, mb, a)
+                        : launch_gemm<1, 64>(ctx, ma, mb, a)));
+  if (a.splits == 1) return 0;
+  const size_t MN = (size_t)M * N, blocks = (MN + 255) / 256, cap = (size_t)ctx->sm_count * 8;
+  gemm_sum_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, ctx->stream>>>(a.D, a.splits, MN, N, D, bias, accumulate, act);
+  B200_LAUNCHED();
+  return 0;
 }
 
 }  // namespace b200
