@@ -297,7 +297,8 @@ int softmax_loss_bwd(b200_ctx *ctx, int loss_kind, const float *y, const float *
 // the weights (K x N floats, N <= 16) sit in shared memory.  With sixteen lanes a sample, each adding all the products
 // of an output, the chain of K additions was the kernel's time (500 -> 10, 77 samples: 20 us forward, 16 us backward;
 // now 8.8 and 7.5 us).
-constexpr int FCS_THREADS = 256, FCS_N = 16;
+constexpr int FCS_N = 16;
+constexpr size_t FCS_MAX_BYTES = 192 * 1024;  // of weights in shared memory
 
 // the sum of acc[j] over the lanes, in lane j of each half-warp: sums of halves, which leave half the values a step
 __device__ __forceinline__ float lanes_sum16(float *acc) {
@@ -314,16 +315,18 @@ __device__ __forceinline__ float lanes_sum16(float *acc) {
 }
 
 // z = x W + b (fully_connected_op_internal.h:15-36), y = softmax(z) (softmax_layer.h:24-34)
-__global__ void __launch_bounds__(FCS_THREADS) fc_softmax_fwd16_kernel(const float *__restrict__ x,
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) fc_softmax_fwd16_kernel(const float *__restrict__ x,
                                                                        const float *__restrict__ W,
                                                                        const float *__restrict__ bias,
                                                                        float *__restrict__ z, float *__restrict__ y,
                                                                        int K, int N, int B) {
   extern __shared__ float fcs_w[];  // [K][N]
-#pragma unroll 8
-  for (int i = threadIdx.x; i < K * N; i += FCS_THREADS) fcs_w[i] = W[i];
+  for (int i = threadIdx.x; i < K * N; i += THREADS) cp_async4(fcs_w + i, W + i, true);
+  cp_async_commit();
+  cp_async_wait<0>();
   __syncthreads();
-  const int n = (blockIdx.x * FCS_THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31, j = lane & 15;
+  const int n = (blockIdx.x * THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31, j = lane & 15;
   if (n >= B) return;
   const float *xr = x + (size_t)n * K;
   float acc[FCS_N];
@@ -352,17 +355,19 @@ __global__ void __launch_bounds__(FCS_THREADS) fc_softmax_fwd16_kernel(const flo
 // dy = loss gradient of (y, t); dz = softmax gradient (as softmax_bwd16_kernel); dx = dz W^T
 // (fully_connected_op_internal.h:45-50), multiplied by the gradient of a relu in front of the layer when
 // `relu_x` (that relu's output = this layer's input) is given (relu_layer.h:31-39)
-__global__ void __launch_bounds__(FCS_THREADS) fc_softmax_bwd16_kernel(const float *__restrict__ y,
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) fc_softmax_bwd16_kernel(const float *__restrict__ y,
                                                                        const float *__restrict__ t, int loss_kind,
                                                                        const float *__restrict__ W,
                                                                        const float *__restrict__ relu_x,
                                                                        float *__restrict__ dy, float *__restrict__ dz,
                                                                        float *__restrict__ dx, int K, int N, int B) {
   extern __shared__ float fcs_w[];  // [K][N]
-#pragma unroll 8
-  for (int i = threadIdx.x; i < K * N; i += FCS_THREADS) fcs_w[i] = W[i];
+  for (int i = threadIdx.x; i < K * N; i += THREADS) cp_async4(fcs_w + i, W + i, true);
+  cp_async_commit();
+  cp_async_wait<0>();
   __syncthreads();
-  const int n = (blockIdx.x * FCS_THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31, j = lane & 15;
+  const int n = (blockIdx.x * THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31, j = lane & 15;
   if (n >= B) return;
   const float factor = 2.0f / (float)N;
   float yj = 0.f, gj = 0.f;
@@ -395,16 +400,25 @@ __global__ void __launch_bounds__(FCS_THREADS) fc_softmax_bwd16_kernel(const flo
   }
 }
 
-bool fc_softmax_fusable(int K, int N) { return N >= 1 && N <= 16 && K >= 1 && (size_t)K * N * sizeof(float) <= 32 * 1024; }
+bool fc_softmax_fusable(int K, int N) { return N >= 1 && N <= 16 && K >= 1 && (size_t)K * N * sizeof(float) <= FCS_MAX_BYTES; }
+
+// eight samples a block; sixteen where the weights leave an SM room for one block only
+template <typename... P, typename... A>
+static int launch_head(b200_ctx *ctx, void (*few)(P...), void (*many)(P...), int K, int N, int B, A... args) {
+  const size_t smem = (size_t)K * N * sizeof(float);
+  const int threads = smem > 64 * 1024 ? 512 : 256;
+  auto kernel = threads == 512 ? many : few;
+  B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<ceil_div(B, threads / 32), threads, smem, ctx->stream>>>(args...);
+  B200_LAUNCHED();
+  return 0;
+}
 
 int fc_softmax_fwd(b200_ctx *ctx, int K, int N, const float *x, const float *W, const float *bias, float *z, float *y,
                    int B) {
   B200_REQUIRE(fc_softmax_fusable(K, N), "fc_softmax_fwd: shape %d x %d not supported", K, N);
   if (B == 0) return 0;
-  fc_softmax_fwd16_kernel<<<ceil_div(B, FCS_THREADS / 32), FCS_THREADS, (size_t)K * N * sizeof(float), ctx->stream>>>(
-    x, W, bias, z, y, K, N, B);
-  B200_LAUNCHED();
-  return 0;
+  return launch_head(ctx, fc_softmax_fwd16_kernel<256>, fc_softmax_fwd16_kernel<512>, K, N, B, x, W, bias, z, y, K, N, B);
 }
 
 int fc_softmax_loss_bwd(b200_ctx *ctx, int loss_kind, int K, int N, const float *y, const float *t, const float *W,
@@ -413,10 +427,8 @@ int fc_softmax_loss_bwd(b200_ctx *ctx, int loss_kind, int K, int N, const float 
   B200_REQUIRE(loss_kind >= B200_LOSS_MSE && loss_kind <= B200_LOSS_CROSS_ENTROPY_MULTICLASS,
                "fc_softmax_loss_bwd: unknown loss %d", loss_kind);
   if (B == 0) return 0;
-  fc_softmax_bwd16_kernel<<<ceil_div(B, FCS_THREADS / 32), FCS_THREADS, (size_t)K * N * sizeof(float), ctx->stream>>>(
-    y, t, loss_kind, W, relu_x, dy, dz, dx, K, N, B);
-  B200_LAUNCHED();
-  return 0;
+  return launch_head(ctx, fc_softmax_bwd16_kernel<256>, fc_softmax_bwd16_kernel<512>, K, N, B, y, t, loss_kind, W, relu_x, dy, dz,
+                     dx, K, N, B);
 }
 
 int loss_value(b200_ctx *ctx, int kind, const float *y, const float *t, float *loss_sum, int dim,

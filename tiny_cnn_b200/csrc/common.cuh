@@ -208,15 +208,31 @@ int merge_rows(b200_ctx *ctx, const float *src, int rows, size_t stride, float *
 // tensor-core GEMM (gemm_tc.cu): D[M][N] (+)= A * Bt^T, operands split into three bf16
 // parts in `scratch` (gemm_tc_scratch_floats floats)
 size_t gemm_tc_scratch_floats(int M, int N, int K);
-int gemm_tc(b200_ctx *ctx, int M, int N, int K, const float *src_a, long long lda, bool a_transposed,
-            const float *src_b, long long ldb, bool b_transposed, float *D, const float *bias,
-            int accumulate, int act, float *scratch);
+struct GemmOperand {
+  const float *src;            // contiguous rows
+  const void *planes = nullptr;  // or its parts, if they exist already (gemm_tc_split; gemm_tc_operand_floats)
+};
+size_t gemm_tc_operand_floats(int rows, int cols);
+int gemm_tc_split(b200_ctx *ctx, const float *src, int rows, int cols, void *planes);
+int gemm_tc(b200_ctx *ctx, int M, int N, int K, const GemmOperand &a, bool a_transposed, const GemmOperand &b,
+            bool b_transposed, float *D, const float *bias, int accumulate, int act, float *scratch);
 
 // `scratch` (fc_scratch_floats floats, may be nullptr) holds the k-slice partial
 // sums small GEMMs are split into, or the split operands of the tensor-core path.
 size_t fc_scratch_floats(const b200_ctx *ctx, int in_size, int out_size, int B);
+// Operands of a layer's products that a step splits once: the input and the weights in the forward pass, which
+// the backward pass reads again, and the output gradient.  Null: not kept.  `*_ready`: split in this step.
+struct FcPlanes {
+  void *x = nullptr, *w = nullptr, *d = nullptr;
+  bool x_ready = false, w_ready = false, d_ready = false;
+};
+bool fc_any_tc(const b200_ctx *ctx, int in_size, int out_size, int B);
+// splits what is missing of those that products of this batch read (x and w; with `grad` d)
+int fc_split(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W, const float *dout, int B, FcPlanes *p,
+             bool grad);
 int fc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
-           const float *bias, float *out, int B, int act, float *scratch, bool w_rows = false);
+           const float *bias, float *out, int B, int act, float *scratch, bool w_rows = false,
+           const FcPlanes *planes = nullptr);
 // sum of a bucket over the ranks of a data-parallel job through peer memory (peer_reduce.cu)
 struct PeerReduce {
   int rank = 0, world = 0;
@@ -240,7 +256,8 @@ int peer_reduce_run(b200_ctx *ctx, const PeerReduce *pr, float *grads);
 
 int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
            const float *dout, float *din, float *dW, float *db, int accumulate, int B,
-           float *scratch, bool w_rows = false);
+           float *scratch, bool w_rows = false,
+           const FcPlanes *planes = nullptr);
 
 int maxpool_fwd(b200_ctx *ctx, const b200_pool_desc &d, const float *in, float *out,
                 int32_t *argmax, int B);

@@ -224,13 +224,37 @@ static int run_gemm(b200_ctx *ctx, int M, int N, int K, const float *A, long lon
   return 0;
 }
 
-// `w_rows`: the weights are stored [out][in] (a convolution whose window is the whole input), not [in][out]
+bool fc_any_tc(const b200_ctx *ctx, int in_size, int out_size, int B) {
+  return use_tc(ctx, B, out_size, in_size) || use_tc(ctx, B, in_size, out_size) || use_tc(ctx, in_size, out_size, B) ||
+         use_tc(ctx, out_size, in_size, B);
+}
+
+int fc_split(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W, const float *dout, int B, FcPlanes *p,
+             bool grad) {
+  const bool fwd = use_tc(ctx, B, out_size, in_size), dx = use_tc(ctx, B, in_size, out_size), dw = use_tc(ctx, in_size, out_size, B);
+  if (!grad) {
+    p->x_ready = p->x && (fwd || dw);
+    p->w_ready = p->w && (fwd || dx);
+    if (p->x_ready) B200_TRY(gemm_tc_split(ctx, in, B, in_size, p->x));
+    if (p->w_ready) B200_TRY(gemm_tc_split(ctx, W, in_size, out_size, p->w));
+  } else if (p->d && (dx || dw)) {
+    B200_TRY(gemm_tc_split(ctx, dout, B, out_size, p->d));
+    p->d_ready = true;
+  }
+  return 0;
+}
+
+static GemmOperand operand(const float *src, const void *planes, bool ready) { return {src, ready ? planes : nullptr}; }
+
+// `w_rows`: the weights are stored [out][in] (a convolution whose window is the whole input), not [in][out]; such a
+// layer keeps no `planes`
 int fc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
-           const float *bias, float *out, int B, int act, float *scratch, bool w_rows) {
+           const float *bias, float *out, int B, int act, float *scratch, bool w_rows, const FcPlanes *planes) {
+  const FcPlanes p = planes ? *planes : FcPlanes();
   if (scratch && use_tc(ctx, B, out_size, in_size))
-    // A = in [B][in]; Bt = W^T: W is [in][out], i.e. K x N, transposed while splitting
-    return gemm_tc(ctx, B, out_size, in_size, in, in_size, false, W, w_rows ? in_size : out_size, !w_rows, out, bias, 0,
-                   act, scratch);
+    // A = in [B][in]; Bt = W^T: W is [in][out], i.e. K x N
+    return gemm_tc(ctx, B, out_size, in_size, operand(in, p.x, p.x_ready), false, operand(W, p.w, p.w_ready), !w_rows, out, bias,
+                   0, act, scratch);
   // M = B, N = out, K = in; A = in (k fast), Bm(k, n) = W[k][n] (n fast) or W[n][k] (k fast)
   if (w_rows)
     return run_gemm<true, false>(ctx, B, out_size, in_size, in, in_size, 1, W, 1, in_size, out, bias, 0, act);
@@ -240,10 +264,11 @@ int fc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const floa
 
 int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
            const float *dout, float *din, float *dW, float *db, int accumulate, int B,
-           float *scratch, bool w_rows) {
+           float *scratch, bool w_rows, const FcPlanes *planes) {
+  const FcPlanes p = planes ? *planes : FcPlanes();
   if (din && scratch && use_tc(ctx, B, in_size, out_size)) {
     // din[B][in] = dout[B][out] * W^T: A = dout; Bt[n = c][k = o] = W[c*out + o] as stored
-    B200_TRY(gemm_tc(ctx, B, in_size, out_size, dout, out_size, false, W, w_rows ? in_size : out_size, w_rows, din,
+    B200_TRY(gemm_tc(ctx, B, in_size, out_size, operand(dout, p.d, p.d_ready), false, operand(W, p.w, p.w_ready), w_rows, din,
                      nullptr, 0, 0, scratch));
   } else if (din && w_rows) {
     B200_TRY((run_gemm<true, true>(ctx, B, in_size, out_size, dout, out_size, 1, W, in_size, 1,
@@ -256,13 +281,14 @@ int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const floa
   }
   if (dW) {
     // dW[in][out] (+)= in^T * dout, or dW[out][in] (+)= dout^T * in
-    const float *p = w_rows ? dout : in, *q = w_rows ? in : dout;
+    const float *l = w_rows ? dout : in, *r = w_rows ? in : dout;
     const int M = w_rows ? out_size : in_size, N = w_rows ? in_size : out_size;
     if (scratch && use_tc(ctx, M, N, B))
-      B200_TRY(gemm_tc(ctx, M, N, B, p, M, true, q, N, true, dW, nullptr, accumulate, 0, scratch));
+      B200_TRY(gemm_tc(ctx, M, N, B, operand(l, p.x, p.x_ready && !w_rows), true, operand(r, p.d, p.d_ready && !w_rows), true, dW,
+                       nullptr, accumulate, 0, scratch));
     else
-      // A(m, k = n) = p[n*M + m] (m fast)
-      B200_TRY((run_gemm<false, true>(ctx, M, N, B, p, 1, M, q, N, 1, dW, nullptr, accumulate, 0)));
+      // A(m, k = n) = l[n*M + m] (m fast)
+      B200_TRY((run_gemm<false, true>(ctx, M, N, B, l, 1, M, r, N, 1, dW, nullptr, accumulate, 0)));
   }
   if (db) {
     col_sum_kernel<<<ceil_div(out_size, 32), dim3(32, 8), 0, ctx->stream>>>(dout, db, B, out_size,

@@ -333,35 +333,43 @@ size_t gemm_tc_scratch_floats(int M, int N, int K) {
   return (words(M, K) + words(N, K)) * 3 / 2 + TC_PART_FLOATS + 128;
 }
 
-// D[M][N] (+)= A * Bt^T with A given as src_a (M x K when !a_transposed, else K x M)
-// and Bt as src_b (N x K when !b_transposed, else K x N).
-int gemm_tc(b200_ctx *ctx, int M, int N, int K, const float *src_a, long long lda, bool a_transposed,
-            const float *src_b, long long ldb, bool b_transposed, float *D, const float *bias,
-            int accumulate, int act, float *scratch) {
+size_t gemm_tc_operand_floats(int rows, int cols) { return (size_t)rows * tc_pitch(cols) * 3 / 2 + 32; }
+
+// the three parts of a matrix with contiguous rows
+int gemm_tc_split(b200_ctx *ctx, const float *src, int rows, int cols, void *planes) {
+  const int pitch = tc_pitch(cols);
+  const long long quads = (long long)rows * pitch / 4;
+  const long long want = (quads + 1023) / 1024, cap = (long long)ctx->sm_count * 8;
+  const int blocks = (int)(want < cap ? want : cap);
+  if (cols % 4 == 0 && ((uintptr_t)src & 15) == 0)
+    tc_split_kernel<true><<<blocks, 256, 0, ctx->stream>>>(src, rows, cols, cols, pitch, static_cast<uint32_t *>(planes));
+  else
+    tc_split_kernel<false><<<blocks, 256, 0, ctx->stream>>>(src, rows, cols, cols, pitch, static_cast<uint32_t *>(planes));
+  B200_LAUNCHED();
+  return 0;
+}
+
+// D[M][N] (+)= A * Bt^T with A given as M x K when !a_transposed, else K x M,
+// and Bt as N x K when !b_transposed, else K x N.  An operand that comes with `planes` is split already.
+int gemm_tc(b200_ctx *ctx, int M, int N, int K, const GemmOperand &oa, bool a_transposed, const GemmOperand &ob,
+            bool b_transposed, float *D, const float *bias, int accumulate, int act, float *scratch) {
   if (M == 0 || N == 0) return 0;
   char *next = reinterpret_cast<char *>(align_up((size_t)reinterpret_cast<uintptr_t>(scratch), 128));
-  auto split = [&](const float *src, long long ld, int rows, int cols) -> void * {
-    const int pitch = tc_pitch(cols);
-    const long long quads = (long long)rows * pitch / 4;
-    const long long want = (quads + 1023) / 1024, cap = (long long)ctx->sm_count * 8;
-    const int blocks = (int)(want < cap ? want : cap);
-    uint32_t *dst = reinterpret_cast<uint32_t *>(next);
-    next += align_up((size_t)rows * pitch * 6, 128);
-    if (cols % 4 == 0 && ld % 4 == 0 && ((uintptr_t)src & 15) == 0)
-      tc_split_kernel<true><<<blocks, 256, 0, ctx->stream>>>(src, rows, cols, ld, pitch, dst);
-    else
-      tc_split_kernel<false><<<blocks, 256, 0, ctx->stream>>>(src, rows, cols, ld, pitch, dst);
-    return dst;
+  auto planes = [&](const GemmOperand &o, int rows, int cols, const void **p) -> int {
+    *p = o.planes ? o.planes : next;
+    if (o.planes) return 0;
+    B200_TRY(gemm_tc_split(ctx, o.src, rows, cols, next));
+    next += align_up((size_t)rows * tc_pitch(cols) * 6, 128);
+    return 0;
   };
   const int ar = a_transposed ? K : M, ac = a_transposed ? M : K, br = b_transposed ? K : N, bc = b_transposed ? N : K;
-  const void *pa = split(src_a, lda, ar, ac);
-  B200_LAUNCHED();
-  const void *pb = split(src_b, ldb, br, bc);
-  B200_LAUNCHED();
+  const void *pa = nullptr, *pb = nullptr;
+  B200_TRY(planes(oa, ar, ac, &pa));
+  B200_TRY(planes(ob, br, bc, &pb));
   // The tile and the split of k: turns that the busiest SM takes times the cycles of a turn: stages of MMAs (N / 2
   // cycles each, a pair's M counts double) or loads (about 22 bytes a cycle and SM), whichever is longer, the
   // epilogue, and for a split k the pass that adds up the partial sums.  (1024 x 784, k = 4096: 118 us in 104 tiles
-  // of 128 x 64, KSPLIT us in 16 tiles of 256 x 256 of four splits.)
+  // of 128 x 64, about 40 us in 16 tiles of 256 x 256 of four splits.)
   struct Shape {
     int cg, bn;
   };

@@ -34,6 +34,7 @@ struct Layer {
   // tensor-core passes: filter blocks of the forward and dX passes, partial weight gradients
   ConvTcUse tc = {};
   float *tc_wt_fwd = nullptr, *tc_wt_dx = nullptr, *tc_part = nullptr;
+  FcPlanes planes;        // fully connected: operands of the tensor-core products, split once a step
   float act_param = 0.f;  // leaky relu: epsilon; elu: alpha
   // batch normalization: shape, constants, this batch's moments, stddev, moving averages, slice sums
   int bn_c = 0, bn_s = 0;
@@ -360,8 +361,11 @@ int net_forward_impl(b200_net *net, const float *x, int B) {
       case B200_LAYER_FC:
         if ((int)i == net->head_fc)
           B200_TRY(fc_softmax_fwd(ctx, L.fc_in, L.fc_out, in, W, b, dst, net->layers[n - 1].out, B));
-        else
-          B200_TRY(fc_fwd(ctx, L.fc_in, L.fc_out, in, W, b, dst, B, L.fused_act, net->scratch));
+        else {
+          L.planes.x_ready = L.planes.w_ready = L.planes.d_ready = false;
+          B200_TRY(fc_split(ctx, L.fc_in, L.fc_out, in, W, nullptr, B, &L.planes, false));
+          B200_TRY(fc_fwd(ctx, L.fc_in, L.fc_out, in, W, b, dst, B, L.fused_act, net->scratch, false, &L.planes));
+        }
         break;
       case B200_LAYER_MAXPOOL:
         B200_TRY(maxpool_fwd(ctx, L.pd, in, dst, L.argmax, B));
@@ -443,13 +447,15 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
   auto fc_backward = [&](Layer &L, bool w_rows, const float *in, float *din, const float *W, float *dW, float *db,
                          bool can_fork) -> int {
     const int n_in = (int)L.in_dim, n_out = (int)L.out_dim;
+    const FcPlanes *planes = w_rows ? nullptr : &L.planes;
+    if (planes) B200_TRY(fc_split(ctx, n_in, n_out, in, W, L.grad, B, &L.planes, true));
     if (!can_fork)
-      return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, dW, db, 0, B, net->scratch, w_rows);
+      return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, dW, db, 0, B, net->scratch, w_rows, planes);
     B200_TRY(fork());
-    rc_side = fc_bwd(ctx, n_in, n_out, in, W, L.grad, nullptr, dW, db, 0, B, net->scratch_side, w_rows);
+    rc_side = fc_bwd(ctx, n_in, n_out, in, W, L.grad, nullptr, dW, db, 0, B, net->scratch_side, w_rows, planes);
     ctx->stream = main_stream;
     if (rc_side) return 0;
-    return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, nullptr, nullptr, 0, B, net->scratch, w_rows);
+    return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, nullptr, nullptr, 0, B, net->scratch, w_rows, planes);
   };
   for (int i = tail_fused ? n - 2 : n - 1; i >= 0 && rc_side == 0; --i) {
     Layer &L = net->layers[i];
@@ -580,6 +586,7 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
     B200_CUDA(cudaStreamWaitEvent(main_stream, net->ev_join, 0));
   }
   if (comm_used) B200_CUDA(cudaStreamWaitEvent(main_stream, net->ev_comm_done, 0));
+  for (Layer &L : net->layers) L.planes.x_ready = L.planes.w_ready = L.planes.d_ready = false;  // of this step only
 
   return rc_side;
 }
@@ -831,6 +838,11 @@ int b200_net_create(b200_ctx *ctx, const b200_layer_spec *specs, int n_layers, i
     size_t need = 0;
     if (L.kind == B200_LAYER_FC || (L.kind == B200_LAYER_CONV && L.tc.fc)) {
       need = fc_scratch_floats(ctx, (int)L.in_dim, (int)L.out_dim, max_batch);
+      if (L.kind == B200_LAYER_FC && fc_any_tc(ctx, L.fc_in, L.fc_out, max_batch)) {
+        net_alloc(net, &L.planes.x, gemm_tc_operand_floats(max_batch, L.fc_in) * f);
+        net_alloc(net, &L.planes.w, gemm_tc_operand_floats(L.fc_in, L.fc_out) * f);
+        net_alloc(net, &L.planes.d, gemm_tc_operand_floats(max_batch, L.fc_out) * f);
+      }
     } else if (L.kind == B200_LAYER_CONV) {
       if ((L.tc.fwd || L.tc.dx || L.tiled) && net->side)
         B200_CUDA(cudaEventCreateWithFlags(&L.ev_prep, cudaEventDisableTiming));
@@ -906,6 +918,7 @@ int b200_net_out_dim(const b200_net *net) { return net ? (int)net->layers.back()
 
 int b200_net_set_params(b200_net *net, const float *host_params) {
   B200_TRY(check_net(net));
+  for (Layer &L : net->layers) L.planes.w_ready = false;
   B200_CUDA(cudaMemcpyAsync(net->params, host_params, net->n_params * sizeof(float),
                             cudaMemcpyHostToDevice, net->ctx->stream));
   B200_CUDA(cudaStreamSynchronize(net->ctx->stream));
