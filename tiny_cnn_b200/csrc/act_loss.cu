@@ -296,9 +296,10 @@ int softmax_loss_bwd(b200_ctx *ctx, int loss_kind, const float *y, const float *
 // (the classifier's last two layers: 64 -> 10 in the CIFAR-10 net).  A warp per sample, the inputs dealt to its lanes;
 // the weights (K x N floats, N <= 16) sit in shared memory.  With sixteen lanes a sample, each adding all the products
 // of an output, the chain of K additions was the kernel's time (500 -> 10, 77 samples: 20 us forward, 16 us backward;
-// now 8.8 and 7.5 us).
-constexpr int FCS_N = 16;
-constexpr size_t FCS_MAX_BYTES = 192 * 1024;  // of weights in shared memory
+// now 3.3 and 3.2 us with the wide form below).
+constexpr int FCS_N = 16, FCS_THREADS = 256;
+constexpr int FCS_NARROW = 256;               // inputs up to which a sample is a warp's work
+constexpr int FCW_THREADS = 512, FCW_WARPS = FCW_THREADS / 32, FCW_SAMPLES = 4;
 
 // the sum of acc[j] over the lanes, in lane j of each half-warp: sums of halves, which leave half the values a step
 __device__ __forceinline__ float lanes_sum16(float *acc) {
@@ -314,61 +315,22 @@ __device__ __forceinline__ float lanes_sum16(float *acc) {
   return acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 16);
 }
 
-// z = x W + b (fully_connected_op_internal.h:15-36), y = softmax(z) (softmax_layer.h:24-34)
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS) fc_softmax_fwd16_kernel(const float *__restrict__ x,
-                                                                       const float *__restrict__ W,
-                                                                       const float *__restrict__ bias,
-                                                                       float *__restrict__ z, float *__restrict__ y,
-                                                                       int K, int N, int B) {
-  extern __shared__ float fcs_w[];  // [K][N]
-  for (int i = threadIdx.x; i < K * N; i += THREADS) cp_async4(fcs_w + i, W + i, true);
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  const int n = (blockIdx.x * THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31, j = lane & 15;
-  if (n >= B) return;
-  const float *xr = x + (size_t)n * K;
-  float acc[FCS_N];
-#pragma unroll
-  for (int i = 0; i < FCS_N; ++i) acc[i] = 0.f;
-#pragma unroll 8
-  for (int k = lane; k < K; k += 32) {
-    const float xk = xr[k];
-    const float *w = fcs_w + k * N;
-#pragma unroll
-    for (int i = 0; i < FCS_N; ++i)
-      if (i < N) acc[i] = fmaf(xk, w[i], acc[i]);
-  }
-  const float sum = lanes_sum16(acc);
+// by a warp: lane j < N holds the products' sum of output j of sample n; z = sum + bias, y = softmax(z)
+__device__ __forceinline__ void head_out(float sum, const float *bias, float *z, float *y, int n, int N) {
+  const int lane = threadIdx.x & 31, j = lane & 15;
   const float zj = (bias != nullptr && j < N) ? sum + bias[j] : sum;
-  const bool live = lane < N;
-  if (live) z[(size_t)n * N + j] = zj;
+  if (lane < N) z[(size_t)n * N + j] = zj;
   float alpha = __shfl_sync(0xffffffffu, zj, 0);
   for (int k = 1; k < N; ++k) alpha = fmaxf(alpha, __shfl_sync(0xffffffffu, zj, k));
   const float ej = expf(zj - alpha);
   float denom = 0.f;
   for (int k = 0; k < N; ++k) denom += __shfl_sync(0xffffffffu, ej, k);
-  if (live) y[(size_t)n * N + j] = ej / denom;
+  if (lane < N) y[(size_t)n * N + j] = ej / denom;
 }
 
-// dy = loss gradient of (y, t); dz = softmax gradient (as softmax_bwd16_kernel); dx = dz W^T
-// (fully_connected_op_internal.h:45-50), multiplied by the gradient of a relu in front of the layer when
-// `relu_x` (that relu's output = this layer's input) is given (relu_layer.h:31-39)
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS) fc_softmax_bwd16_kernel(const float *__restrict__ y,
-                                                                       const float *__restrict__ t, int loss_kind,
-                                                                       const float *__restrict__ W,
-                                                                       const float *__restrict__ relu_x,
-                                                                       float *__restrict__ dy, float *__restrict__ dz,
-                                                                       float *__restrict__ dx, int K, int N, int B) {
-  extern __shared__ float fcs_w[];  // [K][N]
-  for (int i = threadIdx.x; i < K * N; i += THREADS) cp_async4(fcs_w + i, W + i, true);
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  const int n = (blockIdx.x * THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31, j = lane & 15;
-  if (n >= B) return;
+// by a warp: the loss gradient of sample n to dy and the softmax gradient to dz, returned in lane j of each half-warp
+__device__ __forceinline__ float head_grad(const float *y, const float *t, int loss_kind, float *dy, float *dz, int n, int N) {
+  const int lane = threadIdx.x & 31, j = lane & 15;
   const float factor = 2.0f / (float)N;
   float yj = 0.f, gj = 0.f;
   if (j < N) {
@@ -384,6 +346,54 @@ __global__ void __launch_bounds__(THREADS) fc_softmax_bwd16_kernel(const float *
     s = __fadd_rn(s, __fmul_rn(gk, df));
   }
   if (lane < N) dz[(size_t)n * N + j] = s;
+  return s;
+}
+
+// z = x W + b (fully_connected_op_internal.h:15-36), y = softmax(z) (softmax_layer.h:24-34)
+__global__ void __launch_bounds__(FCS_THREADS) fc_softmax_fwd16_kernel(const float *__restrict__ x,
+                                                                       const float *__restrict__ W,
+                                                                       const float *__restrict__ bias,
+                                                                       float *__restrict__ z, float *__restrict__ y,
+                                                                       int K, int N, int B) {
+  extern __shared__ float fcs_w[];  // [K][N]
+  for (int i = threadIdx.x; i < K * N; i += FCS_THREADS) cp_async4(fcs_w + i, W + i, true);
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  const int n = (blockIdx.x * FCS_THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (n >= B) return;
+  const float *xr = x + (size_t)n * K;
+  float acc[FCS_N];
+#pragma unroll
+  for (int i = 0; i < FCS_N; ++i) acc[i] = 0.f;
+#pragma unroll 8
+  for (int k = lane; k < K; k += 32) {
+    const float xk = xr[k];
+    const float *w = fcs_w + k * N;
+#pragma unroll
+    for (int i = 0; i < FCS_N; ++i)
+      if (i < N) acc[i] = fmaf(xk, w[i], acc[i]);
+  }
+  head_out(lanes_sum16(acc), bias, z, y, n, N);
+}
+
+// dy = loss gradient of (y, t); dz = softmax gradient (as softmax_bwd16_kernel); dx = dz W^T
+// (fully_connected_op_internal.h:45-50), multiplied by the gradient of a relu in front of the layer when
+// `relu_x` (that relu's output = this layer's input) is given (relu_layer.h:31-39)
+__global__ void __launch_bounds__(FCS_THREADS) fc_softmax_bwd16_kernel(const float *__restrict__ y,
+                                                                       const float *__restrict__ t, int loss_kind,
+                                                                       const float *__restrict__ W,
+                                                                       const float *__restrict__ relu_x,
+                                                                       float *__restrict__ dy, float *__restrict__ dz,
+                                                                       float *__restrict__ dx, int K, int N, int B) {
+  extern __shared__ float fcs_w[];  // [K][N]
+  for (int i = threadIdx.x; i < K * N; i += FCS_THREADS) cp_async4(fcs_w + i, W + i, true);
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  const int n = (blockIdx.x * FCS_THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (n >= B) return;
+  const float s = head_grad(y, t, loss_kind, dy, dz, n, N);
   if (dx == nullptr) return;
   float d[FCS_N];
 #pragma unroll
@@ -400,25 +410,95 @@ __global__ void __launch_bounds__(THREADS) fc_softmax_bwd16_kernel(const float *
   }
 }
 
-bool fc_softmax_fusable(int K, int N) { return N >= 1 && N <= 16 && K >= 1 && (size_t)K * N * sizeof(float) <= FCS_MAX_BYTES; }
-
-// eight samples a block; sixteen where the weights leave an SM room for one block only
-template <typename... P, typename... A>
-static int launch_head(b200_ctx *ctx, void (*few)(P...), void (*many)(P...), int K, int N, int B, A... args) {
-  const size_t smem = (size_t)K * N * sizeof(float);
-  const int threads = smem > 64 * 1024 ? 512 : 256;
-  auto kernel = threads == 512 ? many : few;
-  B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<ceil_div(B, threads / 32), threads, smem, ctx->stream>>>(args...);
-  B200_LAUNCHED();
-  return 0;
+// The same for longer inputs: a block takes four samples, its threads deal the inputs out, and a row of weights is read
+// once for the four of them.  (4096 -> 10, 1024 samples, a warp a sample: 37 us each way, bound by the shared-memory
+// reads of the weights; now 21 and 20 us.)
+__global__ void __launch_bounds__(FCW_THREADS) fc_softmax_fwd_wide_kernel(const float *__restrict__ x,
+                                                                          const float *__restrict__ W,
+                                                                          const float *__restrict__ bias, float *__restrict__ z,
+                                                                          float *__restrict__ y, int K, int N, int B) {
+  __shared__ float sums[FCW_SAMPLES][FCW_WARPS][FCS_N];
+  const int n0 = blockIdx.x * FCW_SAMPLES, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float acc[FCW_SAMPLES][FCS_N];
+#pragma unroll
+  for (int s = 0; s < FCW_SAMPLES; ++s)
+#pragma unroll
+    for (int i = 0; i < FCS_N; ++i) acc[s][i] = 0.f;
+#pragma unroll 2
+  for (int k = threadIdx.x; k < K; k += FCW_THREADS) {
+    float xk[FCW_SAMPLES];
+#pragma unroll
+    for (int s = 0; s < FCW_SAMPLES; ++s) xk[s] = x[(size_t)min(n0 + s, B - 1) * K + k];
+#pragma unroll
+    for (int i = 0; i < FCS_N; ++i)
+      if (i < N) {
+        const float w = W[(size_t)k * N + i];
+#pragma unroll
+        for (int s = 0; s < FCW_SAMPLES; ++s) acc[s][i] = fmaf(xk[s], w, acc[s][i]);
+      }
+  }
+#pragma unroll
+  for (int s = 0; s < FCW_SAMPLES; ++s) {
+    const float v = lanes_sum16(acc[s]);
+    if (lane < FCS_N) sums[s][warp][lane] = v;
+  }
+  __syncthreads();
+  const int n = n0 + warp;
+  if (warp >= FCW_SAMPLES || n >= B) return;
+  float sum = 0.f;
+  for (int w = 0; w < FCW_WARPS; ++w) sum += sums[warp][w][lane & 15];
+  head_out(sum, bias, z, y, n, N);
 }
+
+__global__ void __launch_bounds__(FCW_THREADS) fc_softmax_bwd_wide_kernel(const float *__restrict__ y,
+                                                                          const float *__restrict__ t, int loss_kind,
+                                                                          const float *__restrict__ W,
+                                                                          const float *__restrict__ relu_x,
+                                                                          float *__restrict__ dy, float *__restrict__ dz,
+                                                                          float *__restrict__ dx, int K, int N, int B) {
+  __shared__ float ds[FCW_SAMPLES][FCS_N];
+  const int n0 = blockIdx.x * FCW_SAMPLES, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < FCW_SAMPLES && n0 + warp < B) {
+    const float s = head_grad(y, t, loss_kind, dy, dz, n0 + warp, N);
+    if (lane < FCS_N) ds[warp][lane] = s;
+  }
+  __syncthreads();
+  if (dx == nullptr) return;
+  const int samples = min(FCW_SAMPLES, B - n0);
+#pragma unroll 2
+  for (int c = threadIdx.x; c < K; c += FCW_THREADS) {  // dx_c = sum_i dz_i W[c][i]
+    float a[FCW_SAMPLES], gate[FCW_SAMPLES];
+#pragma unroll
+    for (int s = 0; s < FCW_SAMPLES; ++s) {
+      a[s] = 0.f;
+      gate[s] = relu_x != nullptr ? relu_x[(size_t)min(n0 + s, B - 1) * K + c] : 1.f;
+    }
+#pragma unroll
+    for (int i = 0; i < FCS_N; ++i)
+      if (i < N) {
+        const float w = W[(size_t)c * N + i];
+#pragma unroll
+        for (int s = 0; s < FCW_SAMPLES; ++s) a[s] = fmaf(ds[s][i], w, a[s]);
+      }
+#pragma unroll
+    for (int s = 0; s < FCW_SAMPLES; ++s)
+      if (s < samples) dx[(size_t)(n0 + s) * K + c] = gate[s] > 0.f ? a[s] : 0.f;
+  }
+}
+
+bool fc_softmax_fusable(int K, int N) { return N >= 1 && N <= FCS_N && K >= 1; }
 
 int fc_softmax_fwd(b200_ctx *ctx, int K, int N, const float *x, const float *W, const float *bias, float *z, float *y,
                    int B) {
   B200_REQUIRE(fc_softmax_fusable(K, N), "fc_softmax_fwd: shape %d x %d not supported", K, N);
   if (B == 0) return 0;
-  return launch_head(ctx, fc_softmax_fwd16_kernel<256>, fc_softmax_fwd16_kernel<512>, K, N, B, x, W, bias, z, y, K, N, B);
+  if (K <= FCS_NARROW)
+    fc_softmax_fwd16_kernel<<<ceil_div(B, FCS_THREADS / 32), FCS_THREADS, (size_t)K * N * sizeof(float), ctx->stream>>>(
+      x, W, bias, z, y, K, N, B);
+  else
+    fc_softmax_fwd_wide_kernel<<<ceil_div(B, FCW_SAMPLES), FCW_THREADS, 0, ctx->stream>>>(x, W, bias, z, y, K, N, B);
+  B200_LAUNCHED();
+  return 0;
 }
 
 int fc_softmax_loss_bwd(b200_ctx *ctx, int loss_kind, int K, int N, const float *y, const float *t, const float *W,
@@ -427,8 +507,14 @@ int fc_softmax_loss_bwd(b200_ctx *ctx, int loss_kind, int K, int N, const float 
   B200_REQUIRE(loss_kind >= B200_LOSS_MSE && loss_kind <= B200_LOSS_CROSS_ENTROPY_MULTICLASS,
                "fc_softmax_loss_bwd: unknown loss %d", loss_kind);
   if (B == 0) return 0;
-  return launch_head(ctx, fc_softmax_bwd16_kernel<256>, fc_softmax_bwd16_kernel<512>, K, N, B, y, t, loss_kind, W, relu_x, dy, dz,
-                     dx, K, N, B);
+  if (K <= FCS_NARROW)
+    fc_softmax_bwd16_kernel<<<ceil_div(B, FCS_THREADS / 32), FCS_THREADS, (size_t)K * N * sizeof(float), ctx->stream>>>(
+      y, t, loss_kind, W, relu_x, dy, dz, dx, K, N, B);
+  else
+    fc_softmax_bwd_wide_kernel<<<ceil_div(B, FCW_SAMPLES), FCW_THREADS, 0, ctx->stream>>>(y, t, loss_kind, W, relu_x, dy, dz, dx,
+                                                                                         K, N, B);
+  B200_LAUNCHED();
+  return 0;
 }
 
 int loss_value(b200_ctx *ctx, int kind, const float *y, const float *t, float *loss_sum, int dim,
