@@ -101,6 +101,11 @@ def _f32(*shape, device):
     return torch.empty(*shape, dtype=torch.float32, device=device)
 
 
+def _sums(n, device, zero):
+    """Buffer of a gradient summed over the batch; the kernels write all of it unless they add to it."""
+    return (torch.zeros if zero else torch.empty)(n, dtype=torch.float32, device=device)
+
+
 def conv_in_len(d: ConvDesc) -> int:
     padded = d.input_is_padded or not d.pad_same
     return d.in_c * (d.inp_h * d.inp_w if padded else d.in_h * d.in_w)
@@ -129,9 +134,10 @@ def conv2d_grad_op(ctx: Context, d: ConvDesc, x, W, dout, need_dx=True, dW=None,
     (dx, dW, db) with dW/db summed over the batch."""
     B = x.shape[0]
     dx = _f32(B, conv_in_len(d), device=x.device) if need_dx else None
-    dW = torch.zeros(conv_w_len(d), dtype=torch.float32, device=x.device) if dW is None else dW
+    zero = accumulate or B == 0 or bool(d.tbl)
+    dW = _sums(conv_w_len(d), x.device, zero) if dW is None else dW
     if d.has_bias and db is None:
-        db = torch.zeros(d.out_c, dtype=torch.float32, device=x.device)
+        db = _sums(d.out_c, x.device, zero)
     check(ctx.lib.b200_conv2d_bwd(ctx.handle, C.byref(d), ptr(x), ptr(W), ptr(dout), ptr(dx),
                                   ptr(dW), ptr(db), int(accumulate), B))
     return dx, dW, db
@@ -151,9 +157,10 @@ def fully_connected_grad_op(ctx: Context, in_size, out_size, x, W, dout, has_bia
     """FullyConnectedGradOp::compute (tiny_dnn/core/kernels/fully_connected_grad_op.h:22-52)."""
     B = x.shape[0]
     dx = _f32(B, in_size, device=x.device) if need_dx else None
-    dW = torch.zeros(in_size * out_size, dtype=torch.float32, device=x.device) if dW is None else dW
+    zero = accumulate or B == 0
+    dW = _sums(in_size * out_size, x.device, zero) if dW is None else dW
     if has_bias and db is None:
-        db = torch.zeros(out_size, dtype=torch.float32, device=x.device)
+        db = _sums(out_size, x.device, zero)
     check(ctx.lib.b200_fc_bwd(ctx.handle, in_size, out_size, ptr(x), ptr(W), ptr(dout), ptr(dx),
                               ptr(dW), ptr(db), int(accumulate), B))
     return dx, dW, db
