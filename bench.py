@@ -250,15 +250,13 @@ def time_kernels(ctx, torch, ops, reps=20):
 
 # DRAM traffic per launch (dram__bytes_read.sum + dram__bytes_write.sum) from the ncu captures
 # summarised under profiles/; None where no capture of that launch exists
-# (profiles/conv_tc_kernel_conv2_fwd_b256_ncu_full.md; conv2's dX launch is the same kernel on
-# tensors of the same sizes -- 32 -> 32 channels, the same 512 tiles -- so the figure stands for both)
-NCU_DRAM_BYTES = {"conv2_fwd": 17.04e6, "conv2_dx": 17.04e6}
+NCU_DRAM_BYTES = {}
 
 
 def conv_rooflines(kt, peaks):
     """Per-kernel table and the roofline object of the dominant kernel.  Tensor-core passes
-    compute every fp32 product as three TF32 products, so their ceiling in algorithmic
-    (fp32-equivalent) flop/s is the TF32 rate / 3 = the measured bf16 rate / 6."""
+    compute every fp32 product as six bf16 products (conv1's as three TF32 products at half the
+    rate), so their ceiling in algorithmic (fp32-equivalent) flop/s is the measured bf16 rate / 6."""
     peak_fp32 = SM_COUNT * FP32_LANES * 2 * 1.965e9 / 1e12
     bf16 = peaks.get("bf16_tflops")
     peak_tc = (bf16 if bf16 else 1590.0) / 6.0
@@ -268,9 +266,9 @@ def conv_rooflines(kt, peaks):
         tf = v["flops"] / (v["ms"] * 1e-3) / 1e12
         peak = peak_tc if v["tensor"] else peak_fp32
         kernels[k] = {"ms": round(v["ms"], 4), "op_ms": round(v["op_ms"], 4), "tflops": round(tf, 3),
-                      "engine": "tcgen05 3xTF32" if v["tensor"] else "fp32 FFMA",
+                      "engine": "tcgen05 bf16x3" if v["tensor"] else "fp32 FFMA",
                       "frac_of_peak": round(tf / peak, 4)}
-    # the kernel function with the largest share of the step: conv_tc_kernel runs the forward and
+    # the kernel function with the largest share of the step: conv_gather_kernel runs the forward and
     # dX passes of every tensor-core layer; report its longest launch
     fam = [k for k, v in kt.items() if v["tensor"] and not k.endswith("_dw")]
     pool = fam if fam else list(kt)
@@ -284,17 +282,17 @@ def conv_rooflines(kt, peaks):
     conv_fl = sum(x["flops"] for x in kt.values())
     op_tf = v["flops"] / (v["op_ms"] * 1e-3) / 1e12
     roofline = {
-        "kernel": ("conv_tc_kernel" if tensor else "conv FFMA kernel") + f" ({dom})",
+        "kernel": ("conv_gather_kernel" if tensor else "conv FFMA kernel") + f" ({dom})",
         "bound": "tensor" if tensor else "fp32",
         "achieved": round(tf, 3), "peak": round(peak, 2), "unit": "TFLOP/s", "frac": round(tf / peak, 4),
         # the same pass as the operator call issues it: the main kernel plus the layout kernels it needs
-        # (tall hi/lo copies, filter matrices, partial-row merges)
+        # (filter matrices, sums of partial results)
         "achieved_op": round(op_tf, 3), "frac_op": round(op_tf / peak, 4),
         "traffic": NCU_DRAM_BYTES.get(dom),
-        "peak_source": (f"algorithmic fp32 flop/s; ceiling = bf16 tensor peak {bf16} TFLOP/s {src} / 2 (TF32 rate) "
-                        "/ 3 (three TF32 products per fp32 product)") if tensor else
+        "peak_source": (f"algorithmic fp32 flop/s; ceiling = bf16 tensor peak {bf16} TFLOP/s {src} / 6 "
+                        "(six bf16 products per fp32 product)") if tensor else
                        "fp32 FFMA: 148 SMs x 128 lanes x 2 flop x clocks.max.sm 1965 MHz (no measured fp32 figure)",
-        "tensor_pipe_tflops": round(3 * tf, 1) if tensor else None,
+        "tensor_pipe_tflops": round(6 * tf, 1) if tensor else None,
         "conv_main_kernels_all": {"ms": round(conv_ms, 4), "tflops": round(conv_fl / (conv_ms * 1e-3) / 1e12, 3)},
         "conv_operator_calls_all": {"ms": round(conv_op_ms, 4),
                                     "tflops": round(conv_fl / (conv_op_ms * 1e-3) / 1e12, 3)},
@@ -520,8 +518,8 @@ def run_b200(args, rank, world, local_rank):
                        "how": f"blocks of {args.steps} steps between barriers, CUDA events, max over ranks, "
                               f"repeated until {MIN_TIMED_MS:.0f} ms were timed; the median block is reported"},
             "notes": {
-                "arithmetic": "fp32 results; conv2/conv3 passes on tcgen05 tensor cores as 3xTF32 (hi/lo split, fp32 "
-                              "accumulation) -- also conv1 forward and dW; conv1 dX and the rest fp32 FFMA",
+                "arithmetic": "fp32 results; conv2/conv3 passes on tcgen05 tensor cores, three bf16 parts of every operand, "
+                              "six products, fp32 accumulation; conv1 forward and dW as 3xTF32; conv1 dX and the rest fp32 FFMA",
                 "step": ("CUDA graph of forward+backward+update" if world == 1 else
                          "one CUDA graph: forward+backward with the gradients of all layers but the first pushed to the "
                          "peers over NVLink from a side branch as soon as they exist, then first-layer push + "

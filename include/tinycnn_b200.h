@@ -68,12 +68,11 @@ B200_API int b200_ctx_sync(b200_ctx *ctx);
 
 /*
  * Context options.  "fc_tensor_cores": 0 = fully-connected GEMMs always on the
- * fp32 FFMA kernels, 1 (default) = large ones on the tensor cores with the
- * 3xTF32 split (fp32-level accuracy), 2 = every GEMM the tensor-core kernel can
- * take.  "conv_tensor_cores": 0 = convolutions never on the tensor cores,
- * 1 (default) = stride-1 layers with at least 16 input and 16 output
- * channels, 2 = every pass the tensor-core kernels can take (stride 1,
- * dilation 1, windows up to 8x8, at most 256 channels either side).  Unknown names are an error.
+ * fp32 FFMA kernels, 1 (default) = large ones on the tensor cores with every
+ * operand split into three bf16 parts (fp32-level accuracy), 2 = every GEMM the
+ * tensor-core kernel can take.  "conv_tensor_cores": 0 = convolutions never on the tensor cores,
+ * 1 (default) = every pass they can take except the gradient with respect to an
+ * input of at most 4 channels where an FFMA kernel takes it, 2 = that one too.  Unknown names are an error.
  */
 B200_API int b200_ctx_set_option(b200_ctx *ctx, const char *name, int value);
 
@@ -619,9 +618,7 @@ B200_API float *b200_net_grads_ptr(b200_net *net);
 B200_API float *b200_net_output_ptr(b200_net *net);
 /* Device pointer to the output of layer `i` / its gradient dE/d out, [batch][dim] CHW rows
  * (tests).  A layer whose activation was folded into its producer has no output of its own
- * (NULL).  The gradient of a convolution whose backward kernels all read the pixel-major copy
- * is kept in that form only, and this buffer is then not written; set the environment variable
- * B200_NET_KEEP_GRADS=1 before b200_net_create to have every gradient here as well. */
+ * (NULL). */
 B200_API float *b200_net_layer_out_ptr(b200_net *net, int i);
 B200_API float *b200_net_layer_grad_ptr(b200_net *net, int i);
 

@@ -90,10 +90,10 @@ struct b200_ctx {
   // device word a kernel sets when a bounded wait ran out; read by b200_ctx_sync
   int *dev_err = nullptr;
 
-  // fully-connected GEMMs on the tensor cores (3xTF32): 0 never, 1 when large, 2 whenever legal
+  // fully-connected GEMMs on the tensor cores (three bf16 parts of every operand): 0 never, 1 when large, 2 whenever legal
   int fc_tensor_cores = 1;
-  // convolutions on the tensor cores: 0 never, 1 for layers with at least 16 channels on
-  // both sides, 2 whenever the geometry allows
+  // convolutions on the tensor cores: 0 never, 1 where they are the faster kernels (conv_tc_use), 2 whenever the
+  // geometry allows
   int conv_tensor_cores = 1;
 
   // tile shapes already chosen, keyed by the problem's dimensions

@@ -934,12 +934,13 @@ int conv_gather_dx(b200_ctx *ctx, const ConvGeom &g, const float *dout, const fl
 
 // Which kernels take the passes of a layer.  The gather kernels take what they can: on layers of 3 to 256
 // channels, 7 to 64 pixels and 1 to 256 samples they were the fastest for 120 of 132 passes timed against the
-// FFMA and general kernels.  Two kinds of layer stay with other kernels:
+// FFMA and general kernels; the others were narrow layers.  Two kinds of layer stay with other kernels:
 //   dX into at most 4 channels: an MMA is 16 columns wide and would be three quarters padding, while
 //     the FFMA kernel for few outputs reads each gradient once (32x32, 32 -> 3 channels, 5x5, 256 samples:
 //     42 us against 104 us);
 //   forward and dW of layers whose whole window has at most 96 / 128 values: the im2col kernels keep all
-//     taps of a pixel in one operand row (same layer: forward 27 us against 32, dW 42 us against 78).
+//     taps of a pixel in one operand row (same layer: forward 24 us against 32, dW with its sums 42 us against 44
+//     with the window's columns folded into the channels).
 ConvTcUse conv_tc_use(const b200_ctx *ctx, const ConvGeom &g, int algo) {
   ConvTcUse u = {false, false, false, false, false, false};
   if (algo == 1 || algo == 2 || (algo != 3 && ctx->conv_tensor_cores == 0)) return u;
