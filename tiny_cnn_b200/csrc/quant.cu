@@ -141,7 +141,7 @@ __device__ __forceinline__ void filter_range(const float *__restrict__ W, int ns
   float mn = W[0], mx = W[0];
   size_t total = (size_t)nseg * seg_len;
   for (size_t t = threadIdx.x; t < total; t += blockDim.x) {
-    size_t s = t / seg_len, e = t - s * seg_len;
+    size_t s = nseg == 1 ? 0 : t / seg_len, e = t - s * seg_len;
     float v = W[s * seg_stride + e];
     mn = fminf(mn, v);
     mx = fmaxf(mx, v);
@@ -713,7 +713,10 @@ __global__ void __launch_bounds__(256) q_fc_range_kernel(const float *__restrict
     for (int i = threadIdx.x; i < out_size; i += 256) wsum[i] = 0u;
 }
 
-// blocks [0, B * rblocks): 1024 bytes of a sample's row; behind them 32 outputs x 256 inputs of the filter each
+// The first blocks take 32 outputs x 128 inputs of the filter each, the others 1024 bytes of a sample's row.  Bound by the latency
+// of a filter block's chain (range, then loads and conversions in double precision), so those start first and are short
+// (9216 -> 256, 128 samples: 18.3 us with 256 inputs a block behind the rows, now 12.07 us).
+constexpr int QF_CIN = 128;
 __global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restrict__ in, int in_size, int B, int pitch,
                                                             int rblocks, const float *__restrict__ W, int out_size,
                                                             const float *__restrict__ bias, int nbias,
@@ -721,17 +724,26 @@ __global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restr
                                                             QGlobal *out_qg, uint8_t *__restrict__ inq,
                                                             uint8_t *__restrict__ Wt, uint8_t *__restrict__ bq,
                                                             unsigned *__restrict__ wsum) {
-  if ((int)blockIdx.x < B * rblocks) {
-    const int n = blockIdx.x / rblocks, j0 = (blockIdx.x - n * rblocks) * 1024 + threadIdx.x * 4;
+  const int b = blockIdx.x, fblocks = gridDim.x - B * rblocks;
+  if (b >= fblocks) {
+    const int n = (b - fblocks) / rblocks, j0 = (b - fblocks - n * rblocks) * 1024 + threadIdx.x * 4;
     const float *r = in + (size_t)n * in_size;
     QScale q;
     q.set(qs[n].min_in, qs[n].max_in);
     int sum = 0;
     if (j0 < pitch) {  // pitch is a multiple of 4
       unsigned w = 0;
+      float x[4];
+      if (j0 + 4 <= in_size && ((uintptr_t)(r + j0) & 15) == 0) {
+        const float4 y = *reinterpret_cast<const float4 *>(r + j0);
+        x[0] = y.x, x[1] = y.y, x[2] = y.z, x[3] = y.w;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = j0 + k < in_size ? r[j0 + k] : 0.f;
+      }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const unsigned v = j0 + k < in_size ? q.of(r[j0 + k]) : 0u;
+        const unsigned v = j0 + k < in_size ? q.of(x[k]) : 0u;
         w |= v << (8 * k);
         sum += (int)v;
       }
@@ -742,11 +754,17 @@ __global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restr
     return;
   }
   __shared__ QGlobal qg;
-  __shared__ uint8_t tile[256][36];
+  __shared__ uint8_t tile[QF_CIN][36];
+  const int oblocks = (out_size + 31) / 32;
+  const int i0 = b % oblocks * 32, c0 = b / oblocks * QF_CIN, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float x[QF_CIN / 8];  // on their way while the range is found
+#pragma unroll
+  for (int k = 0; k < QF_CIN / 8; ++k) {
+    const int c = c0 + warp + 8 * k, i = i0 + lane;
+    x[k] = c < in_size && i < out_size ? W[(size_t)c * out_size + i] : 0.f;
+  }
   // the partial results stand in for the filter: same extremes, and when all are equal so is W[0]
   filter_range(part, 1, 0, (size_t)2 * nparts, bias, nbias, qg);
-  const int b = blockIdx.x - B * rblocks, oblocks = (out_size + 31) / 32;
-  const int i0 = b % oblocks * 32, c0 = b / oblocks * 256, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (b == 0) {
     if (threadIdx.x == 0) *out_qg = qg;
     for (int j = threadIdx.x; j < nbias; j += 256) bq[j] = (uint8_t)f2q<8>(bias[j], qg.min_b, qg.max_b);
@@ -754,23 +772,22 @@ __global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restr
   QScale q;
   q.set(qg.min_f, qg.max_f);
   unsigned sum = 0;
-#pragma unroll 8
-  for (int j = warp; j < 256; j += 8) {
-    const int c = c0 + j, i = i0 + lane;
-    const unsigned v = c < in_size && i < out_size ? q.of(W[(size_t)c * out_size + i]) : 0u;
+#pragma unroll
+  for (int k = 0; k < QF_CIN / 8; ++k) {
+    const int j = warp + 8 * k;
+    const unsigned v = c0 + j < in_size && i0 + lane < out_size ? q.of(x[k]) : 0u;
     tile[j][lane] = (uint8_t)v;
     sum += v;
   }
   if (i0 + lane < out_size && sum) atomicAdd(&wsum[i0 + lane], sum);
   __syncthreads();
-  // a warp writes rows of 256 bytes, a lane 8 bytes of each
+  // a warp writes rows of 128 bytes, a lane 4 bytes of each
   for (int r = warp; r < 32; r += 8) {
     if (i0 + r >= out_size) break;
-    uint2 v;
-    unsigned char *d = reinterpret_cast<unsigned char *>(&v);
+    unsigned v = 0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) d[k] = tile[lane * 8 + k][r];
-    if (c0 + lane * 8 < pitch) *reinterpret_cast<uint2 *>(Wt + (size_t)(i0 + r) * pitch + c0 + lane * 8) = v;
+    for (int k = 0; k < 4; ++k) v |= (unsigned)tile[lane * 4 + k][r] << (8 * k);
+    if (c0 + lane * 4 < pitch) *reinterpret_cast<unsigned *>(Wt + (size_t)(i0 + r) * pitch + c0 + lane * 4) = v;
   }
 }
 
@@ -1107,7 +1124,7 @@ int qfc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const flo
   if (wblocks > Q_PART_BLOCKS) wblocks = Q_PART_BLOCKS;
   q_fc_range_kernel<<<B + wblocks, 256, 0, st>>>(in, in_size, B, W, lenW, out_size, s.qs, s.part, s.acc, wsum);
   B200_LAUNCHED();
-  const int rblocks = ceil_div(pitch, 1024), fblocks = ceil_div(out_size, 32) * ceil_div(pitch, 256);
+  const int rblocks = ceil_div(pitch, 1024), fblocks = ceil_div(out_size, 32) * ceil_div(pitch, QF_CIN);
   q_fc_quantize_kernel<<<B * rblocks + fblocks, 256, 0, st>>>(in, in_size, B, pitch, rblocks, W, out_size, bias, nbias, s.part,
                                                              wblocks, s.qs, s.qg, s.inq, s.Wq, s.bq, wsum);
   B200_LAUNCHED();
