@@ -257,10 +257,19 @@ int peer_reduce_sum_early(b200_ctx *ctx, const PeerReduce *pr, float *grads);
 int peer_reduce_finish(b200_ctx *ctx, const PeerReduce *pr, float *grads, int late_pushed, int early_summed);
 int peer_reduce_run(b200_ctx *ctx, const PeerReduce *pr, float *grads);
 
+// dX beside its gradient through an activation in front of the layer: dst = dX through activation `act` with output y
+struct FcActGrad {
+  const float *y;
+  float *dst;
+  int act;
+  float param;
+};
+bool fc_dx_takes_act(const b200_ctx *ctx, int in_size, int out_size, int B, bool scratch);
 int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
            const float *dout, float *din, float *dW, float *db, int accumulate, int B,
            float *scratch, bool w_rows = false,
-           const FcPlanes *planes = nullptr);
+           const FcPlanes *planes = nullptr,
+           const FcActGrad *ag = nullptr);
 
 int maxpool_fwd(b200_ctx *ctx, const b200_pool_desc &d, const float *in, float *out,
                 int32_t *argmax, int B);

@@ -22,22 +22,19 @@ constexpr int GK = 16;  // tile depth
 // C[m][n] (+)= sum_k A(m,k) * Bm(k,n) (+ bias[n]), then optional activation.
 // A(m,k) = A[m*a_m + k*a_k], Bm(k,n) = Bm[k*b_k + n*b_n], C row-major ldc = N.
 // A_KFAST / B_NFAST say which index is contiguous so tile loads coalesce.
-// With gridDim.z > 1 block z of a cluster reduces k in [z*k_per, (z+1)*k_per).
 template <int BT, int TT, bool A_KFAST, bool B_NFAST>
 __global__ void __launch_bounds__(256) sgemm_kernel(int M, int N, int K, const float *__restrict__ A,
                                                     long long a_m, long long a_k,
                                                     const float *__restrict__ Bm, long long b_k,
                                                     long long b_n, float *__restrict__ C,
                                                     const float *__restrict__ bias, int accumulate,
-                                                    int act, int k_per) {
+                                                    int act) {
   static_assert(BT / TT == 16, "256 threads as 16 x 16");
   __shared__ __align__(16) float As[GK][BT + 4];
   __shared__ __align__(16) float Bs[GK][BT + 4];
   const int tid = threadIdx.x;
   const int m0 = blockIdx.y * BT, n0 = blockIdx.x * BT;
   const int tm = (tid / 16) * TT, tn = (tid % 16) * TT;
-  const int kbeg = blockIdx.z * k_per;
-  const int kend = min(K, kbeg + k_per);
   float acc[TT][TT];
 #pragma unroll
   for (int i = 0; i < TT; ++i)
@@ -53,12 +50,12 @@ __global__ void __launch_bounds__(256) sgemm_kernel(int M, int N, int K, const f
       const int mm = A_KFAST ? idx / GK : idx % BT, kk = A_KFAST ? idx % GK : idx / BT;
       const int nn = B_NFAST ? idx % BT : idx / GK, kb = B_NFAST ? idx / BT : idx % GK;
       const int m = m0 + mm, n = n0 + nn;
-      ar[e] = (m < M && k0 + kk < kend) ? A[m * a_m + (k0 + kk) * a_k] : 0.f;
-      br[e] = (n < N && k0 + kb < kend) ? Bm[(k0 + kb) * b_k + n * b_n] : 0.f;
+      ar[e] = (m < M && k0 + kk < K) ? A[m * a_m + (k0 + kk) * a_k] : 0.f;
+      br[e] = (n < N && k0 + kb < K) ? Bm[(k0 + kb) * b_k + n * b_n] : 0.f;
     }
   };
-  fetch(kbeg);
-  for (int k0 = kbeg; k0 < kend; k0 += GK) {
+  fetch(0);
+  for (int k0 = 0; k0 < K; k0 += GK) {
 #pragma unroll
     for (int e = 0; e < PER; ++e) {
       const int idx = tid + e * 256;
@@ -66,7 +63,7 @@ __global__ void __launch_bounds__(256) sgemm_kernel(int M, int N, int K, const f
       Bs[B_NFAST ? idx / BT : idx % GK][B_NFAST ? idx % BT : idx / GK] = br[e];
     }
     __syncthreads();
-    if (k0 + GK < kend) fetch(k0 + GK);
+    if (k0 + GK < K) fetch(k0 + GK);
 #pragma unroll
     for (int kk = 0; kk < GK; ++kk) {
       float av[TT], bv[TT];
@@ -82,48 +79,195 @@ __global__ void __launch_bounds__(256) sgemm_kernel(int M, int N, int K, const f
     }
     __syncthreads();
   }
-  auto store = [&](int m, int n, float v) {
-    if (m >= M || n >= N) return;
-    const size_t ci = (size_t)m * N + n;
-    if (bias) v += bias[n];
-    if (accumulate) v += C[ci];
-    C[ci] = apply_act(v, act);
+#pragma unroll
+  for (int i = 0; i < TT; ++i)
+#pragma unroll
+    for (int j = 0; j < TT; ++j) {
+      const int m = m0 + tm + i, n = n0 + tn + j;
+      if (m >= M || n >= N) continue;
+      const size_t ci = (size_t)m * N + n;
+      float v = acc[i][j];
+      if (bias) v += bias[n];
+      if (accumulate) v += C[ci];
+      C[ci] = apply_act(v, act);
+    }
+}
+
+// The same product for the sizes whose 64x64 tiles do not fill the chip.  What bounds such a product is latency: a
+// block has a few hundred k's.  So its loads are asked for at once, 16 bytes each where the operand allows it (up to
+// four stages of 64 k's; a slice of up to 256 k's pays one trip to memory), in the operand's own layout, and four groups
+// of 64 threads share a stage's k's, 4 x 4 outputs a thread: eight 16-byte reads of shared memory for 64
+// multiplications.  The groups' sums are added first, then those of the cluster's blocks.
+// (784-500-500-10 with 77 samples: the first layer 10.9 us with 16 k's a stage and 2 x 2 outputs a thread, which the loads'
+// latency and four 4-byte reads for four multiplications held up, now 7.5; with 4096 hidden units the step of 77 samples went
+// from 941 to 449 us, of 8 from 411 to 265.)
+struct FcTileArgs {
+  int M, N, K, k_per;
+  const float *A, *Bm;   // rows are contiguous: A [M][K] (A_KFAST) or [K][M], Bm [K][N] (B_NFAST) or [N][K]
+  int lda, ldb, va, vb;  // va, vb: 16-byte copies (rows and first value lie on 16-byte boundaries)
+  float *C;
+  const float *bias;
+  int accumulate, act;
+  float *col_sum;        // optional (B_NFAST): (+)= the sums of Bm over k, the bias gradient beside dW
+  const float *y;        // optional: C2 = C through the gradient of an activation whose output is y
+  float *C2;
+  int y_act;
+  float y_param;
+};
+
+constexpr int FT = 32, FT_K = 64, FT_STAGES = 4, FT_GROUPS = 4;
+constexpr int FT_KP = FT_K + 4;                // pitch of a row of k's: eight rows' 16 bytes on different banks
+constexpr int FT_OP = FT * FT_KP;              // floats of one operand's stage (either layout)
+constexpr int FT_SMEM = FT_STAGES * 2 * FT_OP * 4;
+
+template <bool A_KFAST, bool B_NFAST>
+__global__ void __launch_bounds__(256) fc_tile_kernel(const __grid_constant__ FcTileArgs a) {
+  extern __shared__ __align__(16) float fsm[];
+  __shared__ __align__(16) float psum[(FT + 1) * FT];  // the block's sums, and those of Bm
+  const int tid = threadIdx.x, group = tid >> 6, tm = (tid >> 3) & 7, tn = tid & 7;
+  const int m0 = blockIdx.y * FT, n0 = blockIdx.x * FT;
+  const int kbeg = blockIdx.z * a.k_per, kend = min(a.K, kbeg + a.k_per);
+  const int nst = (kend - kbeg + FT_K - 1) / FT_K;
+  // rows of 64 k's, or k rows of 32 values; outside the matrix and the slice zero
+  auto load = [&](float *dst, const float *src, int ld, bool kfast, int r0, int rows, int k0, int vec) {
+    if (vec) {
+#pragma unroll
+      for (int e = 0; e < FT * FT_K / 4 / 256; ++e) {
+        const int p = tid + e * 256, r = kfast ? p / (FT_K / 4) : p % (FT / 4) * 4, k = kfast ? p % (FT_K / 4) * 4 : p / (FT / 4);
+        const bool ok = r0 + r < rows && k0 + k < kend;
+        const size_t at = kfast ? (size_t)(r0 + r) * ld + k0 + k : (size_t)(k0 + k) * ld + r0 + r;
+        cp_async16(dst + (kfast ? r * FT_KP + k : k * FT + r), src + (ok ? at : 0), ok);
+      }
+    } else {
+#pragma unroll 4
+      for (int e = 0; e < FT * FT_K / 256; ++e) {
+        const int p = tid + e * 256, r = kfast ? p / FT_K : p % FT, k = kfast ? p % FT_K : p / FT;
+        const bool ok = r0 + r < rows && k0 + k < kend;
+        const size_t at = kfast ? (size_t)(r0 + r) * ld + k0 + k : (size_t)(k0 + k) * ld + r0 + r;
+        cp_async4(dst + (kfast ? r * FT_KP + k : k * FT + r), src + (ok ? at : 0), ok);
+      }
+    }
   };
-  if (gridDim.z == 1) {
+  auto fetch = [&](int i) {
+    if (i < nst) {
+      float *d = fsm + (i % FT_STAGES) * 2 * FT_OP;
+      load(d, a.A, a.lda, A_KFAST, m0, a.M, kbeg + i * FT_K, a.va);
+      load(d + FT_OP, a.Bm, a.ldb, !B_NFAST, n0, a.N, kbeg + i * FT_K, a.vb);
+    }
+    cp_async_commit();
+  };
+  const bool sums = B_NFAST && a.col_sum && blockIdx.y == 0;
+  float acc[4][4], cs[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < TT; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < TT; ++j) store(m0 + tm + i, n0 + tn + j, acc[i][j]);
-    return;
-  }
-  if constexpr (BT == 32) {
-    __shared__ float part[32 * 32];
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 #pragma unroll
-    for (int i = 0; i < TT; ++i)
+  for (int i = 0; i < FT_STAGES - 1; ++i) fetch(i);
+  for (int st = 0; st < nst; ++st) {
+    fetch(st + FT_STAGES - 1);  // into the stage that was read before the last barrier
+    cp_async_wait<FT_STAGES - 1>();
+    __syncthreads();
+    const float *as = fsm + (st % FT_STAGES) * 2 * FT_OP, *bs = as + FT_OP;
+    // rows of k's: a thread has every eighth row, so that a warp's rows are neighbours; k rows: four values side by side
 #pragma unroll
-      for (int j = 0; j < TT; ++j) part[(tm + i) * 32 + tn + j] = acc[i][j];
-    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
-    const int Z = gridDim.z;
-    const uint32_t at = smem_u32(part);
-    for (int e = blockIdx.z * 256 + tid; e < 1024; e += Z * 256) {
-      float v[8];
+    for (int kk = 0; kk < FT_K / FT_GROUPS; kk += 4) {
+      const int k = group * (FT_K / FT_GROUPS) + kk;
+      float av[4][4], bv[4][4];  // [k][row]
 #pragma unroll
-      for (int z = 0; z < 8; ++z) {
-        v[z] = 0.f;
-        if (z < Z) {
-          uint32_t ra;
-          asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(at + 4u * e), "r"(z));
-          asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v[z]) : "r"(ra) : "memory");
+      for (int i = 0; i < 4; ++i) {
+        const float4 x = *reinterpret_cast<const float4 *>(A_KFAST ? as + (i * 8 + tm) * FT_KP + k : as + (k + i) * FT + tm * 4);
+        const float4 z = *reinterpret_cast<const float4 *>(B_NFAST ? bs + (k + i) * FT + tn * 4 : bs + (i * 8 + tn) * FT_KP + k);
+        const float xv[4] = {x.x, x.y, x.z, x.w}, zv[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (A_KFAST) av[j][i] = xv[j];
+          else av[i][j] = xv[j];
+          if (B_NFAST) bv[i][j] = zv[j];
+          else bv[j][i] = zv[j];
         }
       }
-      float sum = v[0];
 #pragma unroll
-      for (int z = 1; z < 8; ++z)
-        if (z < Z) sum += v[z];
-      store(m0 + e / 32, n0 + e % 32, sum);
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[q][i], bv[q][j], acc[i][j]);
+      if (B_NFAST && sums)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) cs[j] += (bv[0][j] + bv[1][j]) + (bv[2][j] + bv[3][j]);
     }
-    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+    __syncthreads();
   }
+  // the groups' sums, in the stages' place: [group][row][32], row 32 the sums of Bm
+  cp_async_wait<0>();
+  float *part = fsm + group * (FT + 1) * FT;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = A_KFAST ? i * 8 + tm : tm * 4 + i;
+    if (B_NFAST)
+      *reinterpret_cast<float4 *>(part + m * FT + tn * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    else
+#pragma unroll
+      for (int j = 0; j < 4; ++j) part[m * FT + j * 8 + tn] = acc[i][j];
+  }
+  if (B_NFAST && sums && tm == 0) *reinterpret_cast<float4 *>(part + FT * FT + tn * 4) = make_float4(cs[0], cs[1], cs[2], cs[3]);
+  __syncthreads();
+  const int quads = (FT * FT + (sums ? FT : 0)) / 4;
+  for (int e = tid; e < quads; e += 256) {
+    float4 v = reinterpret_cast<const float4 *>(fsm)[e];
+#pragma unroll
+    for (int g = 1; g < FT_GROUPS; ++g) {
+      const float4 w = reinterpret_cast<const float4 *>(fsm + g * (FT + 1) * FT)[e];
+      v.x += w.x, v.y += w.y, v.z += w.z, v.w += w.w;
+    }
+    reinterpret_cast<float4 *>(psum)[e] = v;
+  }
+  const int Z = gridDim.z;
+  if (Z == 1)
+    __syncthreads();
+  else
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+  const uint32_t at = smem_u32(psum);
+  const int share = (quads + Z - 1) / Z, last = min(quads, ((int)blockIdx.z + 1) * share);
+  for (int e = blockIdx.z * share + tid; e < last; e += 256) {
+    float v[8][4];
+#pragma unroll
+    for (int z = 0; z < 8; ++z)
+      if (z < Z) {
+        uint32_t ra = at + 16u * e;
+        if (Z > 1) asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(at + 16u * e), "r"(z));
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                     : "=f"(v[z][0]), "=f"(v[z][1]), "=f"(v[z][2]), "=f"(v[z][3])
+                     : "r"(ra)
+                     : "memory");
+      }
+#pragma unroll
+    for (int z = 1; z < 8; ++z)
+      if (z < Z)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[0][j] += v[z][j];
+    const int m = m0 + e / (FT / 4), n = n0 + e % (FT / 4) * 4;
+    if (e >= FT * FT / 4) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (n + j < a.N) a.col_sum[n + j] = a.accumulate ? a.col_sum[n + j] + v[0][j] : v[0][j];
+      continue;
+    }
+    if (m >= a.M) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (n + j >= a.N) break;
+      const size_t ci = (size_t)m * a.N + n + j;
+      float r = v[0][j];
+      if (a.bias) r += a.bias[n + j];
+      if (a.accumulate) r += a.C[ci];
+      r = apply_act(r, a.act);
+      a.C[ci] = r;
+      if (a.C2) a.C2[ci] = act_grad(a.y_act, a.y_param, a.y[ci], r);
+    }
+  }
+  if (Z > 1) asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
 }
 
 // db[i] (+)= sum_n dout[n*N + i]: 32 columns x 8 row-lanes per block, lanes
@@ -169,7 +313,7 @@ static GemmPlan plan_gemm(const b200_ctx *ctx, int M, int N, int K) {
   int max_by_k = ceil_div(K > 0 ? K : 1, 64);               // at least 64 of k per slice
   int s = want < max_by_k ? want : max_by_k;
   if (s < 1) s = 1;
-  int k_per = ceil_div(ceil_div(K > 0 ? K : 1, s), GK) * GK;
+  int k_per = ceil_div(ceil_div(K > 0 ? K : 1, s), GK) * GK;  // whole 16-byte pieces of a row
   p.k_per = k_per;
   p.slices = ceil_div(K > 0 ? K : 1, k_per);
   return p;
@@ -195,20 +339,33 @@ size_t fc_scratch_floats(const b200_ctx *ctx, int in_size, int out_size, int B, 
   return need;
 }
 
+// Product with operands in contiguous rows: A [M][K] (A_KFAST) or [K][M], Bm [K][N] (B_NFAST) or [N][K].  `col_sum` and `ag` (see
+// FcTileArgs) are taken by the small tiles alone: they are asked for where plan_gemm gives those.
 template <bool A_KFAST, bool B_NFAST>
-static int run_gemm(b200_ctx *ctx, int M, int N, int K, const float *A, long long a_m,
-                    long long a_k, const float *Bm, long long b_k, long long b_n, float *C,
-                    const float *bias, int accumulate, int act) {
+static int run_gemm(b200_ctx *ctx, int M, int N, int K, const float *A, const float *Bm, float *C, const float *bias, int accumulate,
+                    int act, float *col_sum = nullptr, const FcActGrad *ag = nullptr) {
   if (M == 0 || N == 0) return 0;
-  GemmPlan p = plan_gemm(ctx, M, N, K);
-  dim3 grid(ceil_div(N, p.tile), ceil_div(M, p.tile), p.slices);
+  const GemmPlan p = plan_gemm(ctx, M, N, K);
+  const dim3 grid(ceil_div(N, p.tile), ceil_div(M, p.tile), p.slices);
+  const int lda = A_KFAST ? K : M, ldb = B_NFAST ? N : K;
   if (p.tile == 64) {
-    sgemm_kernel<64, 4, A_KFAST, B_NFAST><<<grid, 256, 0, ctx->stream>>>(
-      M, N, K, A, a_m, a_k, Bm, b_k, b_n, C, bias, accumulate, act, p.k_per);
+    sgemm_kernel<64, 4, A_KFAST, B_NFAST><<<grid, 256, 0, ctx->stream>>>(M, N, K, A, A_KFAST ? lda : 1, A_KFAST ? 1 : lda, Bm,
+                                                                         B_NFAST ? ldb : 1, B_NFAST ? 1 : ldb, C, bias,
+                                                                         accumulate, act);
   } else {
+    FcTileArgs a = {};
+    a.M = M, a.N = N, a.K = K, a.k_per = p.k_per;
+    a.A = A, a.Bm = Bm, a.lda = lda, a.ldb = ldb;
+    a.va = lda % 4 == 0 && ((uintptr_t)A & 15) == 0;
+    a.vb = ldb % 4 == 0 && ((uintptr_t)Bm & 15) == 0;
+    a.C = C, a.bias = bias, a.accumulate = accumulate, a.act = act;
+    a.col_sum = col_sum;
+    if (ag) a.y = ag->y, a.C2 = ag->dst, a.y_act = ag->act, a.y_param = ag->param;
+    B200_CUDA(cudaFuncSetAttribute(fc_tile_kernel<A_KFAST, B_NFAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM));
     cudaLaunchConfig_t c = {};
     c.gridDim = grid;
     c.blockDim = dim3(256);
+    c.dynamicSmemBytes = FT_SMEM;
     c.stream = ctx->stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -216,8 +373,7 @@ static int run_gemm(b200_ctx *ctx, int M, int N, int K, const float *A, long lon
     at[0].val.clusterDim.z = (unsigned)p.slices;
     c.attrs = at;
     c.numAttrs = 1;
-    B200_CUDA(cudaLaunchKernelEx(&c, sgemm_kernel<32, 2, A_KFAST, B_NFAST>, M, N, K, A, a_m, a_k, Bm, b_k, b_n, C, bias,
-                                 accumulate, act, p.k_per));
+    B200_CUDA(cudaLaunchKernelEx(&c, fc_tile_kernel<A_KFAST, B_NFAST>, a));
   }
   B200_LAUNCHED();
   return 0;
@@ -262,29 +418,30 @@ int fc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const floa
     return gemm_tc(ctx, B, out_size, in_size, operand(in, p.x, p.x_ready), false, operand(W, p.w, p.w_ready), !w_rows, out, bias,
                    0, act, scratch);
   // M = B, N = out, K = in; A = in (k fast), Bm(k, n) = W[k][n] (n fast) or W[n][k] (k fast)
-  if (w_rows)
-    return run_gemm<true, false>(ctx, B, out_size, in_size, in, in_size, 1, W, 1, in_size, out, bias, 0, act);
-  return run_gemm<true, true>(ctx, B, out_size, in_size, in, in_size, 1, W, out_size, 1, out, bias,
-                              0, act);
+  if (w_rows) return run_gemm<true, false>(ctx, B, out_size, in_size, in, W, out, bias, 0, act);
+  return run_gemm<true, true>(ctx, B, out_size, in_size, in, W, out, bias, 0, act);
+}
+
+// whether the dX pass can also form the gradient through an activation in front of the layer
+bool fc_dx_takes_act(const b200_ctx *ctx, int in_size, int out_size, int B, bool scratch) {
+  return !(scratch && use_tc(ctx, B, in_size, out_size)) && plan_gemm(ctx, B, in_size, out_size).tile == FT;
 }
 
 int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
            const float *dout, float *din, float *dW, float *db, int accumulate, int B,
-           float *scratch, bool w_rows, const FcPlanes *planes) {
+           float *scratch, bool w_rows, const FcPlanes *planes, const FcActGrad *ag) {
   const FcPlanes p = planes ? *planes : FcPlanes();
   if (din && scratch && use_tc(ctx, B, in_size, out_size)) {
     // din[B][in] = dout[B][out] * W^T: A = dout; Bt[n = c][k = o] = W[c*out + o] as stored
     B200_TRY(gemm_tc(ctx, B, in_size, out_size, operand(dout, p.d, p.d_ready), false, operand(W, p.w, p.w_ready), w_rows, din,
                      nullptr, 0, 0, scratch));
   } else if (din && w_rows) {
-    B200_TRY((run_gemm<true, true>(ctx, B, in_size, out_size, dout, out_size, 1, W, in_size, 1,
-                                   din, nullptr, 0, 0)));
+    B200_TRY((run_gemm<true, true>(ctx, B, in_size, out_size, dout, W, din, nullptr, 0, 0, nullptr, ag)));
   } else if (din) {
-    // din[B][in] = dout[B][out] * W^T : M = B, N = in, K = out;
-    // Bm(k = o, n = c) = W[c*out + o] -> b_k = 1, b_n = out (k fast)
-    B200_TRY((run_gemm<true, false>(ctx, B, in_size, out_size, dout, out_size, 1, W, 1, out_size,
-                                    din, nullptr, 0, 0)));
+    // din[B][in] = dout[B][out] * W^T : M = B, N = in, K = out; Bm(k = o, n = c) = W[c*out + o] (k fast)
+    B200_TRY((run_gemm<true, false>(ctx, B, in_size, out_size, dout, W, din, nullptr, 0, 0, nullptr, ag)));
   }
+  bool db_done = false;
   if (dW) {
     // dW[in][out] (+)= in^T * dout, or dW[out][in] (+)= dout^T * in
     const float *l = w_rows ? dout : in, *r = w_rows ? in : dout;
@@ -292,11 +449,13 @@ int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const floa
     if (scratch && use_tc(ctx, M, N, B))
       B200_TRY(gemm_tc(ctx, M, N, B, operand(l, p.x, p.x_ready && !w_rows), true, operand(r, p.d, p.d_ready && !w_rows), true, dW,
                        nullptr, accumulate, 0, scratch));
-    else
-      // A(m, k = n) = l[n*M + m] (m fast)
-      B200_TRY((run_gemm<false, true>(ctx, M, N, B, l, 1, M, r, N, 1, dW, nullptr, accumulate, 0)));
+    else {
+      // A(m, k = n) = l[n*M + m] (m fast); the bias gradient is the sum of the right operand over k
+      db_done = db && !w_rows && plan_gemm(ctx, M, N, B).tile == FT;
+      B200_TRY((run_gemm<false, true>(ctx, M, N, B, l, r, dW, nullptr, accumulate, 0, db_done ? db : nullptr)));
+    }
   }
-  if (db) {
+  if (db && !db_done) {
     col_sum_kernel<<<ceil_div(out_size, 32), dim3(32, 8), 0, ctx->stream>>>(dout, db, B, out_size,
                                                                            accumulate);
     B200_LAUNCHED();

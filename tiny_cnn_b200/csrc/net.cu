@@ -472,19 +472,30 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
   // The sums over a tensor-core dW kernel's partial results go to a third stream: behind their kernel they would hold
   // up the next layer's dW on the side branch.  With peers they stay there, since the gradients leave early.
   bool sums_used = false;
+  int act_done = -1;  // the activation layer whose gradient came with the dX of the layer behind it
   // a fully-connected layer, or a convolution that is one (w_rows)
   auto fc_backward = [&](Layer &L, bool w_rows, const float *in, float *din, const float *W, float *dW, float *db,
-                         bool can_fork) -> int {
+                         bool can_fork, int before) -> int {
     const int n_in = (int)L.in_dim, n_out = (int)L.out_dim;
+    FcActGrad ag = {};  // an activation in front of the layer: its gradient with the dX
+    if (net->fuse && din && before >= 0) {
+      Layer &A = net->layers[before];
+      float *target = before > 0 ? net->layers[before - 1].grad : net->input_grad ? net->in_grad : nullptr;
+      if (act_of_layer(A.kind) != B200_ACT_NONE && A.kind != B200_LAYER_SOFTMAX && target && !A.bwd_done_by_next && fc_dx_takes_act(ctx, n_in, n_out, B, net->scratch != nullptr)) {
+        ag = {A.out, target, act_of_layer(A.kind), A.act_param};
+        act_done = before;
+      }
+    }
     const FcPlanes *planes = w_rows ? nullptr : &L.planes;
     if (planes) B200_TRY(fc_split(ctx, n_in, n_out, in, W, L.grad, B, &L.planes, true));
     if (!can_fork)
-      return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, dW, db, 0, B, net->scratch, w_rows, planes);
+      return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, dW, db, 0, B, net->scratch, w_rows, planes, ag.dst ? &ag : nullptr);
     B200_TRY(fork());
     rc_side = fc_bwd(ctx, n_in, n_out, in, W, L.grad, nullptr, dW, db, 0, B, net->scratch_side, w_rows, planes);
     ctx->stream = main_stream;
     if (rc_side) return 0;
-    return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, nullptr, nullptr, 0, B, net->scratch, w_rows, planes);
+    return fc_bwd(ctx, n_in, n_out, in, W, L.grad, din, nullptr, nullptr, 0, B, net->scratch, w_rows, planes,
+                  ag.dst ? &ag : nullptr);
   };
   for (int i = tail_fused ? n - 2 : n - 1; i >= 0 && rc_side == 0; --i) {
     Layer &L = net->layers[i];
@@ -500,7 +511,7 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
     switch (L.kind) {
       case B200_LAYER_CONV: {
         if (L.tc.fc) {
-          B200_TRY(fc_backward(L, true, in, din, W, dW, db, can_fork));
+          B200_TRY(fc_backward(L, true, in, din, W, dW, db, can_fork, i - 1));
           break;
         }
         bool tiled_bwd = L.tiled && L.g.OW <= 64;
@@ -555,7 +566,7 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
         break;
       }
       case B200_LAYER_FC:
-        B200_TRY(fc_backward(L, false, in, din, W, dW, db, can_fork));
+        B200_TRY(fc_backward(L, false, in, din, W, dW, db, can_fork, i - 1));
         break;
       case B200_LAYER_MAXPOOL:
         if (L.relu_bwd_fused) {
@@ -578,6 +589,7 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
       case B200_LAYER_SIGMOID:
       case B200_LAYER_LEAKY_RELU:
       case B200_LAYER_ELU:
+        if (i == act_done) break;
         if (L.bwd_done_by_next) break;  // the pooling layer after it already wrote din
         if (din)
           B200_TRY(act_bwd(ctx, act_of_layer(L.kind), L.out, L.grad, din, (int)L.out_dim, B, L.act_param));
