@@ -87,6 +87,9 @@ struct b200_ctx {
   void *pinned = nullptr;
   size_t pinned_bytes = 0;
 
+  // recorded when every block of the next dX kernel has begun (launch_kernel clears it); null: not asked for
+  cudaEvent_t started = nullptr;
+
   // device word a kernel sets when a bounded wait ran out; read by b200_ctx_sync
   int *dev_err = nullptr;
 
@@ -104,6 +107,34 @@ struct b200_ctx {
 };
 
 namespace b200 {
+
+// a launch with clusters of `cluster` blocks along x that records ctx->started
+template <typename... Params, typename... Args>
+int launch_kernel(b200_ctx *ctx, void (*kernel)(Params...), dim3 grid, int threads, size_t smem, int cluster, const Args &...args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = ctx->stream;
+  cudaLaunchAttribute at[2];
+  if (cluster > 1) {
+    at[c.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[c.numAttrs].val.clusterDim.x = (unsigned)cluster;
+    at[c.numAttrs].val.clusterDim.y = at[c.numAttrs].val.clusterDim.z = 1;
+    ++c.numAttrs;
+  }
+  if (ctx->started) {
+    at[c.numAttrs].id = cudaLaunchAttributeLaunchCompletionEvent;
+    at[c.numAttrs].val.launchCompletionEvent.event = ctx->started;
+    at[c.numAttrs].val.launchCompletionEvent.flags = 0;
+    ++c.numAttrs;
+    ctx->started = nullptr;
+  }
+  c.attrs = at;
+  B200_CUDA(cudaLaunchKernelEx(&c, kernel, args...));
+  B200_LAUNCHED();
+  return 0;
+}
 
 int ctx_scratch(b200_ctx *ctx, size_t bytes, void **out);
 int ctx_arena(b200_ctx *ctx, size_t bytes, void **out);
@@ -151,6 +182,7 @@ int conv_tiled_fwd(b200_ctx *ctx, const ConvGeom &g, const float *in, const floa
 int conv_tiled_dx_prep(b200_ctx *ctx, const ConvGeom &g, const float *W, float *scratch);
 int conv_tiled_dx(b200_ctx *ctx, const ConvGeom &g, const float *W, const float *dout,
                   float *din, int B, float *scratch, int prep = 1);
+int conv_tiled_dx_blocks(const b200_ctx *ctx, const ConvGeom &g, int B);  // blocks of the kernel for few channels; 0: another one
 // Writes `*splits` partial sums of [dW | db] (row length conv_weight_len + OC)
 // into scratch; the caller merges them in row order.
 int conv_tiled_dw_partials(b200_ctx *ctx, const ConvGeom &g, const float *in,
@@ -165,6 +197,7 @@ int conv_gather_prep(b200_ctx *ctx, const ConvGeom &g, const float *W, float *wt
 int conv_gather_fwd(b200_ctx *ctx, const ConvGeom &g, const float *in, const float *wt, const float *bias, float *out,
                     int B, int act);
 int conv_gather_dx(b200_ctx *ctx, const ConvGeom &g, const float *dout, const float *wt, float *din, int B);
+int conv_gather_dx_blocks(const b200_ctx *ctx, const ConvGeom &g, int B);  // SMs that it takes
 // dW and db the same way (conv_gather_dw.cu), any stride; `part` holds conv_gather_dw_floats of `plan_batch`, the batch that
 // the tiling is chosen for (at least B)
 bool conv_gather_dw_ok(const b200_ctx *ctx, const ConvGeom &g);

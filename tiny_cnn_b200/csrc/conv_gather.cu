@@ -763,6 +763,41 @@ int least_units(const GatherPlan &p) {
   return n;
 }
 
+// CTA pair or single CTAs, and S: the least time of the busiest SM, tile after tile, a tile taking the
+// longer of its MMAs (N / 2 cycles each, with a floor; pairs measured 1.2 x as fast) and its loads (about
+// 40 cycles for 32 places of a channel pair).
+struct GatherShape {
+  int CG, S, ks, blocks;
+};
+
+GatherShape gather_shape(const b200_ctx *ctx, const GatherPlan &p, int B) {
+  GatherShape sh = {1, 1, 1, 0};
+  long long best = -1;
+  for (int cg = 2; cg >= 1; --cg) {
+    for (int S = p.S; S >= 1; S /= 2) {
+      const int ks = S == 1 && p.ND >= 2 && least_units(p) >= 2 ? 2 : 1;
+      const long long slots = ctx->sm_count / cg;
+      long long tiles = 0, tile_cost = 0;
+      for (int i = 0; i < p.nphases; ++i) {
+        const ConvPhase &q = p.ph[i];
+        tiles += ((long long)B * q.PH * q.PW + cg * S * 128 - 1) / (cg * S * 128);
+        const long long units = (long long)p.nslab * ((q.kslab + 31) / 32) * S;
+        // about 900 cycles of an issuer's instructions a unit
+        const long long issue = S * ks > 1 ? 450 : 900;
+        const long long mma = units * (p.NP * 6 > issue ? p.NP * 6 : issue) * (cg == 2 ? 5 : 6) / 5;
+        const long long load = (long long)p.nslab * ((p.CS + 1) / 2) * ((rows_needed(q, p, S * 128) * q.pitch + 31) / 32) * 40;
+        tile_cost += mma > load ? mma : load;
+      }
+      const long long cost = (tiles * p.ngroups + slots - 1) / slots * (tile_cost / p.nphases + 2000);
+      if (best < 0 || cost < best) {
+        best = cost;
+        sh = {cg, S, ks, (int)min(tiles * p.ngroups, slots) * cg};
+      }
+    }
+  }
+  return sh;
+}
+
 int launch_conv_gather(b200_ctx *ctx, const GatherPlan &p, const ConvGeom &g, int for_dx, const float *in, const float *filt,
                        const float *bias, float *out, int B, int act) {
   // the kernel counts pixels and tiles in 32 bits
@@ -804,35 +839,10 @@ int launch_conv_gather(b200_ctx *ctx, const GatherPlan &p, const ConvGeom &g, in
   a.nphases = p.nphases;
   a.koff_len = p.koff_len;
   a.act = act;
-  // CTA pair or single CTAs, and S: the least time of the busiest SM, tile after tile, a tile taking the
-  // longer of its MMAs (N / 2 cycles each, with a floor; pairs measured 1.2 x as fast) and its loads (about
-  // 40 cycles for 32 places of a channel pair).
-  long long best = -1;
-  int CG = 1;
-  for (int cg = 2; cg >= 1; --cg) {
-    for (int S = p.S; S >= 1; S /= 2) {
-      const int ks = S == 1 && p.ND >= 2 && least_units(p) >= 2 ? 2 : 1;
-      const long long slots = ctx->sm_count / cg;
-      long long tiles = 0, tile_cost = 0;
-      for (int i = 0; i < p.nphases; ++i) {
-        const ConvPhase &q = p.ph[i];
-        tiles += ((long long)B * q.PH * q.PW + cg * S * 128 - 1) / (cg * S * 128);
-        const long long units = (long long)p.nslab * ((q.kslab + 31) / 32) * S;
-        // about 900 cycles of an issuer's instructions a unit
-        const long long issue = S * ks > 1 ? 450 : 900;
-        const long long mma = units * (p.NP * 6 > issue ? p.NP * 6 : issue) * (cg == 2 ? 5 : 6) / 5;
-        const long long load = (long long)p.nslab * ((p.CS + 1) / 2) * ((rows_needed(q, p, S * 128) * q.pitch + 31) / 32) * 40;
-        tile_cost += mma > load ? mma : load;
-      }
-      const long long cost = (tiles * p.ngroups + slots - 1) / slots * (tile_cost / p.nphases + 2000);
-      if (best < 0 || cost < best) {
-        best = cost;
-        CG = cg;
-        a.S = S;
-        a.ks = ks;
-      }
-    }
-  }
+  const GatherShape sh = gather_shape(ctx, p, B);
+  const int CG = sh.CG;
+  a.S = sh.S;
+  a.ks = sh.ks;
   int tile0 = 0;
   for (int i = 0; i < p.nphases; ++i) {
     a.ph[i] = p.ph[i];
@@ -850,8 +860,7 @@ int launch_conv_gather(b200_ctx *ctx, const GatherPlan &p, const ConvGeom &g, in
   }
   a.nf = nf;
   const size_t smem = base + nf * FB;
-  const int units = a.ntiles * a.ngroups, slots = ctx->sm_count / CG;
-  const int grid = (units < slots ? units : slots) * CG;
+  const int units = a.ntiles * a.ngroups, grid = sh.blocks;
 #ifdef B200_TC_TIMING
   static const bool timing = getenv("B200_TC_TIMING") != nullptr;
   if (timing) B200_CUDA(cudaMalloc(&a.dbg, (size_t)grid * 16 * sizeof(long long)));
@@ -870,10 +879,7 @@ int launch_conv_gather(b200_ctx *ctx, const GatherPlan &p, const ConvGeom &g, in
   }
   auto launch = [&](auto one, auto pair) -> int {
     B200_CUDA(cudaFuncSetAttribute(CG == 2 ? pair : one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (CG == 2) return launch_pair(ctx, pair, grid, CV_THREADS, smem, a);
-    one<<<grid, CV_THREADS, smem, ctx->stream>>>(a);
-    B200_LAUNCHED();
-    return 0;
+    return launch_kernel(ctx, CG == 2 ? pair : one, dim3((unsigned)grid), CV_THREADS, smem, CG, a);
   };
   if (p.V == 2)
     B200_TRY(launch(conv_gather_kernel<1, 2>, conv_gather_kernel<2, 2>));
@@ -935,6 +941,10 @@ int conv_gather_fwd(b200_ctx *ctx, const ConvGeom &g, const float *in, const flo
 
 int conv_gather_dx(b200_ctx *ctx, const ConvGeom &g, const float *dout, const float *wt, float *din, int B) {
   return launch_conv_gather(ctx, gather_plan(ctx, g, 1), g, 1, dout, wt, nullptr, din, B, B200_ACT_NONE);
+}
+
+int conv_gather_dx_blocks(const b200_ctx *ctx, const ConvGeom &g, int B) {
+  return gather_shape(ctx, gather_plan(ctx, g, 1), B).blocks;
 }
 
 // Which kernels take the passes of a layer.  The gather kernels take what they can: on layers of 3 to 256

@@ -876,15 +876,22 @@ static int launch_fewout(b200_ctx *ctx, const FewOutCfg &p, int B) {
   do {                                                                                                   \
     B200_CUDA(cudaFuncSetAttribute(conv_fewout_kernel<KH, KW, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                    (int)smem));                                                          \
-    conv_fewout_kernel<KH, KW, N><<<grid, FO_THREADS, smem, ctx->stream>>>(p);                           \
+    B200_TRY(launch_kernel(ctx, conv_fewout_kernel<KH, KW, N>, grid, FO_THREADS, smem, 1, p));           \
   } while (0)
   if (p.CO == 1) B200_FEWOUT(1);
   else if (p.CO == 2) B200_FEWOUT(2);
   else if (p.CO == 3) B200_FEWOUT(3);
   else B200_FEWOUT(4);
 #undef B200_FEWOUT
-  B200_LAUNCHED();
   return 0;
+}
+
+static bool fewout_takes(const b200_ctx *ctx, const ConvGeom &g) {
+  return g.C <= 4 && padded_channels(g.C) == 4 && fewout_smem(g.OC, g.KH, g.KW) <= ctx->smem_optin;
+}
+
+int conv_tiled_dx_blocks(const b200_ctx *ctx, const ConvGeom &g, int B) {
+  return fewout_takes(ctx, g) ? ceil_div(g.WI, FO_TILE) * ceil_div(g.HI, FO_TILE_H) * B : 0;
 }
 
 // the flipped, transposed filter copy the dX kernels read; depends on the weights only
@@ -904,7 +911,7 @@ int conv_tiled_dx(b200_ctx *ctx, const ConvGeom &g, const float *W, const float 
   if (B == 0) return 0;
   int Cp = padded_channels(g.C);
   if (prep) B200_TRY(conv_tiled_dx_prep(ctx, g, W, scratch));
-  if (g.C <= 4 && Cp == 4 && fewout_smem(g.OC, g.KH, g.KW) <= ctx->smem_optin) {
+  if (fewout_takes(ctx, g)) {
     // few input channels: dX is a convolution with few OUTPUT channels
     FewOutCfg f{};
     f.in = dout;

@@ -408,26 +408,6 @@ __device__ __forceinline__ void tc_fence_after() {
 }
 
 
-// launch with clusters of two CTAs
-template <typename Args>
-static int launch_pair(b200_ctx *ctx, void (*kernel)(Args), int grid, int threads, size_t smem, const Args &a) {
-  cudaLaunchConfig_t c = {};
-  c.gridDim = dim3((unsigned)grid);
-  c.blockDim = dim3((unsigned)threads);
-  c.dynamicSmemBytes = smem;
-  c.stream = ctx->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  c.attrs = at;
-  c.numAttrs = 1;
-  B200_CUDA(cudaLaunchKernelEx(&c, kernel, a));
-  B200_LAUNCHED();
-  return 0;
-}
-
 // ---- host side: tensor-map encoder obtained from the driver at run time ----------------
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
