@@ -83,6 +83,7 @@ struct ConvGatherArgs {
   int iys, ixs, oys, oxs, tdy, tdx;
   int CS, nslab, cstr; // channels per slab (a multiple of V), slabs, places per V channels in shared memory
   int S, NP, ngroups, ND, nf;
+  int Z;               // blocks that share a tile's k's (kernels with SPLIT)
   int ks;              // 2: tiles of one pixel set whose k's are split between the issuers, an accumulator each
   int nphases, ntiles, koff_len;
   int resident;        // the whole filter fits the ring: loaded once
@@ -138,7 +139,22 @@ __device__ __forceinline__ void add_bias_act(float *v, const float *bias, int ac
   }
 }
 
-template <int CG, int V>
+// 64-k blocks of a tile that a block takes, and the 32-k units that these are
+struct KRange {
+  int i0, i1, u0, u1;
+  __device__ __forceinline__ void init(const ConvGatherArgs &a, const ConvPhase &p, int rank) {
+    const int nfb = (p.kslab + 63) >> 6, nkb = (p.kslab + 31) >> 5, n = a.nslab * nfb;
+    i0 = n * rank / a.Z;
+    i1 = n * (rank + 1) / a.Z;
+    u0 = i0 / nfb * nkb + i0 % nfb * 2;
+    u1 = i1 / nfb * nkb + i1 % nfb * 2;
+  }
+};
+
+// SPLIT: a cluster of Z blocks takes one tile of 128 pixels, each a share of its k's, and adds up the sums over distributed
+// shared memory, in the order of the blocks.  For passes whose tiles leave most SMs idle, where the chain over k is what
+// takes the time (9x11, 220 -> 31 channels, 3x3, 5 samples: three tiles of 2000 k's, 32 us, in shares of 256 12 us).
+template <int CG, int V, bool SPLIT>
 __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid_constant__ ConvGatherArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -163,8 +179,10 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(filt_empty + CV_MAX_F);
 
   const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
+  static_assert(!SPLIT || CG == 1, "a tile is split or a pair's");
   const uint32_t rank = CG == 2 ? cluster_rank() : 0;
-  const int cluster = blockIdx.x / CG, nclusters = gridDim.x / CG;
+  const int zrank = SPLIT ? (int)cluster_rank() : 0;
+  const int cluster = SPLIT ? blockIdx.x / a.Z : blockIdx.x / CG, nclusters = SPLIT ? gridDim.x / a.Z : gridDim.x / CG;
   const int nunits = a.ntiles * a.ngroups;
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -207,7 +225,38 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
   constexpr uint32_t tmem_base = 0, tmem_a = tmem_base + CV_D_COLS;
   bool failed = __any_sync(0xffffffffu, *tmem_slot != tmem_base);
 
-  if (warp < CV_EPI_WARPS) {
+  if (SPLIT && warp < CV_EPI_WARPS) {
+    // ---- epilogue of a share: the sums to shared memory, [channel][pixel], where the filter blocks were ----
+    const ConvPhase &p = phase_of(a, cluster / a.ngroups);
+    KRange kr;
+    kr.init(a, p, zrank);
+    const int nu = kr.u1 - kr.u0, quad = warp & 3;
+    float *part = reinterpret_cast<float *>(filt) + quad * 32 + lane;
+    bool have[2];  // with two accumulators the units go to them by parity
+    for (int e = 0; e < 2; ++e) {
+      have[e] = e < a.ks && (a.ks == 1 ? nu >= 1 : nu >= 2 || (nu == 1 && (kr.u0 & 1) == e));
+      if (have[e] && !failed && !mbar_wait_warp_sleep<CV_NAP_EPI>(&acc_full[e], 0)) failed = true;
+    }
+    tc_fence_after();
+    const uint32_t tq0 = tmem_base + ((uint32_t)(quad * 32) << 16);
+    for (int c = (warp >> 2) * 16; c < a.NP; c += 32) {
+      float v[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = 0.f;
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (have[e] && !failed) {
+          uint32_t x[16], y[16];
+          tmem_ld16_nowait(tq0 + (uint32_t)(e * 2 * a.NP + c), x);
+          tmem_ld16_nowait(tq0 + (uint32_t)(e * 2 * a.NP + a.NP + c), y);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(x[j]) + __uint_as_float(y[j]);
+        }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) part[(c + j) * 128] = v[j];
+    }
+  } else if (warp < CV_EPI_WARPS) {
     // ---- epilogue: two warps per TMEM lane quadrant, each takes every other 16 channels -------------
     const size_t plane_o = (size_t)a.OHf * a.OWf;
     const int quad = warp & 3;
@@ -283,7 +332,10 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
       const ConvPhase &p = phase_of(a, unit / a.ngroups);
       const int nkb = (p.kslab + 31) >> 5;
       const int *tab = pixtab + (it & 1) * a.S * 128 + quad * 32 + lane;
-      for (int slab = 0; slab < a.nslab && !failed; ++slab, ++slabs) {
+      KRange kr;
+      if (SPLIT) kr.init(a, p, zrank);
+      const int slab1 = SPLIT ? (kr.u1 + nkb - 1) / nkb : a.nslab;
+      for (int slab = SPLIT ? kr.u0 / nkb : 0; slab < slab1 && !failed; ++slab, ++slabs) {
         const uint32_t rb = slabs & 1;
         tq = tc_clock();
         if (!mbar_wait_warp_sleep<CV_NAP_GATHER>(&raw_full[rb], (slabs >> 1) & 1)) {
@@ -292,7 +344,8 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
         }
         w0 += tc_clock() - tq;
         const uint32_t rbase = smem_u32(raw + rb * (size_t)RB);
-        for (int kb = 0; kb < nkb && !failed; ++kb) {
+        const int kb1 = SPLIT ? min(nkb, kr.u1 - slab * nkb) : nkb;
+        for (int kb = SPLIT ? max(0, kr.u0 - slab * nkb) : 0; kb < kb1 && !failed; ++kb) {
           const uint32_t ko = smem_u32(koff + p.koff0 + kb * (32 / V));
           // A group and its two unit buffers serve the pixel sets of their own parity (alternate units when
           // there is one set): group, buffers and issuer are one pipeline that sees every phase of its barriers.
@@ -378,7 +431,10 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
         postab[pos] = inside ? b * a.C * plane + iy * a.IW + ix : -1;
       }
       asm volatile("bar.sync 1, %0;\n" ::"n"(CV_LOAD_THREADS) : "memory");
-      for (int slab = 0; slab < a.nslab && !failed; ++slab, ++slabs) {
+      KRange kr;
+      if (SPLIT) kr.init(a, p, zrank);
+      const int nkb = (p.kslab + 31) >> 5, slab0 = SPLIT ? kr.u0 / nkb : 0, slab1 = SPLIT ? (kr.u1 + nkb - 1) / nkb : a.nslab;
+      for (int slab = slab0; slab < slab1 && !failed; ++slab, ++slabs) {
         const uint32_t rb = slabs & 1;
         tq = tc_clock();
         if (slabs >= 2 && !mbar_wait_warp_sleep<CV_NAP_LOAD>(&raw_empty[rb], ((slabs >> 1) - 1) & 1)) {
@@ -386,7 +442,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
           break;
         }
         w0 += tc_clock() - tq;
-        if (slab == 0) {
+        if (slab == slab0) {
           int *tab = pixtab + (it & 1) * a.S * 128;
           for (int i = lt; i < a.S * 128; i += CV_LOAD_THREADS) {
             int off = 0;
@@ -438,7 +494,9 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
       const int nblk = a.nslab * ((p.kslab + 63) >> 6);
       const uint32_t *src = a.filt + p.filt + (size_t)grp * nblk * a.NP * 96;
       const int block = (int)(p.filt / (a.NP * 96)) + grp * nblk;
-      for (int i = 0; i < nblk; ++i, ++f) {
+      KRange kr;
+      if (SPLIT) kr.init(a, p, zrank);
+      for (int i = SPLIT ? kr.i0 : 0; i < (SPLIT ? kr.i1 : nblk); ++i, ++f) {
         const uint32_t st = f % a.nf, use = f / a.nf;
         if (use > 0 && !mbar_wait_warp_sleep<CV_NAP_LOAD>(&filt_empty[st], (use - 1) & 1)) {
           failed = true;
@@ -475,9 +533,12 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
     const bool paired = nsets > 1;             // a gather group and its two buffers belong to one issuer
     for (int unit = cluster; unit < nunits && me < nsets; unit += nclusters) {
       const ConvPhase &p = phase_of(a, unit / a.ngroups);
-      const int kslab = p.kslab, nfb = (kslab + 63) >> 6, nblk = a.nslab * nfb, nku = a.nslab * ((kslab + 31) >> 5);
-      int u0 = 0;                              // units of the tile before this block
-      for (int i = 0, fb = 0; i < nblk; ++i, fb = fb + 1 == nfb ? 0 : fb + 1) {
+      KRange kr;
+      if (SPLIT) kr.init(a, p, zrank);
+      const int kslab = p.kslab, nfb = (kslab + 63) >> 6, nblk = SPLIT ? kr.i1 : a.nslab * nfb,
+                nku = SPLIT ? kr.u1 : a.nslab * ((kslab + 31) >> 5), ubeg = SPLIT ? kr.u0 : 0;
+      int u0 = ubeg;                           // units of the tile before this block
+      for (int i = SPLIT ? kr.i0 : 0, fb = SPLIT ? kr.i0 % nfb : 0; i < nblk; ++i, fb = fb + 1 == nfb ? 0 : fb + 1) {
         tq = tc_clock();
         if ((!a.resident || first) && !failed) {
           failed = !mbar_wait_warp_cg<CG>(&filt_full[st], fpar);
@@ -488,7 +549,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
         const int nh = (k16 + 1) >> 1;
         for (int h = a.ks == 2 ? (u0 ^ me) & 1 : 0; h < nh; h += a.ks) {
           const bool last = u0 + h + a.ks >= nku, both = k16 - h * 2 >= 2;
-          const uint32_t more = u0 + h >= a.ks;
+          const uint32_t more = u0 + h - ubeg >= a.ks;
           const uint64_t b1 = f0hi | uni(fst + (uint32_t)(h * 4));
           for (int s = me; s < nsets; s += CV_ISSUERS) {
             uint32_t db = db0 + s;
@@ -500,7 +561,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
             w1 += tc_clock() - tq;
             tq = tc_clock();
             // one issuer alone takes the groups in turn, from group 0 in every tile
-            const bool second = !paired && ((u0 + h) & 1);
+            const bool second = !paired && ((u0 + h) & 1);  // by the unit's number in the tile, as the groups count
             const uint32_t turn = second ? v1++ : v++, ab = (paired ? me : (int)second) * 2 + (turn & 1);
             if (!failed) failed = !mbar_wait_warp_cg<CG>(&a_full[ab], (turn >> 1) & 1);
             w2 += tc_clock() - tq;
@@ -530,8 +591,35 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
   if (failed && a.err) atomicExch(a.err, 3);
   tc_fence_before();
   __syncthreads();
-  if (CG == 2) cluster_sync();
+  if (CG == 2 || SPLIT) cluster_sync();
   if (warp == CV_W_FILT) tmem_dealloc_cg<CG>(tmem_base, 512);
+  if (SPLIT) {
+    // every block adds up each Z-th channel of the tile, a warp 32 pixels of a channel
+    const int tile = cluster / a.ngroups, n0 = (cluster - tile * a.ngroups) * a.NP, n = min(a.N - n0, a.NP);
+    const ConvPhase &p = phase_of(a, tile);
+    const int PHW = p.PH * p.PW, total = a.B * PHW;
+    const size_t plane_o = (size_t)a.OHf * a.OWf;
+    const uint32_t part = smem_u32(filt);
+    for (int e = warp; e < (n - zrank + a.Z - 1) / a.Z * 4; e += CV_THREADS / 32) {
+      const int c = e / 4 * a.Z + zrank, px = e % 4 * 32 + lane, g = (tile - p.tile0) * 128 + px;
+      float v[8];
+#pragma unroll
+      for (int z = 0; z < 8; ++z)
+        if (z < a.Z) {
+          uint32_t ra;
+          asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(part + (uint32_t)(c * 128 + px) * 4u), "r"(z));
+          asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v[z]) : "r"(ra) : "memory");
+        }
+#pragma unroll
+      for (int z = 1; z < 8; ++z)
+        if (z < a.Z) v[0] += v[z];
+      if (g >= total) continue;
+      const int b = g / PHW, r = g - b * PHW, y = r / p.PW, x = r - y * p.PW;
+      a.out[((size_t)b * a.N + n0 + c) * plane_o + (size_t)(y * a.oys + p.oy0) * a.OWf + (x * a.oxs + p.ox0)] =
+        apply_act(v[0] + bias_s[n0 + c], a.act);
+    }
+    cluster_sync();  // nobody leaves while others read its sums
+  }
 }
 
 // ---- filter blocks ---------------------------------------------------------------------------------
@@ -766,32 +854,38 @@ int least_units(const GatherPlan &p) {
 // CTA pair or single CTAs, and S: the least time of the busiest SM, tile after tile, a tile taking the
 // longer of its MMAs (N / 2 cycles each, with a floor; pairs measured 1.2 x as fast) and its loads (about
 // 40 cycles for 32 places of a channel pair).
+// Tiles that leave most SMs idle are split over clusters of Z blocks, each with two blocks of 64 k's or more; as many clusters
+// as surely run at once, however the SMs are grouped; about 2500 cycles for the exchange.
 struct GatherShape {
-  int CG, S, ks, blocks;
+  int CG, S, ks, Z, blocks;
 };
 
 GatherShape gather_shape(const b200_ctx *ctx, const GatherPlan &p, int B) {
-  GatherShape sh = {1, 1, 1, 0};
+  GatherShape sh = {1, 1, 1, 1, 0};
   long long best = -1;
   for (int cg = 2; cg >= 1; --cg) {
     for (int S = p.S; S >= 1; S /= 2) {
       const int ks = S == 1 && p.ND >= 2 && least_units(p) >= 2 ? 2 : 1;
       const long long slots = ctx->sm_count / cg;
-      long long tiles = 0, tile_cost = 0;
+      for (int Z = 1; Z <= (cg * S == 1 ? 8 : 1); Z *= 2) {
+      long long tiles = 0, tile_cost = 0, blocks = 0;
       for (int i = 0; i < p.nphases; ++i) {
         const ConvPhase &q = p.ph[i];
         tiles += ((long long)B * q.PH * q.PW + cg * S * 128 - 1) / (cg * S * 128);
-        const long long units = (long long)p.nslab * ((q.kslab + 31) / 32) * S;
+        const long long units = ((long long)p.nslab * ((q.kslab + 31) / 32) * S + Z - 1) / Z;
+        blocks = max(blocks, (long long)p.nslab * ((q.kslab + 63) / 64));
         // about 900 cycles of an issuer's instructions a unit
         const long long issue = S * ks > 1 ? 450 : 900;
         const long long mma = units * (p.NP * 6 > issue ? p.NP * 6 : issue) * (cg == 2 ? 5 : 6) / 5;
-        const long long load = (long long)p.nslab * ((p.CS + 1) / 2) * ((rows_needed(q, p, S * 128) * q.pitch + 31) / 32) * 40;
+        const long long load = (long long)((p.nslab + Z - 1) / Z) * ((p.CS + 1) / 2) * ((rows_needed(q, p, S * 128) * q.pitch + 31) / 32) * 40;
         tile_cost += mma > load ? mma : load;
       }
-      const long long cost = (tiles * p.ngroups + slots - 1) / slots * (tile_cost / p.nphases + 2000);
+      if (Z > 1 && (blocks < 2 * Z || tiles * p.ngroups > ctx->sm_count / Z * 7 / 8)) break;
+      const long long cost = (tiles * p.ngroups + slots - 1) / slots * (tile_cost / p.nphases + 2000 + (Z > 1 ? 2500 : 0));
       if (best < 0 || cost < best) {
         best = cost;
-        sh = {cg, S, ks, (int)min(tiles * p.ngroups, slots) * cg};
+        sh = {cg, S, ks, Z, (int)min(tiles * p.ngroups, slots) * cg * Z};
+      }
       }
     }
   }
@@ -843,6 +937,7 @@ int launch_conv_gather(b200_ctx *ctx, const GatherPlan &p, const ConvGeom &g, in
   const int CG = sh.CG;
   a.S = sh.S;
   a.ks = sh.ks;
+  a.Z = sh.Z;
   int tile0 = 0;
   for (int i = 0; i < p.nphases; ++i) {
     a.ph[i] = p.ph[i];
@@ -854,7 +949,7 @@ int launch_conv_gather(b200_ctx *ctx, const GatherPlan &p, const ConvGeom &g, in
   int nf = (int)((ctx->smem_optin - base) / FB);
   if (nf > CV_MAX_F) nf = CV_MAX_F;
   const int nblk = p.nslab * ((p.ph[0].kslab + 63) / 64);
-  if (p.nphases == 1 && p.ngroups == 1 && nblk <= nf) {
+  if (p.nphases == 1 && p.ngroups == 1 && nblk <= nf && sh.Z == 1) {
     a.resident = 1;
     nf = nblk;
   }
@@ -877,16 +972,17 @@ int launch_conv_gather(b200_ctx *ctx, const GatherPlan &p, const ConvGeom &g, in
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     B200_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed (%d) for the filter blocks", (int)r);
   }
-  auto launch = [&](auto one, auto pair) -> int {
-    B200_CUDA(cudaFuncSetAttribute(CG == 2 ? pair : one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return launch_kernel(ctx, CG == 2 ? pair : one, dim3((unsigned)grid), CV_THREADS, smem, CG, a);
+  auto launch = [&](auto one, auto pair, auto split) -> int {
+    auto kernel = CG == 2 ? pair : sh.Z > 1 ? split : one;
+    B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    return launch_kernel(ctx, kernel, dim3((unsigned)grid), CV_THREADS, smem, CG * sh.Z, a);
   };
   if (p.V == 2)
-    B200_TRY(launch(conv_gather_kernel<1, 2>, conv_gather_kernel<2, 2>));
+    B200_TRY(launch(conv_gather_kernel<1, 2, false>, conv_gather_kernel<2, 2, false>, conv_gather_kernel<1, 2, true>));
   else if (p.V == 4)
-    B200_TRY(launch(conv_gather_kernel<1, 4>, conv_gather_kernel<2, 4>));
+    B200_TRY(launch(conv_gather_kernel<1, 4, false>, conv_gather_kernel<2, 4, false>, conv_gather_kernel<1, 4, true>));
   else
-    B200_TRY(launch(conv_gather_kernel<1, 8>, conv_gather_kernel<2, 8>));
+    B200_TRY(launch(conv_gather_kernel<1, 8, false>, conv_gather_kernel<2, 8, false>, conv_gather_kernel<1, 8, true>));
 #ifdef B200_TC_TIMING
   if (timing) {  // diagnostic: cycles of the roles and of their waits, averaged over blocks
     std::vector<long long> h((size_t)grid * 16);
@@ -899,9 +995,9 @@ int launch_conv_gather(b200_ctx *ctx, const GatherPlan &p, const ConvGeom &g, in
     int pairs = 0;
     for (int i = 0; i < p.nphases; ++i) pairs += p.ph[i].kslab;
     fprintf(stderr,
-            "[tc-timing] gather %s CG %d S %d NP %d groups %d CS %d slabs %d k/slab %d ring %d grid %d units %d | mma %.0f (filter %.0f "
+            "[tc-timing] gather %s CG %d S %d Z %d NP %d groups %d CS %d slabs %d k/slab %d ring %d grid %d units %d | mma %.0f (filter %.0f "
             "acc %.0f A %.0f) | converter %.0f (raw %.0f A %.0f) | loader %.0f (raw %.0f) | epilogue %.0f (wait %.0f)\n",
-            for_dx ? "dx" : "fwd", CG, a.S, a.NP, a.ngroups, a.CS, a.nslab, pairs, a.nf, grid, units, s[12], s[13], s[14], s[15],
+            for_dx ? "dx" : "fwd", CG, a.S, a.Z, a.NP, a.ngroups, a.CS, a.nslab, pairs, a.nf, grid, units, s[12], s[13], s[14], s[15],
             s[4], s[5], s[6], s[8], s[9], s[0], s[1]);
   }
 #endif
