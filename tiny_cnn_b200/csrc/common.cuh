@@ -90,6 +90,10 @@ struct b200_ctx {
   // recorded when every block of the next dX kernel has begun (launch_kernel clears it); null: not asked for
   cudaEvent_t started = nullptr;
 
+  // second stream of calls whose kernels leave SMs to one another (conv2d_bwd), and the events that tie it to `stream`
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_started = nullptr, ev_join = nullptr;
+
   // device word a kernel sets when a bounded wait ran out; read by b200_ctx_sync
   int *dev_err = nullptr;
 
