@@ -237,8 +237,9 @@ __global__ void __launch_bounds__(BN_THREADS) bn_apply_kernel(const float *__res
                     [&](size_t i, float v) { y[i] = __fdiv_rn(__fsub_rn(v, mean), sd); });
 }
 
-// dx = (dy - mean(dy) - mean(dy*y) * y) / stddev (batch_normalization_layer.h:94-134)
-__global__ void __launch_bounds__(BN_THREADS) bn_bwd_kernel(const float *__restrict__ y, const float *__restrict__ dy,
+// dx = (dy - mean(dy) - mean(dy*y) * y) / stddev (batch_normalization_layer.h:94-134).  Five blocks an SM, so that the grid of about
+// four is there at once: with four a few blocks made a second turn (256 samples of 64 maps of 32x32: 35.8 us, now 31).
+__global__ void __launch_bounds__(BN_THREADS, 5) bn_bwd_kernel(const float *__restrict__ y, const float *__restrict__ dy,
                                                             float *__restrict__ dx, int S, int B, int slices,
                                                             const float *__restrict__ part_d,
                                                             const float *__restrict__ part_dy,
