@@ -10,6 +10,7 @@ namespace b200 {
 // relu_layer.h:25-29, tanh_layer.h:24-28 -- elementwise, float4 where aligned
 __global__ void act_fwd_kernel(int kind, float param, const float *__restrict__ x, float *__restrict__ y,
                                size_t n4, size_t n) {
+  after_previous_kernel();
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   size_t step = (size_t)gridDim.x * blockDim.x;
   const float4 *x4 = reinterpret_cast<const float4 *>(x);
@@ -27,6 +28,7 @@ __global__ void act_fwd_kernel(int kind, float param, const float *__restrict__ 
 
 __global__ void act_bwd_kernel(int kind, float param, const float *__restrict__ y, const float *__restrict__ dy,
                                float *__restrict__ dx, size_t n4, size_t n) {
+  after_previous_kernel();
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   size_t step = (size_t)gridDim.x * blockDim.x;
   const float4 *y4 = reinterpret_cast<const float4 *>(y);
@@ -241,8 +243,8 @@ int act_fwd(b200_ctx *ctx, int kind, const float *x, float *y, int dim, int B, f
       softmax_fwd_kernel<<<ceil_div(B, 32), 32, 0, ctx->stream>>>(x, y, dim, B);
   } else {
     size_t n4 = (aligned16(x) && aligned16(y)) ? n / 4 : 0;
-    act_fwd_kernel<<<grid_for(n4 ? n4 : n, 256, ctx->sm_count), 256, 0, ctx->stream>>>(kind, param, x,
-                                                                                      y, n4, n);
+    B200_TRY(launch_kernel(ctx, act_fwd_kernel, dim3(grid_for(n4 ? n4 : n, 256, ctx->sm_count)), dim3(256), 0, 1, kind, param,
+                           x, y, n4, n));
   }
   B200_LAUNCHED();
   return 0;
@@ -260,8 +262,8 @@ int act_bwd(b200_ctx *ctx, int kind, const float *y, const float *dy, float *dx,
       softmax_bwd_kernel<<<ceil_div(B, 32), 32, 0, ctx->stream>>>(y, const_cast<float *>(dy), dx, dim, B, nullptr, 0);
   } else {
     size_t n4 = (aligned16(y) && aligned16(dy) && aligned16(dx)) ? n / 4 : 0;
-    act_bwd_kernel<<<grid_for(n4 ? n4 : n, 256, ctx->sm_count), 256, 0, ctx->stream>>>(
-      kind, param, y, dy, dx, n4, n);
+    B200_TRY(launch_kernel(ctx, act_bwd_kernel, dim3(grid_for(n4 ? n4 : n, 256, ctx->sm_count)), dim3(256), 0, 1, kind, param,
+                           y, dy, dx, n4, n));
   }
   B200_LAUNCHED();
   return 0;
@@ -355,6 +357,7 @@ __global__ void __launch_bounds__(FCS_THREADS) fc_softmax_fwd16_kernel(const flo
                                                                        const float *__restrict__ bias,
                                                                        float *__restrict__ z, float *__restrict__ y,
                                                                        int K, int N, int B) {
+  after_previous_kernel();
   extern __shared__ float fcs_w[];  // [K][N]
   for (int i = threadIdx.x; i < K * N; i += FCS_THREADS) cp_async4(fcs_w + i, W + i, true);
   cp_async_commit();
@@ -386,6 +389,7 @@ __global__ void __launch_bounds__(FCS_THREADS) fc_softmax_bwd16_kernel(const flo
                                                                        const float *__restrict__ relu_x,
                                                                        float *__restrict__ dy, float *__restrict__ dz,
                                                                        float *__restrict__ dx, int K, int N, int B) {
+  after_previous_kernel();
   extern __shared__ float fcs_w[];  // [K][N]
   for (int i = threadIdx.x; i < K * N; i += FCS_THREADS) cp_async4(fcs_w + i, W + i, true);
   cp_async_commit();
@@ -417,6 +421,7 @@ __global__ void __launch_bounds__(FCW_THREADS) fc_softmax_fwd_wide_kernel(const 
                                                                           const float *__restrict__ W,
                                                                           const float *__restrict__ bias, float *__restrict__ z,
                                                                           float *__restrict__ y, int K, int N, int B) {
+  after_previous_kernel();
   __shared__ float sums[FCW_SAMPLES][FCW_WARPS][FCS_N];
   const int n0 = blockIdx.x * FCW_SAMPLES, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float acc[FCW_SAMPLES][FCS_N];
@@ -456,6 +461,7 @@ __global__ void __launch_bounds__(FCW_THREADS) fc_softmax_bwd_wide_kernel(const 
                                                                           const float *__restrict__ relu_x,
                                                                           float *__restrict__ dy, float *__restrict__ dz,
                                                                           float *__restrict__ dx, int K, int N, int B) {
+  after_previous_kernel();
   __shared__ float ds[FCW_SAMPLES][FCS_N];
   const int n0 = blockIdx.x * FCW_SAMPLES, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < FCW_SAMPLES && n0 + warp < B) {
@@ -493,11 +499,11 @@ int fc_softmax_fwd(b200_ctx *ctx, int K, int N, const float *x, const float *W, 
   B200_REQUIRE(fc_softmax_fusable(K, N), "fc_softmax_fwd: shape %d x %d not supported", K, N);
   if (B == 0) return 0;
   if (K <= FCS_NARROW)
-    fc_softmax_fwd16_kernel<<<ceil_div(B, FCS_THREADS / 32), FCS_THREADS, (size_t)K * N * sizeof(float), ctx->stream>>>(
-      x, W, bias, z, y, K, N, B);
+    B200_TRY(launch_kernel(ctx, fc_softmax_fwd16_kernel, dim3(ceil_div(B, FCS_THREADS / 32)), dim3(FCS_THREADS),
+                           (size_t)K * N * sizeof(float), 1, x, W, bias, z, y, K, N, B));
   else
-    fc_softmax_fwd_wide_kernel<<<ceil_div(B, FCW_SAMPLES), FCW_THREADS, 0, ctx->stream>>>(x, W, bias, z, y, K, N, B);
-  B200_LAUNCHED();
+    B200_TRY(launch_kernel(ctx, fc_softmax_fwd_wide_kernel, dim3(ceil_div(B, FCW_SAMPLES)), dim3(FCW_THREADS), 0, 1, x, W,
+                           bias, z, y, K, N, B));
   return 0;
 }
 
@@ -508,12 +514,11 @@ int fc_softmax_loss_bwd(b200_ctx *ctx, int loss_kind, int K, int N, const float 
                "fc_softmax_loss_bwd: unknown loss %d", loss_kind);
   if (B == 0) return 0;
   if (K <= FCS_NARROW)
-    fc_softmax_bwd16_kernel<<<ceil_div(B, FCS_THREADS / 32), FCS_THREADS, (size_t)K * N * sizeof(float), ctx->stream>>>(
-      y, t, loss_kind, W, relu_x, dy, dz, dx, K, N, B);
+    B200_TRY(launch_kernel(ctx, fc_softmax_bwd16_kernel, dim3(ceil_div(B, FCS_THREADS / 32)), dim3(FCS_THREADS),
+                           (size_t)K * N * sizeof(float), 1, y, t, loss_kind, W, relu_x, dy, dz, dx, K, N, B));
   else
-    fc_softmax_bwd_wide_kernel<<<ceil_div(B, FCW_SAMPLES), FCW_THREADS, 0, ctx->stream>>>(y, t, loss_kind, W, relu_x, dy, dz, dx,
-                                                                                         K, N, B);
-  B200_LAUNCHED();
+    B200_TRY(launch_kernel(ctx, fc_softmax_bwd_wide_kernel, dim3(ceil_div(B, FCW_SAMPLES)), dim3(FCW_THREADS), 0, 1, y, t,
+                           loss_kind, W, relu_x, dy, dz, dx, K, N, B));
   return 0;
 }
 

@@ -108,14 +108,14 @@ int conv_bwd_impl(b200_ctx *ctx, const b200_conv_desc *d, const float *in, const
     const int rc = tc_dx ? conv_gather_dx(ctx, g, dout, s_dx, din, batch) : conv_tiled_dx(ctx, g, W, dout, din, batch, s_dx, 0);
     ctx->started = nullptr;
     B200_TRY(rc);
-    B200_CUDA(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-    B200_CUDA(cudaStreamWaitEvent(ctx->side, ctx->ev_started, 0));
+    B200_TRY(stream_wait(ctx, ctx->side, ctx->ev_fork));
+    B200_TRY(stream_wait(ctx, ctx->side, ctx->ev_started));
     ctx->stream = ctx->side;
     const int rc_dw = tc.dw_small ? conv_dw_small(ctx, g, in, dout, batch, s_dw, dW, db, accumulate)
                                   : conv_gather_dw(ctx, g, in, dout, batch, s_dw, dW, db, accumulate, batch);
     ctx->stream = main;
     B200_CUDA(cudaEventRecord(ctx->ev_join, ctx->side));  // also behind a launch that failed: what began ends before the call's successors
-    B200_CUDA(cudaStreamWaitEvent(main, ctx->ev_join, 0));
+    B200_TRY(stream_wait(ctx, main, ctx->ev_join));
     return rc_dw;
   }
   if (tc_dx) {

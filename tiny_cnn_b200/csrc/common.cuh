@@ -90,6 +90,10 @@ struct b200_ctx {
   // recorded when every block of the next dX kernel has begun (launch_kernel clears it); null: not asked for
   cudaEvent_t started = nullptr;
 
+  // kernels may be launched while the one before them in the stream runs (launch_kernel); not the one behind a wait for another
+  // stream, which only costs the driver time
+  bool overlap = true, waited = false;
+
   // second stream of calls whose kernels leave SMs to one another (conv2d_bwd), and the events that tie it to `stream`
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_started = nullptr, ev_join = nullptr;
@@ -112,21 +116,36 @@ struct b200_ctx {
 
 namespace b200 {
 
-// a launch with clusters of `cluster` blocks along x that records ctx->started
+// `stream`, the context's or one beside it, goes on behind `e`
+inline int stream_wait(b200_ctx *ctx, cudaStream_t stream, cudaEvent_t e) {
+  ctx->waited = true;
+  B200_CUDA(cudaStreamWaitEvent(stream, e, 0));
+  return 0;
+}
+
+// A launch with clusters of `cluster` blocks that records ctx->started.  The kernel begins with
+// after_previous_kernel: its launch and what it sets up overlap the end of the kernel before it.
 template <typename... Params, typename... Args>
-int launch_kernel(b200_ctx *ctx, void (*kernel)(Params...), dim3 grid, int threads, size_t smem, int cluster, const Args &...args) {
+int launch_kernel(b200_ctx *ctx, void (*kernel)(Params...), dim3 grid, dim3 threads, size_t smem, dim3 cluster, const Args &...args) {
   cudaLaunchConfig_t c = {};
   c.gridDim = grid;
-  c.blockDim = dim3((unsigned)threads);
+  c.blockDim = threads;
   c.dynamicSmemBytes = smem;
   c.stream = ctx->stream;
-  cudaLaunchAttribute at[2];
-  if (cluster > 1) {
-    at[c.numAttrs].id = cudaLaunchAttributeClusterDimension;
-    at[c.numAttrs].val.clusterDim.x = (unsigned)cluster;
-    at[c.numAttrs].val.clusterDim.y = at[c.numAttrs].val.clusterDim.z = 1;
+  cudaLaunchAttribute at[3];
+  if (ctx->overlap && !ctx->waited) {
+    at[c.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[c.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     ++c.numAttrs;
   }
+  if (cluster.x * cluster.y * cluster.z > 1) {
+    at[c.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[c.numAttrs].val.clusterDim.x = cluster.x;
+    at[c.numAttrs].val.clusterDim.y = cluster.y;
+    at[c.numAttrs].val.clusterDim.z = cluster.z;
+    ++c.numAttrs;
+  }
+  ctx->waited = false;
   if (ctx->started) {
     at[c.numAttrs].id = cudaLaunchAttributeLaunchCompletionEvent;
     at[c.numAttrs].val.launchCompletionEvent.event = ctx->started;

@@ -214,6 +214,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1) conv_gather_kernel(const __grid
       koff[p.koff0 + k] = (c * a.cstr + jy * a.tdy * p.pitch + jx * a.tdx) * (2 * V);
     }
   }
+  wait_for_previous_kernel();
   for (int n = tid; n < a.ngroups * a.NP; n += CV_THREADS) bias_s[n] = (a.bias && n < a.N) ? a.bias[n] : 0.f;
   if (warp == CV_W_FILT) tmem_alloc_cg<CG>(tmem_slot, 512);
   tc_fence_before();
@@ -639,6 +640,7 @@ __global__ void __launch_bounds__(256) conv_gather_prep_kernel(const float *__re
                                                                int C, int OC, int KH, int KW,
                                                                const __grid_constant__ FilterSet s0,
                                                                const __grid_constant__ FilterSet s1) {
+  after_previous_kernel();
   const FilterSet &s = blockIdx.y == 0 ? s0 : s1;
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < s.total; i += gridDim.x * 256ll) {
     int ph = 0;
@@ -1025,8 +1027,8 @@ int conv_gather_prep(b200_ctx *ctx, const ConvGeom &g, const float *W, float *wt
   const long long total = s[0].total > s[1].total ? s[0].total : s[1].total;
   long long blocks = (total + 255) / 256;
   if (blocks > ctx->sm_count * 8) blocks = ctx->sm_count * 8;
-  conv_gather_prep_kernel<<<dim3((unsigned)blocks, n), 256, 0, ctx->stream>>>(W, g.tbl, g.C, g.OC, g.KH, g.KW, s[0], s[1]);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, conv_gather_prep_kernel, dim3((unsigned)blocks, n), dim3(256), 0, 1, W, g.tbl, g.C, g.OC, g.KH,
+                         g.KW, s[0], s[1]));
   return 0;
 }
 

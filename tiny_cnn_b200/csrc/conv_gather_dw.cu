@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv_gather_dw_kernel(const __g
     gtab[t] = (ry * a.GC + cg) * 16;
     if (e == 0 && (t >> 1) < ((a.steps + 1) & ~1)) rtab[t >> 1] = ((ry * a.sub * a.SW + cg * 8) * (int)RBY) >> 4;
   }
+  wait_for_previous_kernel();
   if (warp == DW_W_MMA) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
@@ -454,6 +455,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv_gather_dw_kernel(const __g
 __global__ void __launch_bounds__(256) conv_gather_dw_finish_kernel(const __grid_constant__ ConvDwArgs a, int rows, int spread,
                                                                     float *__restrict__ dW, float *__restrict__ db,
                                                                     const uint8_t *__restrict__ tbl, int accumulate) {
+  after_previous_kernel();
   __shared__ float4 lanes[8][32];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int nblk = spread ? rows : (rows + 7) / 8;
@@ -781,8 +783,7 @@ int conv_gather_dw(b200_ctx *ctx, const ConvGeom &g, const float *in, const floa
   if (timing) B200_CUDA(cudaMalloc(&a.dbg, (size_t)grid * 16 * sizeof(long long)));
   if (timing) B200_CUDA(cudaMemset(a.dbg, 0, (size_t)grid * 16 * sizeof(long long)));
 #endif
-  kernel<<<grid, DW_THREADS, smem, ctx->stream>>>(a);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, kernel, dim3(grid), DW_THREADS, smem, 1, a));
 #ifdef B200_TC_TIMING
   if (timing) {  // diagnostic: cycles of the roles and of their waits, averaged over blocks
     std::vector<long long> h((size_t)grid * 16);
@@ -817,8 +818,8 @@ int conv_gather_dw_finish(b200_ctx *ctx, const ConvGeom &g, int B, const float *
   }
   const int spread = most > 12;
   const int blocks = (spread ? rows : (rows + 7) / 8) + (a.bpart ? g.OC : 0);
-  conv_gather_dw_finish_kernel<<<blocks, dim3(32, 8), 0, ctx->stream>>>(a, rows, spread, dW, db, g.tbl, accumulate);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, conv_gather_dw_finish_kernel, dim3(blocks), dim3(32, 8), 0, 1, a, rows, spread, dW, db, g.tbl,
+                         accumulate));
   return 0;
 }
 

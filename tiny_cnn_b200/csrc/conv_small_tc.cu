@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(TFS_THREADS, 1)
     }
     mbar_fence_init();
   }
+  wait_for_previous_kernel();
   for (int o = tid; o < a.OCp; o += TFS_THREADS) bias_s[o] = (a.bias && o < a.OC) ? a.bias[o] : 0.f;
   if (warp == W_TMA) tmem_alloc(tmem_slot, (uint32_t)a.tmem_cols);
   tc_fence_before();
@@ -457,8 +458,7 @@ int conv_fwd_small(b200_ctx *ctx, const ConvGeom &g, const float *in, const floa
   static const bool timing = getenv("B200_TC_TIMING") != nullptr;
   if (timing) B200_CUDA(cudaMalloc(&a.dbg, (size_t)a.nblocks * 12 * sizeof(long long)));
 #endif
-  conv_fwd_small_tc_kernel<<<a.nblocks, TFS_THREADS, smem, ctx->stream>>>(x_map, a);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, conv_fwd_small_tc_kernel, dim3(a.nblocks), dim3(TFS_THREADS), smem, 1, x_map, a));
 #ifdef B200_TC_TIMING
   if (timing) {  // diagnostic: cycles of the four roles and of their waits, averaged over blocks
     std::vector<long long> h((size_t)a.nblocks * 12);
@@ -564,13 +564,13 @@ __device__ __forceinline__ void dw_finish_block(const DwFinishArgs &a, const int
   }
 }
 
-__global__ void __launch_bounds__(256) dw_finish_kernel(const DwFinishArgs a) { dw_finish_block(a, (int)blockIdx.x); }
+__global__ void __launch_bounds__(256) dw_finish_kernel(const DwFinishArgs a) {
+  after_previous_kernel(); dw_finish_block(a, (int)blockIdx.x); }
 
 int dw_finish_blocks(const DwFinishArgs &a) { return (a.row_w + 31) / 32 + (a.db != nullptr ? a.OC : 0); }
 
 int launch_dw_finish(b200_ctx *ctx, const DwFinishArgs &a) {
-  dw_finish_kernel<<<dw_finish_blocks(a), dim3(32, 8), 0, ctx->stream>>>(a);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, dw_finish_kernel, dim3(dw_finish_blocks(a)), dim3(32, 8), 0, 1, a));
   return 0;
 }
 
@@ -630,6 +630,7 @@ __global__ void __launch_bounds__(TCS_THREADS, 1)
     mbar_init(accum, 1);
     mbar_fence_init();
   }
+  wait_for_previous_kernel();
   if (warp == TCS_CONV_WARPS) tmem_alloc(tmem_slot, (uint32_t)a.tmem_cols);
   tc_fence_before();
   __syncthreads();
@@ -927,8 +928,7 @@ int conv_dw_small(b200_ctx *ctx, const ConvGeom &g, const float *in, const float
   static const bool timing = getenv("B200_TC_TIMING") != nullptr;
   if (timing) B200_CUDA(cudaMalloc(&a.dbg, (size_t)a.ksplits * 8 * sizeof(long long)));
 #endif
-  conv_dw_small_tc_kernel<<<a.ksplits, TCS_THREADS, smem, ctx->stream>>>(x_map, dy_map, a);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, conv_dw_small_tc_kernel, dim3(a.ksplits), dim3(TCS_THREADS), smem, 1, x_map, dy_map, a));
 #ifdef B200_TC_TIMING
   if (timing) {  // diagnostic: cycles of the three roles and of their waits, averaged over blocks
     std::vector<long long> h((size_t)a.ksplits * 8);

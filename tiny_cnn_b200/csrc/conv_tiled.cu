@@ -48,6 +48,7 @@ __global__ void conv_prep_wt_fwd_kernel(const float *__restrict__ W, float *__re
 __global__ void conv_prep_wt_dx_kernel(const float *__restrict__ W, float *__restrict__ wt, int C,
                                        int OC, int Cp, int KH, int KW,
                                        const uint8_t *__restrict__ tbl) {
+  after_previous_kernel();
   int KK = KH * KW;
   int total = OC * KK * Cp;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -737,6 +738,7 @@ __global__ void __launch_bounds__(FO_THREADS) conv_fewout_kernel(const FewOutCfg
   const int tid = threadIdx.x, z = tid / FO_PATCHES, t = tid - z * FO_PATCHES, tx = t & 7, ty = t >> 3;
   const int b = blockIdx.y, tile = blockIdx.x;
   const int x0 = (tile % p.tiles_x) * FO_TILE, y0 = (tile / p.tiles_x) * FO_TILE_H;
+  wait_for_previous_kernel();
   for (int i = tid; i < p.CI * KK; i += FO_THREADS)
     reinterpret_cast<float4 *>(wsm)[i] = reinterpret_cast<const float4 *>(p.wt)[i];
   const float *img = p.in + (size_t)b * p.CI * p.HI * p.WI;
@@ -899,9 +901,8 @@ int conv_tiled_dx_prep(b200_ctx *ctx, const ConvGeom &g, const float *W, float *
   int KK = g.KH * g.KW;
   int Cp = padded_channels(g.C);
   int total = g.OC * KK * Cp;
-  conv_prep_wt_dx_kernel<<<ceil_div(total, 256), 256, 0, ctx->stream>>>(W, scratch, g.C, g.OC, Cp,
-                                                                       g.KH, g.KW, g.tbl);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, conv_prep_wt_dx_kernel, dim3(ceil_div(total, 256)), dim3(256), 0, 1, W, scratch, g.C, g.OC, Cp,
+                         g.KH, g.KW, g.tbl));
   return 0;
 }
 

@@ -8,6 +8,21 @@
 
 namespace b200 {
 
+// The first thing that a kernel launched by launch_kernel does, or the first behind what it sets up without memory: such a
+// kernel may begin while the one before it in the stream runs, and goes on here when that one has ended and its
+// stores are there.  The condition, always true, is not known to the compiler, which therefore moves no load ahead of it.
+__device__ __forceinline__ void wait_for_previous_kernel() {
+  unsigned blocks;
+  asm volatile("mov.u32 %0, %%nctaid.x;\n" : "=r"(blocks));
+  if (blocks != 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+// The same in a kernel that leaves room on its SMs: the next one may begin from here on.  (A kernel that takes whole SMs does not
+// let the next one in: its waiting blocks would keep those of other streams out.)
+__device__ __forceinline__ void after_previous_kernel() {
+  wait_for_previous_kernel();
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 __device__ __forceinline__ float apply_act(float v, int act) {
   if (act == B200_ACT_RELU) return fmaxf(0.f, v);
   if (act == B200_ACT_TANH) return tanhf(v);

@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(256) sgemm_kernel(int M, int N, int K, const f
                                                     long long b_n, float *__restrict__ C,
                                                     const float *__restrict__ bias, int accumulate,
                                                     int act) {
+  after_previous_kernel();
   static_assert(BT / TT == 16, "256 threads as 16 x 16");
   __shared__ __align__(16) float As[GK][BT + 4];
   __shared__ __align__(16) float Bs[GK][BT + 4];
@@ -122,6 +123,7 @@ constexpr int FT_SMEM = FT_STAGES * 2 * FT_OP * 4;
 
 template <bool A_KFAST, bool B_NFAST>
 __global__ void __launch_bounds__(256) fc_tile_kernel(const __grid_constant__ FcTileArgs a) {
+  after_previous_kernel();
   extern __shared__ __align__(16) float fsm[];
   __shared__ __align__(16) float psum[(FT + 1) * FT];  // the block's sums, and those of Bm
   const int tid = threadIdx.x, group = tid >> 6, tm = (tid >> 3) & 7, tn = tid & 7;
@@ -274,6 +276,7 @@ __global__ void __launch_bounds__(256) fc_tile_kernel(const __grid_constant__ Fc
 // combined in a fixed order through shared memory
 __global__ void col_sum_kernel(const float *__restrict__ d, float *__restrict__ db, int rows, int N,
                                int accumulate) {
+  after_previous_kernel();
   __shared__ float part[8][33];
   int col = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
@@ -349,9 +352,8 @@ static int run_gemm(b200_ctx *ctx, int M, int N, int K, const float *A, const fl
   const dim3 grid(ceil_div(N, p.tile), ceil_div(M, p.tile), p.slices);
   const int lda = A_KFAST ? K : M, ldb = B_NFAST ? N : K;
   if (p.tile == 64) {
-    sgemm_kernel<64, 4, A_KFAST, B_NFAST><<<grid, 256, 0, ctx->stream>>>(M, N, K, A, A_KFAST ? lda : 1, A_KFAST ? 1 : lda, Bm,
-                                                                         B_NFAST ? ldb : 1, B_NFAST ? 1 : ldb, C, bias,
-                                                                         accumulate, act);
+    return launch_kernel(ctx, sgemm_kernel<64, 4, A_KFAST, B_NFAST>, grid, dim3(256), 0, dim3(1), M, N, K, A, A_KFAST ? lda : 1,
+                         A_KFAST ? 1 : lda, Bm, B_NFAST ? ldb : 1, B_NFAST ? 1 : ldb, C, bias, accumulate, act);
   } else {
     FcTileArgs a = {};
     a.M = M, a.N = N, a.K = K, a.k_per = p.k_per;
@@ -362,21 +364,8 @@ static int run_gemm(b200_ctx *ctx, int M, int N, int K, const float *A, const fl
     a.col_sum = col_sum;
     if (ag) a.y = ag->y, a.C2 = ag->dst, a.y_act = ag->act, a.y_param = ag->param;
     B200_CUDA(cudaFuncSetAttribute(fc_tile_kernel<A_KFAST, B_NFAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM));
-    cudaLaunchConfig_t c = {};
-    c.gridDim = grid;
-    c.blockDim = dim3(256);
-    c.dynamicSmemBytes = FT_SMEM;
-    c.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = (unsigned)p.slices;
-    c.attrs = at;
-    c.numAttrs = 1;
-    B200_CUDA(cudaLaunchKernelEx(&c, fc_tile_kernel<A_KFAST, B_NFAST>, a));
+    return launch_kernel(ctx, fc_tile_kernel<A_KFAST, B_NFAST>, grid, dim3(256), FT_SMEM, dim3(1, 1, p.slices), a);
   }
-  B200_LAUNCHED();
-  return 0;
 }
 
 // whether the product of a pass (0 forward, 1 dX, 2 dW) runs on the tensor cores
@@ -456,9 +445,8 @@ int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const floa
     }
   }
   if (db && !db_done) {
-    col_sum_kernel<<<ceil_div(out_size, 32), dim3(32, 8), 0, ctx->stream>>>(dout, db, B, out_size,
-                                                                           accumulate);
-    B200_LAUNCHED();
+    B200_TRY(launch_kernel(ctx, col_sum_kernel, dim3(ceil_div(out_size, 32)), dim3(32, 8), 0, 1, dout, db, B, out_size,
+                           accumulate));
   }
   return 0;
 }

@@ -339,7 +339,7 @@ int net_forward_impl(b200_net *net, const float *x, int B, bool alone) {
         if (pass == 0 ? !L.tc.fwd && !tc_dx : !dx_copy) continue;
         if (!prep_on_side) {
           B200_CUDA(cudaEventRecord(net->ev_fork, main_stream));
-          B200_CUDA(cudaStreamWaitEvent(net->side, net->ev_fork, 0));
+          B200_TRY(stream_wait(ctx, net->side, net->ev_fork));
           prep_on_side = true;
         }
         ctx->stream = net->side;
@@ -371,7 +371,7 @@ int net_forward_impl(b200_net *net, const float *x, int B, bool alone) {
         const bool tc_dx = L.tc.dx && (i > 0 || net->input_grad);
         if (L.tc.fwd || tc_dx) {
           if (prep_on_side && L.ev_prep)
-            B200_CUDA(cudaStreamWaitEvent(ctx->stream, L.ev_prep, 0));
+            B200_TRY(stream_wait(ctx, ctx->stream, L.ev_prep));
           else
             B200_TRY(conv_gather_prep(ctx, L.g, W, L.tc_wt_fwd, tc_dx ? L.tc_wt_dx : nullptr));
           L.dx_ready = tc_dx;
@@ -424,7 +424,7 @@ int net_forward_impl(b200_net *net, const float *x, int B, bool alone) {
     // everything the side stream was given in this pass ends here (a filter copy made for the
     // backward pass has no reader in the forward pass), so a forward pass alone leaves no open branch
     B200_CUDA(cudaEventRecord(net->ev_join, net->side));
-    B200_CUDA(cudaStreamWaitEvent(ctx->stream, net->ev_join, 0));
+    B200_TRY(stream_wait(ctx, ctx->stream, net->ev_join));
   }
   net->cur_batch = B;
   net->cur_x = x;
@@ -464,7 +464,7 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
   // against 0.374 ms with one).
   auto fork = [&]() -> int {
     B200_CUDA(cudaEventRecord(net->ev_fork, main_stream));
-    B200_CUDA(cudaStreamWaitEvent(net->side, net->ev_fork, 0));
+    B200_TRY(stream_wait(ctx, net->side, net->ev_fork));
     ctx->stream = net->side;
     side_used = true;
     return 0;
@@ -533,7 +533,7 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
           if (!tiled_bwd) return conv_general_dx(ctx, L.g, W, L.grad, din, B);
           // the filter copy was made beside the forward pass (same weights: nothing updates
           // them between the two passes of a step)
-          if (L.dx_prep_side) B200_CUDA(cudaStreamWaitEvent(ctx->stream, L.ev_prep, 0));
+          if (L.dx_prep_side) B200_TRY(stream_wait(ctx, ctx->stream, L.ev_prep));
           if (!L.dx_prep_side) B200_TRY(conv_tiled_dx_prep(ctx, L.g, W, L.wt_dx));
           if (dx_first) ctx->started = net->ev_started;
           return conv_tiled_dx(ctx, L.g, W, L.grad, din, B, L.wt_dx, 0);
@@ -544,7 +544,7 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
           const int rc = dx_pass();
           ctx->started = nullptr;
           B200_TRY(rc);
-          B200_CUDA(cudaStreamWaitEvent(net->side, net->ev_started, 0));
+          B200_TRY(stream_wait(ctx, net->side, net->ev_started));
           ctx->stream = net->side;
         }
         float *part = forked ? net->scratch_side : net->scratch;
@@ -553,7 +553,7 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
           rc_side = conv_gather_dw(ctx, L.g, in, L.grad, B, L.tc_part, dW, db, 0, net->max_batch, !later);
           if (!rc_side && later) {
             B200_CUDA(cudaEventRecord(net->ev_dw, net->side));
-            B200_CUDA(cudaStreamWaitEvent(net->sums, net->ev_dw, 0));
+            B200_TRY(stream_wait(ctx, net->sums, net->ev_dw));
             ctx->stream = net->sums;
             rc_side = conv_gather_dw_finish(ctx, L.g, B, L.tc_part, dW, db, 0, net->max_batch);
             sums_used = true;
@@ -615,10 +615,10 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
       // every weight gradient of layers i.. has been issued (main or side stream): send them to
       // the peers now, from a third stream, while the remaining layers still compute
       B200_CUDA(cudaEventRecord(net->ev_comm_main, main_stream));
-      B200_CUDA(cudaStreamWaitEvent(net->comm, net->ev_comm_main, 0));
+      B200_TRY(stream_wait(ctx, net->comm, net->ev_comm_main));
       if (side_used) {
         B200_CUDA(cudaEventRecord(net->ev_comm_side, net->side));
-        B200_CUDA(cudaStreamWaitEvent(net->comm, net->ev_comm_side, 0));
+        B200_TRY(stream_wait(ctx, net->comm, net->ev_comm_side));
       }
       ctx->stream = net->comm;
       int rc = peer_reduce_push_early(ctx, &net->peer, net->grads);
@@ -636,13 +636,13 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
   ctx->stream = main_stream;
   if (sums_used) {
     B200_CUDA(cudaEventRecord(net->ev_dw, net->sums));
-    B200_CUDA(cudaStreamWaitEvent(main_stream, net->ev_dw, 0));
+    B200_TRY(stream_wait(ctx, main_stream, net->ev_dw));
   }
   if (side_used) {  // the optimizer (or the caller's all-reduce) follows on the main stream
     B200_CUDA(cudaEventRecord(net->ev_join, net->side));
-    B200_CUDA(cudaStreamWaitEvent(main_stream, net->ev_join, 0));
+    B200_TRY(stream_wait(ctx, main_stream, net->ev_join));
   }
-  if (comm_used) B200_CUDA(cudaStreamWaitEvent(main_stream, net->ev_comm_done, 0));
+  if (comm_used) B200_TRY(stream_wait(ctx, main_stream, net->ev_comm_done));
   net_drop_prepared(net);
   return rc_side;
 }
@@ -1216,7 +1216,11 @@ static int run_captured(b200_net *net, int slot_idx, const std::string &key, F b
   cudaGraph_t graph = nullptr;
   unsigned long long before = g_launches.load();
   B200_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
+  // In a graph a kernel starts microseconds after the one before it anyhow, and blocks that wait on an SM shift which of two
+  // branches gets it: steps of the CIFAR-10 network of 12 samples took 131 us for 111, of 64 samples 159 for 174.
+  net->ctx->overlap = false;
   int r = body();
+  net->ctx->overlap = true;
   cudaError_t ce = cudaStreamEndCapture(st, &graph);
   unsigned long long recorded = g_launches.load() - before;
   if (r != 0) {
@@ -1404,16 +1408,16 @@ int b200_net_fit_host_enqueue(b200_net *net, const float *x_host, const float *t
       int run_nb = 0;
       B200_TRY(fit_step_rows(net, nb, batch, &run_nb));
       const int buf = (int)(net->fit_toggle++ & 1u);
-      if (net->stage_used[buf]) B200_CUDA(cudaStreamWaitEvent(net->copy_stream, net->stage_free[buf], 0));
+      if (net->stage_used[buf]) B200_TRY(stream_wait(net->ctx, net->copy_stream, net->stage_free[buf]));
       net->stage_used[buf] = true;
       B200_CUDA(cudaMemcpyAsync(net->x_stage[buf], x_host + (size_t)i * in_dim, in_dim * nb * sizeof(float),
                                 cudaMemcpyHostToDevice, net->copy_stream));
       B200_CUDA(cudaMemcpyAsync(net->t_stage[buf], t_host + (size_t)i * out_dim, out_dim * nb * sizeof(float),
                                 cudaMemcpyHostToDevice, net->copy_stream));
       B200_CUDA(cudaEventRecord(net->up_done[buf], net->copy_stream));
-      B200_CUDA(cudaStreamWaitEvent(st, net->up_done[buf], 0));
+      B200_TRY(stream_wait(net->ctx, st, net->up_done[buf]));
       if (nb == batch) {
-        if (out_host && net->out_stage_used[buf]) B200_CUDA(cudaStreamWaitEvent(st, net->d2h_done[buf], 0));
+        if (out_host && net->out_stage_used[buf]) B200_TRY(stream_wait(net->ctx, st, net->d2h_done[buf]));
         net->fit_out_copy = out_host ? net->out_stage[buf] : nullptr;
         int rc = b200_net_train_step(net, net->x_stage[buf], net->t_stage[buf], batch, loss_kind, opt_kind, h);
         net->fit_out_copy = nullptr;
@@ -1421,7 +1425,7 @@ int b200_net_fit_host_enqueue(b200_net *net, const float *x_host, const float *t
         B200_CUDA(cudaEventRecord(net->stage_free[buf], st));  // the step reads its input to the end (first layer's dW)
         if (out_host) {
           net->out_stage_used[buf] = true;
-          B200_CUDA(cudaStreamWaitEvent(net->d2h_stream, net->stage_free[buf], 0));
+          B200_TRY(stream_wait(net->ctx, net->d2h_stream, net->stage_free[buf]));
           B200_CUDA(cudaMemcpyAsync(out_host + (size_t)i * out_dim, net->out_stage[buf], out_dim * nb * sizeof(float),
                                     cudaMemcpyDeviceToHost, net->d2h_stream));
           B200_CUDA(cudaEventRecord(net->d2h_done[buf], net->d2h_stream));
@@ -1490,13 +1494,13 @@ int b200_net_fit_u8_host(b200_net *net, const b200_image_desc *d, const uint8_t 
       int run_nb = 0;
       B200_TRY(fit_step_rows(net, nb, batch, &run_nb));
       const int buf = (int)(step & 1);
-      if (step >= 2) B200_CUDA(cudaStreamWaitEvent(net->copy_stream, net->stage_free[buf], 0));
+      if (step >= 2) B200_TRY(stream_wait(net->ctx, net->copy_stream, net->stage_free[buf]));
       B200_CUDA(cudaMemcpyAsync(net->u8_stage[buf], images_host + (size_t)i * img_bytes, img_bytes * nb,
                                 cudaMemcpyHostToDevice, net->copy_stream));
       B200_CUDA(cudaMemcpyAsync(net->label_stage[buf], labels_host + i, (size_t)nb, cudaMemcpyHostToDevice,
                                 net->copy_stream));
       B200_CUDA(cudaEventRecord(net->up_done[buf], net->copy_stream));
-      B200_CUDA(cudaStreamWaitEvent(st, net->up_done[buf], 0));
+      B200_TRY(stream_wait(net->ctx, st, net->up_done[buf]));
       B200_TRY(fit_rows_to_fixed(net));
       // scale / pad the bytes into the step's fixed input rows, labels into its target rows
       B200_TRY(images_u8_to_float(net->ctx, d, net->u8_stage[buf], nb, net->x_dev));

@@ -720,6 +720,7 @@ __host__ __device__ __forceinline__ int reduce_entries(const SmallStep &L, int B
 
 __global__ void __launch_bounds__(256) small_reduce_kernel(const __grid_constant__ SmallNet net, const float *__restrict__ x,
                                                            int B) {
+  after_previous_kernel();
   __shared__ float lanes[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   int s = 0, blk = blockIdx.x, per_block;
@@ -914,8 +915,7 @@ int small_net_run(b200_ctx *ctx, const SmallNet &n, const float *x, const float 
   int blocks = 0;
   for (int i = 0; i < n.n; ++i) blocks += ceil_div(n.step[i].w_len + n.step[i].b_len, reduce_entries(n.step[i], B));
   if (blocks == 0) return 0;
-  small_reduce_kernel<<<blocks, 256, 0, ctx->stream>>>(n, x, B);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, small_reduce_kernel, dim3(blocks), dim3(256), 0, 1, n, x, B));
   return 0;
 }
 

@@ -97,6 +97,7 @@ __device__ __forceinline__ void pieces_map(int c, int C, int S4, int n0, int n1,
 // left the variance with five digits.)
 __global__ void __launch_bounds__(BN_THREADS) bn_moments_kernel(const float *__restrict__ x, int S, int B,
                                                                 double2 *__restrict__ part, int vec4) {
+  after_previous_kernel();
   const int c = blockIdx.x, C = gridDim.x, z = blockIdx.y, Z = gridDim.y;
   const int n0 = (int)((long long)B * z / Z), n1 = (int)((long long)B * (z + 1) / Z);
   double s1 = 0., s2 = 0.;
@@ -163,6 +164,7 @@ __device__ __forceinline__ void merge_slices(const double2 *part, int c, int C, 
 __global__ void __launch_bounds__(BN_THREADS) bn_sum_kernel(const float *__restrict__ x, const float *__restrict__ y,
                                                             int S, int B, float *__restrict__ part_x,
                                                             float *__restrict__ part_xy, int vec4) {
+  after_previous_kernel();
   const int c = blockIdx.x, C = gridDim.x, z = blockIdx.y, Z = gridDim.y;
   const int n0 = (int)((long long)B * z / Z), n1 = (int)((long long)B * (z + 1) / Z);
   float sx = 0.f, sxy = 0.f;
@@ -195,6 +197,7 @@ __global__ void __launch_bounds__(BN_THREADS) bn_apply_kernel(const float *__res
                                                               int B, float eps, int slices,
                                                               const double2 *__restrict__ part, float *mean_io, float *var_io,
                                                               float *__restrict__ stddev, int vec4) {
+  after_previous_kernel();
   const int c = blockIdx.x, C = gridDim.x, z = blockIdx.y, Z = gridDim.y;
   float mean, var;
   if (part != nullptr) {
@@ -244,6 +247,7 @@ __global__ void __launch_bounds__(BN_THREADS, 5) bn_bwd_kernel(const float *__re
                                                             const float *__restrict__ part_d,
                                                             const float *__restrict__ part_dy,
                                                             const float *__restrict__ stddev, int vec4) {
+  after_previous_kernel();
   const int c = blockIdx.x, C = gridDim.x, z = blockIdx.y, Z = gridDim.y;
   const float count = (float)B * (float)S;
   __shared__ Slices p;
@@ -352,11 +356,10 @@ int batchnorm_fwd(b200_ctx *ctx, int channels, int spatial, float eps, const flo
   double2 *part = reinterpret_cast<double2 *>(scratch);
   const int vec4 = spatial % 4 == 0 && aligned16(x) && aligned16(y);
   if (train) {
-    bn_moments_kernel<<<grid, BN_THREADS, 0, ctx->stream>>>(x, spatial, B, part, vec4);
-    B200_LAUNCHED();
+    B200_TRY(launch_kernel(ctx, bn_moments_kernel, dim3(grid), dim3(BN_THREADS), 0, 1, x, spatial, B, part, vec4));
   }
-  bn_apply_kernel<<<grid, BN_THREADS, 0, ctx->stream>>>(x, y, spatial, B, eps, Z, train ? part : nullptr, mean, variance, stddev, vec4);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, bn_apply_kernel, dim3(grid), dim3(BN_THREADS), 0, 1, x, y, spatial, B, eps, Z,
+                         train ? part : nullptr, mean, variance, stddev, vec4));
   return 0;
 }
 
@@ -367,10 +370,9 @@ int batchnorm_bwd(b200_ctx *ctx, int channels, int spatial, const float *y, cons
   const dim3 grid(channels, Z);
   float *part_d = scratch, *part_dy = scratch + (size_t)Z * channels;
   const int vec4 = spatial % 4 == 0 && aligned16(y) && aligned16(dy) && aligned16(dx);
-  bn_sum_kernel<<<grid, BN_THREADS, 0, ctx->stream>>>(dy, y, spatial, B, part_d, part_dy, vec4);
-  B200_LAUNCHED();
-  bn_bwd_kernel<<<grid, BN_THREADS, 0, ctx->stream>>>(y, dy, dx, spatial, B, Z, part_d, part_dy, stddev, vec4);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, bn_sum_kernel, dim3(grid), dim3(BN_THREADS), 0, 1, dy, y, spatial, B, part_d, part_dy, vec4));
+  B200_TRY(launch_kernel(ctx, bn_bwd_kernel, dim3(grid), dim3(BN_THREADS), 0, 1, y, dy, dx, spatial, B, Z, part_d, part_dy,
+                         stddev, vec4));
   return 0;
 }
 

@@ -47,6 +47,7 @@ __global__ void maxpool_fwd_kernel(const __grid_constant__ b200_pool_desc d, con
                                    float *__restrict__ out, int32_t *__restrict__ argmax, I total,
                                    const __grid_constant__ Divider<I> ow, const __grid_constant__ Divider<I> oh,
                                    const __grid_constant__ Divider<I> ch) {
+  after_previous_kernel();
   I idx = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
   const I step = (I)gridDim.x * (I)blockDim.x;
   const I in_row = (I)d.in_c * d.in_h * d.in_w;
@@ -81,6 +82,7 @@ __global__ void maxpool_bwd_kernel(const __grid_constant__ b200_pool_desc d, con
                                    const __grid_constant__ Divider<I> iw, const __grid_constant__ Divider<I> ih,
                                    const __grid_constant__ Divider<I> ch, const __grid_constant__ Divider<I> sh,
                                    const __grid_constant__ Divider<I> sw) {
+  after_previous_kernel();
   I idx = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
   const I step = (I)gridDim.x * (I)blockDim.x;
   const I out_row = (I)d.in_c * d.out_h * d.out_w;
@@ -106,6 +108,7 @@ __global__ void maxpool2x2_fwd_kernel(int in_w, int in_h, int out_w, int out_h, 
                                       const float *__restrict__ in, float *__restrict__ out,
                                       int32_t *__restrict__ argmax, int in_c, const __grid_constant__ Divider<I> d_ow2,
                                       const __grid_constant__ Divider<I> d_oh, const __grid_constant__ Divider<I> d_ch) {
+  after_previous_kernel();
   const I ow2 = (I)(out_w >> 1);  // output pairs per row
   const I total = (I)planes * (I)out_h * ow2;
   I idx = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
@@ -148,6 +151,7 @@ __global__ void maxpool2x2_bwd_kernel(int in_w, int in_h, int out_w, int out_h, 
                                       const float *__restrict__ pooled_y, float *__restrict__ din, int in_c,
                                       const __grid_constant__ Divider<I> d_ow2, const __grid_constant__ Divider<I> d_oh,
                                       const __grid_constant__ Divider<I> d_ch) {
+  after_previous_kernel();
   const I ow2 = (I)(out_w >> 1), oh = (I)out_h, ic = (I)in_c;
   const I total = (I)planes * oh * ow2;
   I idx = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
@@ -311,12 +315,10 @@ static bool pool2x2_fast(const b200_pool_desc &d) {
 
 // f(I) with the type that indexes the layer's tensors, and a step past their ends
 template <typename F>
-static void by_size(const b200_pool_desc &d, int B, F f) {
+static int by_size(const b200_pool_desc &d, int B, F f) {
   const long long rows = (long long)B * d.in_c, in = rows * d.in_h * d.in_w, out = rows * d.out_h * d.out_w;
-  if ((in > out ? in : out) < (1LL << 31))
-    f(0u);
-  else
-    f(0ll);
+  if ((in > out ? in : out) < (1LL << 31)) return f(0u);
+  return f(0ll);
 }
 
 int maxpool_fwd(b200_ctx *ctx, const b200_pool_desc &d, const float *in, float *out,
@@ -326,21 +328,19 @@ int maxpool_fwd(b200_ctx *ctx, const b200_pool_desc &d, const float *in, float *
   if (total == 0) return 0;
   if (pool2x2_fast(d) && aligned16(in) && aligned16(out) && aligned16(argmax)) {
     long long planes = (long long)B * d.in_c;
-    by_size(d, B, [&](auto one) {
+    B200_TRY(by_size(d, B, [&](auto one) {
       using I = decltype(one);
-      maxpool2x2_fwd_kernel<I><<<grid_for(total / 2, 256, ctx->sm_count), 256, 0, ctx->stream>>>(
-        d.in_w, d.in_h, d.out_w, d.out_h, planes, in, out, argmax, d.in_c, Divider<I>(d.out_w / 2), Divider<I>(d.out_h),
-        Divider<I>(d.in_c));
-    });
-    B200_LAUNCHED();
+      return launch_kernel(ctx, maxpool2x2_fwd_kernel<I>, dim3(grid_for(total / 2, 256, ctx->sm_count)), dim3(256), 0, 1,
+                           d.in_w, d.in_h, d.out_w, d.out_h, planes, in, out, argmax, d.in_c, Divider<I>(d.out_w / 2),
+                           Divider<I>(d.out_h), Divider<I>(d.in_c));
+    }));
     return 0;
   }
-  by_size(d, B, [&](auto one) {
+  B200_TRY(by_size(d, B, [&](auto one) {
     using I = decltype(one);
-    maxpool_fwd_kernel<I><<<grid_for(total, 256, ctx->sm_count), 256, 0, ctx->stream>>>(
-      d, in, out, argmax, (I)total, Divider<I>(d.out_w), Divider<I>(d.out_h), Divider<I>(d.in_c));
-  });
-  B200_LAUNCHED();
+    return launch_kernel(ctx, maxpool_fwd_kernel<I>, dim3(grid_for(total, 256, ctx->sm_count)), dim3(256), 0, 1, d, in, out,
+                         argmax, (I)total, Divider<I>(d.out_w), Divider<I>(d.out_h), Divider<I>(d.in_c));
+  }));
   return 0;
 }
 
@@ -357,22 +357,20 @@ int maxpool_bwd(b200_ctx *ctx, const b200_pool_desc &d, const float *dout, const
   if (fast) {
     long long planes = (long long)B * d.in_c;
     long long work = planes * d.out_h * (d.out_w / 2);
-    by_size(d, B, [&](auto one) {
+    B200_TRY(by_size(d, B, [&](auto one) {
       using I = decltype(one);
-      maxpool2x2_bwd_kernel<I><<<grid_for(work, 256, ctx->sm_count), 256, 0, ctx->stream>>>(
-        d.in_w, d.in_h, d.out_w, d.out_h, planes, dout, argmax, pooled_y, din, d.in_c, Divider<I>(d.out_w / 2), Divider<I>(d.out_h),
-        Divider<I>(d.in_c));
-    });
-    B200_LAUNCHED();
+      return launch_kernel(ctx, maxpool2x2_bwd_kernel<I>, dim3(grid_for(work, 256, ctx->sm_count)), dim3(256), 0, 1, d.in_w,
+                           d.in_h, d.out_w, d.out_h, planes, dout, argmax, pooled_y, din, d.in_c, Divider<I>(d.out_w / 2),
+                           Divider<I>(d.out_h), Divider<I>(d.in_c));
+    }));
     return 0;
   }
-  by_size(d, B, [&](auto one) {
+  B200_TRY(by_size(d, B, [&](auto one) {
     using I = decltype(one);
-    maxpool_bwd_kernel<I><<<grid_for(total, 256, ctx->sm_count), 256, 0, ctx->stream>>>(
-      d, dout, argmax, din, (I)total, Divider<I>(d.in_w), Divider<I>(d.in_h), Divider<I>(d.in_c), Divider<I>(d.stride_h),
-      Divider<I>(d.stride_w));
-  });
-  B200_LAUNCHED();
+    return launch_kernel(ctx, maxpool_bwd_kernel<I>, dim3(grid_for(total, 256, ctx->sm_count)), dim3(256), 0, 1, d, dout,
+                         argmax, din, (I)total, Divider<I>(d.in_w), Divider<I>(d.in_h), Divider<I>(d.in_c),
+                         Divider<I>(d.stride_h), Divider<I>(d.stride_w));
+  }));
   return 0;
 }
 

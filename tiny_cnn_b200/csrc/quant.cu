@@ -431,6 +431,7 @@ __global__ void __launch_bounds__(256) q_conv_filter_kernel(const float *__restr
                                                             const float *__restrict__ bias, int nbias, QGlobal *out_qg,
                                                             uint8_t *__restrict__ Wq, uint8_t *__restrict__ bq,
                                                             unsigned *__restrict__ wsum) {
+  after_previous_kernel();
   __shared__ QGlobal qg;
   __shared__ unsigned part[8];
   filter_range(W, nseg, seg_stride, seg_len, bias, nbias, qg);
@@ -487,6 +488,7 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
   unsigned *xsum = psum + a.rows * a.WI;                                             // [per] over the window
   int *acc = a.acc_smem ? reinterpret_cast<int *>(xsum + a.per) : reinterpret_cast<int *>(a.out) + (size_t)n * a.OC * npix + p0;
   const int acc_step = a.acc_smem ? a.per : npix;                                    // from output channel to output channel
+  wait_for_previous_kernel();
   for (int i = tid; i < a.ntiles * 8 * a.pitch / 16; i += QC_THREADS) cp_async16(ws + 16 * i, a.Wq + 16 * i, true);
   cp_async_commit();
   for (int i = tid; i < a.ksteps * 4; i += QC_THREADS) {
@@ -1066,24 +1068,13 @@ int qconv_fwd(b200_ctx *ctx, const b200_conv_desc *d, const float *in, const flo
       QScratch s;
       B200_TRY(q_carve(ctx, 1, 0, (size_t)a.ntiles * 8 * a.pitch, g.OC, (size_t)a.ntiles * 8, &s));
       unsigned *wsum = reinterpret_cast<unsigned *>(s.acc);
-      q_conv_filter_kernel<<<a.ntiles * 8, 256, 0, st>>>(W, g.C, plane, (size_t)g.KH * g.KH, g.C, a.Cp, g.OC, g.KH * g.KW,
-                                                        a.pitch, bias, nbias, s.qg, s.Wq, s.bq, wsum);
-      B200_LAUNCHED();
+      B200_TRY(launch_kernel(ctx, q_conv_filter_kernel, dim3(a.ntiles * 8), dim3(256), 0, 1, W, g.C, plane,
+                             (size_t)g.KH * g.KH, g.C, a.Cp, g.OC, g.KH * g.KW, a.pitch, bias, nbias, s.qg, s.Wq, s.bq,
+                             wsum));
       a.Wq = s.Wq, a.bq = s.bq, a.wsum = wsum, a.qg = s.qg;
       B200_CUDA(cudaFuncSetAttribute(q_conv_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      cudaLaunchConfig_t c = {};
-      c.gridDim = dim3((unsigned)(B * nc));
-      c.blockDim = dim3(QC_THREADS);
-      c.dynamicSmemBytes = smem;
-      c.stream = st;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = (unsigned)nc;
-      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-      c.attrs = at;
-      c.numAttrs = 1;
-      B200_CUDA(cudaLaunchKernelEx(&c, q_conv_fused_kernel, a));
-      B200_LAUNCHED();
+      B200_TRY(launch_kernel(ctx, q_conv_fused_kernel, dim3((unsigned)(B * nc)), dim3(QC_THREADS), smem, dim3((unsigned)nc),
+                             a));
       return 0;
     }
   }
