@@ -132,6 +132,17 @@ __global__ void q_input_range_kernel(const float *__restrict__ in, size_t row_le
 
 // ---- 2. filter / bias ranges ---------------------------------------------------
 
+__device__ __forceinline__ void widen_ranges(float w0, float b0, int nbias, float *mn, float *mx, float *bmn, float *bmx) {
+  if (*mn == *mx) {
+    *mx = __fadd_rn(w0, 1e-3f);
+    *mn = __fsub_rn(w0, 1e-3f);
+  }
+  if (nbias > 0 && *bmn == *bmx) {
+    *bmx = __fadd_rn(b0, 1e-3f);
+    *bmn = __fsub_rn(b0, 1e-3f);
+  }
+}
+
 // By a whole block.  Filter: `nseg` segments of `seg_len` elements every
 // `seg_stride`, seeded with W[0]; equal min/max widen to W[0] -+ 1e-3.
 // Bias: all `nbias` elements, seeded with 0; equal min/max widen to b[0] -+ 1e-3.
@@ -171,14 +182,7 @@ __device__ __forceinline__ void filter_range(const float *__restrict__ W, int ns
     bmn = warp_min(lane < nw ? s4[2][lane] : s4[2][0]);
     bmx = warp_max(lane < nw ? s4[3][lane] : s4[3][0]);
     if (lane == 0) {
-      if (mn == mx) {
-        mx = __fadd_rn(W[0], 1e-3f);
-        mn = __fsub_rn(W[0], 1e-3f);
-      }
-      if (nbias > 0 && bmn == bmx) {
-        bmx = __fadd_rn(bias[0], 1e-3f);
-        bmn = __fsub_rn(bias[0], 1e-3f);
-      }
+      widen_ranges(W[0], nbias > 0 ? bias[0] : 0.f, nbias, &mn, &mx, &bmn, &bmx);
       qg.min_f = mn;
       qg.max_f = mx;
       qg.min_b = bmn;
@@ -378,24 +382,41 @@ __global__ void q_requant_dequant_kernel(const int *__restrict__ acc, size_t out
 // (blocks exchange theirs), quantizes the input rows that it needs into shared memory with the channels fastest,
 // takes the products, exchanges the accumulators' extremes and requantizes.  In eight launches each step read and
 // wrote memory (28x28x32 -> 64, 5x5, 128 samples: 247 us, of which the dp4a products 174 us and the requantizing
-// 20 us; this 65 us).  What bounds it: the products' shared-memory reads, 8 bytes a lane for every two
-// 16 x 8 x 32 products of a fragment, and then the requantizing's 64-bit integer multiplications.
+// 20 us; in one 66 us with the sums in shared memory, a filter fragment read for every unit, and values quantized in double
+// precision and requantized in 64 bits; this 53 us).  Cycles of a block there: range 8 k, quantizing 15 k, byte sums 5 k, products 24 k (were
+// 40 k; shared-memory reads), extremes 8 k, requantizing 28 k.
 // A k step is 32 bytes: four groups of 8 channels, wherever in the window they lie (`tab`); channels are
 // padded to 8, the filter's rows to 32 bytes with zeros.
-struct QScale {  // f2q<8> of one range: the same operations, the ones that do not depend on the value done once
+__device__ __noinline__ unsigned quantize_in_double(float v, double scale, double low) {
+  const long long q = (long long)__dsub_rn(round(__dmul_rn((double)v, scale)), low);
+  return (unsigned)(q > 0 ? (q < 255 ? q : 255) : 0);
+}
+
+// f2q<8> of one range: the same operations, the ones that do not depend on the value done once.  Almost every value needs no
+// double: the 32-bit product is off by 2^-23 of itself at most, so where its distance from the nearest whole number is that
+// far from one half, the exact product rounds to the same one.  (In double alone, with a 64-bit conversion, a value took three times
+// as many instructions: 9216 -> 256 with 128 samples spent 12 us on them.)
+struct QScale {
   double scale, low;
-  bool flat;
+  float scale32;
+  int low32;
+  bool flat, quick;
   __device__ __forceinline__ void set(float rmin, float rmax) {
     flat = rmin == rmax;
     const double range_adjust = __ddiv_rn(256.0, __dsub_rn(256.0, 1.0));
     const double range = __dmul_rn((double)__fsub_rn(rmax, rmin), range_adjust);
     scale = __ddiv_rn(256.0, range);
     low = round(__dmul_rn((double)rmin, scale));
+    scale32 = (float)scale;
+    quick = fabs(low) < 2097152.0 && scale > 1e-30 && scale < 1e30;
+    low32 = quick ? (int)low : 0;
   }
   __device__ __forceinline__ unsigned of(float v) const {
     if (flat) return 0u;
-    const long long q = (long long)__dsub_rn(round(__dmul_rn((double)v, scale)), low);
-    return (unsigned)(q > 0 ? (q < 255 ? q : 255) : 0);
+    const float f = __fmul_rn(v, scale32), t = __fadd_rn(f, 12582912.f);  // 1.5 * 2^23: the whole number is in the last bits
+    if (quick && fabsf(f) < 2097152.f && fabsf(__fsub_rn(f, __fsub_rn(t, 12582912.f))) < 0.5f - fabsf(f) * 2.4e-7f)
+      return (unsigned)min(255, max(0, __float_as_int(t) - 0x4b400000 - low32));
+    return quantize_in_double(v, scale, low);
   }
 };
 
@@ -417,6 +438,7 @@ struct QConvArgs {
   int C, HI, WI, OC, OH, OW, KH, KW, SH, SW, has_bias;
   int Cp, ksteps, pitch, ntiles;  // channels padded to 8; k steps; bytes of a filter row; 8-channel tiles of the outputs
   int per, rows;                  // output pixels of a block (a multiple of 16), most input rows it needs
+  int copies;                     // of the table of results: 32 or 1
   int acc_smem;                   // the accumulators wait in shared memory, not in the output's place
 };
 
@@ -469,11 +491,47 @@ __device__ __forceinline__ unsigned q_remote(const void *p, int rank) {  // a wo
   return v;
 }
 
+__device__ __noinline__ int requant_in_64_bits(int acc, const QSample &s) { return requant_one(acc, s); }
+
+// requant_one in 32 bits where that decides it.  The quotient before rounding is off by `bound` at most: three roundings of the
+// product and two of the sum, relative to the largest accumulator of the sample, and the 64-bit form's own cut at
+// 2^-16.  Above zero that form rounds to the nearest whole number, below zero to the one under it; a value further than the
+// bound from a half, and from zero, does so for certain.  One in some thousands goes the long way.
+struct QQuick {
+  float scale, offset, bound;
+  int out;
+  bool on;
+  __device__ __forceinline__ void set(const QSample &s) {
+    scale = __fmul_rn(__ll2float_rn(s.range_scale_fp), 3.5527136788005009e-15f);  // 2^-48
+    offset = __fmul_rn(__ll2float_rn(s.input_offset_fp), 1.52587890625e-5f);      // 2^-16
+    const float most = __fadd_rn(__fmul_rn(fmaxf(fabsf((float)s.acc_min), fabsf((float)s.acc_max)), scale), fabsf(offset));
+    bound = __fadd_rn(2e-5f, __fmul_rn(most, 5e-7f));
+    on = s.output_offset_fp > -2097152 && s.output_offset_fp < 2097152 && most < 1048576.f && scale > 1e-30f;
+    out = on ? (int)s.output_offset_fp + 0x4b400000 : 0;
+  }
+  __device__ __forceinline__ int of(int acc, const QSample &s) const {
+    const float f = __fadd_rn(__fmul_rn((float)acc, scale), offset), t = __fadd_rn(f, 12582912.f);  // 1.5 * 2^23
+    if (on && fabsf(__fsub_rn(f, __fsub_rn(t, 12582912.f))) < 0.5f - bound && fabsf(f) > bound)
+      return min(255, max(0, __float_as_int(t) - out + (__float_as_int(f) >> 31)));
+    return requant_in_64_bits(acc, s);
+  }
+};
+__device__ __forceinline__ uint2 q_lds8(unsigned at) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "r"(at));
+  return v;
+}
+
+constexpr int QC_UNITS = 5;  // units of 16 pixels x 32 outputs whose sums a warp keeps in registers
+
+// REGS: the sums wait for the sample's extremes in registers, not in shared memory or in the output's place
+template <bool REGS>
 __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __grid_constant__ QConvArgs a) {
   extern __shared__ __align__(16) uint8_t qsm[];
   __shared__ float rmin[QC_WARPS], rmax[QC_WARPS], range[2];
   __shared__ int amin[QC_WARPS], amax[QC_WARPS], extremes[2];
   __shared__ QSample smp;
+  __shared__ QQuick quick;
   __shared__ float lut[256];
   int nc, rank;
   asm("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(nc));
@@ -500,8 +558,19 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
   {
     float mn = in[0], mx = in[0];
     const int scan = a.HI * a.HI, parts = max(1, QC_WARPS * nc / a.C), span = (scan + parts - 1) / parts;
+    const bool vec = ((plane | scan) & 3) == 0 && parts == 1 && ((uintptr_t)in & 15) == 0;
     for (int u = rank * QC_WARPS + warp; u < a.C * parts; u += nc * QC_WARPS) {
       const int c = u / parts, b = (u - c * parts) * span;
+      if (vec) {  // a plane's loads asked for at once
+        const float4 *p = reinterpret_cast<const float4 *>(in + (size_t)c * plane);
+#pragma unroll 8
+        for (int e = lane; e < scan / 4; e += 32) {
+          const float4 v = p[e];
+          mn = fminf(mn, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
+          mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+        }
+        continue;
+      }
 #pragma unroll 8
       for (int e = b + lane; e < min(scan, b + span); e += 32) {
         const float v = in[(size_t)c * plane + e];
@@ -525,11 +594,11 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
       }
     }
     q_cluster_sync(nc);
+    if (warp == 0 && nc > 1) {  // a lane a block: one after the other they take 250 cycles each
+      mn = warp_min(__uint_as_float(q_remote(&range[0], lane & (nc - 1))));
+      mx = warp_max(__uint_as_float(q_remote(&range[1], lane & (nc - 1))));
+    }
     if (tid == 0) {
-      for (int r = 0; r < nc && nc > 1; ++r) {
-        mn = fminf(mn, __uint_as_float(q_remote(&range[0], r)));
-        mx = fmaxf(mx, __uint_as_float(q_remote(&range[1], r)));
-      }
       smp.min_in = mn;
       smp.max_in = mx;
       sample_params(smp, *a.qg, 0);
@@ -539,16 +608,30 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
   {
     QScale q;
     q.set(smp.min_in, smp.max_in);
-    const int groups = a.Cp / 4;
-#pragma unroll 2
-    for (int j = tid; j < places * groups; j += QC_THREADS) {
-      const int cg = j / places, p = j - cg * places;
-      const float *src = in + (size_t)cg * 4 * plane + iy0 * a.WI + p;
-      unsigned w = 0;
+    const int groups = a.Cp / 8;
+    int cg = tid / places, p = tid - cg * places;  // eight channels of a place
+    const int stepg = QC_THREADS / places, stepp = QC_THREADS - stepg * places;
+    float next[8];
+    auto fetch = [&]() {
+      const float *src = in + (size_t)cg * 8 * plane + iy0 * a.WI + p;
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (cg * 4 + k < a.C) w |= q.of(src[(size_t)k * plane]) << (8 * k);
-      *reinterpret_cast<unsigned *>(xs + (size_t)p * a.Cp + cg * 4) = w;
+      for (int k = 0; k < 8; ++k) next[k] = cg < groups && cg * 8 + k < a.C ? src[(size_t)k * plane] : 0.f;
+    };
+    if (places > 0) fetch();
+    while (places > 0 && cg < groups) {
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = next[k];
+      const int c0 = cg * 8;
+      uint8_t *dst = xs + (size_t)p * a.Cp + c0;
+      cg += stepg, p += stepp;
+      if (p >= places) p -= places, ++cg;
+      fetch();  // the next place's values are on their way meanwhile
+      unsigned w[2] = {0u, 0u};
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (c0 + k < a.C) w[k >> 2] |= q.of(v[k]) << (8 * (k & 3));
+      *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
     }
   }
   cp_async_wait<0>();
@@ -575,18 +658,15 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
   const unsigned off_f = (unsigned)a.qg->off_f, off_in = (unsigned)smp.off_in, both = (unsigned)(KK * a.C) * off_f * off_in;
   const int mtiles = (p1 - p0 + 15) / 16, ngroups = (a.ntiles + 3) / 4, g = lane >> 2, q = lane & 3;
   int mn = INT_MAX, mx = INT_MIN;
-  for (int u = warp; u < mtiles * ngroups; u += QC_WARPS) {
+  auto products = [&](int u, unsigned(&c)[4][4]) {
     const int ng = u / mtiles, m = u - ng * mtiles, nt = min(4, a.ntiles - ng * 4);
     const uint8_t *x[2];
-    int pix[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      pix[e] = m * 16 + g + 8 * e;
-      const int p = min(p0 + pix[e], p1 - 1), y = p / a.OW;
+      const int p = min(p0 + m * 16 + g + 8 * e, p1 - 1), y = p / a.OW;
       x[e] = xs + ((size_t)(y * a.SH - iy0) * a.WI + (p - y * a.OW) * a.SW) * a.Cp;
     }
     const uint8_t *w = ws + (size_t)(ng * 32 + g) * a.pitch + q * 8;
-    unsigned c[4][4];
 #pragma unroll
     for (int t = 0; t < 4; ++t)
 #pragma unroll
@@ -601,18 +681,96 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
         mma_u8(c[t], a0, a1, b);
       }
     }
+  };
+  // f(output channel, pixel, sum) for what this lane holds of a unit
+  auto each = [&](int u, const unsigned(&c)[4][4], auto f) {
+    const int ng = u / mtiles, m = u - ng * mtiles;
 #pragma unroll
     for (int t = 0; t < 4; ++t)
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int o = (ng * 4 + t) * 8 + q * 2 + (k & 1), p = pix[k >> 1];
-        if (t >= nt || o >= a.OC || p >= p1 - p0) continue;
-        int v = (int)(c[t][k] - off_in * a.wsum[o] - off_f * xsum[p] + both);
-        if (a.has_bias) v += (int)a.bq[o] - smp.zero_total;
+        const int o = (ng * 4 + t) * 8 + q * 2 + (k & 1), p = m * 16 + g + 8 * (k >> 1);
+        if (o < a.OC && p < p1 - p0) f(o, p, c[t][k]);
+      }
+  };
+  auto value = [&](int o, int p, unsigned sum) {
+    const int v = (int)(sum - off_in * a.wsum[o] - off_f * xsum[p] + both);
+    return a.has_bias ? v + (int)a.bq[o] - smp.zero_total : v;
+  };
+  const int units = mtiles * ngroups;
+  // REGS: a warp's units are pixels of one group of outputs, so that a filter fragment serves all of them: 14 reads of
+  // shared memory for 20 products (unit by unit 30, and these reads are what the products take their time for)
+  const int wper = REGS ? QC_WARPS / ngroups : 1, wgroup = warp / wper, wfirst = wgroup < ngroups ? warp - wgroup * wper : mtiles;
+  auto unit_of = [&](int i) { return wgroup * mtiles + wfirst + i * wper; };
+  auto has = [&](int i) { return wfirst + i * wper < mtiles; };
+  unsigned c[REGS ? QC_UNITS : 1][4][4];
+  if (REGS) {
+    unsigned x[QC_UNITS][2];
+#pragma unroll
+    for (int i = 0; i < QC_UNITS; ++i) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int p = min(p0 + (wfirst + i * wper) * 16 + g + 8 * e, p1 - 1), y = p / a.OW;
+        x[i][e] = smem_u32(xs) + (unsigned)((y * a.SH - iy0) * a.WI + (p - y * a.OW) * a.SW) * a.Cp;
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) c[i][t][k] = 0;
+    }
+    if (wfirst < mtiles) {
+      const int nt = min(4, a.ntiles - wgroup * 4);
+      const unsigned w = smem_u32(ws) + (unsigned)((wgroup * 32 + g) * a.pitch + q * 8);
+      const unsigned step[4] = {0u, nt > 1 ? 8u * a.pitch : 0u, nt > 2 ? 16u * a.pitch : 0u, nt > 3 ? 24u * a.pitch : 0u};
+      for (int ks = 0; ks < a.ksteps; ++ks) {
+        const unsigned off = (unsigned)tab[ks * 4 + q];
+        uint2 f[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) f[t] = q_lds8(w + step[t] + ks * 32);
+#pragma unroll
+        for (int i = 0; i < QC_UNITS; ++i) {
+          if (!has(i)) break;
+          const uint2 a0 = q_lds8(x[i][0] + off), a1 = q_lds8(x[i][1] + off);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) mma_u8(c[i][t], a0, a1, f[t]);
+        }
+      }
+    }
+    unsigned of_out[4][2];  // what belongs to an output
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int o = (wgroup * 4 + t) * 8 + q * 2 + k;
+        of_out[t][k] = wgroup < ngroups && o < a.OC ? both - off_in * a.wsum[o] + (a.has_bias ? (unsigned)((int)a.bq[o] - smp.zero_total) : 0u) : 0u;
+      }
+#pragma unroll
+    for (int i = 0; i < QC_UNITS; ++i) {
+      if (!has(i)) break;
+      const int m = wfirst + i * wper;
+      const int pa = m * 16 + g, pb = pa + 8;
+      const unsigned xa = pa < p1 - p0 ? off_f * xsum[pa] : 0u, xb = pb < p1 - p0 ? off_f * xsum[pb] : 0u;
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int o = (wgroup * 4 + t) * 8 + q * 2 + (k & 1);
+          c[i][t][k] += of_out[t][k & 1] - (k < 2 ? xa : xb);
+          if (o >= a.OC || (k < 2 ? pa : pb) >= p1 - p0) continue;
+          mn = min(mn, (int)c[i][t][k]);
+          mx = max(mx, (int)c[i][t][k]);
+        }
+    }
+  } else {
+    for (int u = warp; u < units; u += QC_WARPS) {
+      products(u, c[0]);
+      each(u, c[0], [&](int o, int p, unsigned sum) {
+        const int v = value(o, p, sum);
         acc[(size_t)o * acc_step + p] = v;
         mn = min(mn, v);
         mx = max(mx, v);
-      }
+      });
+    }
   }
   mn = warp_min_i(mn);
   mx = warp_max_i(mx);
@@ -630,24 +788,41 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
     }
   }
   q_cluster_sync(nc);
+  if (warp == 0 && nc > 1) {
+    mn = warp_min_i((int)q_remote(&extremes[0], lane & (nc - 1)));
+    mx = warp_max_i((int)q_remote(&extremes[1], lane & (nc - 1)));
+  }
   if (tid == 0) {
-    for (int r = 0; r < nc && nc > 1; ++r) {
-      mn = min(mn, (int)q_remote(&extremes[0], r));
-      mx = max(mx, (int)q_remote(&extremes[1], r));
-    }
     smp.acc_min = mn;
     smp.acc_max = mx;
     requant_params(smp);
+    quick.set(smp);
   }
   q_cluster_sync(nc);  // nobody leaves while others may read its extremes
   const QSample s = smp;
-  if (tid < 256) lut[tid] = q2f<8>(tid, s.min_new, s.max_new);
+  // the 256 results: a copy for every lane where filter and input were, so that no two lanes want the same bank
+  float *table = a.copies > 1 ? reinterpret_cast<float *>(qsm) : lut;
+  if (a.copies > 1) {
+    for (int i = warp; i < 256; i += QC_WARPS) table[i * 32 + lane] = q2f<8>(i, s.min_new, s.max_new);
+  } else if (tid < 256) {
+    lut[tid] = q2f<8>(tid, s.min_new, s.max_new);
+  }
   __syncthreads();
+  const int tstep = a.copies, tlane = lane & (a.copies - 1);
   float *out = a.out + (size_t)n * a.OC * npix + p0;
+  const QQuick qk = quick;
+  if (REGS) {
+#pragma unroll
+    for (int i = 0; i < QC_UNITS; ++i) {
+      if (!has(i)) break;
+      each(unit_of(i), c[i], [&](int o, int p, unsigned v) { out[(size_t)o * npix + p] = table[qk.of((int)v, smp) * tstep + tlane]; });
+    }
+    return;
+  }
   const int count = p1 - p0;
   for (int i = tid; i < a.OC * count; i += QC_THREADS) {
     const int o = i / count, p = i - o * count;
-    out[(size_t)o * npix + p] = lut[requant_one(acc[(size_t)o * acc_step + p], s)];
+    out[(size_t)o * npix + p] = table[qk.of(acc[(size_t)o * acc_step + p], smp) * tstep + tlane];
   }
 }
 
@@ -656,12 +831,14 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
 // Four launches: ranges of the samples and of the filter (B + `wblocks` blocks), quantizing (the filter transposed to
 // [out][in]), the byte products (tensor cores as above; tiles of 64 samples x 64 outputs, the inputs dealt to
 // enough blocks to fill the chip, whole-number sums added in any order), and a sample's requantizing by one block.
-// In nine launches 9216 -> 256 of 128 samples took 64 us, now 34 us; what is left is reading the filter twice
-// and the gaps between the launches.
+// In nine launches 9216 -> 256 of 128 samples took 64 us, in four 34 us, and 23 us since a launch overlaps the end of the one
+// before it and few values are quantized in double precision; what is left is reading the filter twice and four chains of
+// load, arithmetic and store.
 __global__ void __launch_bounds__(256) q_fc_range_kernel(const float *__restrict__ in, int in_size, int B,
                                                          const float *__restrict__ W, size_t lenW, int out_size, QSample *qs,
                                                          float *__restrict__ part, int *__restrict__ acc,
                                                          unsigned *__restrict__ wsum) {
+  after_previous_kernel();
   const bool row = (int)blockIdx.x < B;
   const int w = blockIdx.x - B, nw = gridDim.x - B;
   const float *v = row ? in + (size_t)blockIdx.x * in_size : W;
@@ -716,8 +893,9 @@ __global__ void __launch_bounds__(256) q_fc_range_kernel(const float *__restrict
 }
 
 // The first blocks take 32 outputs x 128 inputs of the filter each, the others 1024 bytes of a sample's row.  Bound by the latency
-// of a filter block's chain (range, then loads and conversions in double precision), so those start first and are short
-// (9216 -> 256, 128 samples: 18.3 us with 256 inputs a block behind the rows, now 12.07 us).
+// of a filter block's chain (range, then loads and conversions), so those start first, are short, and ask for their part of the
+// filter before they wait for the ranges (9216 -> 256, 128 samples: 18.3 us with 256 inputs a block behind the rows, 12.07 us
+// with every value in double precision and all loads behind the wait).
 constexpr int QF_CIN = 128;
 __global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restrict__ in, int in_size, int B, int pitch,
                                                             int rblocks, const float *__restrict__ W, int out_size,
@@ -728,6 +906,7 @@ __global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restr
                                                             unsigned *__restrict__ wsum) {
   const int b = blockIdx.x, fblocks = gridDim.x - B * rblocks;
   if (b >= fblocks) {
+    after_previous_kernel();
     const int n = (b - fblocks) / rblocks, j0 = (b - fblocks - n * rblocks) * 1024 + threadIdx.x * 4;
     const float *r = in + (size_t)n * in_size;
     QScale q;
@@ -765,6 +944,7 @@ __global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restr
     const int c = c0 + warp + 8 * k, i = i0 + lane;
     x[k] = c < in_size && i < out_size ? W[(size_t)c * out_size + i] : 0.f;
   }
+  after_previous_kernel();  // the filter's values, which the ranges' kernel only read, may be asked for ahead of it
   // the partial results stand in for the filter: same extremes, and when all are equal so is W[0]
   filter_range(part, 1, 0, (size_t)2 * nparts, bias, nbias, qg);
   if (b == 0) {
@@ -808,6 +988,7 @@ __global__ void __launch_bounds__(256) q_fc_gemm_kernel(int B, int out_size, int
 #pragma unroll
     for (int k = 0; k < 4; ++k) c[t][k] = 0;
   const uint8_t *xa = xs + ((warp >> 1) * 16 + g) * ROW + q * 8, *wb = ws + ((warp & 1) * 32 + g) * ROW + q * 8;
+  after_previous_kernel();
   for (int kb = k0; kb < k1; kb += QF_K) {
     for (int i = tid; i < 128 * (QF_K / 16); i += 256) {
       const int r = i / (QF_K / 16), at = i % (QF_K / 16) * 16, k = kb + at;
@@ -841,6 +1022,7 @@ __global__ void __launch_bounds__(256) q_fc_requant_kernel(int in_size, int out_
                                                            const int *__restrict__ acc, const QSample *__restrict__ qs,
                                                            const QGlobal *__restrict__ qg, const unsigned *__restrict__ wsum,
                                                            const uint8_t *__restrict__ bq, float *__restrict__ out) {
+  after_previous_kernel();
   __shared__ QSample s;
   __shared__ int smn[8], smx[8];
   const int n = blockIdx.x, tid = threadIdx.x;
@@ -879,6 +1061,244 @@ __global__ void __launch_bounds__(256) q_fc_requant_kernel(int in_size, int out_
   __syncthreads();
   const QSample t = s;
   for (int i = tid; i < out_size; i += 256) out[(size_t)n * out_size + i] = q2f<8>(requant_one(value(i), t), t.min_new, t.max_new);
+}
+
+// ---- 5d. small fully-connected layers in one launch --------------------------------------------------
+//
+// What bounds the four launches above on a small layer is the chain: range, quantizing, products, requantizing, with a launch and
+// a trip to memory each (232 -> 21, 125 samples: 22.6 us, most of it the host's).  Here one cluster of up to eight blocks goes
+// through the phases with two cluster barriers between them.  A block takes a slice of at most 256 inputs, 64
+// outputs and 128 samples; it reads its values of the filter and the samples once, into registers, finds their
+// ranges, waits for the other blocks', quantizes what it holds into shared memory, and adds its products -- already with the
+// zero points' terms, so that no sums over bytes are exchanged -- to the accumulators.  Behind the second barrier
+// a warp requantizes a sample.  (That layer 11.7 us, 64 -> 10 of one sample 9.0 for 19.0.  With a grid of up to 144 blocks and
+// grid barriers 9216 -> 256 of 128 samples took 43 us, where the launches take 23.)
+constexpr int QO_THREADS = 512, QO_WARPS = QO_THREADS / 32, QO_M = 128, QO_N = 64, QO_BLOCKS = 8;
+constexpr int QO_ROW = 256 + 32;  // bytes from row to row in shared memory: rows on different banks
+constexpr int QO_SMEM = (QO_M + QO_N) * QO_ROW;
+
+struct QFcArgs {
+  const float *in, *W, *bias;
+  float *out;
+  int B, in_size, out_size, nbias;
+  int klog, slices, ntiles;   // inputs of a slice as a power of two
+  int vec;                    // rows of the input start on 16-byte boundaries
+  float2 *wpart, *xpart;      // ranges of the blocks' filter values [blocks] and of the samples' slices [parts][B]
+  float2 *xrange;             // [B]
+  int *acc;                   // [B][out_size]
+};
+
+__global__ void __launch_bounds__(QO_THREADS, 1) q_fc_whole_kernel(const __grid_constant__ QFcArgs a) {
+  extern __shared__ __align__(16) uint8_t qsm[];
+  __shared__ QScale xq[QO_M], wq, bq;
+  __shared__ int xoff[QO_M], xsum[QO_M], wsum[QO_N], off_f;
+  __shared__ QGlobal qg;
+  __shared__ float wmn[QO_WARPS], wmx[QO_WARPS];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ks = blockIdx.x % a.slices, nt = blockIdx.x / a.slices % a.ntiles, mt = blockIdx.x / a.slices / a.ntiles;
+  const int m0 = mt * QO_M, n0 = nt * QO_N, k0 = ks << a.klog, wlog = a.klog - 2, words = 1 << wlog;  // words of four inputs
+  const int nk = min(a.in_size - k0, 1 << a.klog), rows = min(a.B - m0, QO_M);
+  after_previous_kernel();
+  // ---- values and their ranges ----
+  float x[16][4], w[8][4];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {  // word kq of row r
+    if (j * 4 >= words || (warp * 32 + j * QO_THREADS) >> wlog >= rows) break;
+    const int p = tid + j * QO_THREADS, r = p >> wlog, k = (p & (words - 1)) * 4;
+    const float *src = a.in + (size_t)(m0 + r) * a.in_size + k0 + k;
+    const bool live = r < rows;
+    if (a.vec) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (live && k < nk) v = *reinterpret_cast<const float4 *>(src);
+      x[j][0] = v.x, x[j][1] = v.y, x[j][2] = v.z, x[j][3] = v.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[j][e] = live && k + e < nk ? src[e] : 0.f;
+    }
+  }
+  const int n = tid & (QO_N - 1), q0 = tid >> 6;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {  // words q0 + 8 j of output n
+    if (j * 8 >= words) break;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int k = (q0 + 8 * j) * 4 + e;
+      w[j][e] = n0 + n < a.out_size && k < nk ? a.W[(size_t)(k0 + k) * a.out_size + n0 + n] : 0.f;
+    }
+  }
+  if (a.slices > 1)
+    for (size_t i = blockIdx.x * (size_t)QO_THREADS + tid; i < (size_t)a.B * a.out_size; i += (size_t)gridDim.x * QO_THREADS)
+      a.acc[i] = 0;
+  {
+    float mn = a.W[0], mx = mn;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (j * 8 >= words) break;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (n0 + n < a.out_size && (q0 + 8 * j) * 4 + e < nk) mn = fminf(mn, w[j][e]), mx = fmaxf(mx, w[j][e]);
+    }
+    mn = warp_min(mn);
+    mx = warp_max(mx);
+    if (lane == 0) wmn[warp] = mn, wmx[warp] = mx;
+  }
+  // the blocks of a slice's output tiles share its rows
+  const int halves = words > 32 ? 2 : 1, span = min(words, 32);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (j * 4 >= words || (warp * 32 + j * QO_THREADS) >> wlog >= rows) break;
+    if (j % a.ntiles != nt) continue;
+    const int p = tid + j * QO_THREADS, r = p >> wlog, k = (p & (words - 1)) * 4;
+    const bool live = r < rows;
+    float mn = live ? a.in[(size_t)(m0 + r) * a.in_size] : 0.f, mx = mn;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (live && k + e < nk) mn = fminf(mn, x[j][e]), mx = fmaxf(mx, x[j][e]);
+    for (int o = span >> 1; o > 0; o >>= 1) {
+      mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if (live && (lane & (span - 1)) == 0)
+      a.xpart[(size_t)(ks * halves + (halves == 2 ? (p >> 5) & 1 : 0)) * a.B + m0 + r] = make_float2(mn, mx);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    float mn = wmn[0], mx = wmx[0];
+    for (int i = 1; i < QO_WARPS; ++i) mn = fminf(mn, wmn[i]), mx = fmaxf(mx, wmx[i]);
+    a.wpart[blockIdx.x] = make_float2(mn, mx);
+  }
+  q_cluster_sync(2);
+  // ---- scales: a thread a sample, a warp the filter and the biases ----
+  if (tid < QO_M) {
+    if (tid < rows) {
+      float mn = a.in[(size_t)(m0 + tid) * a.in_size], mx = mn;
+#pragma unroll 8
+      for (int i = 0; i < a.slices * halves; ++i) {
+        const float2 v = __ldcg(a.xpart + (size_t)i * a.B + m0 + tid);
+        mn = fminf(mn, v.x);
+        mx = fmaxf(mx, v.y);
+      }
+      xq[tid].set(mn, mx);
+      xoff[tid] = (int)f2q_unclamped<8>(0.0f, mn, mx);
+      if (ks == 0 && nt == 0) a.xrange[m0 + tid] = make_float2(mn, mx);
+    }
+  } else if (warp == QO_M / 32) {
+    float mn = a.W[0], mx = mn, bmn = 0.f, bmx = 0.f;
+    for (int i = lane; i < (int)gridDim.x; i += 32) {
+      const float2 v = __ldcg(a.wpart + i);
+      mn = fminf(mn, v.x);
+      mx = fmaxf(mx, v.y);
+    }
+    for (int i = lane; i < a.nbias; i += 32) {
+      bmn = fminf(bmn, a.bias[i]);
+      bmx = fmaxf(bmx, a.bias[i]);
+    }
+    mn = warp_min(mn), mx = warp_max(mx), bmn = warp_min(bmn), bmx = warp_max(bmx);
+    if (lane == 0) {
+      widen_ranges(a.W[0], a.nbias > 0 ? a.bias[0] : 0.f, a.nbias, &mn, &mx, &bmn, &bmx);
+      qg.min_f = mn, qg.max_f = mx, qg.min_b = bmn, qg.max_b = bmx;
+      off_f = qg.off_f = (int)f2q_unclamped<8>(0.0f, mn, mx);
+      wq.set(mn, mx);
+      bq.set(bmn, bmx);
+    }
+  }
+  __syncthreads();
+  // ---- bytes, the inputs of a row side by side ----
+  uint8_t *xs = qsm, *ws = qsm + QO_M * QO_ROW;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (j * 4 >= words || (warp * 32 + j * QO_THREADS) >> wlog >= rows) break;  // rows behind the last are multiplied and not used
+    const int p = tid + j * QO_THREADS, r = p >> wlog, k = (p & (words - 1)) * 4;
+    unsigned v = 0;
+    if (r < rows)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (k + e < nk) v |= xq[r].of(x[j][e]) << (8 * e);
+    *reinterpret_cast<unsigned *>(xs + r * QO_ROW + k) = v;
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (j * 8 >= words) break;
+    const int k = (q0 + 8 * j) * 4;
+    unsigned v = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (n0 + n < a.out_size && k + e < nk) v |= wq.of(w[j][e]) << (8 * e);
+    *reinterpret_cast<unsigned *>(ws + n * QO_ROW + k) = v;
+  }
+  __syncthreads();
+  if (tid < QO_M + QO_N) {  // byte sums of the rows (the filter's lie behind the samples')
+    unsigned s = 0;
+    for (int i = 0; i < words; i += 4) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(qsm + tid * QO_ROW + i * 4);
+      s = __dp4a(v.x, 0x01010101u, __dp4a(v.y, 0x01010101u, __dp4a(v.z, 0x01010101u, __dp4a(v.w, 0x01010101u, s))));
+    }
+    (tid < QO_M ? xsum[tid] : wsum[tid - QO_M]) = (int)s;
+  }
+  // ---- products: a warp 16 samples x 32 outputs ----
+  const int g = lane >> 2, q = lane & 3, mw = warp & 7, nw = warp >> 3;
+  unsigned c[4][4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[t][k] = 0;
+  if (mw * 16 < rows) {
+    const uint8_t *xa = xs + (mw * 16 + g) * QO_ROW + q * 8, *wb = ws + (nw * 32 + g) * QO_ROW + q * 8;
+    for (int s = 0; s < words / 8; ++s) {
+      const uint2 a0 = *reinterpret_cast<const uint2 *>(xa + s * 32), a1 = *reinterpret_cast<const uint2 *>(xa + 8 * QO_ROW + s * 32);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) mma_u8(c[t], a0, a1, *reinterpret_cast<const uint2 *>(wb + t * 8 * QO_ROW + s * 32));
+    }
+  }
+  __syncthreads();
+  // through shared memory, so that a warp adds to 32 neighbours
+  int *st = reinterpret_cast<int *>(qsm);
+  constexpr int SP = QO_N + 2;
+  static_assert(QO_M * SP * 4 <= QO_SMEM, "the sums take the bytes' place");
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int m = mw * 16 + g + (k >> 1) * 8, o = nw * 32 + t * 8 + q * 2 + (k & 1);
+      if (m < rows)
+        st[m * SP + o] = (int)(c[t][k] - (unsigned)xoff[m] * (unsigned)wsum[o] - (unsigned)off_f * (unsigned)xsum[m] +
+                               (unsigned)nk * (unsigned)off_f * (unsigned)xoff[m]);
+    }
+  __syncthreads();
+  for (int i = tid; i < rows * QO_N; i += QO_THREADS) {
+    const int m = i / QO_N, o = i % QO_N;
+    if (n0 + o >= a.out_size) continue;
+    int *dst = a.acc + (size_t)(m0 + m) * a.out_size + n0 + o;
+    if (a.slices > 1)
+      atomicAdd(dst, st[m * SP + o]);
+    else
+      *dst = st[m * SP + o];
+  }
+  q_cluster_sync(2);
+  // ---- a warp requantizes a sample ----
+  for (int r = blockIdx.x + (int)gridDim.x * warp; r < a.B; r += (int)gridDim.x * QO_WARPS) {
+    QSample s = {};
+    const float2 range = __ldcg(a.xrange + r);
+    s.min_in = range.x;
+    s.max_in = range.y;
+    sample_params(s, qg, 1);
+    const int *acc = a.acc + (size_t)r * a.out_size;
+    auto value = [&](int i) {
+      const int v = __ldcg(acc + i);
+      return a.nbias ? (int)((unsigned)v + bq.of(a.bias[i]) - (unsigned)s.zero_total) : v;
+    };
+    int mn = INT_MAX, mx = INT_MIN;
+    for (int i = lane; i < a.out_size; i += 32) {
+      const int v = value(i);
+      mn = min(mn, v);
+      mx = max(mx, v);
+    }
+    s.acc_min = warp_min_i(mn);
+    s.acc_max = warp_max_i(mx);
+    requant_params(s);
+    for (int i = lane; i < a.out_size; i += 32)
+      a.out[(size_t)r * a.out_size + i] = q2f<8>(requant_one(value(i), s), s.min_new, s.max_new);
+  }
 }
 
 // ---- 7. the forms for chained quantized layers ("eq") -----------------------------------------
@@ -1051,15 +1471,20 @@ int qconv_fwd(b200_ctx *ctx, const b200_conv_desc *d, const float *in, const flo
     const int npix = g.OH * g.OW;
     // blocks of a sample: as many as leave every sample a place; more where the rows of one do not fit
     int nc = 8;
-    while (nc > 1 && (long long)B * nc > ctx->sm_count) nc /= 2;
+    while (nc > 1 && ((long long)B * nc > ctx->sm_count || (nc - 1) * 16 >= npix)) nc /= 2;  // 16 pixels each
     size_t smem = 0;
+    bool regs = false;
     for (; nc <= 8; nc *= 2) {
       a.per = (ceil_div(npix, nc) + 15) / 16 * 16;
       const int rows = (a.per + g.OW - 2) / g.OW * g.SH + g.KH;  // a run of `per` pixels needs at most that many
       a.rows = rows < g.HI ? rows : g.HI;
       smem = (size_t)a.ntiles * 8 * a.pitch + (size_t)a.rows * g.WI * a.Cp +
              4 * ((size_t)a.ksteps * 4 + (size_t)a.rows * g.WI + a.per);
-      const size_t with_acc = smem + 4 * (size_t)g.OC * a.per;
+      const int groups = (a.ntiles + 3) / 4;
+      // a warp's only unit needs no more code than that
+      regs = groups <= QC_WARPS && a.per / 16 <= QC_WARPS / groups * QC_UNITS && a.per / 16 * groups > QC_WARPS;
+      a.copies = smem >= 32 * 256 * sizeof(float) ? 32 : 1;
+      const size_t with_acc = smem + (regs ? 0 : 4 * (size_t)g.OC * a.per);
       a.acc_smem = with_acc + 4096 <= ctx->smem_optin;  // beside the kernel's own shared variables
       if (a.acc_smem) smem = with_acc;
       if (smem + 4096 <= ctx->smem_optin) break;
@@ -1072,9 +1497,9 @@ int qconv_fwd(b200_ctx *ctx, const b200_conv_desc *d, const float *in, const flo
                              (size_t)g.KH * g.KH, g.C, a.Cp, g.OC, g.KH * g.KW, a.pitch, bias, nbias, s.qg, s.Wq, s.bq,
                              wsum));
       a.Wq = s.Wq, a.bq = s.bq, a.wsum = wsum, a.qg = s.qg;
-      B200_CUDA(cudaFuncSetAttribute(q_conv_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      B200_TRY(launch_kernel(ctx, q_conv_fused_kernel, dim3((unsigned)(B * nc)), dim3(QC_THREADS), smem, dim3((unsigned)nc),
-                             a));
+      auto kernel = regs ? q_conv_fused_kernel<true> : q_conv_fused_kernel<false>;
+      B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      B200_TRY(launch_kernel(ctx, kernel, dim3((unsigned)(B * nc)), dim3(QC_THREADS), smem, dim3((unsigned)nc), a));
       return 0;
     }
   }
@@ -1106,19 +1531,39 @@ int qfc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const flo
   if (B == 0) return 0;
   const size_t lenW = (size_t)in_size * out_size;
   const int nbias = bias ? out_size : 0;
+  // one cluster where the slices and tiles of the layer are few enough: the smallest slices for which that is so
+  for (int klog = 5; klog <= 8; ++klog) {
+    const long long slices = ceil_div(in_size, 1 << klog), tiles = (long long)ceil_div(out_size, QO_N) * ceil_div(B, QO_M);
+    if (slices * tiles > QO_BLOCKS) continue;
+    const int blocks = (int)(slices * tiles), parts = (int)slices * (klog > 7 ? 2 : 1);
+    QFcArgs a = {};
+    a.in = in, a.W = W, a.bias = bias, a.out = out;
+    a.B = B, a.in_size = in_size, a.out_size = out_size, a.nbias = nbias;
+    a.klog = klog, a.slices = (int)slices, a.ntiles = ceil_div(out_size, QO_N);
+    a.vec = in_size % 4 == 0 && ((uintptr_t)in & 15) == 0;
+    const size_t o_x = align_up(sizeof(float2) * blocks, 256), o_r = align_up(o_x + sizeof(float2) * parts * B, 256),
+                 o_acc = align_up(o_r + sizeof(float2) * B, 256);
+    void *base = nullptr;
+    B200_TRY(ctx_scratch(ctx, o_acc + sizeof(int) * (size_t)B * out_size, &base));
+    char *p = static_cast<char *>(base);
+    a.wpart = reinterpret_cast<float2 *>(p);
+    a.xpart = reinterpret_cast<float2 *>(p + o_x);
+    a.xrange = reinterpret_cast<float2 *>(p + o_r);
+    a.acc = reinterpret_cast<int *>(p + o_acc);
+    B200_CUDA(cudaFuncSetAttribute(q_fc_whole_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, QO_SMEM));
+    return launch_kernel(ctx, q_fc_whole_kernel, dim3((unsigned)blocks), dim3(QO_THREADS), QO_SMEM, dim3((unsigned)blocks), a);
+  }
   const int pitch = (in_size + 31) / 32 * 32;  // bytes per quantized row, zero padded
   QScratch s;
   B200_TRY(q_carve(ctx, B, pitch, (size_t)pitch * out_size, out_size, (size_t)out_size + ceil_div(out_size, B), &s));
   unsigned *wsum = reinterpret_cast<unsigned *>(s.acc + (size_t)B * out_size);
-  cudaStream_t st = ctx->stream;
   int wblocks = blocks_for(lenW, 4096);
   if (wblocks > Q_PART_BLOCKS) wblocks = Q_PART_BLOCKS;
-  q_fc_range_kernel<<<B + wblocks, 256, 0, st>>>(in, in_size, B, W, lenW, out_size, s.qs, s.part, s.acc, wsum);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, q_fc_range_kernel, dim3(B + wblocks), dim3(256), 0, 1, in, in_size, B, W, lenW, out_size, s.qs,
+                         s.part, s.acc, wsum));
   const int rblocks = ceil_div(pitch, 1024), fblocks = ceil_div(out_size, 32) * ceil_div(pitch, QF_CIN);
-  q_fc_quantize_kernel<<<B * rblocks + fblocks, 256, 0, st>>>(in, in_size, B, pitch, rblocks, W, out_size, bias, nbias, s.part,
-                                                             wblocks, s.qs, s.qg, s.inq, s.Wq, s.bq, wsum);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, q_fc_quantize_kernel, dim3(B * rblocks + fblocks), dim3(256), 0, 1, in, in_size, B, pitch,
+                         rblocks, W, out_size, bias, nbias, s.part, wblocks, s.qs, s.qg, s.inq, s.Wq, s.bq, wsum));
   // the inputs dealt out so that two blocks an SM have work, 128 bytes at least
   const int tiles = ceil_div(out_size, 64) * ceil_div(B, 64);
   int splits = ceil_div(2 * ctx->sm_count, tiles);
@@ -1126,11 +1571,10 @@ int qfc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const flo
   const int per = (ceil_div(pitch, splits) + 31) / 32 * 32;
   constexpr int gemm_smem = 128 * (QF_K + 32);
   B200_CUDA(cudaFuncSetAttribute(q_fc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem));
-  q_fc_gemm_kernel<<<dim3(ceil_div(out_size, 64), ceil_div(B, 64), ceil_div(pitch, per)), 256, gemm_smem, st>>>(
-    B, out_size, pitch, per, s.inq, s.Wq, s.acc);
-  B200_LAUNCHED();
-  q_fc_requant_kernel<<<B, 256, 0, st>>>(in_size, out_size, nbias > 0, s.acc, s.qs, s.qg, wsum, s.bq, out);
-  B200_LAUNCHED();
+  B200_TRY(launch_kernel(ctx, q_fc_gemm_kernel, dim3(ceil_div(out_size, 64), ceil_div(B, 64), ceil_div(pitch, per)),
+                         dim3(256), gemm_smem, 1, B, out_size, pitch, per, s.inq, s.Wq, s.acc));
+  B200_TRY(launch_kernel(ctx, q_fc_requant_kernel, dim3(B), dim3(256), 0, 1, in_size, out_size, nbias > 0, s.acc, s.qs, s.qg,
+                         wsum, s.bq, out));
   return 0;
 }
 
