@@ -7,17 +7,34 @@
 //   db       db[N]     += column sums of dout         (:62-67)
 //
 // Large problems use 64x64 tiles.  Small ones (the CIFAR net's 1024->64 and
-// 64->10 layers give 4..64 such tiles on 148 SMs) use 32x32 tiles and split
+// 64->10 layers give 4..64 such tiles on 148 SMs) use tiles of 1024 results and split
 // the reduction dimension over a cluster of up to eight blocks; each block then
 // adds up its share of the tile over the cluster's shared memory, slice after slice,
 // so the result does not depend on scheduling.  (With the slices in global memory and
 // a second kernel to add them, a 784-500-500-10 step of 77 samples took 13 us more.)
+#include <type_traits>
+
 #include "common.cuh"
 #include "device_utils.cuh"
 
 namespace b200 {
 
 constexpr int GK = 16;  // tile depth
+
+// four neighbouring results, of which `left` exist: (+)= v (+ bias), then an optional activation; in one store where rows allow
+// it (vc).  Four stores of four bytes each took as long as everything else together where the sums are short (4096x4096 from
+// 8 samples, dW: 76 us, now 46).
+__device__ __forceinline__ void store_row(float *c, int left, float *v, const float *bias, int accumulate, int act, int vc) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (j < left) {
+      if (bias) v[j] += bias[j];
+      if (accumulate) v[j] += c[j];
+      v[j] = apply_act(v[j], act);
+      if (!vc) c[j] = v[j];
+    }
+  if (vc && left > 0) *reinterpret_cast<float4 *>(c) = make_float4(v[0], v[1], v[2], v[3]);
+}
 
 // C[m][n] (+)= sum_k A(m,k) * Bm(k,n) (+ bias[n]), then optional activation.
 // A(m,k) = A[m*a_m + k*a_k], Bm(k,n) = Bm[k*b_k + n*b_n], C row-major ldc = N.
@@ -28,9 +45,9 @@ __global__ void __launch_bounds__(256) sgemm_kernel(int M, int N, int K, const f
                                                     const float *__restrict__ Bm, long long b_k,
                                                     long long b_n, float *__restrict__ C,
                                                     const float *__restrict__ bias, int accumulate,
-                                                    int act) {
+                                                    int act, int vc) {
   after_previous_kernel();
-  static_assert(BT / TT == 16, "256 threads as 16 x 16");
+  static_assert(BT / TT == 16 && TT == 4, "256 threads as 16 x 16");
   __shared__ __align__(16) float As[GK][BT + 4];
   __shared__ __align__(16) float Bs[GK][BT + 4];
   const int tid = threadIdx.x;
@@ -81,17 +98,12 @@ __global__ void __launch_bounds__(256) sgemm_kernel(int M, int N, int K, const f
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < TT; ++i)
-#pragma unroll
-    for (int j = 0; j < TT; ++j) {
-      const int m = m0 + tm + i, n = n0 + tn + j;
-      if (m >= M || n >= N) continue;
-      const size_t ci = (size_t)m * N + n;
-      float v = acc[i][j];
-      if (bias) v += bias[n];
-      if (accumulate) v += C[ci];
-      C[ci] = apply_act(v, act);
-    }
+  for (int i = 0; i < TT; ++i) {
+    const int m = m0 + tm + i;
+    if (m >= M) break;
+    const size_t ci = (size_t)m * N + n0 + tn;
+    store_row(C + ci, N - n0 - tn, acc[i], bias ? bias + n0 + tn : nullptr, accumulate, act, vc);
+  }
 }
 
 // The same product for the sizes whose 64x64 tiles do not fill the chip.  What bounds such a product is latency: a
@@ -106,6 +118,7 @@ struct FcTileArgs {
   int M, N, K, k_per;
   const float *A, *Bm;   // rows are contiguous: A [M][K] (A_KFAST) or [K][M], Bm [K][N] (B_NFAST) or [N][K]
   int lda, ldb, va, vb;  // va, vb: 16-byte copies (rows and first value lie on 16-byte boundaries)
+  int vc;                // 16-byte stores, the same of C, C2 and y
   float *C;
   const float *bias;
   int accumulate, act;
@@ -116,45 +129,51 @@ struct FcTileArgs {
   float y_param;
 };
 
-constexpr int FT = 32, FT_K = 64, FT_STAGES = 4, FT_GROUPS = 4;
+constexpr int FT_K = 64, FT_GROUPS = 4;
 constexpr int FT_KP = FT_K + 4;                // pitch of a row of k's: eight rows' 16 bytes on different banks
-constexpr int FT_OP = FT * FT_KP;              // floats of one operand's stage (either layout)
-constexpr int FT_SMEM = FT_STAGES * 2 * FT_OP * 4;
+// Tiles of 1024 results: 32 x 32, and 16 x 64 or 8 x 128 for a mini-batch of at most 16 or 8 samples, which would leave the rest of 32
+// rows empty: the weights then decide, and a block reads four times as many for the same multiplications.
+__host__ __device__ constexpr int ft_cols(int FM) { return 1024 / FM; }
+__host__ __device__ constexpr int ft_stages(int FM) { return FM == 8 ? 3 : 4; }
+__host__ __device__ constexpr int ft_smem(int FM) { return ft_stages(FM) * (FM + ft_cols(FM)) * FT_KP * 4; }
 
-template <bool A_KFAST, bool B_NFAST>
+template <int FM, bool A_KFAST, bool B_NFAST>
 __global__ void __launch_bounds__(256) fc_tile_kernel(const __grid_constant__ FcTileArgs a) {
   after_previous_kernel();
   extern __shared__ __align__(16) float fsm[];
-  __shared__ __align__(16) float psum[(FT + 1) * FT];  // the block's sums, and those of Bm
-  const int tid = threadIdx.x, group = tid >> 6, tm = (tid >> 3) & 7, tn = tid & 7;
-  const int m0 = blockIdx.y * FT, n0 = blockIdx.x * FT;
+  constexpr int FN = ft_cols(FM), XM = FM / 4, XN = FN / 4, ST = ft_stages(FM), OP_A = FM * FT_KP, STAGE = (FM + FN) * FT_KP;
+  __shared__ __align__(16) float psum[(FM + 1) * FN];  // the block's sums, and those of Bm
+  const int tid = threadIdx.x, group = tid >> 6, tm = (tid & 63) / XN, tn = tid % XN;
+  const int m0 = blockIdx.y * FM, n0 = blockIdx.x * FN;
   const int kbeg = blockIdx.z * a.k_per, kend = min(a.K, kbeg + a.k_per);
   const int nst = (kend - kbeg + FT_K - 1) / FT_K;
-  // rows of 64 k's, or k rows of 32 values; outside the matrix and the slice zero
-  auto load = [&](float *dst, const float *src, int ld, bool kfast, int r0, int rows, int k0, int vec) {
+  // T rows of 64 k's, or 64 k rows of T values; outside the matrix and the slice zero
+  auto load = [&](auto tile, float *dst, const float *src, int ld, bool kfast, int r0, int rows, int k0, int vec) {
+    constexpr int T = decltype(tile)::value;
     if (vec) {
 #pragma unroll
-      for (int e = 0; e < FT * FT_K / 4 / 256; ++e) {
-        const int p = tid + e * 256, r = kfast ? p / (FT_K / 4) : p % (FT / 4) * 4, k = kfast ? p % (FT_K / 4) * 4 : p / (FT / 4);
+      for (int e = 0; e < (T * FT_K / 4 + 255) / 256; ++e) {
+        const int p = tid + e * 256, r = kfast ? p / (FT_K / 4) : p % (T / 4) * 4, k = kfast ? p % (FT_K / 4) * 4 : p / (T / 4);
+        if (T * FT_K / 4 < 256 && p >= T * FT_K / 4) break;
         const bool ok = r0 + r < rows && k0 + k < kend;
         const size_t at = kfast ? (size_t)(r0 + r) * ld + k0 + k : (size_t)(k0 + k) * ld + r0 + r;
-        cp_async16(dst + (kfast ? r * FT_KP + k : k * FT + r), src + (ok ? at : 0), ok);
+        cp_async16(dst + (kfast ? r * FT_KP + k : k * T + r), src + (ok ? at : 0), ok);
       }
     } else {
 #pragma unroll 4
-      for (int e = 0; e < FT * FT_K / 256; ++e) {
-        const int p = tid + e * 256, r = kfast ? p / FT_K : p % FT, k = kfast ? p % FT_K : p / FT;
+      for (int e = 0; e < T * FT_K / 256; ++e) {
+        const int p = tid + e * 256, r = kfast ? p / FT_K : p % T, k = kfast ? p % FT_K : p / T;
         const bool ok = r0 + r < rows && k0 + k < kend;
         const size_t at = kfast ? (size_t)(r0 + r) * ld + k0 + k : (size_t)(k0 + k) * ld + r0 + r;
-        cp_async4(dst + (kfast ? r * FT_KP + k : k * FT + r), src + (ok ? at : 0), ok);
+        cp_async4(dst + (kfast ? r * FT_KP + k : k * T + r), src + (ok ? at : 0), ok);
       }
     }
   };
   auto fetch = [&](int i) {
     if (i < nst) {
-      float *d = fsm + (i % FT_STAGES) * 2 * FT_OP;
-      load(d, a.A, a.lda, A_KFAST, m0, a.M, kbeg + i * FT_K, a.va);
-      load(d + FT_OP, a.Bm, a.ldb, !B_NFAST, n0, a.N, kbeg + i * FT_K, a.vb);
+      float *d = fsm + (i % ST) * STAGE;
+      load(std::integral_constant<int, FM>(), d, a.A, a.lda, A_KFAST, m0, a.M, kbeg + i * FT_K, a.va);
+      load(std::integral_constant<int, FN>(), d + OP_A, a.Bm, a.ldb, !B_NFAST, n0, a.N, kbeg + i * FT_K, a.vb);
     }
     cp_async_commit();
   };
@@ -165,21 +184,21 @@ __global__ void __launch_bounds__(256) fc_tile_kernel(const __grid_constant__ Fc
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 #pragma unroll
-  for (int i = 0; i < FT_STAGES - 1; ++i) fetch(i);
+  for (int i = 0; i < ST - 1; ++i) fetch(i);
   for (int st = 0; st < nst; ++st) {
-    fetch(st + FT_STAGES - 1);  // into the stage that was read before the last barrier
-    cp_async_wait<FT_STAGES - 1>();
+    fetch(st + ST - 1);  // into the stage that was read before the last barrier
+    cp_async_wait<ST - 1>();
     __syncthreads();
-    const float *as = fsm + (st % FT_STAGES) * 2 * FT_OP, *bs = as + FT_OP;
-    // rows of k's: a thread has every eighth row, so that a warp's rows are neighbours; k rows: four values side by side
+    const float *as = fsm + (st % ST) * STAGE, *bs = as + OP_A;
+    // rows of k's: a thread's four are XM or XN apart, so that a warp's rows are neighbours; k rows: four values side by side
 #pragma unroll
     for (int kk = 0; kk < FT_K / FT_GROUPS; kk += 4) {
       const int k = group * (FT_K / FT_GROUPS) + kk;
       float av[4][4], bv[4][4];  // [k][row]
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float4 x = *reinterpret_cast<const float4 *>(A_KFAST ? as + (i * 8 + tm) * FT_KP + k : as + (k + i) * FT + tm * 4);
-        const float4 z = *reinterpret_cast<const float4 *>(B_NFAST ? bs + (k + i) * FT + tn * 4 : bs + (i * 8 + tn) * FT_KP + k);
+        const float4 x = *reinterpret_cast<const float4 *>(A_KFAST ? as + (i * XM + tm) * FT_KP + k : as + (k + i) * FM + tm * 4);
+        const float4 z = *reinterpret_cast<const float4 *>(B_NFAST ? bs + (k + i) * FN + tn * 4 : bs + (i * XN + tn) * FT_KP + k);
         const float xv[4] = {x.x, x.y, x.z, x.w}, zv[4] = {z.x, z.y, z.z, z.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -201,26 +220,26 @@ __global__ void __launch_bounds__(256) fc_tile_kernel(const __grid_constant__ Fc
     }
     __syncthreads();
   }
-  // the groups' sums, in the stages' place: [group][row][32], row 32 the sums of Bm
+  // the groups' sums, in the stages' place: [group][row][FN], row FM the sums of Bm
   cp_async_wait<0>();
-  float *part = fsm + group * (FT + 1) * FT;
+  float *part = fsm + group * (FM + 1) * FN;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int m = A_KFAST ? i * 8 + tm : tm * 4 + i;
+    const int m = A_KFAST ? i * XM + tm : tm * 4 + i;
     if (B_NFAST)
-      *reinterpret_cast<float4 *>(part + m * FT + tn * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      *reinterpret_cast<float4 *>(part + m * FN + tn * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
     else
 #pragma unroll
-      for (int j = 0; j < 4; ++j) part[m * FT + j * 8 + tn] = acc[i][j];
+      for (int j = 0; j < 4; ++j) part[m * FN + j * XN + tn] = acc[i][j];
   }
-  if (B_NFAST && sums && tm == 0) *reinterpret_cast<float4 *>(part + FT * FT + tn * 4) = make_float4(cs[0], cs[1], cs[2], cs[3]);
+  if (B_NFAST && sums && tm == 0) *reinterpret_cast<float4 *>(part + FM * FN + tn * 4) = make_float4(cs[0], cs[1], cs[2], cs[3]);
   __syncthreads();
-  const int quads = (FT * FT + (sums ? FT : 0)) / 4;
+  const int quads = (FM * FN + (sums ? FN : 0)) / 4;
   for (int e = tid; e < quads; e += 256) {
     float4 v = reinterpret_cast<const float4 *>(fsm)[e];
 #pragma unroll
     for (int g = 1; g < FT_GROUPS; ++g) {
-      const float4 w = reinterpret_cast<const float4 *>(fsm + g * (FT + 1) * FT)[e];
+      const float4 w = reinterpret_cast<const float4 *>(fsm + g * (FM + 1) * FN)[e];
       v.x += w.x, v.y += w.y, v.z += w.z, v.w += w.w;
     }
     reinterpret_cast<float4 *>(psum)[e] = v;
@@ -249,24 +268,20 @@ __global__ void __launch_bounds__(256) fc_tile_kernel(const __grid_constant__ Fc
       if (z < Z)
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[0][j] += v[z][j];
-    const int m = m0 + e / (FT / 4), n = n0 + e % (FT / 4) * 4;
-    if (e >= FT * FT / 4) {
+    const int m = m0 + e / XN, n = n0 + e % XN * 4;
+    if (e >= FM * FN / 4) {
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         if (n + j < a.N) a.col_sum[n + j] = a.accumulate ? a.col_sum[n + j] + v[0][j] : v[0][j];
       continue;
     }
     if (m >= a.M) continue;
+    const size_t ci = (size_t)m * a.N + n;
+    store_row(a.C + ci, a.N - n, v[0], a.bias ? a.bias + n : nullptr, a.accumulate, a.act, a.vc);
+    if (a.C2) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (n + j >= a.N) break;
-      const size_t ci = (size_t)m * a.N + n + j;
-      float r = v[0][j];
-      if (a.bias) r += a.bias[n + j];
-      if (a.accumulate) r += a.C[ci];
-      r = apply_act(r, a.act);
-      a.C[ci] = r;
-      if (a.C2) a.C2[ci] = act_grad(a.y_act, a.y_param, a.y[ci], r);
+      for (int j = 0; j < 4; ++j) v[0][j] = n + j < a.N ? act_grad(a.y_act, a.y_param, a.y[ci + j], v[0][j]) : 0.f;
+      store_row(a.C2 + ci, a.N - n, v[0], nullptr, 0, B200_ACT_NONE, a.vc);
     }
   }
   if (Z > 1) asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
@@ -293,9 +308,9 @@ __global__ void col_sum_kernel(const float *__restrict__ d, float *__restrict__ 
   }
 }
 
-// Plan of one GEMM: tile size and k slices.
+// Plan of one GEMM: tile and k slices.
 struct GemmPlan {
-  int tile;    // 64 or 32
+  int tile;    // rows of a tile: 64 (of 64 x 64), or 32, 16 or 8 of fc_tile_kernel's
   int slices;  // >= 1
   int k_per;
 };
@@ -303,18 +318,18 @@ struct GemmPlan {
 static GemmPlan plan_gemm(const b200_ctx *ctx, int M, int N, int K) {
   GemmPlan p;
   long long t64 = (long long)ceil_div(M, 64) * ceil_div(N, 64);
-  if (t64 >= ctx->sm_count) {
+  if (t64 >= ctx->sm_count && M > 16) {
     p.tile = 64;
     p.slices = 1;
     p.k_per = K > 0 ? K : 1;
     return p;
   }
-  p.tile = 32;
-  long long t32 = (long long)ceil_div(M, 32) * ceil_div(N, 32);
-  int want = (int)((2LL * ctx->sm_count + t32 - 1) / t32);  // fill the machine twice
-  if (want > 8) want = 8;                                    // what a cluster may have anywhere
+  p.tile = M <= 8 && N >= 128 ? 8 : M <= 16 && N >= 64 ? 16 : 32;
+  const long long tiles = (long long)ceil_div(M, p.tile) * ceil_div(N, ft_cols(p.tile));
+  int want = (int)((2LL * ctx->sm_count + tiles - 1) / tiles);  // fill the machine twice
+  if (want > 8) want = 8;                                       // what a cluster may have anywhere
   // at least 64 of k per slice, 128 where the tiles are one for every SM already (500x500, 77 samples, dW: two slices 9.9 us)
-  int max_by_k = ceil_div(K > 0 ? K : 1, t32 >= ctx->sm_count ? 128 : 64);
+  int max_by_k = ceil_div(K > 0 ? K : 1, tiles >= ctx->sm_count ? 128 : 64);
   int s = want < max_by_k ? want : max_by_k;
   if (s < 1) s = 1;
   int k_per = ceil_div(ceil_div(K > 0 ? K : 1, s), GK) * GK;  // whole 16-byte pieces of a row
@@ -350,23 +365,32 @@ static int run_gemm(b200_ctx *ctx, int M, int N, int K, const float *A, const fl
                     int act, float *col_sum = nullptr, const FcActGrad *ag = nullptr) {
   if (M == 0 || N == 0) return 0;
   const GemmPlan p = plan_gemm(ctx, M, N, K);
-  const dim3 grid(ceil_div(N, p.tile), ceil_div(M, p.tile), p.slices);
   const int lda = A_KFAST ? K : M, ldb = B_NFAST ? N : K;
+  const auto aligned = [](const void *q) { return ((uintptr_t)q & 15) == 0; };
   if (p.tile == 64) {
+    const dim3 grid(ceil_div(N, 64), ceil_div(M, 64));
     return launch_kernel(ctx, sgemm_kernel<64, 4, A_KFAST, B_NFAST>, grid, dim3(256), 0, dim3(1), M, N, K, A, A_KFAST ? lda : 1,
-                         A_KFAST ? 1 : lda, Bm, B_NFAST ? ldb : 1, B_NFAST ? 1 : ldb, C, bias, accumulate, act);
-  } else {
-    FcTileArgs a = {};
-    a.M = M, a.N = N, a.K = K, a.k_per = p.k_per;
-    a.A = A, a.Bm = Bm, a.lda = lda, a.ldb = ldb;
-    a.va = lda % 4 == 0 && ((uintptr_t)A & 15) == 0;
-    a.vb = ldb % 4 == 0 && ((uintptr_t)Bm & 15) == 0;
-    a.C = C, a.bias = bias, a.accumulate = accumulate, a.act = act;
-    a.col_sum = col_sum;
-    if (ag) a.y = ag->y, a.C2 = ag->dst, a.y_act = ag->act, a.y_param = ag->param;
-    B200_CUDA(cudaFuncSetAttribute(fc_tile_kernel<A_KFAST, B_NFAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM));
-    return launch_kernel(ctx, fc_tile_kernel<A_KFAST, B_NFAST>, grid, dim3(256), FT_SMEM, dim3(1, 1, p.slices), a);
+                         A_KFAST ? 1 : lda, Bm, B_NFAST ? ldb : 1, B_NFAST ? 1 : ldb, C, bias, accumulate, act,
+                         N % 4 == 0 && aligned(C));
   }
+  FcTileArgs a = {};
+  a.M = M, a.N = N, a.K = K, a.k_per = p.k_per;
+  a.A = A, a.Bm = Bm, a.lda = lda, a.ldb = ldb;
+  a.va = lda % 4 == 0 && aligned(A);
+  a.vb = ldb % 4 == 0 && aligned(Bm);
+  a.vc = N % 4 == 0 && aligned(C) && (!ag || (aligned(ag->dst) && aligned(ag->y)));
+  a.C = C, a.bias = bias, a.accumulate = accumulate, a.act = act;
+  a.col_sum = col_sum;
+  if (ag) a.y = ag->y, a.C2 = ag->dst, a.y_act = ag->act, a.y_param = ag->param;
+  auto run = [&](auto rows) -> int {
+    constexpr int FM = decltype(rows)::value;
+    B200_CUDA(cudaFuncSetAttribute(fc_tile_kernel<FM, A_KFAST, B_NFAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, ft_smem(FM)));
+    return launch_kernel(ctx, fc_tile_kernel<FM, A_KFAST, B_NFAST>, dim3(ceil_div(N, ft_cols(FM)), ceil_div(M, FM), p.slices),
+                         dim3(256), ft_smem(FM), dim3(1, 1, p.slices), a);
+  };
+  if (p.tile == 8) return run(std::integral_constant<int, 8>());
+  if (p.tile == 16) return run(std::integral_constant<int, 16>());
+  return run(std::integral_constant<int, 32>());
 }
 
 // whether the product of a pass (0 forward, 1 dX, 2 dW) runs on the tensor cores
@@ -414,7 +438,7 @@ int fc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const floa
 
 // whether the dX pass can also form the gradient through an activation in front of the layer
 bool fc_dx_takes_act(const b200_ctx *ctx, int in_size, int out_size, int B, bool scratch) {
-  return !(scratch && use_tc(ctx, B, in_size, out_size)) && plan_gemm(ctx, B, in_size, out_size).tile == FT;
+  return !(scratch && use_tc(ctx, B, in_size, out_size)) && plan_gemm(ctx, B, in_size, out_size).tile != 64;
 }
 
 int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
@@ -441,7 +465,7 @@ int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const floa
                        nullptr, accumulate, 0, scratch));
     else {
       // A(m, k = n) = l[n*M + m] (m fast); the bias gradient is the sum of the right operand over k
-      db_done = db && !w_rows && plan_gemm(ctx, M, N, B).tile == FT;
+      db_done = db && !w_rows && plan_gemm(ctx, M, N, B).tile != 64;
       B200_TRY((run_gemm<false, true>(ctx, M, N, B, l, r, dW, nullptr, accumulate, 0, db_done ? db : nullptr)));
     }
   }

@@ -85,7 +85,10 @@ __global__ void opt_update_kernel(int kind, OptParams h, const float *__restrict
 
 // Whole flat parameter buffer in one launch; the segment an element belongs to
 // selects Adam's (b1_t, b2_t), which differ per tensor because adam::update
-// advances them once per call (optimizer.h:125-126).
+// advances them once per call (optimizer.h:125-126).  V neighbours a thread: four, with 16-byte accesses, where HBM bounds it
+// (20.5 million parameters, momentum: 85.0 us one by one, 63.2 now, 6.5 TB/s); one where a thread has no more than that
+// to do and the chain of load, arithmetic and store is what takes the time (60 thousand: a step 1.4 us slower with four).
+template <int V>
 __global__ void opt_update_segments_kernel(int kind, OptParams h, const float *__restrict__ grads,
                                            float *__restrict__ W, float *__restrict__ s0,
                                            float *__restrict__ s1,
@@ -94,13 +97,31 @@ __global__ void opt_update_segments_kernel(int kind, OptParams h, const float *_
                                            const int *__restrict__ skip_if) {
   after_previous_kernel();
   if (skip_if && *skip_if != 0) return;
-  size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  size_t step = (size_t)gridDim.x * blockDim.x;
-  for (; i < total; i += step) {
+  const bool two = opt_two_states(kind);
+  const size_t step = (size_t)gridDim.x * blockDim.x, groups = (total + V - 1) / V;
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < groups; q += step) {
+    const size_t i = V * q;
+    const int n = total - i < V ? (int)(total - i) : V;
+    float g[V], w[V], a[V], b[V] = {};
+    if (V == 4 && n == 4) {
+      auto load = [&](float *v, const float *from) {
+        const float4 x = reinterpret_cast<const float4 *>(from)[q];
+        v[0] = x.x, v[1 % V] = x.y, v[2 % V] = x.z, v[3 % V] = x.w;
+      };
+      load(g, grads), load(w, W), load(a, s0);
+      if (two) load(b, s1);
+    } else {
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const size_t k = i + (e < n ? e : 0);
+        g[e] = grads[k], w[e] = W[k], a[e] = s0[k], b[e] = two ? s1[k] : 0.f;
+      }
+    }
     OptParams hp = h;
-    if (opt_two_states(kind)) {
-      // binary search of the segment containing i
-      int lo = 0, hi = n_segs - 1;
+    int lo = 0;
+    if (two) {
+      // binary search of the segment containing i; the others lie there or behind it
+      int hi = n_segs - 1;
       while (lo < hi) {
         int mid = (lo + hi + 1) >> 1;
         if (segs[mid].offset <= i)
@@ -108,15 +129,30 @@ __global__ void opt_update_segments_kernel(int kind, OptParams h, const float *_
         else
           hi = mid - 1;
       }
-      hp.b1_t = pow_tab[2 * lo];
-      hp.b2_t = pow_tab[2 * lo + 1];
     }
-    float g = grads[i];
-    float w = W[i], a = s0[i], b = opt_two_states(kind) ? s1[i] : 0.f;
-    opt_apply(kind, hp, g, w, a, b);
-    W[i] = w;
-    s0[i] = a;
-    if (opt_two_states(kind)) s1[i] = b;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      if (two) {
+        if (e > 0)
+          while (lo + 1 < n_segs && segs[lo + 1].offset <= i + e) ++lo;
+        hp.b1_t = pow_tab[2 * lo];
+        hp.b2_t = pow_tab[2 * lo + 1];
+      }
+      opt_apply(kind, hp, g[e], w[e], a[e], b[e]);
+    }
+    if (V == 4 && n == 4) {
+      reinterpret_cast<float4 *>(W)[q] = make_float4(w[0], w[1 % V], w[2 % V], w[3 % V]);
+      reinterpret_cast<float4 *>(s0)[q] = make_float4(a[0], a[1 % V], a[2 % V], a[3 % V]);
+      if (two) reinterpret_cast<float4 *>(s1)[q] = make_float4(b[0], b[1 % V], b[2 % V], b[3 % V]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < V; ++e)
+        if (e < n) {
+          W[i + e] = w[e];
+          s0[i + e] = a[e];
+          if (two) s1[i + e] = b[e];
+        }
+    }
   }
 }
 
@@ -178,8 +214,11 @@ int opt_update_segments(b200_ctx *ctx, int kind, const b200_opt_hyper &h, const 
                         size_t total, float *pow_tab, const int *skip_if) {
   B200_REQUIRE(kind >= B200_OPT_ADAGRAD && kind <= B200_OPT_NESTEROV_MOMENTUM, "unknown optimizer %d", kind);
   if (total == 0) return 0;
-  B200_TRY(launch_kernel(ctx, opt_update_segments_kernel, dim3(grid_for(total, 256, ctx->sm_count)), dim3(256), 0, 1, kind,
-                         to_params(h), grads, W, s0, s1, segs_dev, n_segs, total, pow_tab, skip_if));
+  // four a thread where one by one would not fit the largest grid
+  const bool wide = total > (size_t)ctx->sm_count * 16 * 256;
+  B200_TRY(launch_kernel(ctx, wide ? opt_update_segments_kernel<4> : opt_update_segments_kernel<1>,
+                         dim3(grid_for(wide ? (total + 3) / 4 : total, 256, ctx->sm_count)), dim3(256), 0, 1, kind, to_params(h), grads, W,
+                         s0, s1, segs_dev, n_segs, total, pow_tab, skip_if));
   return 0;
 }
 
