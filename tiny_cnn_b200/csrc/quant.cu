@@ -383,8 +383,9 @@ __global__ void q_requant_dequant_kernel(const int *__restrict__ acc, size_t out
 // takes the products, exchanges the accumulators' extremes and requantizes.  In eight launches each step read and
 // wrote memory (28x28x32 -> 64, 5x5, 128 samples: 247 us, of which the dp4a products 174 us and the requantizing
 // 20 us; in one 66 us with the sums in shared memory, a filter fragment read for every unit, and values quantized in double
-// precision and requantized in 64 bits; this 53 us).  Cycles of a block there: range 8 k, quantizing 15 k, byte sums 5 k, products 24 k (were
-// 40 k; shared-memory reads), extremes 8 k, requantizing 28 k.
+// precision and requantized in 64 bits; this 39 us).  Cycles of a block there: range 7 k (11 k where each warp read planes of its
+// own), quantizing 8 k (15 k from global memory, a branch for every value), window sums 4 k, products 24 k (40 k; shared-memory
+// reads), extremes 9 k, requantizing 15 k (28 k with a branch for every value, the stores four bytes each).
 // A k step is 32 bytes: four groups of 8 channels, wherever in the window they lie (`tab`); channels are
 // padded to 8, the filter's rows to 32 bytes with zeros.
 __device__ __noinline__ unsigned quantize_in_double(float v, double scale, double low) {
@@ -411,14 +412,39 @@ struct QScale {
     quick = fabs(low) < 2097152.0 && scale > 1e-30 && scale < 1e30;
     low32 = quick ? (int)low : 0;
   }
+  // the value by 32 bits alone, and whether they decide it
+  __device__ __forceinline__ unsigned in32(float v, bool &ok) const {
+    const float f = __fmul_rn(v, scale32), t = __fadd_rn(f, 12582912.f);  // 1.5 * 2^23: the whole number is in the last bits
+    ok = fabsf(f) < 2097152.f && fabsf(__fsub_rn(f, __fsub_rn(t, 12582912.f))) < 0.5f - fabsf(f) * 2.4e-7f;
+    return (unsigned)min(255, max(0, __float_as_int(t) - 0x4b400000 - low32));
+  }
   __device__ __forceinline__ unsigned of(float v) const {
     if (flat) return 0u;
-    const float f = __fmul_rn(v, scale32), t = __fadd_rn(f, 12582912.f);  // 1.5 * 2^23: the whole number is in the last bits
-    if (quick && fabsf(f) < 2097152.f && fabsf(__fsub_rn(f, __fsub_rn(t, 12582912.f))) < 0.5f - fabsf(f) * 2.4e-7f)
-      return (unsigned)min(255, max(0, __float_as_int(t) - 0x4b400000 - low32));
-    return quantize_in_double(v, scale, low);
+    bool ok;
+    const unsigned r = in32(v, ok);
+    return quick && ok ? r : quantize_in_double(v, scale, low);
+  }
+  // four values to the bytes of a word: one branch for all, so that their chains overlap
+  __device__ __forceinline__ unsigned of4(const float *v) const {
+    if (flat) return 0u;
+    unsigned w = 0u;
+    bool all = quick;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      bool ok;
+      w |= in32(v[k], ok) << (8 * k);
+      all = all && ok;
+    }
+    if (all) return w;
+    w = 0u;
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) w |= quantize_in_double(k == 0 ? v[0] : k == 1 ? v[1] : k == 2 ? v[2] : v[3], scale, low) << (8 * k);
+    return w;
   }
 };
+
+// a word whose first `left` bytes are set
+__device__ __forceinline__ unsigned first_bytes(int left) { return left >= 4 ? ~0u : left > 0 ? (1u << (8 * left)) - 1u : 0u; }
 
 __device__ __forceinline__ void mma_u8(unsigned *c, const uint2 &a0, const uint2 &a1, const uint2 &b) {
   // lane (g, q) holds bytes 8 q .. 8 q + 7 of rows g and g + 8 and of column g: the order of the k's is free as long
@@ -439,6 +465,7 @@ struct QConvArgs {
   int Cp, ksteps, pitch, ntiles;  // channels padded to 8; k steps; bytes of a filter row; 8-channel tiles of the outputs
   int per, rows;                  // output pixels of a block (a multiple of 16), most input rows it needs
   int copies;                     // of the table of results: 32 or 1
+  int raw;                        // the input rows wait in shared memory for their range
   int acc_smem;                   // the accumulators wait in shared memory, not in the output's place
 };
 
@@ -491,29 +518,28 @@ __device__ __forceinline__ unsigned q_remote(const void *p, int rank) {  // a wo
   return v;
 }
 
-__device__ __noinline__ int requant_in_64_bits(int acc, const QSample &s) { return requant_one(acc, s); }
-
-// requant_one in 32 bits where that decides it.  The quotient before rounding is off by `bound` at most: three roundings of the
-// product and two of the sum, relative to the largest accumulator of the sample, and the 64-bit form's own cut at
-// 2^-16.  Above zero that form rounds to the nearest whole number, below zero to the one under it; a value further than the
-// bound from a half, and from zero, does so for certain.  One in some thousands goes the long way.
+// requant_one in 32 bits.  With scale = hi * 2^32 + lo, lo signed, floor(acc * scale / 2^32) = acc * hi + floor(acc * lo / 2^32), and
+// modulo 2^32 that is enough where the sum fits an int32, which it does for every accumulator if it does for the least and
+// the largest.  Otherwise (`on` not set) in 64 bits.
 struct QQuick {
-  float scale, offset, bound;
-  int out;
+  int hi, lo, offset, out;
   bool on;
   __device__ __forceinline__ void set(const QSample &s) {
-    scale = __fmul_rn(__ll2float_rn(s.range_scale_fp), 3.5527136788005009e-15f);  // 2^-48
-    offset = __fmul_rn(__ll2float_rn(s.input_offset_fp), 1.52587890625e-5f);      // 2^-16
-    const float most = __fadd_rn(__fmul_rn(fmaxf(fabsf((float)s.acc_min), fabsf((float)s.acc_max)), scale), fabsf(offset));
-    bound = __fadd_rn(2e-5f, __fmul_rn(most, 5e-7f));
-    on = s.output_offset_fp > -2097152 && s.output_offset_fp < 2097152 && most < 1048576.f && scale > 1e-30f;
-    out = on ? (int)s.output_offset_fp + 0x4b400000 : 0;
+    lo = (int)(unsigned)s.range_scale_fp;
+    hi = (int)(unsigned)(((unsigned long long)s.range_scale_fp - (unsigned long long)(long long)lo) >> 32);
+    offset = (int)(unsigned)s.input_offset_fp;
+    out = (int)(unsigned)s.output_offset_fp;
+    const double most = fmax(fabs((double)s.acc_min), fabs((double)s.acc_max)) * fabs((double)s.range_scale_fp);
+    on = most < 4e18 && fabs((double)s.input_offset_fp) < 4e18 && fits(s.acc_min, s) && fits(s.acc_max, s) &&
+         s.output_offset_fp > -(1LL << 30) && s.output_offset_fp < (1LL << 30);
   }
-  __device__ __forceinline__ int of(int acc, const QSample &s) const {
-    const float f = __fadd_rn(__fmul_rn((float)acc, scale), offset), t = __fadd_rn(f, 12582912.f);  // 1.5 * 2^23
-    if (on && fabsf(__fsub_rn(f, __fsub_rn(t, 12582912.f))) < 0.5f - bound && fabsf(f) > bound)
-      return min(255, max(0, __float_as_int(t) - out + (__float_as_int(f) >> 31)));
-    return requant_in_64_bits(acc, s);
+  __device__ __forceinline__ static bool fits(int acc, const QSample &s) {
+    const long long v = (((long long)acc * s.range_scale_fp) >> 32) + s.input_offset_fp;
+    return v > -(1LL << 31) + 65536 && v < (1LL << 31) - 65536;
+  }
+  __device__ __forceinline__ int of(int acc) const {
+    const int v = (int)((unsigned)acc * (unsigned)hi + (unsigned)__mulhi(acc, lo) + (unsigned)offset), below = v >> 31;
+    return min(255, max(0, ((v + ((32768 ^ below) - below)) >> 16) - out));
   }
 };
 __device__ __forceinline__ uint2 q_lds8(unsigned at) {
@@ -522,7 +548,8 @@ __device__ __forceinline__ uint2 q_lds8(unsigned at) {
   return v;
 }
 
-constexpr int QC_UNITS = 5;  // units of 16 pixels x 32 outputs whose sums a warp keeps in registers
+constexpr int QC_UNITS = 5;   // units of 16 pixels x 32 outputs whose sums a warp keeps in registers
+constexpr int QC_STAGE = 20;  // words from output to output of a unit in shared memory
 
 // REGS: the sums wait for the sample's extremes in registers, not in shared memory or in the output's place
 template <bool REGS>
@@ -546,6 +573,7 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
   unsigned *xsum = psum + a.rows * a.WI;                                             // [per] over the window
   int *acc = a.acc_smem ? reinterpret_cast<int *>(xsum + a.per) : reinterpret_cast<int *>(a.out) + (size_t)n * a.OC * npix + p0;
   const int acc_step = a.acc_smem ? a.per : npix;                                    // from output channel to output channel
+  float *raw = reinterpret_cast<float *>(((uintptr_t)(xsum + a.per) + 15) & ~(uintptr_t)15);  // [C][places], in the accumulators' place
   wait_for_previous_kernel();
   for (int i = tid; i < a.ntiles * 8 * a.pitch / 16; i += QC_THREADS) cp_async16(ws + 16 * i, a.Wq + 16 * i, true);
   cp_async_commit();
@@ -554,12 +582,62 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
     tab[i] = (tap / a.KW * a.WI + tap % a.KW) * a.Cp + c;
   }
   const float *in = a.in + (size_t)n * a.C * plane;
+  if (a.raw) {
+    const bool vec = ((plane | places | (iy0 * a.WI)) & 3) == 0 && ((uintptr_t)in & 15) == 0;
+    const int unit = vec ? 4 : 1, pu = max(1, places / unit), stepc = QC_THREADS / pu, stepp = QC_THREADS - stepc * pu;
+    int c = places > 0 ? tid / pu : a.C, p = tid % pu;
+    while (c < a.C) {
+      const float *src = in + (size_t)c * plane + iy0 * a.WI + p * unit;
+      if (vec)
+        cp_async16(raw + c * places + p * 4, src, true);
+      else
+        cp_async4(raw + c * places + p, src, true);
+      c += stepc, p += stepp;
+      if (p >= pu) p -= pu, ++c;
+    }
+    cp_async_commit();
+  }
+  for (int i = tid; i < places; i += QC_THREADS) psum[i] = 0u;
   // the range: the reference scans the first HI * HI values of every plane, starting from the first value
   {
     float mn = in[0], mx = in[0];
     const int scan = a.HI * a.HI, parts = max(1, QC_WARPS * nc / a.C), span = (scan + parts - 1) / parts;
     const bool vec = ((plane | scan) & 3) == 0 && parts == 1 && ((uintptr_t)in & 15) == 0;
-    for (int u = rank * QC_WARPS + warp; u < a.C * parts; u += nc * QC_WARPS) {
+    if (a.raw) {
+      // the rows behind the last window, then what the blocks hold: together the whole planes
+      const int end = ((a.OH - 1) * a.SH + a.KH) * a.WI;
+      if (p1 == npix && p1 > p0 && end < scan)
+        for (int c = warp; c < a.C; c += QC_WARPS)
+          for (int e = end + lane; e < scan; e += 32) {
+            const float v = in[(size_t)c * plane + e];
+            mn = fminf(mn, v);
+            mx = fmaxf(mx, v);
+          }
+      cp_async_wait<0>();
+      __syncthreads();
+      const int most = min(places, scan - iy0 * a.WI);  // of a plane's values here
+      if (most == places) {
+        const float4 *r4 = reinterpret_cast<const float4 *>(raw);
+        const int len = a.C * places;
+#pragma unroll 4
+        for (int e = tid; e < len / 4; e += QC_THREADS) {
+          const float4 v = r4[e];
+          mn = fminf(mn, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
+          mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+        }
+        if (tid < (len & 3)) {
+          mn = fminf(mn, raw[(len & ~3) + tid]);
+          mx = fmaxf(mx, raw[(len & ~3) + tid]);
+        }
+      } else {
+        for (int c = warp; c < a.C; c += QC_WARPS)
+          for (int e = lane; e < most; e += 32) {
+            mn = fminf(mn, raw[c * places + e]);
+            mx = fmaxf(mx, raw[c * places + e]);
+          }
+      }
+    }
+    for (int u = rank * QC_WARPS + warp; !a.raw && u < a.C * parts; u += nc * QC_WARPS) {
       const int c = u / parts, b = (u - c * parts) * span;
       if (vec) {  // a plane's loads asked for at once
         const float4 *p = reinterpret_cast<const float4 *>(in + (size_t)c * plane);
@@ -611,39 +689,44 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
     const int groups = a.Cp / 8;
     int cg = tid / places, p = tid - cg * places;  // eight channels of a place
     const int stepg = QC_THREADS / places, stepp = QC_THREADS - stepg * places;
-    float next[8];
-    auto fetch = [&]() {
-      const float *src = in + (size_t)cg * 8 * plane + iy0 * a.WI + p;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) next[k] = cg < groups && cg * 8 + k < a.C ? src[(size_t)k * plane] : 0.f;
+    // with the sums of a place's bytes
+    auto write = [&](int c0, int p, const float(&v)[8]) {
+      const int left = a.C - c0;  // channels behind the last are zero bytes
+      const unsigned w0 = q.of4(v) & first_bytes(left), w1 = q.of4(v + 4) & first_bytes(left - 4);
+      *reinterpret_cast<uint2 *>(xs + (size_t)p * a.Cp + c0) = make_uint2(w0, w1);
+      atomicAdd(psum + p, __dp4a(w1, 0x01010101u, __dp4a(w0, 0x01010101u, 0u)));
     };
-    if (places > 0) fetch();
-    while (places > 0 && cg < groups) {
-      float v[8];
+    if (a.raw) {
+      while (places > 0 && cg < groups) {
+        const float *src = raw + cg * 8 * places + p;
+        float v[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = next[k];
-      const int c0 = cg * 8;
-      uint8_t *dst = xs + (size_t)p * a.Cp + c0;
-      cg += stepg, p += stepp;
-      if (p >= places) p -= places, ++cg;
-      fetch();  // the next place's values are on their way meanwhile
-      unsigned w[2] = {0u, 0u};
+        for (int k = 0; k < 8; ++k) v[k] = cg * 8 + k < a.C ? src[k * places] : 0.f;
+        write(cg * 8, p, v);
+        cg += stepg, p += stepp;
+        if (p >= places) p -= places, ++cg;
+      }
+    } else {
+      float next[8];
+      auto fetch = [&]() {
+        const float *src = in + (size_t)cg * 8 * plane + iy0 * a.WI + p;
 #pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (c0 + k < a.C) w[k >> 2] |= q.of(v[k]) << (8 * (k & 3));
-      *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
+        for (int k = 0; k < 8; ++k) next[k] = cg < groups && cg * 8 + k < a.C ? src[(size_t)k * plane] : 0.f;
+      };
+      if (places > 0) fetch();
+      while (places > 0 && cg < groups) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = next[k];
+        const int c0 = cg * 8, at = p;
+        cg += stepg, p += stepp;
+        if (p >= places) p -= places, ++cg;
+        fetch();  // the next place's values are on their way meanwhile
+        write(c0, at, v);
+      }
     }
   }
   cp_async_wait<0>();
-  __syncthreads();
-  for (int p = tid; p < places; p += QC_THREADS) {
-    unsigned s = 0;
-    for (int k = 0; k < a.Cp; k += 8) {
-      const uint2 x = *reinterpret_cast<const uint2 *>(xs + (size_t)p * a.Cp + k);
-      s = __dp4a(x.y, 0x01010101u, __dp4a(x.x, 0x01010101u, s));
-    }
-    psum[p] = s;
-  }
   __syncthreads();
   for (int p = tid; p < p1 - p0; p += QC_THREADS) {
     const int y = (p0 + p) / a.OW, x = p0 + p - y * a.OW;
@@ -801,28 +884,60 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
   q_cluster_sync(nc);  // nobody leaves while others may read its extremes
   const QSample s = smp;
   // the 256 results: a copy for every lane where filter and input were, so that no two lanes want the same bank
-  float *table = a.copies > 1 ? reinterpret_cast<float *>(qsm) : lut;
-  if (a.copies > 1) {
-    for (int i = warp; i < 256; i += QC_WARPS) table[i * 32 + lane] = q2f<8>(i, s.min_new, s.max_new);
-  } else if (tid < 256) {
-    lut[tid] = q2f<8>(tid, s.min_new, s.max_new);
-  }
+  if (tid < 256) lut[tid] = q2f<8>(tid, s.min_new, s.max_new);
   __syncthreads();
+  const float *table = lut;
+  if (a.copies > 1) {
+    float *t = reinterpret_cast<float *>(qsm);
+    for (int i = warp; i < 256; i += QC_WARPS) t[i * 32 + lane] = lut[i];
+    __syncthreads();
+    table = t;
+  }
   const int tstep = a.copies, tlane = lane & (a.copies - 1);
   float *out = a.out + (size_t)n * a.OC * npix + p0;
   const QQuick qk = quick;
+  auto requant = [&](int v) { return qk.on ? qk.of(v) : requant_one(v, s); };
   if (REGS) {
-#pragma unroll
+    // A unit at a time through the warp's own shared memory, four neighbouring pixels a lane: only the way there is written out
+    // for each of the 80 registers, and rows of 64 bytes are stored.
+    int *mine = reinterpret_cast<int *>(qsm + 32 * 256 * sizeof(float)) + warp * (32 * QC_STAGE);
+    const bool vec = (npix & 3) == 0 && ((uintptr_t)a.out & 15) == 0;  // p0 is a multiple of 16
+#pragma unroll 1
     for (int i = 0; i < QC_UNITS; ++i) {
       if (!has(i)) break;
-      each(unit_of(i), c[i], [&](int o, int p, unsigned v) { out[(size_t)o * npix + p] = table[qk.of((int)v, smp) * tstep + tlane]; });
+#pragma unroll
+      for (int u = 0; u < QC_UNITS; ++u) {
+        if (u != i) continue;
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mine[(t * 8 + q * 2 + (k & 1)) * QC_STAGE + g + 8 * (k >> 1)] = (int)c[u][t][k];
+      }
+      __syncwarp();
+      const int p = (wfirst + i * wper) * 16 + (lane & 3) * 4, left = p1 - p0 - p;
+#pragma unroll 1
+      for (int t = 0; t < 4; ++t) {
+        const int o = (wgroup * 4 + t) * 8 + g;
+        if (o >= a.OC || left <= 0) continue;
+        const int4 v = *reinterpret_cast<const int4 *>(mine + (t * 8 + g) * QC_STAGE + (lane & 3) * 4);
+        const int r4[4] = {v.x, v.y, v.z, v.w};
+        float r[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[e] = table[requant(r4[e]) * tstep + tlane];
+        float *dst = out + (size_t)o * npix + p;
+        if (vec && left >= 4)
+          *reinterpret_cast<float4 *>(dst) = make_float4(r[0], r[1], r[2], r[3]);
+        else
+          for (int e = 0; e < 4 && e < left; ++e) dst[e] = e == 0 ? r[0] : e == 1 ? r[1] : e == 2 ? r[2] : r[3];
+      }
+      __syncwarp();
     }
     return;
   }
   const int count = p1 - p0;
   for (int i = tid; i < a.OC * count; i += QC_THREADS) {
     const int o = i / count, p = i - o * count;
-    out[(size_t)o * npix + p] = table[qk.of(acc[(size_t)o * acc_step + p], smp) * tstep + tlane];
+    out[(size_t)o * npix + p] = table[requant(acc[(size_t)o * acc_step + p]) * tstep + tlane];
   }
 }
 
@@ -913,7 +1028,6 @@ __global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restr
     q.set(qs[n].min_in, qs[n].max_in);
     int sum = 0;
     if (j0 < pitch) {  // pitch is a multiple of 4
-      unsigned w = 0;
       float x[4];
       if (j0 + 4 <= in_size && ((uintptr_t)(r + j0) & 15) == 0) {
         const float4 y = *reinterpret_cast<const float4 *>(r + j0);
@@ -922,12 +1036,8 @@ __global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restr
 #pragma unroll
         for (int k = 0; k < 4; ++k) x[k] = j0 + k < in_size ? r[j0 + k] : 0.f;
       }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const unsigned v = j0 + k < in_size ? q.of(x[k]) : 0u;
-        w |= v << (8 * k);
-        sum += (int)v;
-      }
+      const unsigned w = q.of4(x) & first_bytes(in_size - j0);
+      sum = (int)__dp4a(w, 0x01010101u, 0u);
       *reinterpret_cast<unsigned *>(inq + (size_t)n * pitch + j0) = w;
     }
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -955,11 +1065,11 @@ __global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restr
   q.set(qg.min_f, qg.max_f);
   unsigned sum = 0;
 #pragma unroll
-  for (int k = 0; k < QF_CIN / 8; ++k) {
-    const int j = warp + 8 * k;
-    const unsigned v = c0 + j < in_size && i0 + lane < out_size ? q.of(x[k]) : 0u;
-    tile[j][lane] = (uint8_t)v;
-    sum += v;
+  for (int k = 0; k < QF_CIN / 8; k += 4) {
+    const unsigned v = q.of4(x + k) & first_bytes(i0 + lane < out_size ? (in_size - c0 - warp + 7) / 8 - k : 0);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) tile[warp + 8 * (k + e)][lane] = (uint8_t)(v >> (8 * e));
+    sum = __dp4a(v, 0x01010101u, sum);
   }
   if (i0 + lane < out_size && sum) atomicAdd(&wsum[i0 + lane], sum);
   __syncthreads();
@@ -1209,22 +1319,13 @@ __global__ void __launch_bounds__(QO_THREADS, 1) q_fc_whole_kernel(const __grid_
   for (int j = 0; j < 16; ++j) {
     if (j * 4 >= words || (warp * 32 + j * QO_THREADS) >> wlog >= rows) break;  // rows behind the last are multiplied and not used
     const int p = tid + j * QO_THREADS, r = p >> wlog, k = (p & (words - 1)) * 4;
-    unsigned v = 0;
-    if (r < rows)
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (k + e < nk) v |= xq[r].of(x[j][e]) << (8 * e);
-    *reinterpret_cast<unsigned *>(xs + r * QO_ROW + k) = v;
+    *reinterpret_cast<unsigned *>(xs + r * QO_ROW + k) = r < rows ? xq[r].of4(x[j]) & first_bytes(nk - k) : 0u;
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     if (j * 8 >= words) break;
     const int k = (q0 + 8 * j) * 4;
-    unsigned v = 0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (n0 + n < a.out_size && k + e < nk) v |= wq.of(w[j][e]) << (8 * e);
-    *reinterpret_cast<unsigned *>(ws + n * QO_ROW + k) = v;
+    *reinterpret_cast<unsigned *>(ws + n * QO_ROW + k) = n0 + n < a.out_size ? wq.of4(w[j]) & first_bytes(nk - k) : 0u;
   }
   __syncthreads();
   if (tid < QO_M + QO_N) {  // byte sums of the rows (the filter's lie behind the samples')
@@ -1483,10 +1584,16 @@ int qconv_fwd(b200_ctx *ctx, const b200_conv_desc *d, const float *in, const flo
       const int groups = (a.ntiles + 3) / 4;
       // a warp's only unit needs no more code than that
       regs = groups <= QC_WARPS && a.per / 16 <= QC_WARPS / groups * QC_UNITS && a.per / 16 * groups > QC_WARPS;
-      a.copies = smem >= 32 * 256 * sizeof(float) ? 32 : 1;
-      const size_t with_acc = smem + (regs ? 0 : 4 * (size_t)g.OC * a.per);
+      // once the products are done the results' table and the units on their way out take the place of everything else
+      const size_t behind = 32 * 256 * sizeof(float) + (size_t)QC_WARPS * 32 * QC_STAGE * sizeof(int);
+      a.copies = regs || smem >= 32 * 256 * sizeof(float) ? 32 : 1;
+      const size_t with_acc = smem + (regs ? 0 : 4 * (size_t)g.OC * a.per), with_raw = smem + 16 + 4 * (size_t)g.C * a.rows * g.WI;
       a.acc_smem = with_acc + 4096 <= ctx->smem_optin;  // beside the kernel's own shared variables
       if (a.acc_smem) smem = with_acc;
+      // read once where the rows of all blocks make up the planes and the range lies inside a plane
+      a.raw = with_raw + 4096 <= ctx->smem_optin && g.SH <= g.KH && g.HI <= g.WI;
+      if (a.raw && with_raw > smem) smem = with_raw;
+      if (regs && behind > smem) smem = behind;
       if (smem + 4096 <= ctx->smem_optin) break;
     }
     if (nc <= 8) {
