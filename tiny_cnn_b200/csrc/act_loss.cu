@@ -2,6 +2,8 @@
 // that sit between the contraction kernels on the training step.
 #include <float.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "device_utils.cuh"
 
@@ -301,7 +303,12 @@ int softmax_loss_bwd(b200_ctx *ctx, int loss_kind, const float *y, const float *
 // now 3.3 and 3.2 us with the wide form below).
 constexpr int FCS_N = 16, FCS_THREADS = 256;
 constexpr int FCS_NARROW = 256;               // inputs up to which a sample is a warp's work
+constexpr int FCS_WIDE = 1024;                // inputs up to which four samples are a block's work (forward)
 constexpr int FCW_THREADS = 512, FCW_WARPS = FCW_THREADS / 32, FCW_SAMPLES = 4;
+constexpr int FCL_THREADS = 256, FCL_WARPS = FCL_THREADS / 32;
+constexpr int FCL_GROUP = 4, FCL_SAMPLES = FCL_WARPS * FCL_GROUP;  // forward: samples of a warp, of a block
+constexpr int FCL_CHUNK = 128;                                     // forward: rows of weights in shared memory, twice
+constexpr int FCL_BWD = 16;                                        // backward: most samples of a block
 
 // the sum of acc[j] over the lanes, in lane j of each half-warp: sums of halves, which leave half the values a step
 __device__ __forceinline__ float lanes_sum16(float *acc) {
@@ -338,7 +345,7 @@ __device__ __forceinline__ float head_grad(const float *y, const float *t, int l
   if (j < N) {
     yj = y[(size_t)n * N + j];
     gj = loss_grad_one(loss_kind, yj, t[(size_t)n * N + j], factor);
-    if (lane < N) dy[(size_t)n * N + j] = gj;
+    if (dy != nullptr && lane < N) dy[(size_t)n * N + j] = gj;
   }
   float s = 0.f;
   for (int k = 0; k < N; ++k) {
@@ -347,7 +354,7 @@ __device__ __forceinline__ float head_grad(const float *y, const float *t, int l
     const float df = (k == j) ? __fmul_rn(yj, __fsub_rn(1.f, yj)) : __fmul_rn(-yk, yj);
     s = __fadd_rn(s, __fmul_rn(gk, df));
   }
-  if (lane < N) dz[(size_t)n * N + j] = s;
+  if (dz != nullptr && lane < N) dz[(size_t)n * N + j] = s;
   return s;
 }
 
@@ -415,8 +422,7 @@ __global__ void __launch_bounds__(FCS_THREADS) fc_softmax_bwd16_kernel(const flo
 }
 
 // The same for longer inputs: a block takes four samples, its threads deal the inputs out, and a row of weights is read
-// once for the four of them.  (4096 -> 10, 1024 samples, a warp a sample: 37 us each way, bound by the shared-memory
-// reads of the weights; now 21 and 20 us.)
+// once for the four of them.
 __global__ void __launch_bounds__(FCW_THREADS) fc_softmax_fwd_wide_kernel(const float *__restrict__ x,
                                                                           const float *__restrict__ W,
                                                                           const float *__restrict__ bias, float *__restrict__ z,
@@ -455,40 +461,139 @@ __global__ void __launch_bounds__(FCW_THREADS) fc_softmax_fwd_wide_kernel(const 
   head_out(sum, bias, z, y, n, N);
 }
 
-__global__ void __launch_bounds__(FCW_THREADS) fc_softmax_bwd_wide_kernel(const float *__restrict__ y,
+// The longest inputs: the blocks of a cluster share the inputs of 32 samples out and add their sums over distributed shared memory.
+// A block's rows of weights lie in shared memory, at an odd pitch, for all its samples, and a value read from there serves four
+// of them.  NP is N rounded up to a multiple of four: a test of every output would put each product behind the one before.
+// (4096 -> 10: with 1024 samples 21.5 us with the kernel above, which the strided reads of the weights hold up, ten lines of the L1
+// cache a load, 9.9 with this one; with 8 samples 12.5 and 7.2.  500 -> 10, 77 samples: 3.4 and 4.5, the cluster's barriers.)
+template <int NP>
+__global__ void __launch_bounds__(FCL_THREADS) fc_softmax_fwd_cluster_kernel(const float *__restrict__ x,
+                                                                          const float *__restrict__ W,
+                                                                          const float *__restrict__ bias, float *__restrict__ z,
+                                                                          float *__restrict__ y, int K, int per, int N, int B) {
+  after_previous_kernel();
+  __shared__ float rows[2][FCL_CHUNK * (NP + 1)];
+  __shared__ float sums[FCL_SAMPLES][FCS_N];
+  const int blocks = gridDim.y, rank = blockIdx.y, n0 = blockIdx.x * FCL_SAMPLES, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int pitch = NP + 1;
+  const int first = n0 + warp * FCL_GROUP, end = min(K, (rank + 1) * per);
+  float acc[FCL_GROUP][FCS_N];
+#pragma unroll
+  for (int s = 0; s < FCL_GROUP; ++s)
+#pragma unroll
+    for (int i = 0; i < FCS_N; ++i) acc[s][i] = 0.f;
+  constexpr int XK = FCL_CHUNK / 32;
+  float next[FCL_GROUP][XK];  // a chunk's values and rows are on their way while the one before is multiplied
+  auto fetch = [&](int k0, float *to) {
+#pragma unroll
+    for (int i = threadIdx.x; i < FCL_CHUNK * NP; i += FCL_THREADS) {
+      const int r = i / NP, o = i - r * NP;
+      const bool ok = k0 + r < end && o < N;
+      cp_async4(to + r * pitch + o, W + (ok ? (size_t)(k0 + r) * N + o : 0), ok);
+    }
+    cp_async_commit();
+#pragma unroll
+    for (int s = 0; s < FCL_GROUP; ++s)
+#pragma unroll
+      for (int j = 0; j < XK; ++j) {
+        const int k = k0 + lane + 32 * j;
+        next[s][j] = first + s < B && k < end ? x[(size_t)(first + s) * K + k] : 0.f;
+      }
+  };
+  int buf = 0;
+  fetch(rank * per, rows[0]);
+  for (int k0 = rank * per; k0 < end; k0 += FCL_CHUNK, buf ^= 1) {
+    float xk[FCL_GROUP][XK];
+#pragma unroll
+    for (int s = 0; s < FCL_GROUP; ++s)
+#pragma unroll
+      for (int j = 0; j < XK; ++j) xk[s][j] = next[s][j];
+    cp_async_wait<0>();
+    __syncthreads();
+    if (k0 + FCL_CHUNK < end) fetch(k0 + FCL_CHUNK, rows[buf ^ 1]);
+    if (first < B) {
+#pragma unroll
+      for (int j = 0; j < XK; ++j)
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          const float w = rows[buf][(lane + 32 * j) * pitch + i];
+#pragma unroll
+          for (int s = 0; s < FCL_GROUP; ++s) acc[s][i] = fmaf(xk[s][j], w, acc[s][i]);
+        }
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < FCL_GROUP; ++s) {
+    const float v = lanes_sum16(acc[s]);
+    if (lane < FCS_N) sums[warp * FCL_GROUP + s][lane] = v;
+  }
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+  for (int s = rank + blocks * warp; s < FCL_SAMPLES && n0 + s < B; s += blocks * FCL_WARPS) {  // a warp a sample
+    float sum = 0.f;
+    const unsigned at = smem_u32(&sums[s][lane & 15]);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      if (b == blocks) break;
+      float v;
+      unsigned remote;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(at), "r"(b));
+      asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(remote) : "memory");
+      sum += v;
+    }
+    head_out(sum, bias, z, y, n0 + s, N);
+  }
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+
+// Backward a thread keeps the weights of one input in registers for up to 16 samples.  (4096 -> 10, 1024 samples: 19.5 us with a row of
+// weights read again for every four, from the L1 cache as above, now 12.5, of which writing dX and reading what the relu gave
+// take 5; 8 samples: 9.7 us with all inputs in one block, now 2.9.)
+template <int NP>
+__global__ void __launch_bounds__(FCL_THREADS) fc_softmax_bwd_wide_kernel(const float *__restrict__ y,
                                                                           const float *__restrict__ t, int loss_kind,
                                                                           const float *__restrict__ W,
                                                                           const float *__restrict__ relu_x,
                                                                           float *__restrict__ dy, float *__restrict__ dz,
-                                                                          float *__restrict__ dx, int K, int N, int B) {
+                                                                          float *__restrict__ dx, int K, int N, int B, int per) {
   after_previous_kernel();
-  __shared__ float ds[FCW_SAMPLES][FCS_N];
-  const int n0 = blockIdx.x * FCW_SAMPLES, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < FCW_SAMPLES && n0 + warp < B) {
-    const float s = head_grad(y, t, loss_kind, dy, dz, n0 + warp, N);
-    if (lane < FCS_N) ds[warp][lane] = s;
+  __shared__ __align__(16) float ds[FCL_BWD][FCS_N];
+  const int n0 = blockIdx.x * per, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, samples = min(per, B - n0);
+  int c = blockIdx.y * FCL_THREADS + threadIdx.x;
+  const bool writes = blockIdx.y == 0, gated = relu_x != nullptr && dx != nullptr;
+  float w[NP], gate[4];
+  auto weights = [&]() {
+#pragma unroll
+    for (int i = 0; i < NP; ++i) w[i] = c < K && i < N ? W[(size_t)c * N + i] : 0.f;
+  };
+  auto gates = [&](int s0) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) gate[e] = !gated ? 1.f : c < K && s0 + e < samples ? relu_x[(size_t)(n0 + s0 + e) * K + c] : 0.f;
+  };
+  if (dx != nullptr) weights();
+  gates(0);
+  for (int s = warp; s < samples; s += FCL_WARPS) {
+    const float g = head_grad(y, t, loss_kind, writes ? dy : nullptr, writes ? dz : nullptr, n0 + s, N);
+    if (lane < FCS_N) ds[s][lane] = g;
   }
   __syncthreads();
   if (dx == nullptr) return;
-  const int samples = min(FCW_SAMPLES, B - n0);
-#pragma unroll 2
-  for (int c = threadIdx.x; c < K; c += FCW_THREADS) {  // dx_c = sum_i dz_i W[c][i]
-    float a[FCW_SAMPLES], gate[FCW_SAMPLES];
+  while (c < K) {
+    for (int s0 = 0; s0 < samples; s0 += 4) {  // dx_c = sum_i dz_i W[c][i]
+      float a[4], now[4];
 #pragma unroll
-    for (int s = 0; s < FCW_SAMPLES; ++s) {
-      a[s] = 0.f;
-      gate[s] = relu_x != nullptr ? relu_x[(size_t)min(n0 + s, B - 1) * K + c] : 1.f;
+      for (int e = 0; e < 4; ++e) a[e] = 0.f, now[e] = gate[e];
+      if (s0 + 4 < samples) gates(s0 + 4);
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int i = 0; i < NP; ++i) a[e] = fmaf(ds[s0 + e][i], w[i], a[e]);  // behind N both are zero
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (s0 + e < samples) dx[(size_t)(n0 + s0 + e) * K + c] = now[e] > 0.f ? a[e] : 0.f;
     }
-#pragma unroll
-    for (int i = 0; i < FCS_N; ++i)
-      if (i < N) {
-        const float w = W[(size_t)c * N + i];
-#pragma unroll
-        for (int s = 0; s < FCW_SAMPLES; ++s) a[s] = fmaf(ds[s][i], w, a[s]);
-      }
-#pragma unroll
-    for (int s = 0; s < FCW_SAMPLES; ++s)
-      if (s < samples) dx[(size_t)(n0 + s) * K + c] = gate[s] > 0.f ? a[s] : 0.f;
+    c += gridDim.y * FCL_THREADS;
+    weights();
+    gates(0);
   }
 }
 
@@ -501,9 +606,17 @@ int fc_softmax_fwd(b200_ctx *ctx, int K, int N, const float *x, const float *W, 
   if (K <= FCS_NARROW)
     B200_TRY(launch_kernel(ctx, fc_softmax_fwd16_kernel, dim3(ceil_div(B, FCS_THREADS / 32)), dim3(FCS_THREADS),
                            (size_t)K * N * sizeof(float), 1, x, W, bias, z, y, K, N, B));
-  else
+  else if (K <= FCS_WIDE)
     B200_TRY(launch_kernel(ctx, fc_softmax_fwd_wide_kernel, dim3(ceil_div(B, FCW_SAMPLES)), dim3(FCW_THREADS), 0, 1, x, W,
                            bias, z, y, K, N, B));
+  else {
+    const int blocks = 8, per = ceil_div(ceil_div(K, blocks), 32) * 32;
+    auto kernel = N <= 4   ? fc_softmax_fwd_cluster_kernel<4>
+                  : N <= 8 ? fc_softmax_fwd_cluster_kernel<8>
+                  : N <= 12 ? fc_softmax_fwd_cluster_kernel<12> : fc_softmax_fwd_cluster_kernel<16>;
+    B200_TRY(launch_kernel(ctx, kernel, dim3(ceil_div(B, FCL_SAMPLES), blocks), dim3(FCL_THREADS), 0, dim3(1, blocks), x, W, bias, z, y,
+                           K, per, N, B));
+  }
   return 0;
 }
 
@@ -516,9 +629,16 @@ int fc_softmax_loss_bwd(b200_ctx *ctx, int loss_kind, int K, int N, const float 
   if (K <= FCS_NARROW)
     B200_TRY(launch_kernel(ctx, fc_softmax_bwd16_kernel, dim3(ceil_div(B, FCS_THREADS / 32)), dim3(FCS_THREADS),
                            (size_t)K * N * sizeof(float), 1, y, t, loss_kind, W, relu_x, dy, dz, dx, K, N, B));
-  else
-    B200_TRY(launch_kernel(ctx, fc_softmax_bwd_wide_kernel, dim3(ceil_div(B, FCW_SAMPLES)), dim3(FCW_THREADS), 0, 1, y, t,
-                           loss_kind, W, relu_x, dy, dz, dx, K, N, B));
+  else {
+    auto kernel = N <= 4   ? fc_softmax_bwd_wide_kernel<4>
+                  : N <= 8 ? fc_softmax_bwd_wide_kernel<8>
+                  : N <= 12 ? fc_softmax_bwd_wide_kernel<12> : fc_softmax_bwd_wide_kernel<16>;
+    const int across = dx ? std::min(ceil_div(K, FCL_THREADS), 65535) : 1;
+    // four samples a block, whose loads then are all on their way at once, until they fill the chip
+    const int per = (long long)ceil_div(B, 4) * across <= 4LL * ctx->sm_count ? 4 : FCL_BWD;
+    B200_TRY(launch_kernel(ctx, kernel, dim3(ceil_div(B, per), across), dim3(FCL_THREADS), 0, 1, y, t, loss_kind, W, relu_x, dy, dz,
+                           dx, K, N, B, per));
+  }
   return 0;
 }
 

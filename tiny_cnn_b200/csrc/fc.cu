@@ -287,25 +287,49 @@ __global__ void __launch_bounds__(256) fc_tile_kernel(const __grid_constant__ Fc
   if (Z > 1) asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
 }
 
-// db[i] (+)= sum_n dout[n*N + i]: 32 columns x 8 row-lanes per block, lanes
-// combined in a fixed order through shared memory
-__global__ void col_sum_kernel(const float *__restrict__ d, float *__restrict__ db, int rows, int N,
-                               int accumulate) {
+// db[i] (+)= sum_n dout[n*N + i].  A block sums 128 columns, a warp of it every eighth row, four values of a row a lane; from 128
+// rows on the blocks of a cluster share the rows out.  All sums are added in a fixed order.  (4096 columns of 1024 rows: 13.5 us
+// with 32 columns a block, whose pieces of 128 bytes and chains of 128 rows held it up, 8.4 now.)
+constexpr int CS_COLS = 128;
+__global__ void __launch_bounds__(256) col_sum_kernel(const float *__restrict__ d, float *__restrict__ db, int rows, int N,
+                                                      int accumulate) {
   after_previous_kernel();
-  __shared__ float part[8][33];
-  int col = blockIdx.x * 32 + threadIdx.x;
-  float s = 0.f;
-  if (col < N)
-#pragma unroll 8
-    for (int r = threadIdx.y; r < rows; r += 8) s += d[(size_t)r * N + col];
-  part[threadIdx.y][threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.y == 0 && col < N) {
-    float t = part[0][threadIdx.x];
+  __shared__ float part[8][CS_COLS];
+  const int Z = gridDim.y, rank = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = blockIdx.x * CS_COLS;
+  float s[4] = {};
+  const float *from[4];
 #pragma unroll
-    for (int l = 1; l < 8; ++l) t += part[l][threadIdx.x];
-    db[col] = accumulate ? db[col] + t : t;
+  for (int j = 0; j < 4; ++j) from[j] = d + min(c0 + lane + 32 * j, N - 1);
+#pragma unroll 8
+  for (int r = rank * 8 + warp; r < rows; r += 8 * Z)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s[j] += from[j][(size_t)r * N];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) part[warp][lane + 32 * j] = s[j];
+  __syncthreads();
+  const int c = threadIdx.x;
+  float t = 0.f;
+  if (c < CS_COLS) {
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += part[w][c];
+    part[0][c] = t;
   }
+  if (Z > 1) {
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+    if (c < CS_COLS && c * Z / CS_COLS == rank) {
+      const unsigned at = smem_u32(&part[0][c]);
+      t = 0.f;
+      for (int z = 0; z < Z; ++z) {
+        float v;
+        unsigned remote;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(at), "r"(z));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(remote) : "memory");
+        t += v;
+      }
+    }
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+  }
+  if (c < CS_COLS && c * Z / CS_COLS == rank && c0 + c < N) db[c0 + c] = accumulate ? db[c0 + c] + t : t;
 }
 
 // Plan of one GEMM: tile and k slices.
@@ -470,8 +494,9 @@ int fc_bwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const floa
     }
   }
   if (db && !db_done) {
-    B200_TRY(launch_kernel(ctx, col_sum_kernel, dim3(ceil_div(out_size, 32)), dim3(32, 8), 0, 1, dout, db, B, out_size,
-                           accumulate));
+    const int blocks = B >= 512 ? 8 : B >= 256 ? 4 : B >= 128 ? 2 : 1;
+    B200_TRY(launch_kernel(ctx, col_sum_kernel, dim3(ceil_div(out_size, CS_COLS), blocks), dim3(256), 0, dim3(1, blocks), dout, db, B,
+                           out_size, accumulate));
   }
   return 0;
 }
