@@ -370,10 +370,11 @@ struct SmallStep {
   float *part, *dW, *db;
   int32_t *argmax;
 };
-constexpr int SN_MAX_STEPS = 16;
+constexpr int SN_MAX_STEPS = 16, SN_MAX_CTAS = 8;
 struct SmallNet {
   int n, in_dim, n_act, n_wts;
-  int clusters[4];   // clusters of 1, 2, 4, 8 CTAs that run at once
+  int clusters[SN_MAX_CTAS];  // clusters of 1, 2, ... CTAs that run at once
+  SmallDiv by_ctas;           // of a launch: CTAs of a sample
   int *err;
   SmallStep step[SN_MAX_STEPS];
 };

@@ -191,7 +191,7 @@ void net_drop_prepared(b200_net *net) {
 // Steps of the whole-network kernels, if every layer is one that they have and the values of a sample fit an SM
 int net_small_plan(b200_net *net) {
   b200_ctx *ctx = net->ctx;
-  int clusters[4];  // of an earlier call: the addresses do not change them
+  int clusters[SN_MAX_CTAS];  // of an earlier call: the addresses do not change them
   memcpy(clusters, net->small.clusters, sizeof clusters);
   net->small = {};
   const int n = (int)net->layers.size();

@@ -3,7 +3,7 @@
 //
 // What bounds such a network layer by layer is not a kernel's work but the launches: LeNet-5 is 0.4 million
 // products a sample, and a training step was 41 kernels of 1 to 15 us with a gap behind each (16 samples: 178 us,
-// now 60 us; a prediction of one sample: 67 us, now 21 us).  Here a cluster of up to eight CTAs takes
+// now 53 us; a prediction of one sample: 67 us, now 21 us).  Here a cluster of up to eight CTAs takes
 // one sample: every CTA keeps all activations and gradients of the sample in shared memory, computes a share of each
 // layer's values and copies them into the shared memory of the others (DSMEM).  The phases of a step are bound by
 // the latency of a few hundred dependent instructions: divisions are multiplications by constants from the host, the
@@ -36,7 +36,8 @@ constexpr int SN_WHOLE = 8192;  // weights of a fully-connected layer up to whic
 // be any number of steps ahead of it, and a barrier used again could take their bytes for those of the earlier step.
 constexpr int SN_EXCHANGES = 2 * SN_MAX_STEPS;  // at most one a step each way
 struct Cluster {
-  int n, rank, shift;   // n = 1 << shift
+  int n, rank, shift;   // n <= 1 << shift
+  SmallDiv by_n;
   uint64_t *bar;   // [SN_EXCHANGES]
   uint32_t step;   // exchanges so far
   bool failed;
@@ -66,10 +67,10 @@ struct Cluster {
     const uint32_t end = smem_u32(p + first + count);
     uint32_t at = smem_u32(p + first), head = min((16u - (at & 15u)) & 15u, end - at);
     const uint32_t bulk = (end - at - head) & ~15u;
-    const int to = threadIdx.x & (n - 1);
+    const int to = threadIdx.x & ((1 << shift) - 1);
     for (int piece = threadIdx.x >> shift; piece < 7; piece += 32 >> shift) {
       // piece 0: the bulk, 1 to 3: values before it, 4 to 6 after
-      if (to == rank) continue;
+      if (to == rank || to >= n) continue;
       uint32_t rb;
       asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(rb) : "r"(smem_u32(b)), "r"(to));
       const uint32_t src = piece == 0 ? at + head : piece < 4 ? at + (piece - 1) * 4 : at + head + bulk + (piece - 4) * 4;
@@ -98,7 +99,7 @@ __device__ __forceinline__ void cluster_barrier() {
 
 // this CTA's share of n values
 __device__ __forceinline__ void share(const Cluster &cl, int n, int *first, int *count) {
-  const int per = (n + cl.n - 1) >> cl.shift;
+  const int per = cl.by_n.of(n + cl.n - 1);
   *first = min(n, cl.rank * per);
   *count = min(n, *first + per) - *first;
 }
@@ -394,7 +395,8 @@ __global__ void __launch_bounds__(SN_THREADS, 1) small_net_kernel(const __grid_c
   cl.failed = false;
   asm("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(cl.n));
   asm("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(cl.rank));
-  cl.shift = 31 - __clz(cl.n);
+  cl.shift = cl.n > 1 ? 32 - __clz(cl.n - 1) : 0;
+  cl.by_n = net.by_ctas;
   const int sample = blockIdx.x / cl.n, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_act = (net.n_act + 3) & ~3;
   float *act = sm, *grd = sm + n_act, *wts = grd + (backward ? n_act : 0), *scratch = wts + net.n_wts;
@@ -819,12 +821,14 @@ int small_launch(b200_ctx *ctx, SmallKernel kernel, int nc, int B, size_t smem, 
   return 0;
 }
 
-// CTAs for one sample, as a power of two: up to eight (what a cluster may have anywhere), as many as let all samples run at once; how
-// many clusters the chip holds depends on how its SMs are grouped
+// CTAs for one sample: up to eight (what a cluster may have anywhere), as many as let all samples run at once; how many clusters the
+// chip holds depends on how its SMs are grouped (15 of eight, 22 of six, 26 of five, 33 of four, 45 of three, 74 of two).  Any number, not
+// powers of two alone: a LeNet-5 step of 16 samples 60 us with four CTAs a sample, 53 with six; of 40 samples 88 with two, 70 with
+// three.  More than eight is no faster: one sample 49 us with eight, 51 with sixteen, which have to send to each other.
 int small_cluster(const SmallNet &n, int B) {
-  for (int k = 3; k > 0; --k)
-    if (B <= n.clusters[k]) return k;
-  return 0;
+  int nc = SN_MAX_CTAS;
+  while (nc > 1 && B > n.clusters[nc - 1]) --nc;
+  return nc;
 }
 
 }  // namespace
@@ -844,12 +848,12 @@ bool small_net_fits(const b200_ctx *ctx, const SmallNet &n) {
 // sums over the samples read a sample's values, or its row of partial sums, for every weight.  Windows other than 3 and
 // 5 wide have no tiled form.  Layer by layer: launches, then the values that pass through memory; average pooling's
 // backward pass is the slow one.
-//   (LeNet-5 step: 16 samples 62 us against 110, 592 samples 531 against 785; 3x3 16 -> 16 -> 16 -> 4 on 16x16 maps: one
+//   (LeNet-5 step: 16 samples 53 us against 110, 592 samples 531 against 785; 3x3 16 -> 16 -> 16 -> 4 on 16x16 maps: one
 // sample 62 against 69, 256 samples 575 against 141; 784-64-64-10: 148 samples 58 against 42, predicted 15 against 19.)
 bool small_net_pays(const SmallNet &n, int B, bool train) {
   if (n.n == 0) return false;
-  const int k = small_cluster(n, B), nc = 1 << k;
-  const double turns = (B + n.clusters[k] - 1) / n.clusters[k];
+  const int nc = small_cluster(n, B);
+  const double turns = (B + n.clusters[nc - 1] - 1) / n.clusters[nc - 1];
   double weights = 0, tiled = 0, slow = 0, square = 0, fc = 0, fc_all = 0, values = 0, rows = 0;  // of a CTA; of all
   double launches = 0, through = 0, averaged = 0;                                                  // layer by layer
   for (int i = 0; i < n.n; ++i) {
@@ -887,13 +891,13 @@ bool small_net_pays(const SmallNet &n, int B, bool train) {
 }
 
 int small_net_plan(b200_ctx *ctx, SmallNet *n) {
-  for (int k = 0; k < 4; ++k) {
+  for (int nc = 1; nc <= SN_MAX_CTAS; ++nc) {
     SmallNet m = *n;
-    place_params(ctx, &m, 1 << k, 1);
+    place_params(ctx, &m, nc, 1);
     cudaLaunchConfig_t c;
     cudaLaunchAttribute at;
-    B200_TRY(small_launch(ctx, small_net_kernel<1>, 1 << k, 1, small_smem(m, 1), &c, &at));
-    B200_CUDA(cudaOccupancyMaxActiveClusters(&n->clusters[k], small_net_kernel<1>, &c));
+    B200_TRY(small_launch(ctx, small_net_kernel<1>, nc, 1, small_smem(m, 1), &c, &at));
+    B200_CUDA(cudaOccupancyMaxActiveClusters(&n->clusters[nc - 1], small_net_kernel<1>, &c));
   }
   return 0;
 }
@@ -902,13 +906,14 @@ int small_net_run(b200_ctx *ctx, const SmallNet &n, const float *x, const float 
                   int backward, int loss) {
   B200_REQUIRE(!backward || (loss >= B200_LOSS_MSE && loss <= B200_LOSS_CROSS_ENTROPY_MULTICLASS),
                "loss_grad: unknown loss %d", loss);
-  const int k = small_cluster(n, B);
+  const int nc = small_cluster(n, B);
   SmallNet m = n;
-  place_params(ctx, &m, 1 << k, backward);
+  m.by_ctas.set(nc);
+  place_params(ctx, &m, nc, backward);
   cudaLaunchConfig_t c;
   cudaLaunchAttribute at;
   const SmallKernel kernel = backward == 0 ? small_net_kernel<0> : backward == 1 ? small_net_kernel<1> : small_net_kernel<2>;
-  B200_TRY(small_launch(ctx, kernel, 1 << k, B, small_smem(m, backward), &c, &at));
+  B200_TRY(small_launch(ctx, kernel, nc, B, small_smem(m, backward), &c, &at));
   B200_CUDA(cudaLaunchKernelEx(&c, kernel, m, x, t, in_grad, loss));
   B200_LAUNCHED();
   if (!backward) return 0;
