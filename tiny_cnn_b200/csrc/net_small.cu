@@ -3,7 +3,7 @@
 //
 // What bounds such a network layer by layer is not a kernel's work but the launches: LeNet-5 is 0.4 million
 // products a sample, and a training step was 41 kernels of 1 to 15 us with a gap behind each (16 samples: 178 us,
-// now 53 us; a prediction of one sample: 67 us, now 21 us).  Here a cluster of up to eight CTAs takes
+// now 53 us; a prediction of one sample: 67 us, now 19 us).  Here a cluster of up to eight CTAs takes
 // one sample: every CTA keeps all activations and gradients of the sample in shared memory, computes a share of each
 // layer's values and copies them into the shared memory of the others (DSMEM).  The phases of a step are bound by
 // the latency of a few hundred dependent instructions: divisions are multiplications by constants from the host, the
@@ -408,6 +408,7 @@ __global__ void __launch_bounds__(SN_THREADS, 1) small_net_kernel(const __grid_c
   if (tid < SN_EXCHANGES) mbar_fence_init();
   __syncthreads();
   if (cl.n > 1) asm volatile("barrier.cluster.arrive.aligned;\n" ::: "memory");  // waited for before the first exchange
+  if (MODE == 0) after_previous_kernel();  // the others are launched behind it
   // Everything that the sample needs from global memory is asked for at once, weights by bulk copies; the first step's
   // share is waited for here, the rest behind the first step.
   if (tid < net.n) {
@@ -806,21 +807,6 @@ void place_params(const b200_ctx *ctx, SmallNet *n, int nc, int backward) {
 
 using SmallKernel = void (*)(SmallNet, const float *, const float *, float *, int);
 
-int small_launch(b200_ctx *ctx, SmallKernel kernel, int nc, int B, size_t smem, cudaLaunchConfig_t *c, cudaLaunchAttribute *at) {
-  B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  *c = {};
-  c->gridDim = dim3((unsigned)(B * nc));
-  c->blockDim = dim3(SN_THREADS);
-  c->dynamicSmemBytes = smem;
-  c->stream = ctx->stream;
-  at->id = cudaLaunchAttributeClusterDimension;
-  at->val.clusterDim.x = (unsigned)nc;
-  at->val.clusterDim.y = at->val.clusterDim.z = 1;
-  c->attrs = at;
-  c->numAttrs = 1;
-  return 0;
-}
-
 // CTAs for one sample: up to eight (what a cluster may have anywhere), as many as let all samples run at once; how many clusters the
 // chip holds depends on how its SMs are grouped (15 of eight, 22 of six, 26 of five, 33 of four, 45 of three, 74 of two).  Any number, not
 // powers of two alone: a LeNet-5 step of 16 samples 60 us with four CTAs a sample, 53 with six; of 40 samples 88 with two, 70 with
@@ -894,9 +880,19 @@ int small_net_plan(b200_ctx *ctx, SmallNet *n) {
   for (int nc = 1; nc <= SN_MAX_CTAS; ++nc) {
     SmallNet m = *n;
     place_params(ctx, &m, nc, 1);
-    cudaLaunchConfig_t c;
+    const size_t smem = small_smem(m, 1);
+    B200_CUDA(cudaFuncSetAttribute(small_net_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchAttribute at;
-    B200_TRY(small_launch(ctx, small_net_kernel<1>, nc, 1, small_smem(m, 1), &c, &at));
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)nc;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)nc);
+    c.blockDim = dim3(SN_THREADS);
+    c.dynamicSmemBytes = smem;
+    c.stream = ctx->stream;
+    c.attrs = &at;
+    c.numAttrs = 1;
     B200_CUDA(cudaOccupancyMaxActiveClusters(&n->clusters[nc - 1], small_net_kernel<1>, &c));
   }
   return 0;
@@ -910,12 +906,13 @@ int small_net_run(b200_ctx *ctx, const SmallNet &n, const float *x, const float 
   SmallNet m = n;
   m.by_ctas.set(nc);
   place_params(ctx, &m, nc, backward);
-  cudaLaunchConfig_t c;
-  cudaLaunchAttribute at;
   const SmallKernel kernel = backward == 0 ? small_net_kernel<0> : backward == 1 ? small_net_kernel<1> : small_net_kernel<2>;
-  B200_TRY(small_launch(ctx, kernel, nc, B, small_smem(m, backward), &c, &at));
-  B200_CUDA(cudaLaunchKernelEx(&c, kernel, m, x, t, in_grad, loss));
-  B200_LAUNCHED();
+  const size_t smem = small_smem(m, backward);
+  B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // A prediction's launch, plan and barriers overlap the end of the kernel before it (LeNet-5, one sample: 20.5 us a call, 18.6 so), but
+  // not where its clusters only fit if nothing else lies between them: 45 of three CTAs took 28.7 us for 24.6.  Steps are captured.
+  if (backward || (nc > 2 && B * 15 > n.clusters[nc - 1] * 14)) ctx->waited = true;
+  B200_TRY(launch_kernel(ctx, kernel, dim3((unsigned)(B * nc)), dim3(SN_THREADS), smem, dim3((unsigned)nc), m, x, t, in_grad, loss));
   if (!backward) return 0;
   int blocks = 0;
   for (int i = 0; i < n.n; ++i) blocks += ceil_div(n.step[i].w_len + n.step[i].b_len, reduce_entries(n.step[i], B));
