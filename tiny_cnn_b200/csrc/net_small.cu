@@ -15,6 +15,10 @@
 // The arithmetic is that of the layer kernels (products added in fp32); only the order of the sums differs.
 #include <float.h>
 
+#include <algorithm>
+#include <array>
+#include <map>
+#include <mutex>
 #include <type_traits>
 
 #include "common.cuh"
@@ -876,25 +880,34 @@ bool small_net_pays(const SmallNet &n, int B, bool train) {
          1.05 * (11.5 + launches + B * (0.18e-6 * fc_all + 18e-6 * through + 122e-6 * averaged));
 }
 
+// The counts depend on the device alone (a CTA's registers leave no room for a second one on its SM, whatever its shared memory), and the
+// driver takes a tenth of a millisecond and more to work one out: they are asked for once.
 int small_net_plan(b200_ctx *ctx, SmallNet *n) {
-  for (int nc = 1; nc <= SN_MAX_CTAS; ++nc) {
-    SmallNet m = *n;
-    place_params(ctx, &m, nc, 1);
-    const size_t smem = small_smem(m, 1);
+  static std::mutex lock;
+  static std::map<int, std::array<int, SN_MAX_CTAS>> known;
+  std::lock_guard<std::mutex> guard(lock);
+  auto it = known.find(ctx->device);
+  if (it == known.end()) {
+    std::array<int, SN_MAX_CTAS> most;
+    const size_t smem = small_room(ctx);
     B200_CUDA(cudaFuncSetAttribute(small_net_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)nc;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cudaLaunchConfig_t c = {};
-    c.gridDim = dim3((unsigned)nc);
-    c.blockDim = dim3(SN_THREADS);
-    c.dynamicSmemBytes = smem;
-    c.stream = ctx->stream;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    B200_CUDA(cudaOccupancyMaxActiveClusters(&n->clusters[nc - 1], small_net_kernel<1>, &c));
+    for (int nc = 1; nc <= SN_MAX_CTAS; ++nc) {
+      cudaLaunchAttribute at;
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = (unsigned)nc;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cudaLaunchConfig_t c = {};
+      c.gridDim = dim3((unsigned)nc);
+      c.blockDim = dim3(SN_THREADS);
+      c.dynamicSmemBytes = smem;
+      c.stream = ctx->stream;
+      c.attrs = &at;
+      c.numAttrs = 1;
+      B200_CUDA(cudaOccupancyMaxActiveClusters(&most[nc - 1], small_net_kernel<1>, &c));
+    }
+    it = known.emplace(ctx->device, most).first;
   }
+  std::copy(it->second.begin(), it->second.end(), n->clusters);
   return 0;
 }
 
