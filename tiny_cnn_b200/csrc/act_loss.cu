@@ -243,13 +243,12 @@ int act_fwd(b200_ctx *ctx, int kind, const float *x, float *y, int dim, int B, f
       softmax_fwd16_kernel<<<ceil_div(B * 16, 256), 256, 0, ctx->stream>>>(x, y, dim, B);
     else
       softmax_fwd_kernel<<<ceil_div(B, 32), 32, 0, ctx->stream>>>(x, y, dim, B);
-  } else {
-    size_t n4 = (aligned16(x) && aligned16(y)) ? n / 4 : 0;
-    B200_TRY(launch_kernel(ctx, act_fwd_kernel, dim3(grid_for(n4 ? n4 : n, 256, ctx->sm_count)), dim3(256), 0, 1, kind, param,
-                           x, y, n4, n));
+    B200_LAUNCHED();
+    return 0;
   }
-  B200_LAUNCHED();
-  return 0;
+  size_t n4 = (aligned16(x) && aligned16(y)) ? n / 4 : 0;
+  return launch_kernel(ctx, act_fwd_kernel, dim3(grid_for(n4 ? n4 : n, 256, ctx->sm_count)), dim3(256), 0, 1, kind, param, x, y,
+                       n4, n);
 }
 
 int act_bwd(b200_ctx *ctx, int kind, const float *y, const float *dy, float *dx, int dim, int B, float param) {
@@ -262,13 +261,12 @@ int act_bwd(b200_ctx *ctx, int kind, const float *y, const float *dy, float *dx,
                                                                            nullptr, 0);
     else
       softmax_bwd_kernel<<<ceil_div(B, 32), 32, 0, ctx->stream>>>(y, const_cast<float *>(dy), dx, dim, B, nullptr, 0);
-  } else {
-    size_t n4 = (aligned16(y) && aligned16(dy) && aligned16(dx)) ? n / 4 : 0;
-    B200_TRY(launch_kernel(ctx, act_bwd_kernel, dim3(grid_for(n4 ? n4 : n, 256, ctx->sm_count)), dim3(256), 0, 1, kind, param,
-                           y, dy, dx, n4, n));
+    B200_LAUNCHED();
+    return 0;
   }
-  B200_LAUNCHED();
-  return 0;
+  size_t n4 = (aligned16(y) && aligned16(dy) && aligned16(dx)) ? n / 4 : 0;
+  return launch_kernel(ctx, act_bwd_kernel, dim3(grid_for(n4 ? n4 : n, 256, ctx->sm_count)), dim3(256), 0, 1, kind, param, y, dy,
+                       dx, n4, n);
 }
 
 int loss_grad(b200_ctx *ctx, int kind, const float *y, const float *t, float *dy, int dim, int B) {
