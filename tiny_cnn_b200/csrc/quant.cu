@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
     }
     __syncthreads();
   }
-  {
+  if (places > 0) {  // a sample's last blocks may have no pixels: their runs are rounded up to 16
     QScale q;
     q.set(smp.min_in, smp.max_in);
     const int groups = a.Cp / 8;
@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
       atomicAdd(psum + p, __dp4a(w1, 0x01010101u, __dp4a(w0, 0x01010101u, 0u)));
     };
     if (a.raw) {
-      while (places > 0 && cg < groups) {
+      while (cg < groups) {
         const float *src = raw + cg * 8 * places + p;
         float v[8];
 #pragma unroll
@@ -713,8 +713,8 @@ __global__ void __launch_bounds__(QC_THREADS, 1) q_conv_fused_kernel(const __gri
 #pragma unroll
         for (int k = 0; k < 8; ++k) next[k] = cg < groups && cg * 8 + k < a.C ? src[(size_t)k * plane] : 0.f;
       };
-      if (places > 0) fetch();
-      while (places > 0 && cg < groups) {
+      fetch();
+      while (cg < groups) {
         float v[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = next[k];
