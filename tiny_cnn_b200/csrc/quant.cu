@@ -1052,9 +1052,12 @@ __global__ void __launch_bounds__(256) q_fc_quantize_kernel(const float *__restr
 #pragma unroll
   for (int k = 0; k < QF_CIN / 8; ++k) {
     const int c = c0 + warp + 8 * k, i = i0 + lane;
-    x[k] = c < in_size && i < out_size ? W[(size_t)c * out_size + i] : 0.f;
+    x[k] = c < in_size && i < out_size ? __ldcg(W + (size_t)c * out_size + i) : 0.f;
   }
-  after_previous_kernel();  // the filter's values, which the ranges' kernel only read, may be asked for ahead of it
+  // The filter's values may be asked for ahead of this wait: the ranges' kernel, which let this one begin, only read them and had
+  // itself waited for whoever wrote them.  From the L2 cache, where those writes are by then: what the wait also does is
+  // to make an SM's L1 cache forget the lines it held from before.
+  after_previous_kernel();
   // the partial results stand in for the filter: same extremes, and when all are equal so is W[0]
   filter_range(part, 1, 0, (size_t)2 * nparts, bias, nbias, qg);
   if (b == 0) {
