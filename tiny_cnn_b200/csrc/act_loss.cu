@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(FCL_THREADS) fc_softmax_bwd_wide_kernel(const 
   gates(0);
   for (int s = warp; s < samples; s += FCL_WARPS) {
     const float g = head_grad(y, t, loss_kind, writes ? dy : nullptr, writes ? dz : nullptr, n0 + s, N);
-    if (lane < FCS_N) ds[s][lane] = g;
+    if (lane < FCS_N) ds[s][lane] = lane < N ? g : 0.f;  // behind N an infinite gradient leaves no zero
   }
   __syncthreads();
   if (dx == nullptr) return;
