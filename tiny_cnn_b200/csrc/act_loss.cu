@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(FCL_THREADS) fc_softmax_fwd_cluster_kernel(con
       }
   };
   int buf = 0;
-  fetch(rank * per, rows[0]);
+  if (rank * per < end) fetch(rank * per, rows[0]);  // the last blocks' shares may be empty: no copy that nobody waits for
   for (int k0 = rank * per; k0 < end; k0 += FCL_CHUNK, buf ^= 1) {
     float xk[FCL_GROUP][XK];
 #pragma unroll
