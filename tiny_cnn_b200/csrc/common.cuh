@@ -90,8 +90,8 @@ struct b200_ctx {
   // recorded when every block of the next dX kernel has begun (launch_kernel clears it); null: not asked for
   cudaEvent_t started = nullptr;
 
-  // kernels may be launched while the one before them in the stream runs (launch_kernel); not the one behind a wait for another
-  // stream, which only costs the driver time
+  // Kernels may be launched while the one before them in the stream runs (launch_kernel).  `waited`: not the next one, since a
+  // stream of the context was told to wait for an event (stream_wait): behind such a wait it would only cost the driver time.
   bool overlap = true, waited = false;
 
   // second stream of calls whose kernels leave SMs to one another (conv2d_bwd), and the events that tie it to `stream`
@@ -123,17 +123,19 @@ inline int stream_wait(b200_ctx *ctx, cudaStream_t stream, cudaEvent_t e) {
   return 0;
 }
 
-// A launch with clusters of `cluster` blocks that records ctx->started.  The kernel begins with
-// after_previous_kernel: its launch and what it sets up overlap the end of the kernel before it.
+// A launch with clusters of `cluster` blocks that records ctx->started.  `overlap`: the launch and what the kernel sets up may
+// overlap the end of the kernel before it in the stream.  Only for kernels in which every thread runs wait_for_previous_kernel
+// or after_previous_kernel, ahead of all that the kernel before it may have written or may still read.
 template <typename... Params, typename... Args>
-int launch_kernel(b200_ctx *ctx, void (*kernel)(Params...), dim3 grid, dim3 threads, size_t smem, dim3 cluster, const Args &...args) {
+int launch_kernel_as(b200_ctx *ctx, bool overlap, void (*kernel)(Params...), dim3 grid, dim3 threads, size_t smem, dim3 cluster,
+                     const Args &...args) {
   cudaLaunchConfig_t c = {};
   c.gridDim = grid;
   c.blockDim = threads;
   c.dynamicSmemBytes = smem;
   c.stream = ctx->stream;
   cudaLaunchAttribute at[3];
-  if (ctx->overlap && !ctx->waited) {
+  if (overlap) {
     at[c.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[c.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     ++c.numAttrs;
@@ -157,6 +159,12 @@ int launch_kernel(b200_ctx *ctx, void (*kernel)(Params...), dim3 grid, dim3 thre
   B200_CUDA(cudaLaunchKernelEx(&c, kernel, args...));
   B200_LAUNCHED();
   return 0;
+}
+
+// the same, overlapping wherever the context's launches do
+template <typename... Params, typename... Args>
+int launch_kernel(b200_ctx *ctx, void (*kernel)(Params...), dim3 grid, dim3 threads, size_t smem, dim3 cluster, const Args &...args) {
+  return launch_kernel_as(ctx, ctx->overlap && !ctx->waited, kernel, grid, threads, smem, cluster, args...);
 }
 
 int ctx_scratch(b200_ctx *ctx, size_t bytes, void **out);

@@ -1218,9 +1218,10 @@ static int run_captured(b200_net *net, int slot_idx, const std::string &key, F b
   B200_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
   // In a graph a kernel starts microseconds after the one before it anyhow, and blocks that wait on an SM shift which of two
   // branches gets it: steps of the CIFAR-10 network of 12 samples took 131 us for 111, of 64 samples 159 for 174.
+  const bool overlap = net->ctx->overlap;
   net->ctx->overlap = false;
   int r = body();
-  net->ctx->overlap = true;
+  net->ctx->overlap = overlap;
   cudaError_t ce = cudaStreamEndCapture(st, &graph);
   unsigned long long recorded = g_launches.load() - before;
   if (r != 0) {

@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(SN_THREADS, 1) small_net_kernel(const __grid_c
   if (tid < SN_EXCHANGES) mbar_fence_init();
   __syncthreads();
   if (cl.n > 1) asm volatile("barrier.cluster.arrive.aligned;\n" ::: "memory");  // waited for before the first exchange
-  if (MODE == 0) after_previous_kernel();  // the others are launched behind it
+  if (MODE == 0) after_previous_kernel();  // the others are launched behind the end of the kernel before them
   // Everything that the sample needs from global memory is asked for at once, weights by bulk copies; the first step's
   // share is waited for here, the rest behind the first step.
   if (tid < net.n) {
@@ -922,10 +922,13 @@ int small_net_run(b200_ctx *ctx, const SmallNet &n, const float *x, const float 
   const SmallKernel kernel = backward == 0 ? small_net_kernel<0> : backward == 1 ? small_net_kernel<1> : small_net_kernel<2>;
   const size_t smem = small_smem(m, backward);
   B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  // A prediction's launch, plan and barriers overlap the end of the kernel before it (LeNet-5, one sample: 20.5 us a call, 18.6 so), but
-  // not where its clusters only fit if nothing else lies between them: 45 of three CTAs took 28.7 us for 24.6.  Steps are captured.
-  if (backward || (nc > 2 && B * 15 > n.clusters[nc - 1] * 14)) ctx->waited = true;
-  B200_TRY(launch_kernel(ctx, kernel, dim3((unsigned)(B * nc)), dim3(SN_THREADS), smem, dim3((unsigned)nc), m, x, t, in_grad, loss));
+  // A prediction's launch, plan and barriers overlap the end of the kernel before it in the stream (LeNet-5, one sample: 20.5 us a call,
+  // 18.7 so if that is a kernel which lets it in early, as the call before does; behind a copy the same as without), but
+  // not where its clusters only fit if nothing else lies between them: 45 of three CTAs took 28.7 us for 24.6.  The kernels
+  // with a backward pass do not wait for the one before them: steps are captured, where a launch costs little.
+  const bool overlap = !backward && ctx->overlap && !ctx->waited && (nc <= 2 || B * 15 <= n.clusters[nc - 1] * 14);
+  B200_TRY(launch_kernel_as(ctx, overlap, kernel, dim3((unsigned)(B * nc)), dim3(SN_THREADS), smem, dim3((unsigned)nc), m, x, t,
+                            in_grad, loss));
   if (!backward) return 0;
   int blocks = 0;
   for (int i = 0; i < n.n; ++i) blocks += ceil_div(n.step[i].w_len + n.step[i].b_len, reduce_entries(n.step[i], B));
