@@ -922,10 +922,10 @@ int small_net_run(b200_ctx *ctx, const SmallNet &n, const float *x, const float 
   const SmallKernel kernel = backward == 0 ? small_net_kernel<0> : backward == 1 ? small_net_kernel<1> : small_net_kernel<2>;
   const size_t smem = small_smem(m, backward);
   B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  // A prediction's launch, plan and barriers overlap the end of the kernel before it in the stream (LeNet-5, one sample: 20.5 us a call,
-  // 18.7 so if that is a kernel which lets it in early, as the call before does; behind a copy the same as without), but
-  // not where its clusters only fit if nothing else lies between them: 45 of three CTAs took 28.7 us for 24.6.  The kernels
-  // with a backward pass do not wait for the one before them: steps are captured, where a launch costs little.
+  // A prediction's launch, plan and barriers overlap the end of the kernel before it in the stream (LeNet-5, one sample: 20.5 us a call
+  // behind another prediction, 18.7 so; with an elementwise kernel in front of each 22.6 and 20.6; behind an upload 25.5 to 26.6
+  // either way), but not where its clusters only fit if nothing else lies between them: 45 of three CTAs took 28.7 us for
+  // 24.6.  The kernels with a backward pass do not wait for the one before them: steps are captured, where a launch costs little.
   const bool overlap = !backward && ctx->overlap && !ctx->waited && (nc <= 2 || B * 15 <= n.clusters[nc - 1] * 14);
   B200_TRY(launch_kernel_as(ctx, overlap, kernel, dim3((unsigned)(B * nc)), dim3(SN_THREADS), smem, dim3((unsigned)nc), m, x, t,
                             in_grad, loss));
