@@ -94,30 +94,7 @@ int conv_bwd_impl(b200_ctx *ctx, const b200_conv_desc *d, const float *in, const
   void *scratch = nullptr;
   B200_TRY(ctx_scratch(ctx, (align_up(n_dx, 64) + n_dw + 64) * sizeof(float), &scratch));
   float *s_dx = static_cast<float *>(scratch), *s_dw = s_dx + align_up(n_dx, 64);
-  // dX.  Where it leaves SMs idle, dW runs beside it: on the context's second stream, as soon as the dX blocks have begun
-  // (both need most of an SM's shared memory; 14x28, 78 -> 148, 3x3, 2 samples: 12 us of dW behind 25 of dX, now 3).
-  const int dx_blocks = tc_dx ? conv_gather_dx_blocks(ctx, g, batch) : din && tiled ? conv_tiled_dx_blocks(ctx, g, batch) : 0;
-  if ((tc.dw || tc.dw_small) && dx_blocks > 0 && dx_blocks < ctx->sm_count) {
-    const cudaStream_t main = ctx->stream;
-    if (tc_dx)
-      B200_TRY(conv_gather_prep(ctx, g, W, nullptr, s_dx));
-    else
-      B200_TRY(conv_tiled_dx_prep(ctx, g, W, s_dx));
-    B200_CUDA(cudaEventRecord(ctx->ev_fork, main));
-    ctx->started = ctx->ev_started;
-    const int rc = tc_dx ? conv_gather_dx(ctx, g, dout, s_dx, din, batch) : conv_tiled_dx(ctx, g, W, dout, din, batch, s_dx, 0);
-    ctx->started = nullptr;
-    B200_TRY(rc);
-    B200_TRY(stream_wait(ctx, ctx->side, ctx->ev_fork));
-    B200_TRY(stream_wait(ctx, ctx->side, ctx->ev_started));
-    ctx->stream = ctx->side;
-    const int rc_dw = tc.dw_small ? conv_dw_small(ctx, g, in, dout, batch, s_dw, dW, db, accumulate)
-                                  : conv_gather_dw(ctx, g, in, dout, batch, s_dw, dW, db, accumulate, batch);
-    ctx->stream = main;
-    B200_CUDA(cudaEventRecord(ctx->ev_join, ctx->side));  // also behind a launch that failed: what began ends before the call's successors
-    B200_TRY(stream_wait(ctx, main, ctx->ev_join));
-    return rc_dw;
-  }
+  // dX
   if (tc_dx) {
     B200_TRY(conv_gather_prep(ctx, g, W, nullptr, s_dx));
     B200_TRY(conv_gather_dx(ctx, g, dout, s_dx, din, batch));

@@ -94,10 +94,6 @@ struct b200_ctx {
   // stream of the context was told to wait for an event (stream_wait): behind such a wait it would only cost the driver time.
   bool overlap = true, waited = false;
 
-  // second stream of calls whose kernels leave SMs to one another (conv2d_bwd), and the events that tie it to `stream`
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_started = nullptr, ev_join = nullptr;
-
   // device word a kernel sets when a bounded wait ran out; read by b200_ctx_sync
   int *dev_err = nullptr;
 

@@ -175,8 +175,6 @@ int b200_ctx_create(int device, void *stream, b200_ctx **out) {
     B200_CUDA(cudaStreamCreateWithPriority(&c->stream, cudaStreamNonBlocking, -1));
     c->own_stream = true;
   }
-  B200_CUDA(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
-  for (cudaEvent_t *e : {&c->ev_fork, &c->ev_started, &c->ev_join}) B200_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   ctx_load_tiles(c);
   B200_CUDA(cudaMalloc(&c->dev_err, sizeof(int)));
   B200_CUDA(cudaMemset(c->dev_err, 0, sizeof(int)));
@@ -244,9 +242,6 @@ int b200_ctx_destroy(b200_ctx *ctx) {
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   if (ctx->dev_err) cudaFree(ctx->dev_err);
   for (auto &kv : ctx->tbl_cache) cudaFree(kv.second);
-  for (cudaEvent_t e : {ctx->ev_fork, ctx->ev_started, ctx->ev_join})
-    if (e) cudaEventDestroy(e);
-  if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return 0;
