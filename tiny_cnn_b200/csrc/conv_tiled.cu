@@ -47,8 +47,11 @@ __global__ void conv_prep_wt_fwd_kernel(const float *__restrict__ W, float *__re
 // wt[(o*KK + a*KW + b)*Cp + ic] = W[(o*C + ic)*KK + (KH-1-a)*KW + (KW-1-b)]
 __global__ void conv_prep_wt_dx_kernel(const float *__restrict__ W, float *__restrict__ wt, int C,
                                        int OC, int Cp, int KH, int KW,
-                                       const uint8_t *__restrict__ tbl) {
-  after_previous_kernel();
+                                       const uint8_t *__restrict__ tbl, int early) {
+  if (early)
+    after_previous_kernel();
+  else
+    wait_for_previous_kernel();
   int KK = KH * KW;
   int total = OC * KK * Cp;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -871,14 +874,14 @@ static size_t fewout_smem(int CI, int KH, int KW) {
 }
 
 template <int KH, int KW>
-static int launch_fewout(b200_ctx *ctx, const FewOutCfg &p, int B) {
+static int launch_fewout(b200_ctx *ctx, const FewOutCfg &p, int B, bool overlap) {
   size_t smem = fewout_smem(p.CI, KH, KW);
   dim3 grid(p.tiles_x * ceil_div(p.HO, FO_TILE_H), B);
 #define B200_FEWOUT(N)                                                                                   \
   do {                                                                                                   \
     B200_CUDA(cudaFuncSetAttribute(conv_fewout_kernel<KH, KW, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                    (int)smem));                                                          \
-    B200_TRY(launch_kernel(ctx, conv_fewout_kernel<KH, KW, N>, grid, FO_THREADS, smem, 1, p));           \
+    B200_TRY(launch_kernel_as(ctx, overlap, conv_fewout_kernel<KH, KW, N>, grid, FO_THREADS, smem, 1, p)); \
   } while (0)
   if (p.CO == 1) B200_FEWOUT(1);
   else if (p.CO == 2) B200_FEWOUT(2);
@@ -896,14 +899,23 @@ int conv_tiled_dx_blocks(const b200_ctx *ctx, const ConvGeom &g, int B) {
   return fewout_takes(ctx, g) ? ceil_div(g.WI, FO_TILE) * ceil_div(g.HI, FO_TILE_H) * B : 0;
 }
 
-// the flipped, transposed filter copy the dX kernels read; depends on the weights only
-int conv_tiled_dx_prep(b200_ctx *ctx, const ConvGeom &g, const float *W, float *scratch) {
+// Blocks of conv_fewout_kernel, which hold an SM's FFMA pipes to themselves but leave it room for a second one, must not be dealt out
+// while the small blocks of another kernel sit on some SMs: the others then get two, and twice the time, where one each was
+// to be had (16x16, 4 -> 250, 5x5, 64 samples, 128 blocks: a backward call 126 us so, 104 without overlapping launches, 96 now).
+// Fewer blocks than a quarter of the SMs find free ones all the same, and gain a microsecond.
+static bool fewout_crowds(const b200_ctx *ctx, int blocks) { return 4 * blocks > ctx->sm_count; }
+
+static int launch_dx_prep(b200_ctx *ctx, const ConvGeom &g, const float *W, float *scratch, bool early) {
   int KK = g.KH * g.KW;
   int Cp = padded_channels(g.C);
   int total = g.OC * KK * Cp;
-  B200_TRY(launch_kernel(ctx, conv_prep_wt_dx_kernel, dim3(ceil_div(total, 256)), dim3(256), 0, 1, W, scratch, g.C, g.OC, Cp,
-                         g.KH, g.KW, g.tbl));
-  return 0;
+  return launch_kernel(ctx, conv_prep_wt_dx_kernel, dim3(ceil_div(total, 256)), dim3(256), 0, 1, W, scratch, g.C, g.OC, Cp, g.KH, g.KW,
+                       g.tbl, early ? 1 : 0);
+}
+
+// the flipped, transposed filter copy the dX kernels read; depends on the weights only
+int conv_tiled_dx_prep(b200_ctx *ctx, const ConvGeom &g, const float *W, float *scratch) {
+  return launch_dx_prep(ctx, g, W, scratch, true);
 }
 
 // `prep` = 0: `scratch` already holds the filter copy of these weights (conv_tiled_dx_prep)
@@ -911,7 +923,8 @@ int conv_tiled_dx(b200_ctx *ctx, const ConvGeom &g, const float *W, const float 
                   float *din, int B, float *scratch, int prep) {
   if (B == 0) return 0;
   int Cp = padded_channels(g.C);
-  if (prep) B200_TRY(conv_tiled_dx_prep(ctx, g, W, scratch));
+  const bool crowds = fewout_crowds(ctx, conv_tiled_dx_blocks(ctx, g, B));
+  if (prep) B200_TRY(launch_dx_prep(ctx, g, W, scratch, !crowds));
   if (fewout_takes(ctx, g)) {
     // few input channels: dX is a convolution with few OUTPUT channels
     FewOutCfg f{};
@@ -927,8 +940,10 @@ int conv_tiled_dx(b200_ctx *ctx, const ConvGeom &g, const float *W, const float 
     f.pad_t = g.KH - 1 - g.pad_t;
     f.pad_l = g.KW - 1 - g.pad_l;
     f.tiles_x = ceil_div(g.WI, FO_TILE);
-    if (g.KH == 5 && g.KW == 5) return launch_fewout<5, 5>(ctx, f, B);
-    if (g.KH == 3 && g.KW == 3) return launch_fewout<3, 3>(ctx, f, B);
+    // the filter copy's kernel does not let it in early; what else may come before it might
+    const bool overlap = ctx->overlap && !ctx->waited && (prep || !crowds);
+    if (g.KH == 5 && g.KW == 5) return launch_fewout<5, 5>(ctx, f, B, overlap);
+    if (g.KH == 3 && g.KW == 3) return launch_fewout<3, 3>(ctx, f, B, overlap);
   }
   CoreCfg p{};
   p.in = dout;
