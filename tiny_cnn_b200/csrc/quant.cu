@@ -1638,6 +1638,18 @@ int qconv_fwd(b200_ctx *ctx, const b200_conv_desc *d, const float *in, const flo
   return 0;
 }
 
+// Whether one cluster is the faster form, by its microseconds: a start, the words of four inputs and of the filter that a thread
+// quantizes, the samples that a warp requantizes, and how sums are added up (non-negative least squares over 1382 layers of 16 to 2048 inputs, 1 to 256
+// outputs and 1 to 512 samples, off by 6 %).  The four launches take 14.3 to 18 us on all of these: 16 inputs, 33 outputs, 128 samples 28.1 us in
+// one cluster (of one block) and 14.7 in launches; 1626 -> 16, 116 samples 29.6 and 15; 64 -> 10, one sample 7.5 and 14.7.
+static bool q_fc_whole_pays(int klog, int slices, int blocks, int out_size, int B) {
+  const int words = 1 << (klog - 2), rows = B < QO_M ? B : QO_M, each = ceil_div(B, QO_WARPS * blocks);
+  return 4.3 + 0.85 * ceil_div(rows * words, QO_THREADS) + 0.54 * ceil_div(words * QO_N, QO_THREADS) +
+           each * (1.25 + 0.62 * ceil_div(out_size, 32)) + (slices > 1 ? 0.13 * ceil_div(rows * QO_N, QO_THREADS) : 0.0) +
+           (blocks > 1 ? 1.3 : 0.0) <
+         16.0;
+}
+
 int qfc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const float *W,
             const float *bias, float *out, int B) {
   B200_REQUIRE(in_size > 0 && out_size > 0, "quantized fc: non-positive size");
@@ -1648,6 +1660,7 @@ int qfc_fwd(b200_ctx *ctx, int in_size, int out_size, const float *in, const flo
   for (int klog = 5; klog <= 8; ++klog) {
     const long long slices = ceil_div(in_size, 1 << klog), tiles = (long long)ceil_div(out_size, QO_N) * ceil_div(B, QO_M);
     if (slices * tiles > QO_BLOCKS) continue;
+    if (!q_fc_whole_pays(klog, (int)slices, (int)(slices * tiles), out_size, B)) break;
     const int blocks = (int)(slices * tiles), parts = (int)slices * (klog > 7 ? 2 : 1);
     QFcArgs a = {};
     a.in = in, a.W = W, a.bias = bias, a.out = out;
