@@ -811,13 +811,28 @@ void place_params(const b200_ctx *ctx, SmallNet *n, int nc, int backward) {
 
 using SmallKernel = void (*)(SmallNet, const float *, const float *, float *, int);
 
+// Whether B clusters of nc CTAs leave one place in fifteen free: clusters that fill the chip wait for each other's SMs
+bool leaves_room(const SmallNet &n, int nc, int B) { return nc <= 2 || B * 15 <= n.clusters[nc - 1] * 14; }
+
+double small_macs(const SmallNet &n) {  // multiply-adds of a sample's forward pass
+  double macs = 0;
+  for (int i = 0; i < n.n; ++i)
+    macs += n.step[i].kind == SN_CONV ? (double)n.step[i].out_n * n.step[i].C * n.step[i].KH * n.step[i].KW
+            : n.step[i].kind == SN_FC ? (double)n.step[i].w_len : 0.0;
+  return macs;
+}
+
 // CTAs for one sample: up to eight (what a cluster may have anywhere), as many as let all samples run at once; how many clusters the
 // chip holds depends on how its SMs are grouped (15 of eight, 22 of six, 26 of five, 33 of four, 45 of three, 74 of two).  Any number, not
 // powers of two alone: a LeNet-5 step of 16 samples 60 us with four CTAs a sample, 53 with six; of 40 samples 88 with two, 70 with
 // three.  More than eight is no faster: one sample 49 us with eight, 51 with sixteen, which have to send to each other.
-int small_cluster(const SmallNet &n, int B) {
+// A prediction whose clusters fill the chip takes a CTA less, which costs it its share of the products and saves 2 us: 3x3 nets
+// of two layers 18.6 us with 22 samples on clusters of six, 15.7 on clusters of five.  Not where that share is above 50 thousand (LeNet-5, 45
+// samples: 24.8 us with three CTAs, 27.1 with two).
+int small_cluster(const SmallNet &n, int B, bool predict) {
   int nc = SN_MAX_CTAS;
   while (nc > 1 && B > n.clusters[nc - 1]) --nc;
+  if (predict && !leaves_room(n, nc, B) && leaves_room(n, nc - 1, B) && small_macs(n) < 50e3 * nc * (nc - 1)) --nc;
   return nc;
 }
 
@@ -830,19 +845,24 @@ bool small_net_fits(const b200_ctx *ctx, const SmallNet &n) {
   return small_smem(m, 1) <= small_room(ctx);
 }
 
-// Microseconds of a pass either way, fitted (non-negative least squares) to 24 networks of 1 to 7 steps at 17 batches
-// from 1 to 2048, forward alone and as a training step; the fits are off by 10 to 15 % (rms), and taking the cheaper
-// one by them costs 1 % on average against always taking the faster one.  The layers have to win by a tenth (a step: a
-// twentieth), which is where fewest networks lose.
+// Microseconds of a pass either way, fitted (non-negative least squares) to 24 networks of 1 to 7 steps at 17 (predictions) and 29
+// (steps) batches from 1 to 2048.
+//   A step: on clusters of any size and with the layers' kernels as they are; where neither form is three times the other the fits
+// are off by 11 to 13 % (rms), and taking the cheaper one by them costs 1 % on average against always taking the faster
+// one.  (With terms of clusters of 1, 2, 4 and 8 and of the layers' older kernels it cost 7 %, and 784-30-10 went to the
+// whole-network kernels at 22 samples, 31 us against 21.)
+//   A prediction: from those older kernels.  The layers, which have to win by a tenth here, are faster than it knows since a launch
+// overlaps the end of the one before it: that costs 11 % on average over the same networks (784-64-64-10, 16 samples: 15.0 us
+// in one kernel, 9.8 in four).
 //   Whole-network kernels: a phase a step and, for each turn of samples that an SM takes, the products of its CTA; the
 // sums over the samples read a sample's values, or its row of partial sums, for every weight.  Windows other than 3 and
 // 5 wide have no tiled form.  Layer by layer: launches, then the values that pass through memory; average pooling's
-// backward pass is the slow one.
-//   (LeNet-5 step: 16 samples 53 us against 110, 592 samples 531 against 785; 3x3 16 -> 16 -> 16 -> 4 on 16x16 maps: one
-// sample 62 against 69, 256 samples 575 against 141; 784-64-64-10: 148 samples 58 against 42, predicted 15 against 19.)
+// backward pass is the slow one, and a softmax of more than 16 values, which is one thread's work a sample.
+//   (LeNet-5 step: 16 samples 53 us against 104, 592 samples 531 against 785; 3x3 16 -> 16 -> 16 -> 4 on 16x16 maps: 12
+// samples 53 us against 66, 60 samples 122 against 83.)
 bool small_net_pays(const SmallNet &n, int B, bool train) {
   if (n.n == 0) return false;
-  const int nc = small_cluster(n, B);
+  const int nc = small_cluster(n, B, false);
   const double turns = (B + n.clusters[nc - 1] - 1) / n.clusters[nc - 1];
   double weights = 0, tiled = 0, slow = 0, square = 0, fc = 0, fc_all = 0, values = 0, rows = 0;  // of a CTA; of all
   double launches = 0, through = 0, averaged = 0;                                                  // layer by layer
@@ -857,27 +877,29 @@ bool small_net_pays(const SmallNet &n, int B, bool train) {
       if (L.KH == L.KW && (L.KW == 3 || L.KW == 5)) square += macs / nc;
       rows += L.w_len;
       weights += L.w_len;
-      launches += train ? 16.8 : 8.6;
+      launches += train ? 21 : 8.6;
     } else if (L.kind == SN_FC) {
       fc += (double)L.w_len / nc;
       fc_all += L.w_len;
       weights += L.w_len <= SN_WHOLE ? L.w_len : (double)L.w_len / nc * (train ? 2 : 1);
-      launches += train ? 8.7 : 5.1;
+      launches += train ? 6.6 : 5.1;
     } else if (L.kind == SN_MAX) {
-      launches += train ? 4.4 : 4.1;
+      launches += train ? 0.7 : 4.1;
     } else if (L.kind == SN_AVG) {
-      launches += train ? 9.0 : 2.8;
+      launches += train ? 4.2 : 2.8;
+    } else if (L.kind == SN_SOFTMAX && L.out_n > 16 && train) {
+      launches += 0.023 * L.out_n * L.out_n;
     }
-    if (L.own_act) launches += train ? 2.4 : 5.1;
+    if (L.own_act) launches += train ? 5.8 : 5.1;
     (L.kind == SN_AVG ? averaged : through) += v;
   }
   if (!train)
     return 6.5 + turns * (1.8 * n.n + 0.6e-4 * weights + 0.4e-4 * tiled + 1e-4 * slow + 0.18e-4 * fc + 0.075e-3 * values) <
            1.1 * (2.8 + launches + B * (0.083e-6 * fc_all + 4.1e-6 * through + 4.8e-6 * averaged));
   const double chain = B <= 64 ? B : B / 8.0;  // rows that a thread of the sums adds
-  return 11.7 + turns * (4.4 * n.n + 0.8e-4 * weights + 31e-4 * slow + 1.8e-4 * square + 1.7e-4 * fc + 0.4e-3 * values) +
-           0.16 * chain + B * (0.75e-6 * fc_all + 72e-6 * rows) <
-         1.05 * (11.5 + launches + B * (0.18e-6 * fc_all + 18e-6 * through + 122e-6 * averaged));
+  return 7.3 + turns * (4.7 * n.n + 2.2e-4 * weights + 37e-4 * slow + 1.3e-4 * square + 0.06e-4 * fc + 0.47e-3 * values) +
+           0.073 * chain + B * (1.1e-6 * fc_all + 110e-6 * rows) <
+         5.7 + launches + B * (0.77e-6 * fc_all + 19e-6 * through + 140e-6 * averaged);
 }
 
 // The counts depend on the device alone (a CTA's registers leave no room for a second one on its SM, whatever its shared memory), and the
@@ -915,7 +937,7 @@ int small_net_run(b200_ctx *ctx, const SmallNet &n, const float *x, const float 
                   int backward, int loss) {
   B200_REQUIRE(!backward || (loss >= B200_LOSS_MSE && loss <= B200_LOSS_CROSS_ENTROPY_MULTICLASS),
                "loss_grad: unknown loss %d", loss);
-  const int nc = small_cluster(n, B);
+  const int nc = small_cluster(n, B, !backward);
   SmallNet m = n;
   m.by_ctas.set(nc);
   place_params(ctx, &m, nc, backward);
@@ -926,7 +948,7 @@ int small_net_run(b200_ctx *ctx, const SmallNet &n, const float *x, const float 
   // behind another prediction, 18.7 so; with an elementwise kernel in front of each 22.6 and 20.6; behind an upload 25.5 to 26.6
   // either way), but not where its clusters only fit if nothing else lies between them: 45 of three CTAs took 28.7 us for
   // 24.6.  The kernels with a backward pass do not wait for the one before them: steps are captured, where a launch costs little.
-  const bool overlap = !backward && ctx->overlap && !ctx->waited && (nc <= 2 || B * 15 <= n.clusters[nc - 1] * 14);
+  const bool overlap = !backward && ctx->overlap && !ctx->waited && leaves_room(n, nc, B);
   B200_TRY(launch_kernel_as(ctx, overlap, kernel, dim3((unsigned)(B * nc)), dim3(SN_THREADS), smem, dim3((unsigned)nc), m, x, t,
                             in_grad, loss));
   if (!backward) return 0;
