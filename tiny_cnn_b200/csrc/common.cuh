@@ -229,6 +229,7 @@ int conv_gather_dx_blocks(const b200_ctx *ctx, const ConvGeom &g, int B);  // SM
 // the tiling is chosen for (at least B)
 bool conv_gather_dw_ok(const b200_ctx *ctx, const ConvGeom &g);
 size_t conv_gather_dw_floats(const b200_ctx *ctx, const ConvGeom &g, int B);
+int conv_gather_dw_blocks(const b200_ctx *ctx, const ConvGeom &g, int B, int plan_batch);  // SMs that it takes
 int conv_gather_dw(b200_ctx *ctx, const ConvGeom &g, const float *in, const float *dout, int B, float *part, float *dW,
                    float *db, int accumulate, int plan_batch, bool finish = true);
 // the sums over `part` that a call with finish = false left out
@@ -250,6 +251,7 @@ int conv_fwd_small(b200_ctx *ctx, const ConvGeom &g, const float *in, const floa
 ConvTcUse conv_tc_use(const b200_ctx *ctx, const ConvGeom &g, int algo);
 // dW of stride-1 layers with in_c*KH*KW <= 128 on the tensor cores, straight from the CHW tensors
 bool conv_dw_small_ok(const b200_ctx *ctx, const ConvGeom &g);
+int conv_dw_small_splits(const b200_ctx *ctx, const ConvGeom &g, int B);  // blocks of conv_dw_small
 size_t conv_dw_small_floats(const b200_ctx *ctx, const ConvGeom &g, int B);
 int conv_dw_small(b200_ctx *ctx, const ConvGeom &g, const float *in, const float *dout, int B, float *part,
                   float *dW, float *db, int accumulate);

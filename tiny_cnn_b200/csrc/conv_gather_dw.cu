@@ -760,6 +760,16 @@ size_t conv_gather_dw_floats(const b200_ctx *ctx, const ConvGeom &g, int B) {
   return n + (size_t)a.kg[0].splits * a.ocb * a.OB + 64;
 }
 
+static int dw_blocks(const ConvDwArgs &a) { return a.kg[a.nkg - 1].first + a.ocb * a.ccb * a.kg[a.nkg - 1].splits; }
+
+int conv_gather_dw_blocks(const b200_ctx *ctx, const ConvGeom &g, int B, int plan_batch) {
+  ConvDwArgs a;
+  size_t smem;
+  if (!dw_plan(ctx, g, plan_batch, &a, &smem)) return 0;
+  dw_splits(ctx, &a, B);
+  return dw_blocks(a);
+}
+
 int conv_gather_dw(b200_ctx *ctx, const ConvGeom &g, const float *in, const float *dout, int B, float *part, float *dW,
                    float *db, int accumulate, int plan_batch, bool finish) {
   ConvDwArgs a;
@@ -775,8 +785,7 @@ int conv_gather_dw(b200_ctx *ctx, const ConvGeom &g, const float *in, const floa
   const bool vec = g.OW % 4 == 0 && ((uintptr_t)dout & 15) == 0;
   auto kernel = a.fold ? (vec ? conv_gather_dw_kernel<true, true> : conv_gather_dw_kernel<false, true>)
                        : (vec ? conv_gather_dw_kernel<true, false> : conv_gather_dw_kernel<false, false>);
-  const DwKGroup &lastk = a.kg[a.nkg - 1];
-  const int grid = lastk.first + a.ocb * a.ccb * lastk.splits;
+  const int grid = dw_blocks(a);
   B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 #ifdef B200_TC_TIMING
   static const bool timing = getenv("B200_TC_TIMING") != nullptr;

@@ -517,12 +517,17 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
         bool tiled_bwd = L.tiled && L.g.OW <= 64;
         const bool tc_dx = L.tc.dx && din != nullptr;
         // dW first: its launch precedes the dX launch, so a one-block-per-SM dW kernel is resident
-        // when the small blocks of an FFMA dX arrive and both share the SMs.  A dX that leaves SMs idle goes first, and
-        // dW takes what is left once its blocks have begun: behind dW it would wait for the longer kernel, and FFMA blocks
-        // would crowd the SMs that come free first (CIFAR net, 24 samples: 159 us a step with dW first, 137 us; 5 samples 133 and 115).
+        // when the small blocks of an FFMA dX arrive and both share the SMs.  Where the two do not fit side by side, a dX that leaves SMs
+        // idle goes first, and dW takes what is left once its blocks have begun: behind dW it would wait for the longer kernel, and
+        // FFMA blocks would crowd the SMs that come free first (CIFAR net, 5 samples 126 us a step with dW first, 105; 36 samples
+        // 146 and 136).  Where they do fit, the wait only holds dW up (3 samples 114 us with it, 100; two 3x3 layers on 32x32 maps, one
+        // sample 47 and 41).  A tensor-core dX of more than three fifths of the SMs leaves dW a second turn that costs as much as
+        // it gains (CIFAR net, 24 samples 138 us, 129 with dW first; those two layers, 40 samples 81 and 72).
         const bool forked = can_fork && (L.tc.dw || L.tc.dw_small);
         const int dx_blocks = !din || !forked ? 0 : tc_dx ? conv_gather_dx_blocks(ctx, L.g, B) : tiled_bwd ? conv_tiled_dx_blocks(ctx, L.g, B) : 0;
-        const bool dx_first = dx_blocks > 0 && dx_blocks < ctx->sm_count;
+        const int dw_blocks = !forked ? 0 : L.tc.dw ? conv_gather_dw_blocks(ctx, L.g, B, net->max_batch) : conv_dw_small_splits(ctx, L.g, B);
+        const bool dx_first = dx_blocks > 0 && dx_blocks + dw_blocks > ctx->sm_count &&
+                              (tc_dx ? 5 * dx_blocks < 3 * ctx->sm_count : dx_blocks < ctx->sm_count);
         auto dx_pass = [&]() -> int {
           if (!din) return 0;
           if (tc_dx) {
