@@ -298,7 +298,7 @@ int softmax_loss_bwd(b200_ctx *ctx, int loss_kind, const float *y, const float *
 // (the classifier's last two layers: 64 -> 10 in the CIFAR-10 net).  A warp per sample, the inputs dealt to its lanes;
 // the weights (K x N floats, N <= 16) sit in shared memory.  With sixteen lanes a sample, each adding all the products
 // of an output, the chain of K additions was the kernel's time (500 -> 10, 77 samples: 20 us forward, 16 us backward;
-// now 3.3 and 3.2 us with the wide form below).
+// now 3.4 and 2.8 us with the wide forms below).
 constexpr int FCS_N = 16, FCS_THREADS = 256;
 constexpr int FCS_NARROW = 256;               // inputs up to which a sample is a warp's work
 constexpr int FCS_WIDE = 1024;                // inputs up to which four samples are a block's work (forward)

@@ -856,8 +856,11 @@ int least_units(const GatherPlan &p) {
 // CTA pair or single CTAs, and S: the least time of the busiest SM, tile after tile, a tile taking the
 // longer of its MMAs (N / 2 cycles each, with a floor; pairs measured 1.2 x as fast) and its loads (about
 // 40 cycles for 32 places of a channel pair).
-// Tiles that leave most SMs idle are split over clusters of Z blocks, each with two blocks of 64 k's or more; as many clusters
-// as surely run at once, however the SMs are grouped; about 2500 cycles for the exchange.
+// Tiles that leave most SMs idle are split over clusters of Z blocks; as many clusters as surely run at once, however the SMs are
+// grouped; about 2500 cycles for the exchange.  A block has two blocks of 64 k's or more in the phase with the most of them.  In a
+// strided dX the phases with fewer taps then get shares of one or of none; with the bound on the phase with the fewest, Z is smaller and the
+// phase with the most takes the time (14x14, 128 -> 64, 3x3, stride 2, two samples: 11.4 us so, 14.4 with that bound; of 108
+// strided passes 24 were 6 to 22 % slower with it, none faster).
 struct GatherShape {
   int CG, S, ks, Z, blocks;
 };
@@ -870,24 +873,24 @@ GatherShape gather_shape(const b200_ctx *ctx, const GatherPlan &p, int B) {
       const int ks = S == 1 && p.ND >= 2 && least_units(p) >= 2 ? 2 : 1;
       const long long slots = ctx->sm_count / cg;
       for (int Z = 1; Z <= (cg * S == 1 ? 8 : 1); Z *= 2) {
-      long long tiles = 0, tile_cost = 0, blocks = 0;
-      for (int i = 0; i < p.nphases; ++i) {
-        const ConvPhase &q = p.ph[i];
-        tiles += ((long long)B * q.PH * q.PW + cg * S * 128 - 1) / (cg * S * 128);
-        const long long units = ((long long)p.nslab * ((q.kslab + 31) / 32) * S + Z - 1) / Z;
-        blocks = max(blocks, (long long)p.nslab * ((q.kslab + 63) / 64));
-        // about 900 cycles of an issuer's instructions a unit
-        const long long issue = S * ks > 1 ? 450 : 900;
-        const long long mma = units * (p.NP * 6 > issue ? p.NP * 6 : issue) * (cg == 2 ? 5 : 6) / 5;
-        const long long load = (long long)((p.nslab + Z - 1) / Z) * ((p.CS + 1) / 2) * ((rows_needed(q, p, S * 128) * q.pitch + 31) / 32) * 40;
-        tile_cost += mma > load ? mma : load;
-      }
-      if (Z > 1 && (blocks < 2 * Z || tiles * p.ngroups > ctx->sm_count / Z * 7 / 8)) break;
-      const long long cost = (tiles * p.ngroups + slots - 1) / slots * (tile_cost / p.nphases + 2000 + (Z > 1 ? 2500 : 0));
-      if (best < 0 || cost < best) {
-        best = cost;
-        sh = {cg, S, ks, Z, (int)min(tiles * p.ngroups, slots) * cg * Z};
-      }
+        long long tiles = 0, tile_cost = 0, blocks = 0;
+        for (int i = 0; i < p.nphases; ++i) {
+          const ConvPhase &q = p.ph[i];
+          tiles += ((long long)B * q.PH * q.PW + cg * S * 128 - 1) / (cg * S * 128);
+          const long long units = ((long long)p.nslab * ((q.kslab + 31) / 32) * S + Z - 1) / Z;
+          blocks = max(blocks, (long long)p.nslab * ((q.kslab + 63) / 64));
+          // about 900 cycles of an issuer's instructions a unit
+          const long long issue = S * ks > 1 ? 450 : 900;
+          const long long mma = units * (p.NP * 6 > issue ? p.NP * 6 : issue) * (cg == 2 ? 5 : 6) / 5;
+          const long long load = (long long)((p.nslab + Z - 1) / Z) * ((p.CS + 1) / 2) * ((rows_needed(q, p, S * 128) * q.pitch + 31) / 32) * 40;
+          tile_cost += mma > load ? mma : load;
+        }
+        if (Z > 1 && (blocks < 2 * Z || tiles * p.ngroups > ctx->sm_count / Z * 7 / 8)) break;
+        const long long cost = (tiles * p.ngroups + slots - 1) / slots * (tile_cost / p.nphases + 2000 + (Z > 1 ? 2500 : 0));
+        if (best < 0 || cost < best) {
+          best = cost;
+          sh = {cg, S, ks, Z, (int)min(tiles * p.ngroups, slots) * cg * Z};
+        }
       }
     }
   }

@@ -565,7 +565,9 @@ __device__ __forceinline__ void dw_finish_block(const DwFinishArgs &a, const int
 }
 
 __global__ void __launch_bounds__(256) dw_finish_kernel(const DwFinishArgs a) {
-  after_previous_kernel(); dw_finish_block(a, (int)blockIdx.x); }
+  after_previous_kernel();
+  dw_finish_block(a, (int)blockIdx.x);
+}
 
 int dw_finish_blocks(const DwFinishArgs &a) { return (a.row_w + 31) / 32 + (a.db != nullptr ? a.OC : 0); }
 

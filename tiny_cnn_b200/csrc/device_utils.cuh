@@ -8,7 +8,7 @@
 
 namespace b200 {
 
-// The first thing that a kernel launched by launch_kernel does, or the first behind what it sets up without memory: such a
+// The first thing that a kernel launched to overlap (launch_kernel_as) does, or the first behind what it sets up without memory: such a
 // kernel may begin while the one before it in the stream runs, and goes on here when that one has ended and its
 // stores are there.  The condition, always true, is not known to the compiler, which therefore moves no load ahead of it.
 __device__ __forceinline__ void wait_for_previous_kernel() {
@@ -17,7 +17,7 @@ __device__ __forceinline__ void wait_for_previous_kernel() {
   if (blocks != 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 // The same in a kernel that leaves room on its SMs: the next one may begin from here on.  (A kernel that takes whole SMs does not
-// let the next one in: its waiting blocks would keep those of other streams out.)
+// let the next one in: its waiting blocks would keep those of other streams out.  Nor does one whose successor's blocks need an SM each.)
 __device__ __forceinline__ void after_previous_kernel() {
   wait_for_previous_kernel();
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");

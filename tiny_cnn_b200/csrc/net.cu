@@ -481,7 +481,8 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
     if (net->fuse && din && before >= 0) {
       Layer &A = net->layers[before];
       float *target = before > 0 ? net->layers[before - 1].grad : net->input_grad ? net->in_grad : nullptr;
-      if (act_of_layer(A.kind) != B200_ACT_NONE && A.kind != B200_LAYER_SOFTMAX && target && !A.bwd_done_by_next && fc_dx_takes_act(ctx, n_in, n_out, B, net->scratch != nullptr)) {
+      if (act_of_layer(A.kind) != B200_ACT_NONE && A.kind != B200_LAYER_SOFTMAX && target && !A.bwd_done_by_next &&
+          fc_dx_takes_act(ctx, n_in, n_out, B, net->scratch != nullptr)) {
         ag = {A.out, target, act_of_layer(A.kind), A.act_param};
         act_done = before;
       }
@@ -524,7 +525,10 @@ int net_backward_impl(b200_net *net, const float *t, int loss_kind, bool peer_in
         // sample 47 and 41).  A tensor-core dX of more than three fifths of the SMs leaves dW a second turn that costs as much as
         // it gains (CIFAR net, 24 samples 138 us, 129 with dW first; those two layers, 40 samples 81 and 72).
         const bool forked = can_fork && (L.tc.dw || L.tc.dw_small);
-        const int dx_blocks = !din || !forked ? 0 : tc_dx ? conv_gather_dx_blocks(ctx, L.g, B) : tiled_bwd ? conv_tiled_dx_blocks(ctx, L.g, B) : 0;
+        const int dx_blocks = !din || !forked ? 0
+                              : tc_dx         ? conv_gather_dx_blocks(ctx, L.g, B)
+                              : tiled_bwd     ? conv_tiled_dx_blocks(ctx, L.g, B)
+                                              : 0;
         const int dw_blocks = !forked ? 0 : L.tc.dw ? conv_gather_dw_blocks(ctx, L.g, B, net->max_batch) : conv_dw_small_splits(ctx, L.g, B);
         const bool dx_first = dx_blocks > 0 && dx_blocks + dw_blocks > ctx->sm_count &&
                               (tc_dx ? 5 * dx_blocks < 3 * ctx->sm_count : dx_blocks < ctx->sm_count);
