@@ -814,11 +814,14 @@ using SmallKernel = void (*)(SmallNet, const float *, const float *, float *, in
 // Whether B clusters of nc CTAs leave one place in fifteen free: clusters that fill the chip wait for each other's SMs
 bool leaves_room(const SmallNet &n, int nc, int B) { return nc <= 2 || B * 15 <= n.clusters[nc - 1] * 14; }
 
-double small_macs(const SmallNet &n) {  // multiply-adds of a sample's forward pass
+// Multiply-adds of a sample's forward pass, for a choice below `nc` CTAs.  Those of a fully-connected layer, which read a weight
+// each, take 2.5 times as long; three CTAs, whose shares of the weights lie off the 16-byte grid, are no faster at them than two.
+double small_macs(const SmallNet &n, int nc) {
   double macs = 0;
   for (int i = 0; i < n.n; ++i)
-    macs += n.step[i].kind == SN_CONV ? (double)n.step[i].out_n * n.step[i].C * n.step[i].KH * n.step[i].KW
-            : n.step[i].kind == SN_FC ? (double)n.step[i].w_len : 0.0;
+    macs += n.step[i].kind == SN_CONV               ? (double)n.step[i].out_n * n.step[i].C * n.step[i].KH * n.step[i].KW
+            : n.step[i].kind == SN_FC && nc != 3 ? 2.5 * n.step[i].w_len
+                                                    : 0.0;
   return macs;
 }
 
@@ -826,13 +829,18 @@ double small_macs(const SmallNet &n) {  // multiply-adds of a sample's forward p
 // chip holds depends on how its SMs are grouped (15 of eight, 22 of six, 26 of five, 33 of four, 45 of three, 74 of two).  Any number, not
 // powers of two alone: a LeNet-5 step of 16 samples 60 us with four CTAs a sample, 53 with six; of 40 samples 88 with two, 70 with
 // three.  More than eight is no faster: one sample 49 us with eight, 51 with sixteen, which have to send to each other.
-// A prediction whose clusters fill the chip takes a CTA less, which costs it its share of the products and saves 2 us: 3x3 nets
-// of two layers 18.6 us with 22 samples on clusters of six, 15.7 on clusters of five.  Not where that share is above 50 thousand (LeNet-5, 45
-// samples: 24.8 us with three CTAs, 27.1 with two).
+// A prediction whose clusters fill the chip takes the next fewer CTAs that leave room, which costs a larger share of the products and saves
+// 2 us: 3x3 nets of two layers 18.6 us with 22 samples on clusters of six, 15.7 on clusters of five; 784-200-200-10, 26 samples 20.7 on
+// five, 16.8 on four.  Not where that share grows by more than 35 thousand (LeNet-5, 45 samples: 24.8 us with three CTAs, 27.1 with
+// two, 33 samples 22.8 either way; 784-200-200-10, 32 samples 18.7 with four, 19.1 with three).
 int small_cluster(const SmallNet &n, int B, bool predict) {
   int nc = SN_MAX_CTAS;
   while (nc > 1 && B > n.clusters[nc - 1]) --nc;
-  if (predict && !leaves_room(n, nc, B) && leaves_room(n, nc - 1, B) && small_macs(n) < 50e3 * nc * (nc - 1)) --nc;
+  if (predict && !leaves_room(n, nc, B)) {
+    int less = nc - 1;
+    while (!leaves_room(n, less, B)) --less;  // two always do
+    if (small_macs(n, nc) * (1.0 / less - 1.0 / nc) < 35e3) nc = less;
+  }
   return nc;
 }
 
